@@ -54,9 +54,13 @@ struct tg_handle {
   MeshView mv{};
   StateView sv{};
   TileView tv{};
-  double* Pb[3] = {nullptr, nullptr, nullptr};   // rotating state buffers (buffer 0 = current state)
-  double* Wb[3] = {nullptr, nullptr, nullptr};
-  size_t smem_grad0 = 0, smem_grad1 = 0, smem_flux = 0;
+  // rotating state buffers (buffer 0 = current state)
+  D4* Sb[3] = {nullptr, nullptr, nullptr};
+  double* Tb[3] = {nullptr, nullptr, nullptr};
+  double* V1b[3] = {nullptr, nullptr, nullptr};
+  double2* W23b[3] = {nullptr, nullptr, nullptr};
+  size_t smem_grad = 0, smem_flux = 0;
+  int grid_grad = 1, grid_flux = 1, grid_res = 1;   // CTAs that fill the chip once (the kernels walk tiles)
   Scalars* sc = nullptr;       // device
   int* done = nullptr;         // device flag written by k_step_begin
   int* never = nullptr;        // device zero, used by single-phase calls
@@ -71,7 +75,8 @@ struct tg_handle {
   cudaGraph_t wgraph = nullptr;                // a step whose dt the previous step formed
   cudaGraphExec_t wgraph_exec = nullptr;
   bool cold = true;                            // the next step may not find dt_next set
-  bool w_partial[3] = {false, false, false};   // a step left only V5 in this buffer's W (refresh_w)
+  bool w_partial[3] = {false, false, false};   // a step left this buffer's V1 unformed (refresh_w)
+  bool uold_stale = false;                     // steps ran since Uold was stored (they form U_old themselves)
   // state transfers: PrimVar records in the caller's order on the device
   double* raw = nullptr;              // 5 * nv doubles
   const int* old_of_new = nullptr;    // device copy of the vertex permutation
@@ -165,8 +170,8 @@ typedef void (*BfluxKernel)(Params, MeshView, StateView, const int*);
 #define TG_WHOLE_MESH(h) \
   if ((h) && (h)->part.n_parts > 0) return fail((h), TG_NOT_SUPPORTED, "a partition handle steps through tg_part_*");
 
-typedef void (*TileFluxKernel)(Params, MeshView, TileView, StateView, Control, Scalars*, int, int, double*, double*,
-                               int, int, const int*);
+typedef void (*TileFluxKernel)(Params, MeshView, TileView, StateView, Control, Scalars*, int, int, StateView, int, int,
+                               int, const int*);
 
 template <int F>
 BfluxKernel pick_bflux(int recon) {
@@ -191,42 +196,42 @@ BfluxKernel bflux_kernel(int flux, int recon) {
   }
 }
 
-template <int F, int M, bool O>
+template <int F, int M>
 TileFluxKernel pick_tile(int recon) {
   switch (recon) {
-    case RECON_FIRST: return k_tile_flux<F, RECON_FIRST, M, O>;
-    case RECON_SECOND: return k_tile_flux<F, RECON_SECOND, M, O>;
-    case RECON_SECOND_MUSCL: return k_tile_flux<F, RECON_SECOND_MUSCL, M, O>;
-    case RECON_VAN_ALBADA: return k_tile_flux<F, RECON_VAN_ALBADA, M, O>;
-    case RECON_TVD_MINMOD: return k_tile_flux<F, RECON_TVD_MINMOD, M, O>;
-    case RECON_TVB_MINMOD: return k_tile_flux<F, RECON_TVB_MINMOD, M, O>;
-    default: return k_tile_flux<F, RECON_ENO2, M, O>;
+    case RECON_FIRST: return k_tile_flux<F, RECON_FIRST, M>;
+    case RECON_SECOND: return k_tile_flux<F, RECON_SECOND, M>;
+    case RECON_SECOND_MUSCL: return k_tile_flux<F, RECON_SECOND_MUSCL, M>;
+    case RECON_VAN_ALBADA: return k_tile_flux<F, RECON_VAN_ALBADA, M>;
+    case RECON_TVD_MINMOD: return k_tile_flux<F, RECON_TVD_MINMOD, M>;
+    case RECON_TVB_MINMOD: return k_tile_flux<F, RECON_TVB_MINMOD, M>;
+    default: return k_tile_flux<F, RECON_ENO2, M>;
   }
 }
-template <int M, bool O>
+template <int M>
 TileFluxKernel tile_kernel_m(int flux, int recon) {
   switch (flux) {
-    case FLUX_TECNO_ROE: return pick_tile<FLUX_TECNO_ROE, M, O>(recon);
-    case FLUX_TECNO_RUSANOV: return pick_tile<FLUX_TECNO_RUSANOV, M, O>(recon);
-    case FLUX_KEPEC: return k_tile_flux<FLUX_KEPEC, RECON_FIRST, M, O>;
-    case FLUX_KEP: return k_tile_flux<FLUX_KEP, RECON_FIRST, M, O>;
-    case FLUX_ROE_EC: return k_tile_flux<FLUX_ROE_EC, RECON_FIRST, M, O>;
-    default: return k_tile_flux<FLUX_AVG, RECON_FIRST, M, O>;
+    case FLUX_TECNO_ROE: return pick_tile<FLUX_TECNO_ROE, M>(recon);
+    case FLUX_TECNO_RUSANOV: return pick_tile<FLUX_TECNO_RUSANOV, M>(recon);
+    case FLUX_KEPEC: return k_tile_flux<FLUX_KEPEC, RECON_FIRST, M>;
+    case FLUX_KEP: return k_tile_flux<FLUX_KEP, RECON_FIRST, M>;
+    case FLUX_ROE_EC: return k_tile_flux<FLUX_ROE_EC, RECON_FIRST, M>;
+    default: return k_tile_flux<FLUX_AVG, RECON_FIRST, M>;
   }
 }
-size_t flux_smem(int flux, int recon, int lmax, int emax, int cmax) {
-  const bool grad = recon != RECON_FIRST;
+template <int F>
+size_t flux_smem_f(int recon, int lmax, int emax, int cmax, bool dt) {
+  return recon != RECON_FIRST ? FluxSmem<F, RECON_TVD_MINMOD>(lmax, emax, cmax, dt).bytes
+                              : FluxSmem<F, RECON_FIRST>(lmax, emax, cmax, dt).bytes;
+}
+size_t flux_smem(int flux, int recon, int lmax, int emax, int cmax, bool dt) {
   switch (flux) {
-    case FLUX_TECNO_ROE:
-      return grad ? tile_flux_smem_t<FLUX_TECNO_ROE, RECON_TVD_MINMOD>(lmax, emax, cmax)
-                  : tile_flux_smem_t<FLUX_TECNO_ROE, RECON_FIRST>(lmax, emax, cmax);
-    case FLUX_TECNO_RUSANOV:
-      return grad ? tile_flux_smem_t<FLUX_TECNO_RUSANOV, RECON_TVD_MINMOD>(lmax, emax, cmax)
-                  : tile_flux_smem_t<FLUX_TECNO_RUSANOV, RECON_FIRST>(lmax, emax, cmax);
-    case FLUX_KEPEC: return tile_flux_smem_t<FLUX_KEPEC, RECON_FIRST>(lmax, emax, cmax);
-    case FLUX_KEP: return tile_flux_smem_t<FLUX_KEP, RECON_FIRST>(lmax, emax, cmax);
-    case FLUX_ROE_EC: return tile_flux_smem_t<FLUX_ROE_EC, RECON_FIRST>(lmax, emax, cmax);
-    default: return tile_flux_smem_t<FLUX_AVG, RECON_FIRST>(lmax, emax, cmax);
+    case FLUX_TECNO_ROE: return flux_smem_f<FLUX_TECNO_ROE>(recon, lmax, emax, cmax, dt);
+    case FLUX_TECNO_RUSANOV: return flux_smem_f<FLUX_TECNO_RUSANOV>(recon, lmax, emax, cmax, dt);
+    case FLUX_KEPEC: return flux_smem_f<FLUX_KEPEC>(RECON_FIRST, lmax, emax, cmax, dt);
+    case FLUX_KEP: return flux_smem_f<FLUX_KEP>(RECON_FIRST, lmax, emax, cmax, dt);
+    case FLUX_ROE_EC: return flux_smem_f<FLUX_ROE_EC>(RECON_FIRST, lmax, emax, cmax, dt);
+    default: return flux_smem_f<FLUX_AVG>(RECON_FIRST, lmax, emax, cmax, dt);
   }
 }
 
@@ -241,50 +246,46 @@ cudaError_t raise_smem(const void* f, size_t bytes) {
   return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-typedef void (*TileGradKernel)(Params, MeshView, TileView, StateView, Scalars*, int, int, const int*, int);
-// ord: a partition's launches over its tile order (frontier / interior), whose
-// gradient and flux + update kernels are separate instantiations (ORD), so the
-// whole-mesh kernels stay exactly as they are
-TileGradKernel grad_kernel(bool first, bool grad, bool ord = false) {
-  if (first) return grad ? k_tile_grad<true, true> : k_tile_grad<true, false>;
-  return ord ? k_tile_grad<false, true, true> : k_tile_grad<false, true>;
+TileFluxKernel tile_kernel(int flux, int recon, int mode) {
+  return mode == MODE_UPDATE ? tile_kernel_m<MODE_UPDATE>(flux, recon) : tile_kernel_m<MODE_RESIDUAL>(flux, recon);
 }
 
-TileFluxKernel tile_kernel(int flux, int recon, int mode, bool ord = false) {
-  if (ord) return tile_kernel_m<MODE_UPDATE, true>(flux, recon);
-  return mode == MODE_UPDATE ? tile_kernel_m<MODE_UPDATE, false>(flux, recon)
-                             : tile_kernel_m<MODE_RESIDUAL, false>(flux, recon);
-}
-
-// state view of buffer b (the three P/W buffers rotate through the stages)
+// state view of buffer b (the three buffers rotate through the stages)
 StateView view(const tg_handle* h, int b) {
   StateView v = h->sv;
-  v.P = h->Pb[b];
-  v.W = h->Wb[b];
+  v.S = h->Sb[b];
+  v.T = h->Tb[b];
+  v.V1 = h->V1b[b];
+  v.W23 = h->W23b[b];
   return v;
 }
 
 // ---- phases (all enqueue on h->stream; `done` gates work inside graphs)
-// Gradients (when `grad`), plus at the first stage dt and U_old.
-// At a step's first stage with fuse_dt, the first-stage kernel runs when dt and
-// U_old are still to be formed, else a gradient-only launch (warm) takes its place.
-// Tiles [base, base + count) of the handle's tile order (all tiles by default).
-TileView tiles(const tg_handle* h, int base) {
-  TileView v = h->tv;
-  v.base = base;
-  return v;
+// A launch over tiles [base, base + count) of the handle's tile order, all of them by
+// default, by at most `grid` CTAs; returns the grid.  The passes of a partition run as two
+// launches over its frontier and interior tiles, whose CTAs are numbered through.
+int tiles(const tg_handle* h, int base, int count, int grid, TileView* v) {
+  *v = h->tv;
+  const int nt = h->L.ntiles, nf = h->part.n_frontier;
+  if (count < 0) count = nt;
+  v->base = base;
+  v->count = count;
+  v->pbase = 0;
+  v->total = std::min(count, grid);
+  if (h->part.n_parts > 0 && count != nt) {
+    const int gf = std::min(nf, grid), gi = std::min(nt - nf, grid);
+    v->total = gf + gi;
+    v->pbase = base == 0 && count == nf ? 0 : gf;
+  }
+  return std::min(count, grid);
 }
 
-void enqueue_gradient(tg_handle* h, int b, bool first, bool grad, const int* done, int base = 0, int count = -1) {
-  if (!first && !grad) return;
-  if (count < 0) count = h->L.ntiles;
-  if (count == 0) return;
-  const bool ord = h->tv.order != nullptr && !first;   // first-stage passes cover all tiles unordered
-  grad_kernel(first, grad, ord)<<<count, kTileThreads, first ? h->smem_grad1 : h->smem_grad0, h->stream>>>(
-      h->prm, h->mv, tiles(h, base), view(h, b), h->sc, h->L.lmax, h->L.emax, done, 0);
-  if (first && grad && h->prm.fuse_dt)
-    grad_kernel(false, true)<<<count, kTileThreads, h->smem_grad0, h->stream>>>(
-        h->prm, h->mv, tiles(h, base), view(h, b), h->sc, h->L.lmax, h->L.emax, done, 1);
+void enqueue_gradient(tg_handle* h, int b, const int* done, int base = 0, int count = -1) {
+  TileView v;
+  const int grid = tiles(h, base, count, h->grid_grad, &v);
+  if (grid == 0) return;
+  k_tile_grad<<<grid, kTileThreads, h->smem_grad, h->stream>>>(
+      h->prm, h->mv, v, view(h, b), h->L.lmax, h->L.cmax, done);
 }
 
 // boundary-face and viscous contributions, gathered by the tiled flux kernel
@@ -297,18 +298,19 @@ void enqueue_boundary(tg_handle* h, int b, const int* done) {
 
 void enqueue_tile_flux(tg_handle* h, int b, int mode, int r, bool norm, int bout, const int* done, int base = 0,
                        int count = -1) {
-  if (count < 0) count = h->L.ntiles;
-  if (count == 0) return;
-  const bool ord = h->tv.order != nullptr && mode == MODE_UPDATE;
-  tile_kernel(h->prm.flux, h->prm.recon, mode, ord)<<<count, kTileThreads, h->smem_flux, h->stream>>>(
-      h->prm, h->mv, tiles(h, base), view(h, b), h->ctl, h->sc, r, norm ? 1 : 0, h->Pb[bout], h->Wb[bout], h->L.lmax,
-      h->L.emax, done);
+  TileView v;
+  const int grid = tiles(h, base, count, mode == MODE_UPDATE ? h->grid_flux : h->grid_res, &v);
+  if (grid == 0) return;
+  tile_kernel(h->prm.flux, h->prm.recon, mode)<<<grid, kTileThreads, h->smem_flux, h->stream>>>(
+      h->prm, h->mv, v, view(h, b), h->ctl, h->sc, r, norm ? 1 : 0, view(h, bout), h->L.lmax, h->L.emax,
+      h->L.cmax, done);
 }
 
-// Inviscid central-flux steps without strong conditions store only V5 of the entropy
-// variables (w3_only in k_tile_flux).  Steps mark the buffers they wrote; before
-// gradients are formed outside a step, a marked buffer gets all four back from P.
+// Inviscid central-flux steps without strong conditions leave V1 unformed (w3_only in
+// k_tile_flux).  Steps mark the buffers they wrote; before gradients are formed outside
+// a step, a marked buffer gets it back from the state.
 void mark_steps(tg_handle* h) {
+  h->uold_stale = true;
   const bool central = h->prm.flux != FLUX_TECNO_ROE && h->prm.flux != FLUX_TECNO_RUSANOV;
   if (central && h->prm.model == 0 && !h->prm.strong)
     for (int b = 0; b < 3; ++b) h->w_partial[b] = true;
@@ -316,7 +318,7 @@ void mark_steps(tg_handle* h) {
 
 void refresh_w(tg_handle* h, int b) {
   if (!h->w_partial[b]) return;
-  k_prim2ent<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv.nv, h->Pb[b], h->Wb[b]);
+  k_prim2ent<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv.nv, view(h, b), nullptr);
   h->w_partial[b] = false;
 }
 
@@ -326,7 +328,7 @@ int residual_kernels(const tg_handle* h) {
 
 // compute_residual on buffer 0 (gradient, boundary/viscous terms, tiled fluxes -> R)
 void enqueue_residual(tg_handle* h, const int* done) {
-  enqueue_gradient(h, 0, false, true, done);
+  enqueue_gradient(h, 0, done);
   enqueue_boundary(h, 0, done);
   enqueue_tile_flux(h, 0, MODE_RESIDUAL, 0, false, 0, done);
 }
@@ -340,7 +342,7 @@ void enqueue_ssw(tg_handle* h, const int* done) {
 
 void enqueue_dt(tg_handle* h, const int* done) {
   if (h->ctl.time_step <= 0.0)
-    k_dt<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->sc, done);
+    k_dt<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->sc, done, 0);
   k_dt_final<<<1, 1, 0, h->stream>>>(h->ctl, h->sc, done);
   enqueue_ssw(h, done);
 }
@@ -357,7 +359,7 @@ void enqueue_norm_final(tg_handle* h, int nblocks, bool use_sc_iter, long long i
 // stage r reads buffer r and writes buffer (r+1)%3, so the step ends in buffer 0.
 // The last stage's update also forms the residual norms and ends the iteration
 // (its last block).  warm: the previous step's last update formed this step's dt
-// and U_old (dt_next set), so the first-stage dt pass and k_dt_final are left out.
+// (dt_next set), so the dt pass and k_dt_final are left out.
 void enqueue_step(tg_handle* h, bool warm) {
   k_step_begin<<<1, 1, 0, h->stream>>>(h->ctl, h->sc, h->done, warm ? 1 : 0);
   // stage r reads buffer bin and writes bout: ssprk3 0->1->2->0, rk4 0->1->2->1->0,
@@ -366,27 +368,35 @@ void enqueue_step(tg_handle* h, bool warm) {
   for (int r = 0; r < h->ctl.n_rks; ++r) {
     const bool first = (r == 0), last = (r == h->ctl.n_rks - 1);
     const int bin = h->ctl.scheme == 1 ? rk4_in[r] : r, bout = h->ctl.scheme == 1 ? rk4_out[r] : (r + 1) % 3;
-    if (first && h->ctl.time_step > 0.0) {
-      k_store_old<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->done);
-      enqueue_gradient(h, bin, false, h->grads_needed, h->done);
-    } else if (first && warm) {
-      enqueue_gradient(h, bin, false, h->grads_needed, h->done);
-    } else {
-      enqueue_gradient(h, bin, first, h->grads_needed, h->done);   // first stage: + dt, U_old
+    if (first && !warm) {
+      if (h->ctl.time_step <= 0.0)
+        k_dt<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->sc, h->done, 1);
+      k_dt_final<<<1, 1, 0, h->stream>>>(h->ctl, h->sc, h->done);
     }
-    if (first && !warm) k_dt_final<<<1, 1, 0, h->stream>>>(h->ctl, h->sc, h->done);
+    if (h->grads_needed) enqueue_gradient(h, bin, h->done);
     if (first) enqueue_ssw(h, h->done);
     enqueue_boundary(h, bin, h->done);
     enqueue_tile_flux(h, bin, MODE_UPDATE, r, last, bout, h->done);
     if (h->prm.strong && h->mv.nsb > 0)
-      k_strong_bc<<<nblk(h->mv.nsb), kBlock, 0, h->stream>>>(h->mv, h->Pb[bout], h->done);
+      k_strong_bc<<<nblk(h->mv.nsb), kBlock, 0, h->stream>>>(h->mv, view(h, bout), h->done);
   }
 }
 
-// The captured step to replay: the warm one once the host has seen the previous
-// step form dt and U_old for the current state (cold is cleared only then).
+// The captured step to replay: the warm one once the previous step has formed dt for the
+// current state (cold is cleared only then).
 cudaGraphExec_t step_graph(const tg_handle* h) {
   return (h->prm.fuse_dt && !h->cold && h->wgraph_exec) ? h->wgraph_exec : h->graph_exec;
+}
+
+// n replays of the captured step.  A cold step leaves dt_next set (or its loop test ended
+// the run, and the later steps' tests do too), so only the first of them forms its own dt.
+tg_status launch_steps(tg_handle* h, long n) {
+  for (long i = 0; i < n; ++i) {
+    TG_CUDA(h, cudaGraphLaunch(step_graph(h), h->stream));
+    h->cold = false;
+  }
+  if (n > 0) mark_steps(h);
+  return TG_OK;
 }
 
 void drop_graphs(tg_handle* h) {
@@ -398,7 +408,7 @@ void drop_graphs(tg_handle* h) {
   h->graph = h->wgraph = nullptr;
 }
 
-// The state changed outside a captured step: the next step forms dt and U_old itself.
+// The state changed outside a captured step: the next step forms dt itself.
 void clear_dt_next(tg_handle* h) {
   cudaMemsetAsync(&h->sc->dt_next, 0, sizeof(int), h->stream);
   h->cold = true;
@@ -539,8 +549,8 @@ tg_status take_queued_input(tg_handle* h) {
   TG_CUDA(h, cudaStreamWaitEvent(h->stream, h->in_done[slot], 0));
   TG_CUDA(h, cudaMemsetAsync(h->bad, 0, sizeof(int), h->stream));
   k_state_check<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->in_stage[slot], h->bad);
-  k_state_in<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->in_stage[slot], h->old_of_new, h->bad, h->sv.P);
-  k_prim2ent_checked<<<nblk(nv), kBlock, 0, h->stream>>>(h->prm, nv, h->sv.P, h->sv.W, h->bad);
+  k_state_in<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->in_stage[slot], h->old_of_new, h->bad, h->Sb[0], h->Tb[0]);
+  k_prim2ent<<<nblk(nv), kBlock, 0, h->stream>>>(h->prm, nv, view(h, 0), h->bad);
   h->w_partial[0] = false;
   k_scalars_set<<<1, 1, 0, h->stream>>>(h->sc, fresh_scalars(h, t0), h->bad);
   h->in_check = true;
@@ -584,7 +594,7 @@ tg_status capture_step_graph(tg_handle* h) {
 
 void enqueue_phase(tg_handle* h, int phase) {
   switch (phase) {
-    case TG_PHASE_GRADIENT: enqueue_gradient(h, 0, false, true, h->never); break;
+    case TG_PHASE_GRADIENT: enqueue_gradient(h, 0, h->never); break;
     case TG_PHASE_FLUX:
       enqueue_boundary(h, 0, h->never);
       enqueue_tile_flux(h, 0, MODE_RESIDUAL, 0, false, 0, h->never);
@@ -600,13 +610,13 @@ void enqueue_phase(tg_handle* h, int phase) {
 
 // InitialCondition::value (src/ic.h:79-104) at every vertex, on the device, written
 // as PrimVar records in the caller's order into the state staging buffer.
-__global__ void k_state_expr(int nv, const double* __restrict__ x, const double* __restrict__ y,
+__global__ void k_state_expr(int nv, const double2* __restrict__ xy,
                              const int* __restrict__ old_of_new, expr::Field5 f, const double* __restrict__ rnd,
                              int nrnd, double* __restrict__ raw, int* __restrict__ err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
   int e = 0;
-  const double xv = x[i], yv = y[i];
+  const double xv = xy[i].x, yv = xy[i].y;
   double* q = raw + 5 * (size_t)old_of_new[i];
   q[0] = expr::eval5(f, 0, xv, yv, 0.0, rnd, nrnd, &e);   // temperature
   q[2] = expr::eval5(f, 1, xv, yv, 0.0, rnd, nrnd, &e);   // x velocity
@@ -623,12 +633,12 @@ tg_status take_raw_state(tg_handle* h, double t0) {
   tg_status st;
   TG_CUDA(h, cudaMemsetAsync(h->bad, 0, sizeof(int), h->stream));
   k_state_check<<<nblk(nc), kBlock, 0, h->stream>>>(nc, h->raw, h->bad);
-  k_state_in<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->raw, h->old_of_new, h->bad, h->sv.P);
+  k_state_in<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->raw, h->old_of_new, h->bad, h->Sb[0], h->Tb[0]);
   int bad = 0;
   TG_CUDA(h, cudaMemcpyAsync(&bad, h->bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   if ((st = sync(h)) != TG_OK) return st;
   if (bad) return fail(h, TG_INVALID_ARG, "state needs T > 0 and p > 0 (src/fv.cc:388-389)");
-  k_prim2ent<<<nblk(nv), kBlock, 0, h->stream>>>(h->prm, nv, h->sv.P, h->sv.W);
+  k_prim2ent<<<nblk(nv), kBlock, 0, h->stream>>>(h->prm, nv, view(h, 0), nullptr);
   h->w_partial[0] = false;
   const Scalars s = fresh_scalars(h, t0);
   TG_CUDA(h, cudaMemcpyAsync(h->sc, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
@@ -705,6 +715,8 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   k.sqrt_gm1 = std::sqrt(mat->gamma - 1.0);
   k.inv_gamma = 1.0 / mat->gamma;
   k.inv_gm1 = 1.0 / (mat->gamma - 1.0);
+  k.gm1 = mat->gamma - 1.0;
+  k.inv_R = 1.0 / mat->gas_const;
   k.gp1_gm1 = (mat->gamma + 1.0) / (mat->gamma - 1.0);
   k.prandtl = mat->prandtl; k.mu_ref = mat->mu_ref; k.T0 = mat->T_0; k.Tref = mat->T_ref; k.omega = mat->omega;
   k.ev_alpha = mat->ev_mod_alpha; k.ev_beta = mat->ev_mod_beta; k.tvbM = mat->tvb_minmod_coef; k.cfl = opt->cfl;
@@ -722,7 +734,6 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   h->mv.nv = L.nv; h->mv.ne = L.ne; h->mv.nb = L.nb; h->mv.nvu = L.nvu; h->mv.n_int_cells = L.n_int_cells;
   UP(dcarea, dcarea) UP(inv6mc, inv6mc) UP(pweight, pweight)
   UP(e_a, e_a) UP(e_b, e_b) UP(e_nx, e_nx) UP(e_ny, e_ny) UP(e_dx, e_dx) UP(e_dy, e_dy)
-  UP(e_g0x, e_g0x) UP(e_g0y, e_g0y) UP(e_g1x, e_g1x) UP(e_g1y, e_g1y)
   UP(ce_off, ce_off) UP(ce_ent, ce_ent) UP(cb_off, cb_off) UP(cb_ent, cb_ent)
   UP(b_v0, b_v0) UP(b_v1, b_v1) UP(b_kind, b_kind) UP(b_adiab, b_adiab) UP(b_cell, b_cell)
   UP(b_nx, b_nx) UP(b_ny, b_ny) UP(b_val, b_val)
@@ -757,45 +768,107 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
     if ((st = dev_upload(h, sb_ent, &h->mv.sb_ent)) != TG_OK) { tg_destroy(h); return st; }
   }
 #undef UP
+  {
+    // what the update and the local time step read per vertex, and packed tile arrays
+    std::vector<double> ia(L.nv), la(L.nv, 0.0), lv(L.nv, 0.0);
+    for (int v = 0; v < L.nv; ++v) {
+      ia[v] = 1.0 / L.dcarea[v];
+      for (int j = L.ce_off[v]; j < L.ce_off[v + 1]; ++j) {
+        const int e = L.ce_ent[j] >> 1;
+        const double area = std::sqrt(L.e_nx[e] * L.e_nx[e] + L.e_ny[e] * L.e_ny[e]);
+        la[v] += area;
+        lv[v] += area / std::sqrt(L.e_dx[e] * L.e_dx[e] + L.e_dy[e] * L.e_dy[e]);
+      }
+      for (int j = L.cb_off[v]; j < L.cb_off[v + 1]; ++j) {
+        const int ent = L.cb_ent[j], d = ent >> 3;
+        if ((ent & 3) == 0) la[v] += 0.5 * std::sqrt(L.b_nx[d] * L.b_nx[d] + L.b_ny[d] * L.b_ny[d]);
+      }
+    }
+    std::vector<double> xy(2 * (size_t)L.nv);
+    for (int v = 0; v < L.nv; ++v) { xy[2 * (size_t)v] = L.x[v]; xy[2 * (size_t)v + 1] = L.y[v]; }
+    // a partition's tiles: those with a ghost among their vertices (the frontier) first, so
+    // a driver can run the interior while a halo exchange is in flight
+    std::vector<int> order, interior;
+    for (int q = 0; q < L.ntiles; ++q) {
+      bool ghost = false;
+      if (n_parts > 0)
+        for (int i = L.t_loff[q]; i < L.t_loff[q + 1] && !ghost; ++i) ghost = L.lv[i] >= plan.n_owned;
+      (ghost ? order : interior).push_back(q);
+    }
+    h->part.n_frontier = (int)order.size();
+    order.insert(order.end(), interior.begin(), interior.end());
+    std::vector<TileRec> rec(L.ntiles);
+    for (int i = 0; i < L.ntiles; ++i) {
+      const int q = order[i], vb = L.t_vbeg[q], nown = L.t_vbeg[q + 1] - vb;
+      TileRec& x = rec[i];
+      x.l0 = L.t_loff[q]; x.sizes = (L.t_loff[q + 1] - x.l0) | (nown << 16);
+      x.e0 = L.t_eoff[q]; x.NE = L.t_eoff[q + 1] - x.e0;
+      x.vb = vb;
+      x.rel = vb + q;
+      x.cb = L.t_cbase[q];
+      x.nent = L.cv_rel[x.rel + nown];
+      if (L.cb_off[vb + nown] > L.cb_off[vb]) x.nent |= kTileBnd;
+    }
+    // (x, y) pairs stored flat
+    auto up2 = [&](const std::vector<double>& a, const double2** out) {
+      const double* p = nullptr;
+      const tg_status u = dev_upload(h, a, &p);
+      *out = reinterpret_cast<const double2*>(p);
+      return u;
+    };
+    if ((st = dev_upload(h, ia, &h->mv.inv_area)) != TG_OK || (st = dev_upload(h, la, &h->mv.lam_area)) != TG_OK ||
+        (st = dev_upload(h, lv, &h->mv.lam_visc)) != TG_OK || (st = up2(xy, &h->tv.xy)) != TG_OK ||
+        (st = up2(L.te_u, &h->tv.u)) != TG_OK || (st = up2(L.te_n, &h->tv.n)) != TG_OK ||
+        (st = up2(L.gj_g, &h->tv.gjg)) != TG_OK || (st = dev_upload(h, rec, &h->tv.rec)) != TG_OK) {
+      tg_destroy(h);
+      return st;
+    }
+  }
 #define UPT(vec, field) \
   if ((st = dev_upload(h, L.vec, &h->tv.field)) != TG_OK) { tg_destroy(h); return st; }
-  UPT(t_vbeg, vbeg) UPT(t_loff, loff) UPT(t_eoff, eoff) UPT(lv, lv) UPT(te_ab, ab)
-  UPT(te_nx, nx) UPT(te_ny, ny) UPT(te_g0x, g0x) UPT(te_g0y, g0y) UPT(te_g1x, g1x) UPT(te_g1y, g1y)
-  UPT(cv_off, cv_off) UPT(cv_ent, cv_ent) UPT(x, x) UPT(y, y) UPT(te_ux, ux) UPT(te_uy, uy) UPT(te_ar, ar)
-  UPT(te_r, r)
+  UPT(lv, lv) UPT(te_ab, ab) UPT(te_ar, ar) UPT(te_r, r) UPT(cv_rel, crel)
+  UPT(cv_ent, cent) UPT(gj_i, gji)
 #undef UPT
-  h->tv.order = nullptr;
-  h->tv.base = 0;
-  h->tv.total = L.ntiles;
   const size_t nv = L.nv;
   h->nblocks_v = nblk(L.nv);
 #define AL(field, n) \
   if ((st = dev_alloc(h, (n), &h->sv.field)) != TG_OK) { tg_destroy(h); return st; }
-  AL(P, 4 * nv) AL(W, 4 * nv) AL(G, 8 * nv) AL(R, 4 * nv) AL(Uold, 4 * nv) AL(dt, nv)
+  AL(G, 2 * nv) AL(R, 4 * nv) AL(Uold, 4 * nv) AL(dt, nv)
   AL(Fb, 8 * (size_t)L.nb) AL(Fv, 9 * (size_t)L.nvu) AL(Fvb, 3 * (size_t)L.nb)
   AL(part, 4 * (size_t)std::max(h->nblocks_v, L.ntiles)) AL(R2, 4 * nv) AL(ssw, nv)
 #undef AL
-  h->Pb[0] = h->sv.P;
-  h->Wb[0] = h->sv.W;
-  for (int b = 1; b < 3; ++b) {
-    if ((st = dev_alloc(h, 4 * nv, &h->Pb[b])) != TG_OK) { tg_destroy(h); return st; }
-    if ((st = dev_alloc(h, 4 * nv, &h->Wb[b])) != TG_OK) { tg_destroy(h); return st; }
+  for (int b = 0; b < 3; ++b) {
+    if ((st = dev_alloc(h, nv, &h->Sb[b])) != TG_OK || (st = dev_alloc(h, nv, &h->Tb[b])) != TG_OK ||
+        (st = dev_alloc(h, nv, &h->V1b[b])) != TG_OK ||
+        (k.strong && (st = dev_alloc(h, nv, &h->W23b[b])) != TG_OK)) {
+      tg_destroy(h);
+      return st;
+    }
   }
-  h->smem_grad0 = tile_grad_smem(L.lmax, L.emax, L.cmax, false);
-  h->smem_grad1 = tile_grad_smem(L.lmax, L.emax, L.cmax, true);
-  h->smem_flux = flux_smem(mat->flux_scheme, mat->reconstruct_scheme, L.lmax, L.emax, L.cmax);
+  h->sv.S0 = h->Sb[0];
+  h->sv.T0 = h->Tb[0];
+  h->smem_grad = tile_grad_smem(L.lmax, L.cmax);
+  h->smem_flux = flux_smem(mat->flux_scheme, mat->reconstruct_scheme, L.lmax, L.emax, L.cmax, k.fuse_dt);
   {
-    cudaError_t ea = raise_smem((const void*)grad_kernel(true, true), h->smem_grad1);
-    cudaError_t ea2 = raise_smem((const void*)grad_kernel(true, false), h->smem_grad1);
-    cudaError_t eb = raise_smem((const void*)grad_kernel(false, true), h->smem_grad0);
+    cudaError_t ea = raise_smem((const void*)k_tile_grad, h->smem_grad);
     cudaError_t ec = raise_smem((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_UPDATE),
                                 h->smem_flux);
     cudaError_t ed = raise_smem((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_RESIDUAL),
                                 h->smem_flux);
-    if (ea != cudaSuccess || ea2 != cudaSuccess || eb != cudaSuccess || ec != cudaSuccess || ed != cudaSuccess) {
+    if (ea != cudaSuccess || ec != cudaSuccess || ed != cudaSuccess) {
       tg_destroy(h);
       return fail(nullptr, TG_CUDA_ERROR, "tile kernels need more shared memory than the device allows");
     }
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+    auto fill = [&](const void* f, size_t smem) {
+      int per = 1;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kTileThreads, smem) != cudaSuccess || per < 1) per = 1;
+      return per * sms;
+    };
+    h->grid_grad = fill((const void*)k_tile_grad, h->smem_grad);
+    h->grid_flux = fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_UPDATE), h->smem_flux);
+    h->grid_res = fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_RESIDUAL), h->smem_flux);
   }
   if ((st = dev_alloc(h, 1, &h->sc)) != TG_OK) { tg_destroy(h); return st; }
   if ((st = dev_alloc(h, 1, &h->done)) != TG_OK) { tg_destroy(h); return st; }
@@ -820,14 +893,13 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   h->kernels_per_flux = residual_kernels(h);
   // launches of a replayed step: step_begin + gradient passes + per stage (boundary,
   // viscous, tiled flux; the last also forms the norms and ends the step) + Liou /
-  // strong-condition kernels; a step that forms its own dt adds the first-stage dt
-  // pass (and its gradient-only twin) and dt_final, a fixed time step store_old.
+  // strong-condition kernels; a step that forms its own dt adds the dt pass and dt_final,
+  // a fixed time step dt_final alone.
   // The count is that of the steady state: warm steps when the next dt is fused.
   const int tail = (k.liou ? 1 : 0) + (k.strong && h->mv.nsb > 0 ? c.n_rks : 0) + c.n_rks * residual_kernels(h);
   const int grads = h->grads_needed ? c.n_rks : 0;
   if (k.fuse_dt) h->kernels_per_step = 1 + grads + tail;
-  else if (c.time_step > 0.0) h->kernels_per_step = 1 + 1 + grads + 1 + tail;
-  else h->kernels_per_step = 1 + (h->grads_needed ? c.n_rks : 1) + 1 + tail;
+  else h->kernels_per_step = 1 + (c.time_step > 0.0 ? 0 : 1) + grads + 1 + tail;
   if ((st = dev_alloc(h, 5 * (size_t)h->n_caller, &h->raw)) != TG_OK) { tg_destroy(h); return st; }
   if ((st = dev_alloc(h, 1, &h->bad)) != TG_OK) { tg_destroy(h); return st; }
   if ((st = dev_upload(h, L.old_of_new, &h->old_of_new)) != TG_OK) { tg_destroy(h); return st; }
@@ -851,23 +923,6 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
     if ((st = dev_upload(h, plan.send_idx, &P.send_idx)) != TG_OK) { tg_destroy(h); return st; }
     if ((st = dev_upload(h, plan.recv_idx, &P.recv_idx)) != TG_OK) { tg_destroy(h); return st; }
     if ((st = dev_alloc(h, 5 * (size_t)std::max(1, P.n_owned), &P.out)) != TG_OK) { tg_destroy(h); return st; }
-    // frontier tiles (some local vertex is a ghost) first, then the interior ones, so a
-    // driver can run the interior while a halo exchange is in flight
-    std::vector<int> order, interior;
-    for (int t = 0; t < L.ntiles; ++t) {
-      bool ghost = false;
-      for (int i = L.t_loff[t]; i < L.t_loff[t + 1] && !ghost; ++i) ghost = L.lv[i] >= plan.n_owned;
-      (ghost ? order : interior).push_back(t);
-    }
-    P.n_frontier = (int)order.size();
-    order.insert(order.end(), interior.begin(), interior.end());
-    if ((st = dev_upload(h, order, &h->tv.order)) != TG_OK) { tg_destroy(h); return st; }
-    if (raise_smem((const void*)grad_kernel(false, true, true), h->smem_grad0) != cudaSuccess ||
-        raise_smem((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_UPDATE, true),
-                   h->smem_flux) != cudaSuccess) {
-      tg_destroy(h);
-      return fail(nullptr, TG_CUDA_ERROR, "tile kernels need more shared memory than the device allows");
-    }
     c.part = 1;
   }
   cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
@@ -949,7 +1004,7 @@ tg_status tg_set_state_expr(tg_handle* h, const tg_expr* const* fields, const do
   int err = 0;
   if (e == cudaSuccess) {
     const int nv = h->L.nv;
-    k_state_expr<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->tv.x, h->tv.y, h->old_of_new, expr::Field5{dcode, doff, dk},
+    k_state_expr<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->tv.xy, h->old_of_new, expr::Field5{dcode, doff, dk},
                                                      drnd, n_rnd, h->raw, derr);
     e = cudaMemcpyAsync(&err, derr, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -991,7 +1046,7 @@ tg_status tg_get_state(tg_handle* h, double* prim, int n_vertex) {
     // a partition writes the records of the vertices it owns and leaves the others
     const int n = h->part.n_owned;
     std::vector<double> rec(5 * (size_t)n);
-    k_part_state_out<<<nblk(std::max(1, n)), kBlock, 0, h->stream>>>(n, h->L.nv, h->Pb[h->part.cur], h->part.out);
+    k_part_state_out<<<nblk(std::max(1, n)), kBlock, 0, h->stream>>>(n, view(h, h->part.cur), h->part.out);
     TG_CUDA(h, cudaGetLastError());
     TG_CUDA(h, cudaMemcpyAsync(rec.data(), h->part.out, rec.size() * sizeof(double), cudaMemcpyDeviceToHost,
                                h->stream));
@@ -1001,7 +1056,7 @@ tg_status tg_get_state(tg_handle* h, double* prim, int n_vertex) {
     return TG_OK;
   }
   const int nv = h->L.nv;
-  k_state_out<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->sv.P, h->old_of_new, h->raw);
+  k_state_out<<<nblk(nv), kBlock, 0, h->stream>>>(nv, view(h, 0), h->old_of_new, h->raw);
   TG_CUDA(h, cudaGetLastError());
   return state_d2h(h, prim, 5 * (size_t)nv * sizeof(double));
 }
@@ -1010,6 +1065,7 @@ tg_status tg_store_conserved_old(tg_handle* h) {
   TG_WHOLE_MESH(h)
   if (!h) return fail(h, TG_INVALID_ARG, "NULL handle");
   k_store_old<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->never);
+  h->uold_stale = false;
   return sync(h);
 }
 
@@ -1045,8 +1101,8 @@ static tg_status copy_grad_out(tg_handle* h, double* dE_out) {
     double* d = dE_out + 15 * (size_t)h->L.old_of_new[i];
     for (int q = 0; q < 15; ++q) d[q] = 0.0;
     for (int c = 0; c < 4; ++c) {
-      d[3 * var_of[c]] = g[(2 * c) * (size_t)nv + i];
-      d[3 * var_of[c] + 1] = g[(2 * c + 1) * (size_t)nv + i];
+      d[3 * var_of[c]] = g[8 * (size_t)i + 2 * c];
+      d[3 * var_of[c] + 1] = g[8 * (size_t)i + 2 * c + 1];
     }
   }
   return TG_OK;
@@ -1056,7 +1112,7 @@ tg_status tg_gradients(tg_handle* h, double* dE_out) {
   TG_WHOLE_MESH(h)
   if (!h) return fail(h, TG_INVALID_ARG, "NULL handle");
   refresh_w(h, 0);
-  enqueue_gradient(h, 0, false, true, h->never);
+  enqueue_gradient(h, 0, h->never);
   tg_status st = sync(h);
   if (st != TG_OK || !dE_out) return st;
   return copy_grad_out(h, dE_out);
@@ -1082,10 +1138,14 @@ tg_status tg_update(tg_handle* h, int r) {
   TG_WHOLE_MESH(h)
   if (!h) return fail(h, TG_INVALID_ARG, "NULL handle");
   if (r < 0 || r >= h->ctl.n_rks) return fail(h, TG_INVALID_ARG, "stage index out of range for the time scheme");
+  if (h->uold_stale) {   // U_old of a state that steps left: they form it themselves
+    k_store_old<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->never);
+    h->uold_stale = false;
+  }
   enqueue_update(h, r, false, h->never);
   h->w_partial[0] = false;                   // k_update stores all four entropy variables
   if (h->prm.strong && h->mv.nsb > 0)
-    k_strong_bc<<<nblk(h->mv.nsb), kBlock, 0, h->stream>>>(h->mv, h->sv.P, h->never);
+    k_strong_bc<<<nblk(h->mv.nsb), kBlock, 0, h->stream>>>(h->mv, view(h, 0), h->never);
   clear_dt_next(h);
   tg_status st = sync(h);
   if (st != TG_OK) return st;
@@ -1126,9 +1186,7 @@ tg_status tg_step(tg_handle* h, int n_steps, double* info4) {
   tg_status st = capture_step_graph(h);
   if (st != TG_OK) return st;
   if ((st = take_queued_input(h)) != TG_OK) return st;
-  const cudaGraphExec_t g = step_graph(h);
-  for (int i = 0; i < n_steps; ++i) TG_CUDA(h, cudaGraphLaunch(g, h->stream));
-  if (n_steps > 0) mark_steps(h);
+  if ((st = launch_steps(h, n_steps)) != TG_OK) return st;
   Scalars s;
   st = read_scalars(h, &s);
   if (st != TG_OK) return st;
@@ -1182,9 +1240,7 @@ tg_status tg_advance(tg_handle* h, int instance, long max_steps, double* info5) 
   long launched = 0;
   while (launched < max_steps && !s.bad && s.counter <= instance && !run_over(h, s)) {
     const long chunk = std::min<long>(16, max_steps - launched);
-    const cudaGraphExec_t g = step_graph(h);
-    for (long i = 0; i < chunk; ++i) TG_CUDA(h, cudaGraphLaunch(g, h->stream));
-    mark_steps(h);
+    if ((st = launch_steps(h, chunk)) != TG_OK) return st;
     launched += chunk;
     if ((st = read_scalars(h, &s)) != TG_OK) return st;
     h->cold = !s.dt_next;
@@ -1212,6 +1268,8 @@ tg_status tg_update_parameters(tg_handle* h, const tg_material* mat, const tg_bc
   k.sqrt_gm1 = std::sqrt(mat->gamma - 1.0);
   k.inv_gamma = 1.0 / mat->gamma;
   k.inv_gm1 = 1.0 / (mat->gamma - 1.0);
+  k.gm1 = mat->gamma - 1.0;
+  k.inv_R = 1.0 / mat->gas_const;
   k.gp1_gm1 = (mat->gamma + 1.0) / (mat->gamma - 1.0);
   k.prandtl = mat->prandtl; k.mu_ref = mat->mu_ref; k.T0 = mat->T_0; k.Tref = mat->T_ref; k.omega = mat->omega;
   k.ev_alpha = mat->ev_mod_alpha; k.ev_beta = mat->ev_mod_beta; k.tvbM = mat->tvb_minmod_coef;
@@ -1251,13 +1309,13 @@ tg_status tg_output_begin(tg_handle* h, double* prim_out, double* dE_out, int gr
   }
   // the previous snapshot's copies finish before its buffers are written again
   if (h->out_pending) TG_CUDA(h, cudaStreamWaitEvent(h->stream, h->out_done, 0));
-  k_state_out<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->Pb[0], h->old_of_new, h->snap);
+  k_state_out<<<nblk(nv), kBlock, 0, h->stream>>>(nv, view(h, 0), h->old_of_new, h->snap);
   if (dE_out) {
     // the reference writes the dE of its last compute_gradients: the last stage's input
     // state after a step, the current state after compute_forces of a Navier-Stokes run
     const int last_in = h->ctl.scheme == 1 ? 1 : h->ctl.n_rks - 1;
     refresh_w(h, grad_state == TG_GRAD_CURRENT ? 0 : last_in);
-    enqueue_gradient(h, grad_state == TG_GRAD_CURRENT ? 0 : last_in, false, true, h->never);
+    enqueue_gradient(h, grad_state == TG_GRAD_CURRENT ? 0 : last_in, h->never);
     k_grad_out<<<nblk(nv), kBlock, 0, h->stream>>>(nv, h->sv.G, h->old_of_new, h->snap_grad, h->sc,
                                                     grad_state == TG_GRAD_LAST_STAGE ? 1 : 0);
   }
@@ -1302,7 +1360,7 @@ tg_status tg_forces(tg_handle* h, int n_forces, const int* n_tags, const int* ta
   TG_CUDA(h, cudaMemcpyAsync(r, rec.data(), rec.size() * sizeof(int4), cudaMemcpyHostToDevice, h->stream));
   TG_CUDA(h, cudaMemcpyAsync(o, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   // Navier-Stokes forces recompute the gradients of the current state (src/force.cc:123)
-  if (h->prm.model == 1) enqueue_gradient(h, 0, false, true, h->never);
+  if (h->prm.model == 1) enqueue_gradient(h, 0, h->never);
   k_forces<<<n_forces, kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), drec, doff, dout);
   std::vector<double> hout(4 * (size_t)n_forces);
   cudaError_t e = cudaMemcpyAsync(hout.data(), dout, hout.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
@@ -1341,13 +1399,13 @@ tg_status tg_moments_increment(tg_handle* h, int instance, long k) {
     Scalars s;
     if ((st = read_scalars(h, &s)) != TG_OK) return st;
     if (s.iter == 0) {
-      enqueue_gradient(h, 0, false, true, h->never);
+      enqueue_gradient(h, 0, h->never);
     } else if (!h->grads_needed) {
       refresh_w(h, 2);
-      enqueue_gradient(h, 2, false, true, h->never);
+      enqueue_gradient(h, 2, h->never);
     }
   }
-  k_moments_increment<<<nblk(h->L.nv), kBlock, 0, h->stream>>>(h->prm, h->L.nv, h->sv.P, h->sv.G, h->mom_extras,
+  k_moments_increment<<<nblk(h->L.nv), kBlock, 0, h->stream>>>(h->prm, h->L.nv, view(h, 0), h->mom_extras,
                                                                  h->mom_nvar, (long long)k, mom_array(h, instance, 0),
                                                                  mom_array(h, instance, 1), mom_array(h, instance, 2));
   return sync(h);
@@ -1571,8 +1629,7 @@ tg_status tg_part_prime(tg_handle* h) {
   tg_status st = part_check(h);
   if (st != TG_OK) return st;
   if (h->prm.fuse_dt) {
-    grad_kernel(true, false)<<<h->L.ntiles, kTileThreads, h->smem_grad1, h->stream>>>(
-        h->prm, h->mv, h->tv, view(h, 0), h->sc, h->L.lmax, h->L.emax, h->never, 0);
+    k_dt<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->sc, h->never, 0);
     k_part_primed<<<1, 1, 0, h->stream>>>(h->sc);
   }
   h->cold = false;
@@ -1584,7 +1641,6 @@ tg_status tg_part_begin(tg_handle* h) {
   if (st != TG_OK) return st;
   if (h->cold) return fail(h, TG_INVALID_ARG, "tg_part_prime and the scalar exchange come first after a new state");
   k_step_begin<<<1, 1, 0, h->stream>>>(h->ctl, h->sc, h->done, 1);
-  if (h->ctl.time_step > 0.0) k_store_old<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->done);
   return launched(h);
 }
 
@@ -1614,7 +1670,7 @@ tg_status tg_part_gradients(tg_handle* h, int r, int which) {
   int bin, bout, base, count;
   if ((st = part_tiles(h, which, &base, &count)) != TG_OK) return st;
   stage_buffers(h, r, &bin, &bout);
-  enqueue_gradient(h, bin, false, h->grads_needed, h->done, base, count);
+  if (h->grads_needed) enqueue_gradient(h, bin, h->done, base, count);
   return launched(h);
 }
 
@@ -1641,12 +1697,11 @@ tg_status tg_part_pack(tg_handle* h, int field, void* dev_send) {
   tg_status st = part_check(h);
   if (st != TG_OK) return st;
   if (field != TG_HALO_STATE && field != TG_HALO_GRAD) return fail(h, TG_INVALID_ARG, "unknown halo field");
-  const int n = h->part.n_send, nv = h->L.nv;
+  const int n = h->part.n_send;
   if (n == 0) return TG_OK;
   if (!dev_send) return fail(h, TG_INVALID_ARG, "NULL send buffer");
-  const double* A = field == TG_HALO_STATE ? h->Pb[h->part.cur] : h->sv.G;
-  const double* B = field == TG_HALO_STATE ? h->Wb[h->part.cur] : h->sv.G + 4 * (size_t)nv;
-  k_halo_pack<<<nblk(8 * n), kBlock, 0, h->stream>>>(n, h->part.send_idx, nv, A, B, (double*)dev_send);
+  k_halo_pack<<<nblk(2 * n), kBlock, 0, h->stream>>>(n, h->part.send_idx, view(h, h->part.cur),
+                                                      field == TG_HALO_GRAD ? 1 : 0, (double*)dev_send);
   return launched(h);
 }
 
@@ -1654,12 +1709,11 @@ tg_status tg_part_unpack(tg_handle* h, int field, const void* dev_recv) {
   tg_status st = part_check(h);
   if (st != TG_OK) return st;
   if (field != TG_HALO_STATE && field != TG_HALO_GRAD) return fail(h, TG_INVALID_ARG, "unknown halo field");
-  const int n = h->part.n_recv, nv = h->L.nv;
+  const int n = h->part.n_recv;
   if (n == 0) return TG_OK;
   if (!dev_recv) return fail(h, TG_INVALID_ARG, "NULL receive buffer");
-  double* A = field == TG_HALO_STATE ? h->Pb[h->part.cur] : h->sv.G;
-  double* B = field == TG_HALO_STATE ? h->Wb[h->part.cur] : h->sv.G + 4 * (size_t)nv;
-  k_halo_unpack<<<nblk(8 * n), kBlock, 0, h->stream>>>(n, h->part.recv_idx, nv, A, B, (const double*)dev_recv);
+  k_halo_unpack<<<nblk(2 * n), kBlock, 0, h->stream>>>(n, h->part.recv_idx, view(h, h->part.cur),
+                                                        field == TG_HALO_GRAD ? 1 : 0, (const double*)dev_recv);
   return launched(h);
 }
 

@@ -16,8 +16,12 @@ constexpr int kBlock = 256;
 struct MeshView {
   int nv, ne, nb, nvu, n_int_cells;
   const double *dcarea, *inv6mc, *pweight;
+  const double *inv_area;             // 1 / dcarea
+  // local time step: sum of |n| over a vertex's gather list (boundary faces half), and of
+  // |n| / |x_b - x_a| over its edges (viscous runs)
+  const double *lam_area, *lam_visc;
   const int *e_a, *e_b;
-  const double *e_nx, *e_ny, *e_dx, *e_dy, *e_g0x, *e_g0y, *e_g1x, *e_g1y;
+  const double *e_nx, *e_ny, *e_dx, *e_dy;
   const int *ce_off, *ce_ent;
   const int *cb_off, *cb_ent;
   const int *b_v0, *b_v1, *b_kind, *b_adiab, *b_cell;
@@ -44,15 +48,36 @@ __device__ __forceinline__ double vertex_radius(const Params& k, const MeshView&
   return k.axi ? m.v_r[v] : 1.0;
 }
 
-// Device state, structure-of-arrays with component stride nv (or ne, nb ...).
+// A 32-byte record: one sector, moved by one 256-bit access per thread.
+struct alignas(32) D4 {
+  double x, y, z, w;
+};
+__device__ __forceinline__ D4 ld4(const D4* p) {
+  D4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st4(D4* p, double x, double y, double z, double w) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
+}
+
+// Device state.  What the flux of a vertex reads is one 32-byte record
+// S = (u, v, p, V5), so a gather of a neighbour touches one sector and one owned vertex
+// is one access; the temperature and V1 are arrays of their own (the central fluxes read
+// neither).  V2 = -V5 u and V3 = -V5 v are not stored: with V5 = -2 beta they are the
+// products prim2ent forms.  Strong boundary conditions reset u, v, p and T after an update
+// and leave the entropy variables, so their runs keep V2, V3 in W23.
 struct StateView {
-  double* P;      // 4*nv  T,u,v,p
-  double* W;      // 4*nv  V1,V2,V3,V5
-  double* G;      // 8*nv  dV1/dx, dV1/dy, dV2/dx, ..., dV5/dy
-  double* R;      // 4*nv
-  double* Uold;   // 4*nv
+  D4* S;          // nv    u, v, p, V5
+  double* T;      // nv
+  double* V1;     // nv
+  double2* W23;   // nv    V2, V3 (bc_scheme strong only)
+  const D4* S0;   // the state the step started from: U_old is formed from it (not for strong
+  const double* T0;   // conditions' reset vertices: their density comes from T0)
+  D4* G;          // 2*nv  (dV1/dx, dV1/dy, dV2/dx, dV2/dy), (dV3/dx, dV3/dy, dV5/dx, dV5/dy)
+  double* R;      // 4*nv  component-major
+  double* Uold;   // 4*nv  store_conserved_old for the single-phase calls
   double* dt;     // nv
-  double* Fe;     // 4*ne
   double* Fb;     // 4*2*nb
   double* Fv;     // 3*3*nvu  (x-mom, y-mom, energy)
   double* Fvb;    // 3*nb
@@ -97,37 +122,78 @@ struct Control {
   int part;            // a partition of a decomposed mesh: norms wait for the other partitions' sums
 };
 
-__device__ __forceinline__ Prim load_prim(const double* P, int nv, int i) {
+__device__ __forceinline__ Prim load_prim(const StateView& s, int i) {
+  const D4 r = ld4(s.S + i);
   Prim q;
-  q.T = P[i]; q.u = P[nv + i]; q.v = P[2 * nv + i]; q.p = P[3 * nv + i];
+  q.T = s.T[i]; q.u = r.x; q.v = r.y; q.p = r.z;
   return q;
+}
+// The stored entropy variables of a vertex.
+__device__ __forceinline__ Ent load_ent(const Params& k, const StateView& s, int i) {
+  const D4 r = ld4(s.S + i);
+  Ent e;
+  e.f = s.V1[i]; e.l = r.w;
+  if (k.strong) {
+    const double2 w = s.W23[i];
+    e.vx = w.x; e.vy = w.y;
+  } else {
+    e.vx = -r.w * r.x; e.vy = -r.w * r.y;
+  }
+  return e;
+}
+__device__ __forceinline__ void store_state(const Params& k, const StateView& s, int i, const Prim& q, const Ent& e) {
+  st4(s.S + i, q.u, q.v, q.p, e.l);
+  s.T[i] = q.T;
+  s.V1[i] = e.f;
+  if (k.strong) s.W23[i] = make_double2(e.vx, e.vy);
+}
+
+// Entropy variables of a vertex after a boundary condition's single-state form
+// (src/bc.h:615-654).  A condition that changes nothing returns the stored variables; one
+// that keeps T and p (slip, adiabatic no-slip) moves V1 by beta (|u|^2 - |u'|^2) exactly;
+// the others, and strong runs (whose stored variables lag the reset state), form them anew.
+// Without the logarithms a boundary vertex's thread no longer holds its tile's gradient
+// pass back as long (17.7 -> 15.5 us on the 128 x 256 cylinder).
+__device__ __forceinline__ Ent bc_ent(const Params& k, const StateView& s, int kind, int adiabatic, const double* val,
+                                      double nx, double ny, int v) {
+  if (!k.strong && (kind == BC_NONE || kind == BC_FARFIELD || kind == BC_OUTLET || kind == BC_PERIODIC))
+    return load_ent(k, s, v);
+  Prim q = load_prim(s, v);
+  if (!k.strong && (kind == BC_SLIP || (kind == BC_NOSLIP && adiabatic))) {
+    const double q2 = q.u * q.u + q.v * q.v, V5 = s.S[v].w;
+    bc_apply1(kind, adiabatic, val, nx, ny, q);
+    Ent e;
+    e.f = s.V1[v] - 0.5 * V5 * (q2 - (q.u * q.u + q.v * q.v));
+    e.vx = -V5 * q.u; e.vy = -V5 * q.v; e.l = V5;
+    return e;
+  }
+  bc_apply1(kind, adiabatic, val, nx, ny, q);
+  return prim2ent(k, q);
 }
 
 // Boundary correction n_b * (W_b0 + W_b1 - W_0 - W_1)/2 of one boundary face
 // (src/fv.cc:926-966): states after the single-state BC at each face vertex.
 __device__ __forceinline__ void bface_grad_corr(const Params& k, const MeshView& m, const StateView& s, int d,
                                                 double* dW /*4*/) {
-  int v0 = m.b_v0[d], v1 = m.b_v1[d];
-  Prim s0 = load_prim(s.P, m.nv, v0), s1 = load_prim(s.P, m.nv, v1);
-  double nx = m.b_nx[d], ny = m.b_ny[d];
-  bc_apply1(m.b_kind[d], m.b_adiab[d], m.b_val + (size_t)d * 10, nx, ny, s0);
-  bc_apply1(m.b_kind[d], m.b_adiab[d], m.b_val + (size_t)d * 10 + 5, nx, ny, s1);
-  Ent e0 = prim2ent(k, s0), e1 = prim2ent(k, s1);
-  const double* W = s.W;
-  const int nv = m.nv;
-  dW[0] = (e0.f + e1.f - W[v0] - W[v1]) / 2.0;
-  dW[1] = (e0.vx + e1.vx - W[nv + v0] - W[nv + v1]) / 2.0;
-  dW[2] = (e0.vy + e1.vy - W[2 * nv + v0] - W[2 * nv + v1]) / 2.0;
-  dW[3] = (e0.l + e1.l - W[3 * nv + v0] - W[3 * nv + v1]) / 2.0;
+  const int v0 = m.b_v0[d], v1 = m.b_v1[d], kind = m.b_kind[d], ad = m.b_adiab[d];
+  const double nx = m.b_nx[d], ny = m.b_ny[d];
+  const Ent e0 = bc_ent(k, s, kind, ad, m.b_val + (size_t)d * 10, nx, ny, v0);
+  const Ent e1 = bc_ent(k, s, kind, ad, m.b_val + (size_t)d * 10 + 5, nx, ny, v1);
+  const Ent w0 = load_ent(k, s, v0), w1 = load_ent(k, s, v1);
+  dW[0] = (e0.f + e1.f - w0.f - w1.f) * 0.5;
+  dW[1] = (e0.vx + e1.vx - w0.vx - w1.vx) * 0.5;
+  dW[2] = (e0.vy + e1.vy - w0.vy - w1.vy) * 0.5;
+  dW[3] = (e0.l + e1.l - w0.l - w1.l) * 0.5;
 }
 
 // ------------------------------------------------------------------ kernels
 
-__global__ void k_prim2ent(Params k, int nv, const double* __restrict__ P, double* __restrict__ W) {
+// Entropy variables of a state from its primitive one; bad (may be NULL): only when clear.
+__global__ void k_prim2ent(Params k, int nv, StateView s, const int* __restrict__ bad) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nv) return;
-  Ent e = prim2ent(k, load_prim(P, nv, i));
-  W[i] = e.f; W[nv + i] = e.vx; W[2 * nv + i] = e.vy; W[3 * nv + i] = e.l;
+  if (i >= nv || (bad && *bad)) return;
+  const Prim q = load_prim(s, i);
+  store_state(k, s, i, q, prim2ent(k, q));
 }
 
 // A caller state arrives as PrimVar records (T, p, u, v, w; src/primvar.h:17-18) in the caller's
@@ -143,33 +209,27 @@ __global__ void k_state_check(int nv, const double* __restrict__ raw, int* __res
 }
 
 __global__ void k_state_in(int nv, const double* __restrict__ raw, const int* __restrict__ old_of_new,
-                           const int* __restrict__ bad, double* __restrict__ P) {
+                           const int* __restrict__ bad, D4* __restrict__ S, double* __restrict__ T) {
   if (*bad) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
   const double* q = raw + 5 * (size_t)old_of_new[i];
-  P[i] = q[0]; P[nv + i] = q[2]; P[2 * (size_t)nv + i] = q[3]; P[3 * (size_t)nv + i] = q[1];
+  st4(S + i, q[2], q[3], q[1], 0.0);   // V5 and V1 follow (k_prim2ent)
+  T[i] = q[0];
 }
 
-// Device SoA (T, u, v, p) -> PrimVar records in the caller's order (w = 0 in 2D).
-__global__ void k_state_out(int nv, const double* __restrict__ P, const int* __restrict__ old_of_new,
+// Device records -> PrimVar records in the caller's order (w = 0 in 2D).
+__global__ void k_state_out(int nv, StateView s, const int* __restrict__ old_of_new,
                             double* __restrict__ raw) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
   double* q = raw + 5 * (size_t)old_of_new[i];
-  q[0] = P[i]; q[1] = P[3 * (size_t)nv + i]; q[2] = P[nv + i]; q[3] = P[2 * (size_t)nv + i]; q[4] = 0.0;
+  const Prim r = load_prim(s, i);
+  q[0] = r.T; q[1] = r.p; q[2] = r.u; q[3] = r.v; q[4] = 0.0;
 }
 
-// A state handed in asynchronously (tg_set_state_async) becomes current only if
-// k_state_check accepted it: its entropy variables and fresh step bookkeeping.
-__global__ void k_prim2ent_checked(Params k, int nv, const double* __restrict__ P, double* __restrict__ W,
-                                   const int* __restrict__ bad) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nv || *bad) return;
-  Ent e = prim2ent(k, load_prim(P, nv, i));
-  W[i] = e.f; W[nv + i] = e.vx; W[2 * nv + i] = e.vy; W[3 * nv + i] = e.l;
-}
-
+// A state handed in asynchronously (tg_set_state_async) becomes current, with fresh step
+// bookkeeping, only if k_state_check accepted it.
 __global__ void k_scalars_set(Scalars* sc, Scalars s0, const int* __restrict__ bad) {
   if (*bad) return;
   *sc = s0;
@@ -180,20 +240,17 @@ __global__ void k_scalars_set(Scalars* sc, Scalars s0, const int* __restrict__ b
 // zero for the z components and for the fourth (z-momentum) variable.
 // zero_unstepped: all zero while no step has run since the state was set (the
 // reference zeroes dE when a sample starts, src/fv.cc:207-212).
-__global__ void k_grad_out(int nv, const double* __restrict__ G, const int* __restrict__ old_of_new,
+__global__ void k_grad_out(int nv, const D4* __restrict__ G, const int* __restrict__ old_of_new,
                            double* __restrict__ out, const Scalars* __restrict__ sc, int zero_unstepped) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
   double* d = out + 15 * (size_t)old_of_new[i];
-  const int var_of[4] = {0, 1, 2, 4};
 #pragma unroll
   for (int q = 0; q < 15; ++q) d[q] = 0.0;
   if (zero_unstepped && sc->iter == 0) return;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    d[3 * var_of[c]] = G[(size_t)(2 * c) * nv + i];
-    d[3 * var_of[c] + 1] = G[(size_t)(2 * c + 1) * nv + i];
-  }
+  const D4 a = ld4(G + 2 * (size_t)i), b = ld4(G + 2 * (size_t)i + 1);
+  d[0] = a.x; d[1] = a.y; d[3] = a.z; d[4] = a.w;       // variables 0, 1, 2 and 4 of five
+  d[6] = b.x; d[7] = b.y; d[12] = b.z; d[13] = b.w;
 }
 
 // store_conserved_old (src/fv.cc:1626-1630)
@@ -201,7 +258,7 @@ __global__ void k_store_old(Params k, MeshView m, StateView s, const int* __rest
   if (*done) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.nv) return;
-  Cons c = prim2con(k, load_prim(s.P, m.nv, i));
+  Cons c = prim2con(k, load_prim(s, i));
   s.Uold[i] = c.r; s.Uold[m.nv + i] = c.mx; s.Uold[2 * m.nv + i] = c.my; s.Uold[3 * m.nv + i] = c.E;
 }
 
@@ -213,7 +270,7 @@ __global__ void k_bflux(Params k, MeshView m, StateView s, const int* __restrict
   if (t >= 2 * m.nb) return;
   int d = t >> 1, q = t & 1;
   int c = q ? m.b_v1[d] : m.b_v0[d];
-  Prim s0 = load_prim(s.P, m.nv, c), s1 = s0;
+  Prim s0 = load_prim(s, c), s1 = s0;
   double nx = m.b_nx[d], ny = m.b_ny[d];
   int kind = m.b_kind[d];
   bc_apply2(kind, m.b_adiab[d], m.b_val + (size_t)d * 10 + 5 * q, nx, ny, s0, s1);
@@ -233,17 +290,19 @@ __global__ void k_viscous(Params k, MeshView m, StateView s, const int* __restri
   if (*done) return;
   int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= m.nvu) return;
-  const int nv = m.nv;
   int c = m.u_cell[u];
   int v[3] = {m.c_v[3 * c], m.c_v[3 * c + 1], m.c_v[3 * c + 2]};
   const double* n = m.c_n + 6 * (size_t)c;
   // cell gradient: P1 sum, boundary corrections in face order, / (2 area)
+  const Ent w0 = load_ent(k, s, v[0]), w1 = load_ent(k, s, v[1]), w2 = load_ent(k, s, v[2]);
   double dE[8];
+  {
+    const double a[4][3] = {{w0.f, w1.f, w2.f}, {w0.vx, w1.vx, w2.vx}, {w0.vy, w1.vy, w2.vy}, {w0.l, w1.l, w2.l}};
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    double w0 = s.W[q * nv + v[0]], w1 = s.W[q * nv + v[1]], w2 = s.W[q * nv + v[2]];
-    dE[2 * q] = n[0] * w0 + n[2] * w1 + n[4] * w2;
-    dE[2 * q + 1] = n[1] * w0 + n[3] * w1 + n[5] * w2;
+    for (int q = 0; q < 4; ++q) {
+      dE[2 * q] = n[0] * a[q][0] + n[2] * a[q][1] + n[4] * a[q][2];
+      dE[2 * q + 1] = n[1] * a[q][0] + n[3] * a[q][1] + n[5] * a[q][2];
+    }
   }
   for (int j = m.c_bf_off[c]; j < m.c_bf_off[c + 1]; ++j) {
     int d = m.c_bf[j];
@@ -262,10 +321,10 @@ __global__ void k_viscous(Params k, MeshView m, StateView s, const int* __restri
   Ent avg;
   if (u < m.n_int_cells) {
     const double t3 = 1.0 / 3.0;
-    avg.f = s.W[v[0]] * t3 + s.W[v[1]] * t3 + s.W[v[2]] * t3;
-    avg.vx = s.W[nv + v[0]] * t3 + s.W[nv + v[1]] * t3 + s.W[nv + v[2]] * t3;
-    avg.vy = s.W[2 * nv + v[0]] * t3 + s.W[2 * nv + v[1]] * t3 + s.W[2 * nv + v[2]] * t3;
-    avg.l = s.W[3 * nv + v[0]] * t3 + s.W[3 * nv + v[1]] * t3 + s.W[3 * nv + v[2]] * t3;
+    avg.f = w0.f * t3 + w1.f * t3 + w2.f * t3;
+    avg.vx = w0.vx * t3 + w1.vx * t3 + w2.vx * t3;
+    avg.vy = w0.vy * t3 + w1.vy * t3 + w2.vy * t3;
+    avg.l = w0.l * t3 + w1.l * t3 + w2.l * t3;
   } else {
     avg.f = avg.vx = avg.vy = avg.l = 0.0;
     int cnt = m.c_nbr_off[c + 1] - m.c_nbr_off[c];
@@ -273,10 +332,8 @@ __global__ void k_viscous(Params k, MeshView m, StateView s, const int* __restri
       int d = m.c_nbr[j];
       for (int q = 0; q < 2; ++q) {
         int vb = q ? m.bf_face_v1[d] : m.bf_face_v0[d];
-        Prim st = load_prim(s.P, nv, vb);
         const double* val = m.b_val + (size_t)d * 10 + (vb == m.b_v0[d] ? 0 : 5);
-        bc_apply1(m.b_kind[d], m.b_adiab[d], val, m.bf_face_nx[d], m.bf_face_ny[d], st);
-        Ent e = prim2ent(k, st);
+        const Ent e = bc_ent(k, s, m.b_kind[d], m.b_adiab[d], val, m.bf_face_nx[d], m.bf_face_ny[d], vb);
         avg.f += e.f; avg.vx += e.vx; avg.vy += e.vy; avg.l += e.l;
       }
     }
@@ -307,6 +364,16 @@ __device__ __forceinline__ double face_radius(double u, double v, double nx, dou
   return fma(c, area, fabs(fma(u, nx, v * ny)));
 }
 
+// The spectral radius sum of a vertex whose copies all hold its state q, from the sum of
+// |u.n| over its faces: + c sum |n| + (mu / rho) sum |n| / |d|, the geometric sums formed
+// once per mesh.  The last stage's update and k_dt both use it, so a step whose dt is
+// formed either way is the same bit for bit.
+__device__ __forceinline__ double spectral_sum(const Params& k, const MeshView& m, int v, const Prim& q, double un) {
+  double lam = fma(sound_speed(k, q), m.lam_area[v], un);
+  if (k.model == 1) lam = fma(viscosity(k, q.T) * (k.R * q.T) / q.p, m.lam_visc[v], lam);
+  return lam;
+}
+
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -318,43 +385,55 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x)
 
 // Local time step (src/fv.cc:1499-1598): spectral-radius gather, dt = cfl A / sum,
 // block minimum by warp shuffles, then one atomicMin on the (positive) bit pattern.
-__global__ void k_dt(Params k, MeshView m, StateView s, Scalars* sc, const int* __restrict__ done) {
+__global__ void k_dt(Params k, MeshView m, StateView s, Scalars* sc, const int* __restrict__ done, int in_step) {
   if (*done) return;
+  if (in_step && k.fuse_dt && sc->dt_next) return;   // the previous step's last update formed it
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long bits = 0x7ff0000000000000ull;  // +inf
   if (v < m.nv) {
-    const int nv = m.nv;
+    const Prim q0 = load_prim(s, v);
     double lam = 0.0;
+    bool same = true;    // every periodic copy holds this vertex's state, as after any update
     for (int j = m.ce_off[v]; j < m.ce_off[v + 1]; ++j) {
-      int ent = m.ce_ent[j];
-      int e = ent >> 1;
-      int self = (ent & 1) ? m.e_b[e] : m.e_a[e];
-      Prim q = load_prim(s.P, nv, self);
-      double nx = m.e_nx[e], ny = m.e_ny[e];
-      double area = face_area(nx, ny);
-      lam += face_radius(q.u, q.v, nx, ny, sound_speed(k, q), area) * 1.0;
-    }
-    for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
-      int ent = m.cb_ent[j];
-      if ((ent & 3) != 0) continue;
-      int idx = ent >> 2, d = idx >> 1;
-      int self = (idx & 1) ? m.b_v1[d] : m.b_v0[d];
-      Prim q = load_prim(s.P, nv, self);
-      double nx = m.b_nx[d], ny = m.b_ny[d];
-      double area = face_area(nx, ny);
-      lam += 0.5 * face_radius(q.u, q.v, nx, ny, sound_speed(k, q), area);
-    }
-    if (k.model == 1) {
-      for (int j = m.ce_off[v]; j < m.ce_off[v + 1]; ++j) {
-        int ent = m.ce_ent[j];
-        int e = ent >> 1;
-        int self = (ent & 1) ? m.e_b[e] : m.e_a[e];
-        Prim q = load_prim(s.P, nv, self);
-        double nx = m.e_nx[e], ny = m.e_ny[e];
-        double area = face_area(nx, ny);
-        double dl = face_area(m.e_dx[e], m.e_dy[e]);
-        lam += (viscosity(k, q.T) * area / dl / density(k, q)) * 1.0;
+      const int ent = m.ce_ent[j], e = ent >> 1;
+      const int self = (ent & 1) ? m.e_b[e] : m.e_a[e];
+      if (self != v) {
+        const Prim q = load_prim(s, self);
+        same = same && q.u == q0.u && q.v == q0.v && q.T == q0.T && q.p == q0.p;
       }
+      lam += fabs(fma(q0.u, m.e_nx[e], q0.v * m.e_ny[e]));
+    }
+    if (same) {
+      for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
+        const int ent = m.cb_ent[j];
+        if ((ent & 3) != 0) continue;
+        const int d = ent >> 3;
+        lam += 0.5 * fabs(fma(q0.u, m.b_nx[d], q0.v * m.b_ny[d]));
+      }
+      lam = spectral_sum(k, m, v, q0, lam);
+    } else {   // an initial state whose copies differ: each contribution from its own copy
+      lam = 0.0;
+      for (int j = m.ce_off[v]; j < m.ce_off[v + 1]; ++j) {
+        const int ent = m.ce_ent[j], e = ent >> 1;
+        const Prim q = load_prim(s, (ent & 1) ? m.e_b[e] : m.e_a[e]);
+        const double nx = m.e_nx[e], ny = m.e_ny[e];
+        lam += face_radius(q.u, q.v, nx, ny, sound_speed(k, q), face_area(nx, ny));
+      }
+      for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
+        const int ent = m.cb_ent[j];
+        if ((ent & 3) != 0) continue;
+        const int idx = ent >> 2, d = idx >> 1;
+        const Prim q = load_prim(s, (idx & 1) ? m.b_v1[d] : m.b_v0[d]);
+        const double nx = m.b_nx[d], ny = m.b_ny[d];
+        lam += 0.5 * face_radius(q.u, q.v, nx, ny, sound_speed(k, q), face_area(nx, ny));
+      }
+      if (k.model == 1)
+        for (int j = m.ce_off[v]; j < m.ce_off[v + 1]; ++j) {
+          const int ent = m.ce_ent[j], e = ent >> 1;
+          const Prim q = load_prim(s, (ent & 1) ? m.e_b[e] : m.e_a[e]);
+          const double area = face_area(m.e_nx[e], m.e_ny[e]), dl = face_area(m.e_dx[e], m.e_dy[e]);
+          lam += viscosity(k, q.T) * area / dl / density(k, q);
+        }
     }
     double dtv = k.cfl * m.dcarea[v] / lam;
     s.dt[v] = dtv;
@@ -382,7 +461,7 @@ __global__ void k_ssw(Params k, MeshView m, StateView s, const int* __restrict__
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.ne) return;
   const int a = m.e_a[e], b = m.e_b[e];
-  const Prim qa = load_prim(s.P, m.nv, a), qb = load_prim(s.P, m.nv, b);
+  const Prim qa = load_prim(s, a), qb = load_prim(s, b);
   const double nx = m.e_nx[e], ny = m.e_ny[e];
   const double ui = qa.u * nx + qa.v * ny, uj = qb.u * nx + qb.v * ny;
   const double ai = sound_speed(k, qa), aj = sound_speed(k, qb);
@@ -399,17 +478,18 @@ __global__ void k_ssw(Params k, MeshView m, StateView s, const int* __restrict__
 // boundary face's condition applied to its vertices' primitive state in face
 // order; the entropy variables keep their values (the reference does not
 // recompute them), so gradients see the pre-condition state.
-__global__ void k_strong_bc(MeshView m, double* __restrict__ P, const int* __restrict__ done) {
+__global__ void k_strong_bc(MeshView m, StateView s, const int* __restrict__ done) {
   if (*done) return;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= m.nsb) return;
-  const int v = m.sb_v[j], nv = m.nv;
-  Prim q = load_prim(P, nv, v);
+  const int v = m.sb_v[j];
+  Prim q = load_prim(s, v);
   for (int e = m.sb_off[j]; e < m.sb_off[j + 1]; ++e) {
     const int d = m.sb_ent[e] >> 1, slot = m.sb_ent[e] & 1;
     bc_apply1(m.b_kind[d], m.b_adiab[d], m.b_val + (size_t)d * 10 + 5 * slot, m.b_nx[d], m.b_ny[d], q);
   }
-  P[v] = q.T; P[nv + v] = q.u; P[2 * (size_t)nv + v] = q.v; P[3 * (size_t)nv + v] = q.p;
+  st4(s.S + v, q.u, q.v, q.p, s.S[v].w);
+  s.T[v] = q.T;
 }
 
 // bc_scheme strong, in compute_residual_norm (src/fv.cc:1805-1819): the momentum
@@ -517,30 +597,28 @@ __device__ __forceinline__ void norm_and_step_end(const StateView& s, int nblock
 // SSP-RK3 stage (src/fv.cc:1635-1658, src/constants.h:4-6) or the classical RK4
 // stage (src/fv.cc:1667-1679, src/constants.h:9), which accumulates
 // sum_r R_r / rks_r in R2 (zero before the first stage, src/fv.cc:2287-2293).
-// q0 is the stage's input state, uo U_old, factor = dt / area.
-__device__ __forceinline__ Cons rk_stage(const Params& k, const Control& ctl, const StateView& s, int nv, int v, int r,
-                                         const Prim& q0, const double* uo, double factor, double r0, double r1,
-                                         double r2, double r3) {
-  Cons c;
+// c is the stage's input state (conserved), uo U_old, factor = dt / area.
+__device__ __forceinline__ Cons rk_stage(const Control& ctl, const StateView& s, int nv, int v, int r, Cons c,
+                                         const double* uo, double factor, double r0, double r1, double r2, double r3) {
   if (ctl.scheme == 1) {
-    const double rks[4] = {1.0, 1.0 / 2.0, 1.0 / 2.0, 1.0};
-    const double inv = 1.0 / rks[r];
+    // selects, not an indexed table: the stage is a run-time value and a table would live in
+    // local memory
+    const double inv = (r == 1 || r == 2) ? 2.0 : 1.0;   // 1 / rks[r], rks = (1, 1/2, 1/2, 1)
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
     if (r > 0) { a0 = s.R2[v]; a1 = s.R2[nv + v]; a2 = s.R2[2 * nv + v]; a3 = s.R2[3 * nv + v]; }
     a0 += r0 * inv; a1 += r1 * inv; a2 += r2 * inv; a3 += r3 * inv;
     if (r < 3) { s.R2[v] = a0; s.R2[nv + v] = a1; s.R2[2 * nv + v] = a2; s.R2[3 * nv + v] = a3; }
     const bool fin = (r == 3);
-    const double c2 = fin ? -factor / 6.0 : -factor * rks[r < 3 ? r + 1 : 3];
+    const double c2 = fin ? -factor / 6.0 : -factor * (r == 2 ? 1.0 : 0.5);
     c.r = uo[0] * 1.0 + (fin ? a0 : r0) * c2;
     c.mx = uo[1] * 1.0 + (fin ? a1 : r1) * c2;
     c.my = uo[2] * 1.0 + (fin ? a2 : r2) * c2;
     c.E = uo[3] * 1.0 + (fin ? a3 : r3) * c2;
     return c;
   }
-  const double a_rk[3] = {0.0, 3.0 / 4.0, 1.0 / 3.0};
-  const double b_rk[3] = {1.0, 1.0 / 4.0, 2.0 / 3.0};
-  c = prim2con(k, q0);
-  const double br = b_rk[r], ar = a_rk[r], c2 = -factor * br;
+  const double ar = r == 0 ? 0.0 : (r == 1 ? 3.0 / 4.0 : 1.0 / 3.0);
+  const double br = r == 0 ? 1.0 : (r == 1 ? 1.0 / 4.0 : 2.0 / 3.0);
+  const double c2 = -factor * br;
   c.r *= br; c.mx *= br; c.my *= br; c.E *= br;
   c.r += uo[0] * ar + r0 * c2;
   c.mx += uo[1] * ar + r1 * c2;
@@ -557,20 +635,19 @@ __global__ void k_update(Params k, MeshView m, StateView s, Control ctl, Scalars
   double nrm[4] = {0.0, 0.0, 0.0, 0.0};
   if (i < nv) {
     double R0 = s.R[i], R1 = s.R[nv + i], R2 = s.R[2 * nv + i], R3 = s.R[3 * nv + i];
-    double area = m.dcarea[i];
+    const double ia = m.inv_area[i];
     if (do_norm) {
       double w = m.pweight[i];
-      double q0 = R0 / area, q1 = R1 / area, q2 = R2 / area, q3 = R3 / area;
+      double q0 = R0 * ia, q1 = R1 * ia, q2 = R2 * ia, q3 = R3 * ia;
       nrm[0] = q0 * q0 * w; nrm[1] = q1 * q1 * w; nrm[2] = q2 * q2 * w; nrm[3] = q3 * q3 * w;
     }
     double dtv = (ctl.time_mode == 1 || ctl.time_step > 0.0) ? sc->dt_global : s.dt[i];
-    double factor = dtv / (vertex_radius(k, m, i) * area);
+    const double factor = dtv * ia / vertex_radius(k, m, i);
     const double uo[4] = {s.Uold[i], s.Uold[nv + i], s.Uold[2 * nv + i], s.Uold[3 * nv + i]};
-    Cons c = rk_stage(k, ctl, s, nv, i, r, load_prim(s.P, nv, i), uo, factor, R0, R1, R2, R3);
+    Cons c = rk_stage(ctl, s, nv, i, r, prim2con(k, load_prim(s, i)), uo, factor, R0, R1, R2, R3);
     Prim q = con2prim(k, c);
     Ent e = prim2ent(k, q);
-    s.P[i] = q.T; s.P[nv + i] = q.u; s.P[2 * nv + i] = q.v; s.P[3 * nv + i] = q.p;
-    s.W[i] = e.f; s.W[nv + i] = e.vx; s.W[2 * nv + i] = e.vy; s.W[3 * nv + i] = e.l;
+    store_state(k, s, i, q, e);
     bool ok = isfinite(q.T) && isfinite(q.u) && isfinite(q.v) && isfinite(q.p) && q.p > 0.0 && c.r > 0.0;
     if (!ok) atomicOr(&sc->bad, 1);
   }
@@ -599,10 +676,10 @@ __global__ void k_norm_part(MeshView m, StateView s, const int* __restrict__ don
   const int nv = m.nv;
   double nrm[4] = {0.0, 0.0, 0.0, 0.0};
   if (i < nv) {
-    double area = m.dcarea[i], w = m.pweight[i];
+    const double ia = m.inv_area[i], w = m.pweight[i];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      double q = s.R[c * nv + i] / area;
+      double q = s.R[c * nv + i] * ia;
       nrm[c] = q * q * w;
     }
   }
@@ -671,7 +748,7 @@ __global__ void k_global(Params k, MeshView m, StateView s) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double ke = 0.0, en = 0.0;
   if (i < m.nv) {
-    Prim q = load_prim(s.P, m.nv, i);
+    Prim q = load_prim(s, i);
     double w = m.pweight[i], A = m.dcarea[i];
     double rho = density(k, q);
     ke = (0.5 * rho * (q.u * q.u + q.v * q.v) * A) * w;
@@ -703,13 +780,12 @@ __global__ void k_forces(Params k, MeshView m, StateView s, const int4* __restri
                          const int* __restrict__ off, double* __restrict__ out) {
   const int f = blockIdx.x;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  const int nv = m.nv;
   for (int j = off[f] + threadIdx.x; j < off[f + 1]; j += blockDim.x) {
     const int4 r = faces[j];
     const int d = r.x, dq = r.y;
     const int v0 = m.b_v0[d], v1 = m.b_v1[d];
     const double nx = m.b_nx[d], ny = m.b_ny[d];
-    Prim s0 = load_prim(s.P, nv, v0), s1 = load_prim(s.P, nv, v1);
+    Prim s0 = load_prim(s, v0), s1 = load_prim(s, v1);
     if (dq >= 0) {
       bc_apply1(m.b_kind[dq], m.b_adiab[dq], m.b_val + (size_t)dq * 10 + 5 * r.z, m.b_nx[dq], m.b_ny[dq], s0);
       bc_apply1(m.b_kind[dq], m.b_adiab[dq], m.b_val + (size_t)dq * 10 + 5 * r.w, m.b_nx[dq], m.b_ny[dq], s1);
@@ -722,13 +798,17 @@ __global__ void k_forces(Params k, MeshView m, StateView s, const int4* __restri
       const double T = (s0.T + s1.T) / 2.0;
       const double mu = viscosity(k, T);
       const double f0 = 1.0 / e0.l, f1 = 1.0 / e1.l;
-      const double* G = s.G;
-      auto g = [&](int c, int v) { return G[(size_t)c * nv + v]; };
+      const D4 ga[2] = {ld4(s.G + 2 * (size_t)v0), ld4(s.G + 2 * (size_t)v1)};
+      const D4 gb[2] = {ld4(s.G + 2 * (size_t)v0 + 1), ld4(s.G + 2 * (size_t)v1 + 1)};
+      auto g = [&](int c, int w) {   // c = 2 .. 7
+        const D4 &a = ga[w], &b = gb[w];
+        return c == 2 ? a.z : c == 3 ? a.w : c == 4 ? b.x : c == 5 ? b.y : c == 6 ? b.z : b.w;
+      };
       // u = -V2 / V5: grad u = -grad V2 / V5 + V2 grad V5 / V5^2 (src/force.cc:169-179)
-      const double ux0 = g(2, v0) * -f0 + g(6, v0) * (f0 * e0.vx / e0.l), uy0 = g(3, v0) * -f0 + g(7, v0) * (f0 * e0.vx / e0.l);
-      const double ux1 = g(2, v1) * -f1 + g(6, v1) * (f1 * e1.vx / e1.l), uy1 = g(3, v1) * -f1 + g(7, v1) * (f1 * e1.vx / e1.l);
-      const double vx0 = g(4, v0) * -f0 + g(6, v0) * (f0 * e0.vy / e0.l), vy0 = g(5, v0) * -f0 + g(7, v0) * (f0 * e0.vy / e0.l);
-      const double vx1 = g(4, v1) * -f1 + g(6, v1) * (f1 * e1.vy / e1.l), vy1 = g(5, v1) * -f1 + g(7, v1) * (f1 * e1.vy / e1.l);
+      const double ux0 = g(2, 0) * -f0 + g(6, 0) * (f0 * e0.vx / e0.l), uy0 = g(3, 0) * -f0 + g(7, 0) * (f0 * e0.vx / e0.l);
+      const double ux1 = g(2, 1) * -f1 + g(6, 1) * (f1 * e1.vx / e1.l), uy1 = g(3, 1) * -f1 + g(7, 1) * (f1 * e1.vx / e1.l);
+      const double vx0 = g(4, 0) * -f0 + g(6, 0) * (f0 * e0.vy / e0.l), vy0 = g(5, 0) * -f0 + g(7, 0) * (f0 * e0.vy / e0.l);
+      const double vx1 = g(4, 1) * -f1 + g(6, 1) * (f1 * e1.vy / e1.l), vy1 = g(5, 1) * -f1 + g(7, 1) * (f1 * e1.vy / e1.l);
       const double gux = ux0 * 0.5 + ux1 * 0.5, guy = uy0 * 0.5 + uy1 * 0.5;
       const double gvx = vx0 * 0.5 + vx1 * 0.5, gvy = vy0 * 0.5 + vy1 * 0.5;
       const double div = gux + gvy;
@@ -761,21 +841,21 @@ __global__ void k_forces(Params k, MeshView m, StateView s, const int4* __restri
 // then density, mach, entropy, vorticity as selected by `extras` (bits 0-3).
 // Vorticity (src/material.h:623-627) reads the entropy-variable gradients G of
 // the last gradient pass: V2 = 2 beta u, V3 = 2 beta v, V5 = -2 beta.
-__global__ void k_moments_increment(Params k, int nv, const double* __restrict__ P, const double* __restrict__ G,
-                                    int extras, int nvar, long long kk, double* __restrict__ fm,
-                                    double* __restrict__ sm, double* __restrict__ m2) {
+__global__ void k_moments_increment(Params k, int nv, StateView s, int extras, int nvar, long long kk,
+                                    double* __restrict__ fm, double* __restrict__ sm, double* __restrict__ m2) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nv) return;
-  Prim q = load_prim(P, nv, i);
+  Prim q = load_prim(s, i);
   double x[9];
   x[0] = q.T; x[1] = q.p; x[2] = q.u; x[3] = q.v; x[4] = 0.0;
   int j = 5;
   if (extras & 1) x[j++] = density(k, q);
   if (extras & 2) x[j++] = sqrt(q.u * q.u + q.v * q.v) / sound_speed(k, q);
   if (extras & 4) x[j++] = entropy_fn(k, q);
-  if (extras & 8)
-    x[j++] = k.R * q.T * (G[4 * (size_t)nv + i] + q.v * G[6 * (size_t)nv + i] - G[3 * (size_t)nv + i] -
-                          q.u * G[7 * (size_t)nv + i]);
+  if (extras & 8) {
+    const D4 a = ld4(s.G + 2 * (size_t)i), b = ld4(s.G + 2 * (size_t)i + 1);
+    x[j++] = k.R * q.T * (b.x + q.v * b.z - a.w - q.u * b.w);
+  }
   const double K = (double)kk, c1 = 1.0 / K, c2 = (K - 1.0) / K;
   for (int c = 0; c < nvar; ++c) {
     const size_t o = (size_t)c * nv + i;
@@ -815,23 +895,28 @@ __global__ void k_moments_scale(size_t n, double fact3, double fact4, double* __
 
 // ---- domain decomposition (tg_part_*): halo exchange and the exchanged step scalars
 
-// Packs 8 doubles per listed vertex (components 0-3 of A, then 0-3 of B: the P and W
-// of a state buffer, or the two halves of the gradient array) into out[8 * i + c].
-__global__ void k_halo_pack(int n, const int* __restrict__ idx, int nv, const double* __restrict__ A,
-                            const double* __restrict__ B, double* __restrict__ out) {
+// Packs 8 doubles per listed vertex into out[8 * i + c]: a state's record S, T and V1 (the
+// last two unused), or the gradient's two records.
+__global__ void k_halo_pack(int n, const int* __restrict__ idx, StateView s, int grad, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 8 * n) return;
-  const int v = idx[i >> 3], c = i & 7;
-  out[i] = c < 4 ? A[(size_t)c * nv + v] : B[(size_t)(c - 4) * nv + v];
+  if (i >= 2 * n) return;
+  const int v = idx[i >> 1];
+  D4 q{0.0, 0.0, 0.0, 0.0};
+  if (grad) q = ld4(s.G + 2 * (size_t)v + (i & 1));
+  else if ((i & 1) == 0) q = ld4(s.S + v);
+  else { q.x = s.T[v]; q.y = s.V1[v]; }
+  double* o = out + 4 * (size_t)i;     // a caller's buffer: 8-byte aligned
+  o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
 }
 
-__global__ void k_halo_unpack(int n, const int* __restrict__ idx, int nv, double* __restrict__ A,
-                              double* __restrict__ B, const double* __restrict__ in) {
+__global__ void k_halo_unpack(int n, const int* __restrict__ idx, StateView s, int grad, const double* __restrict__ in) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 8 * n) return;
-  const int v = idx[i >> 3], c = i & 7;
-  if (c < 4) A[(size_t)c * nv + v] = in[i];
-  else B[(size_t)(c - 4) * nv + v] = in[i];
+  if (i >= 2 * n) return;
+  const int v = idx[i >> 1];
+  const double* q = in + 4 * (size_t)i;
+  if (grad) st4(s.G + 2 * (size_t)v + (i & 1), q[0], q[1], q[2], q[3]);
+  else if ((i & 1) == 0) st4(s.S + v, q[0], q[1], q[2], q[3]);
+  else { s.T[v] = q[0]; s.V1[v] = q[1]; }
 }
 
 // After the first-stage dt pass of tg_part_prime: its minimum is the next step's.
@@ -867,11 +952,12 @@ __global__ void k_part_import(Scalars* sc, const unsigned long long* __restrict_
 }
 
 // Owned vertices of a partition -> PrimVar records in local order (tg_get_state).
-__global__ void k_part_state_out(int n, int nv, const double* __restrict__ P, double* __restrict__ out) {
+__global__ void k_part_state_out(int n, StateView s, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double* q = out + 5 * (size_t)i;
-  q[0] = P[i]; q[1] = P[3 * (size_t)nv + i]; q[2] = P[nv + i]; q[3] = P[2 * (size_t)nv + i]; q[4] = 0.0;
+  const Prim r = load_prim(s, i);
+  q[0] = r.T; q[1] = r.p; q[2] = r.u; q[3] = r.v; q[4] = 0.0;
 }
 
 }  // namespace tg

@@ -368,15 +368,18 @@ std::string build_tiles(HostLayout& L, int max_owned, int max_local, int max_edg
   const int n_own = L.n_owned >= 0 ? L.n_owned : nv;   // tiles cover the owned vertices only
   if (max_owned <= 0 || max_local > 65535 || max_edges > 32767) return "bad tile limits";
   L.t_vbeg.clear(); L.t_loff.assign(1, 0); L.t_eoff.assign(1, 0); L.lv.clear();
-  L.te_ab.clear(); L.te_nx.clear(); L.te_ny.clear();
-  L.te_g0x.clear(); L.te_g0y.clear(); L.te_g1x.clear(); L.te_g1y.clear();
-  L.te_ux.clear(); L.te_uy.clear(); L.te_ar.clear(); L.te_r.clear();
-  L.cv_off.assign(nv + 1, 0);
-  L.cv_ent.clear();
+  L.te_ab.clear(); L.te_n.clear(); L.te_u.clear(); L.te_ar.clear(); L.te_r.clear();
+  L.t_cbase.clear(); L.cv_rel.clear(); L.cv_ent.clear(); L.gj_g.clear(); L.gj_i.clear();
   L.lmax = L.emax = L.tmax = L.cmax = 0;
   // scratch maps global id -> tile-local id, reset per tile
   std::vector<int> vloc(nv, -1), eloc(L.ne, -1);
   std::vector<int> tv, te;  // current tile's local vertices / edges (global ids)
+  std::vector<int> new_halo, order;
+  // about 1.2 tile edges per edge and 1.6 local vertices per vertex
+  const size_t te_cap = (size_t)L.ne * 5 / 4, ent_cap = (size_t)L.ce_off[n_own] + 8 * (size_t)(n_own / std::max(1, max_owned) + 1);
+  L.te_ab.reserve(te_cap); L.te_n.reserve(2 * te_cap); L.te_u.reserve(2 * te_cap); L.te_ar.reserve(te_cap);
+  L.lv.reserve((size_t)nv * 8 / 5); L.cv_rel.reserve(nv + nv / 64); L.cv_ent.reserve(ent_cap);
+  L.gj_i.reserve(ent_cap); L.gj_g.reserve(2 * ent_cap);
   int v = 0;
   while (v < n_own) {
     int vb = v;
@@ -387,7 +390,7 @@ std::string build_tiles(HostLayout& L, int max_owned, int max_local, int max_edg
     while (v < n_own && nown < max_owned) {
       // tentative: count new edges and new local vertices of vertex v
       int add_e = 0, add_v = (vloc[v] < 0) ? 1 : 0;
-      std::vector<int> new_halo;
+      new_halo.clear();
       for (int j = L.ce_off[v]; j < L.ce_off[v + 1]; ++j) {
         int e = L.ce_ent[j] >> 1;
         if (eloc[e] >= 0) continue;
@@ -415,8 +418,7 @@ std::string build_tiles(HostLayout& L, int max_owned, int max_local, int max_edg
       ++v;
     }
     // reorder local vertices: owned [vb, v) first, in order, then the halo in first-seen order
-    std::vector<int> order;
-    order.reserve(tv.size());
+    order.clear();
     for (int x = vb; x < v; ++x) order.push_back(x);
     for (int x : tv)
       if (x < vb || x >= v) order.push_back(x);
@@ -427,27 +429,53 @@ std::string build_tiles(HostLayout& L, int max_owned, int max_local, int max_edg
     L.t_loff.push_back((int)L.lv.size());
     for (int e : te) {
       L.te_ab.push_back((uint32_t)vloc[L.e_a[e]] | ((uint32_t)vloc[L.e_b[e]] << 16));
-      L.te_nx.push_back(L.e_nx[e]); L.te_ny.push_back(L.e_ny[e]);
-      L.te_g0x.push_back(L.e_g0x[e]); L.te_g0y.push_back(L.e_g0y[e]);
-      L.te_g1x.push_back(L.e_g1x[e]); L.te_g1y.push_back(L.e_g1y[e]);
+      L.te_n.push_back(L.e_nx[e]); L.te_n.push_back(L.e_ny[e]);
       // src/material.cc:69 area = normal.norm(); src/kepec.cc:18 unit = normal * (1/area);
       // a gradient-only edge (zero normal) gets a zero unit normal, so its flux is zero
       double area = std::sqrt(L.e_nx[e] * L.e_nx[e] + L.e_ny[e] * L.e_ny[e] + 0.0 * 0.0);
       double ia = area > 0.0 ? 1.0 / area : 0.0;
-      L.te_ux.push_back(L.e_nx[e] * ia);
-      L.te_uy.push_back(L.e_ny[e] * ia);
+      L.te_u.push_back(L.e_nx[e] * ia);
+      L.te_u.push_back(L.e_ny[e] * ia);
       L.te_ar.push_back(area);
       if (L.axi) L.te_r.push_back(L.e_r[e]);
     }
     L.t_eoff.push_back((int)L.te_ab.size());
+    // the gather lists: 16-byte aligned per tile, with tile-relative offsets
+    const int base = (int)L.cv_ent.size(), nown_t = v - vb;
+    L.t_cbase.push_back(base);
     for (int x = vb; x < v; ++x) {
+      const int rel = (int)L.cv_ent.size() - base;
+      if (rel + (L.ce_off[x + 1] - L.ce_off[x]) > 65535) return "tile gather list too long";
+      L.cv_rel.push_back((uint16_t)rel);
       for (int j = L.ce_off[x]; j < L.ce_off[x + 1]; ++j) {
         int ent = L.ce_ent[j];
         L.cv_ent.push_back((uint16_t)((eloc[ent >> 1] << 1) | (ent & 1)));
       }
-      L.cv_off[x + 1] = (int)L.cv_ent.size();
     }
-    L.cmax = std::max(L.cmax, L.cv_off[v] - L.cv_off[vb] + 1);   // +1: staging starts on an even entry
+    L.cv_rel.push_back((uint16_t)(L.cv_ent.size() - base));
+    // the same entries for the gradient pass, ordered so that the lanes of a warp read
+    // consecutive words: per warp of 32 vertices, every vertex's first entry, then every
+    // second one, ... over the vertices that have one
+    for (int w = 0; w < nown_t; w += 32) {
+      const int lanes = std::min(32, nown_t - w);
+      int deg = 0;
+      for (int i = 0; i < lanes; ++i) deg = std::max(deg, L.ce_off[vb + w + i + 1] - L.ce_off[vb + w + i]);
+      for (int k = 0; k < deg; ++k)
+        for (int i = 0; i < lanes; ++i) {
+          const int x = vb + w + i;
+          if (k >= L.ce_off[x + 1] - L.ce_off[x]) continue;
+          const int ent = L.ce_ent[L.ce_off[x] + k], e = ent >> 1;
+          const bool side = ent & 1;
+          L.gj_g.push_back(side ? L.e_g1x[e] : L.e_g0x[e]);
+          L.gj_g.push_back(side ? L.e_g1y[e] : L.e_g0y[e]);
+          L.gj_i.push_back((uint32_t)vloc[side ? L.e_a[e] : L.e_b[e]] |
+                           ((uint32_t)vloc[side ? L.e_b[e] : L.e_a[e]] << 16));
+        }
+    }
+    while (L.cv_ent.size() & 7) L.cv_ent.push_back(0);
+    L.gj_i.resize(L.cv_ent.size(), 0u);
+    L.gj_g.resize(2 * L.cv_ent.size(), 0.0);
+    L.cmax = std::max(L.cmax, (int)L.cv_ent.size() - base);
     L.lmax = std::max(L.lmax, (int)order.size());
     L.emax = std::max(L.emax, (int)te.size());
     L.tmax = std::max(L.tmax, v - vb);
@@ -455,9 +483,7 @@ std::string build_tiles(HostLayout& L, int max_owned, int max_local, int max_edg
     for (int e : te) eloc[e] = -1;
   }
   L.t_vbeg.push_back(n_own);
-  for (int x = n_own; x < nv; ++x) L.cv_off[x + 1] = L.cv_off[x];   // ghosts: empty lists
   L.ntiles = (int)L.t_vbeg.size() - 1;
-  if (L.cv_ent.size() & 1) L.cv_ent.push_back(0);   // the lists are staged in whole 4-byte words
   return "";
 }
 

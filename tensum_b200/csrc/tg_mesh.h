@@ -65,20 +65,25 @@ struct HostLayout {
   // lv[t_loff[t] .. t_loff[t+1]) lists the owned vertices first, then every
   // other endpoint of the tile's edges.  Its edge list (te_*, t_eoff) holds
   // every edge incident to an owned vertex or to a periodic copy of one, with
-  // endpoints as local indices (la | lb << 16).  cv_off/cv_ent is the owned
-  // vertices' gather list in tile-local edge indices, (local_edge << 1) | side,
-  // in exactly the order of ce_ent, so the tiled kernels sum in the same order.
-  int ntiles = 0, lmax = 0, emax = 0, tmax = 0, cmax = 0;  // cmax: gather entries per tile
+  // endpoints as local indices (la | lb << 16).  cv_ent holds the owned vertices'
+  // gather lists in tile-local edge indices, (local_edge << 1) | side, in exactly
+  // the order of ce_ent, so the tiled kernels sum in the same order; a tile's lists
+  // start at t_cbase[t] (a multiple of 8), vertex i's at cv_rel[t_vbeg[t] + t + i]
+  // relative to that.  gj_g / gj_i are the same entries for the gradient pass
+  // (weights; other | self << 16 as local vertices) in lane order: see build_tiles.
+  int ntiles = 0, lmax = 0, emax = 0, tmax = 0, cmax = 0;  // cmax: padded gather entries per tile
   // A partition's layout owns vertices [0, n_owned) only; the rest are ghosts that
   // the halo exchange fills (no tiles, no gather lists).  -1: every vertex is owned.
   int n_owned = -1;
   std::vector<int> t_vbeg, t_loff, t_eoff, lv;
   std::vector<uint32_t> te_ab;
-  std::vector<double> te_nx, te_ny, te_g0x, te_g0y, te_g1x, te_g1y;
-  std::vector<double> te_ux, te_uy, te_ar;   // n/|n| and |n|, as Material::num_flux forms them
+  std::vector<double> te_n;                  // dual normal (x, y) per tile edge
+  std::vector<double> te_u, te_ar;           // n/|n| (x, y) and |n|, as Material::num_flux forms them
   std::vector<double> te_r;                  // the edge's radius (axisymmetric runs)
-  std::vector<int> cv_off;
-  std::vector<uint16_t> cv_ent;
+  std::vector<int> t_cbase;
+  std::vector<uint16_t> cv_rel, cv_ent;
+  std::vector<double> gj_g;
+  std::vector<uint32_t> gj_i;
 };
 
 // Returns "" on success, else an error message.

@@ -29,6 +29,7 @@ enum : int { BC_NONE = 0, BC_SLIP = 1, BC_NOSLIP = 2, BC_FARFIELD = 3, BC_INLET 
 struct Params {
   double gamma, R, Cp, prandtl;
   double sqrt_gm1, inv_gamma, inv_gm1;   // sqrt(gamma - 1), 1/gamma, 1/(gamma - 1)
+  double gm1, inv_R;                     // gamma - 1, 1/R
   double gp1_gm1;                        // (gamma + 1)/(gamma - 1)
   double mu_ref, T0, Tref, omega;
   double ev_alpha, ev_beta, tvbM;
@@ -70,7 +71,9 @@ __device__ __forceinline__ double logavg(double a, double b) { return 0.5 * (a +
 // 1 / logavg(a, b), for the callers that only ever divide by the log mean
 __device__ __forceinline__ double inv_logavg(double a, double b) { return logavg_F(a, b) / (0.5 * (a + b)); }
 
-__device__ __forceinline__ double density(const Params& k, const Prim& q) { return q.p / (k.R * q.T); }
+// 1/(R T) = 2 beta: the one division density, beta and the conserved state share.
+__device__ __forceinline__ double inv_RT(const Params& k, const Prim& q) { return 1.0 / (k.R * q.T); }
+__device__ __forceinline__ double density(const Params& k, const Prim& q) { return q.p * inv_RT(k, q); }
 __device__ __forceinline__ double sound_speed(const Params& k, const Prim& q) { return sqrt(k.gamma * k.R * q.T); }
 __device__ __forceinline__ double entropy_fn(const Params& k, const Prim& q) {
   return log(q.p) - k.gamma * log(density(k, q));
@@ -91,7 +94,7 @@ __device__ __forceinline__ Cons prim2con(const Params& k, const Prim& q) {   // 
   c.r = rho;
   c.mx = q.u * rho;
   c.my = q.v * rho;
-  c.E = fma(0.5 * fma(q.u, q.u, q.v * q.v), rho, q.p / (k.gamma - 1.0));
+  c.E = fma(0.5 * fma(q.u, q.u, q.v * q.v), rho, q.p * k.inv_gm1);
   return c;
 }
 
@@ -100,34 +103,33 @@ __device__ __forceinline__ Prim con2prim(const Params& k, const Cons& c) {   // 
   double ir = 1.0 / c.r;
   q.u = c.mx * ir;
   q.v = c.my * ir;
-  q.p = (k.gamma - 1.0) * (c.E - 0.5 * (c.mx * c.mx + c.my * c.my) / c.r);
-  q.T = q.p / (k.R * c.r);
+  q.p = k.gm1 * (c.E - 0.5 * (c.mx * q.u + c.my * q.v));
+  q.T = q.p * ir * k.inv_R;
   return q;
 }
 
 // V5 = -2 beta of prim2ent alone, with its operations (no logarithm).
 __device__ __forceinline__ double prim2ent_v5(const Params& k, const Prim& q) {
-  double beta = density(k, q) / (2 * q.p);
-  return -2 * beta;
+  return -inv_RT(k, q);
 }
 
 __device__ __forceinline__ Ent prim2ent(const Params& k, const Prim& q) {   // src/material.h:534-546
   Ent e;
-  double rho = density(k, q);
-  double beta = rho / (2 * q.p);
-  double s = entropy_fn(k, q);
-  e.f = (k.gamma - s) / (k.gamma - 1) - (q.u * q.u + q.v * q.v) * beta;
-  e.vx = q.u * (2 * beta);
-  e.vy = q.v * (2 * beta);
-  e.l = -2 * beta;
+  const double b2 = inv_RT(k, q);          // 2 beta
+  const double s = log(q.p) - k.gamma * log(q.p * b2);
+  e.f = (k.gamma - s) * k.inv_gm1 - (q.u * q.u + q.v * q.v) * (0.5 * b2);
+  e.vx = q.u * b2;
+  e.vy = q.v * b2;
+  e.l = -b2;
   return e;
 }
 
 // ----------------------------------------------------------------- limiters
 __device__ __forceinline__ double minmod_tvd(double a, double b) {          // src/limiter.h:14-27
-  if (a < 0.0 && b < 0.0) return -dmin_(-a, -b);
-  if (a > 0.0 && b > 0.0) return dmin_(a, b);
-  return 0.0;
+  // the smaller magnitude where the signs agree, else zero: one FP64 comparison instead of
+  // five, the signs compared as integers
+  const double x = fabs(a), y = fabs(b), m = x < y ? x : y;
+  return (__double2hiint(a) ^ __double2hiint(b)) >= 0 ? copysign(m, a) : 0.0;
 }
 
 template <int RECON>
@@ -198,66 +200,46 @@ __device__ __forceinline__ void reconstruct1(double l, double r, double gl, doub
 }
 
 // ------------------------------------------------------------------- fluxes
-// Per-vertex quantities every flux reads.  The reference recomputes them for
-// each edge from the primitive state (Density, beta = 0.5/(R T), Entropy,
-// sound_speed ...); evaluating them once per vertex with the same expressions
-// gives the same values.
+// What a flux reads of a vertex: the stored record (u, v, p and V5 = -2 beta = -1/(R T)),
+// V1 = (gamma - s)/(gamma - 1) - beta |u|^2, s = ln p - gamma ln rho
+// (src/kepes_tecno_roe.cc:100-104), and one field that costs a square root or a division
+// per vertex.  Density 2 beta p and beta (src/material.h:596, src/kepec.cc:23) are
+// products with V5, formed per edge; the sound speed only enters the entropy-variable
+// modification of Roe's eigenvalues (ev_alpha), which forms it where it is on.
 struct VRec {
-  double rho;   // p / (R T)                                    src/material.h:596
-  double u, v, p;
-  double beta;  // 0.5 / (R T)                                  src/kepec.cc:23
-  double V1;    // (gamma - s)/(gamma - 1) - beta |u|^2, s = ln p - gamma ln rho   src/kepes_tecno_roe.cc:100-104
-  double a;     // sqrt(gamma R T)                              src/material.h:587
-  double b;     // sqrt(rho / p)                                src/roe_ec.cc:22
+  double u, v, p, V5;
+  double V1;
+  double x;     // KEP: T; Roe-EC: sqrt(rho / p) = sqrt(-V5)   src/roe_ec.cc:22
 };
+__device__ __forceinline__ double rec_rho(const VRec& r) { return -r.V5 * r.p; }
+// sqrt(gamma R T), src/material.h:587
+__device__ __forceinline__ double rec_sound(const Params& k, const VRec& r) { return sqrt(-k.gamma / r.V5); }
 
+// The record of a state given by its primitive variables (a boundary state, or a vertex
+// whose stored entropy variables lag it).
 template <int FLUX>
 __device__ __forceinline__ VRec make_vrec(const Params& k, const Prim& q) {
   VRec r;
-  r.rho = q.p / (k.R * q.T);
+  const double b2 = inv_RT(k, q);          // 2 beta
   r.u = q.u;
   r.v = q.v;
   r.p = q.p;
-  r.beta = 0.5 / (k.R * q.T);
+  r.V5 = -b2;
   r.V1 = 0.0;
-  r.a = 0.0;
-  r.b = 0.0;
+  r.x = 0.0;
   if (FLUX == FLUX_TECNO_ROE || FLUX == FLUX_TECNO_RUSANOV) {
-    double s = log(q.p) - k.gamma * log(r.rho);
-    r.V1 = (k.gamma - s) / (k.gamma - 1.0) - r.beta * (q.u * q.u + q.v * q.v);
+    double s = log(q.p) - k.gamma * log(q.p * b2);
+    r.V1 = (k.gamma - s) * k.inv_gm1 - 0.5 * b2 * (q.u * q.u + q.v * q.v);
   }
-  if (FLUX == FLUX_TECNO_ROE || FLUX == FLUX_KEP) r.a = sqrt(k.gamma * k.R * q.T);
-  if (FLUX == FLUX_ROE_EC) r.b = sqrt(r.rho / q.p);
-  return r;
-}
-
-// The same record from the stored entropy variables: V5 = -2 beta gives
-// beta = -V5/2 and rho = 2 beta p = -V5 p, and V1 is the stored first entropy
-// variable, so no division or logarithm is needed per vertex.  The stored
-// variables come from prim2ent (beta = rho/(2p), src/material.h:534-546), the
-// flux recomputes them from (T, p) (beta = 0.5/(R T)); the two differ in the
-// last ulp only.
-template <int FLUX>
-__device__ __forceinline__ VRec make_vrec_w(const Params& k, double u, double v, double p, double T, double V1,
-                                            double V5) {
-  VRec r;
-  r.rho = -V5 * p;
-  r.u = u;
-  r.v = v;
-  r.p = p;
-  r.beta = -0.5 * V5;
-  r.V1 = V1;
-  r.a = 0.0;
-  r.b = 0.0;
-  if (FLUX == FLUX_TECNO_ROE || FLUX == FLUX_KEP) r.a = sqrt(k.gamma * k.R * T);
-  if (FLUX == FLUX_ROE_EC) r.b = sqrt(-V5);
+  if (FLUX == FLUX_KEP) r.x = q.T;
+  if (FLUX == FLUX_ROE_EC) r.x = sqrt(b2);
   return r;
 }
 
 // The averages the KEPEC and TeCNO fluxes share: the density log mean, the
 // inverse of the beta log mean and p = (rho_l + rho_r) / (2 (beta_l + beta_r)),
-// from two reciprocals and one division instead of five divisions: the
-// beta sum's reciprocal serves beta's log-mean ratio f, 1/beta_ln and p.
+// from two reciprocals and one division instead of five divisions: the reciprocal
+// of the V5 sum (-2 times beta's) serves beta's log-mean ratio f, 1/beta_ln and p.
 __device__ __forceinline__ double logavg_F_of(double f, double a, double b) {
   double u = f * f;
   if (u < 1.0e-2) {
@@ -268,11 +250,12 @@ __device__ __forceinline__ double logavg_F_of(double f, double a, double b) {
   return log(b / a) / 2.0 / f;
 }
 __device__ __forceinline__ void shared_means(const VRec& L, const VRec& R, double& rho, double& ibeta, double& p) {
-  const double sr = L.rho + R.rho, sb = L.beta + R.beta;
-  const double isr = 1.0 / sr, isb = 1.0 / sb;
-  rho = 0.5 * sr / logavg_F_of((R.rho - L.rho) * isr, L.rho, R.rho);
-  ibeta = logavg_F_of((R.beta - L.beta) * isb, L.beta, R.beta) * (2.0 * isb);
-  p = 0.5 * sr * isb;
+  const double rl = rec_rho(L), rr = rec_rho(R);
+  const double sr = rl + rr, sv = L.V5 + R.V5;
+  const double isr = 1.0 / sr, isv = 1.0 / sv;
+  rho = 0.5 * sr / logavg_F_of((rr - rl) * isr, rl, rr);
+  ibeta = logavg_F_of((R.V5 - L.V5) * isv, L.V5, R.V5) * (-4.0 * isv);
+  p = -sr * isv;
 }
 
 __device__ __forceinline__ Flx kepec_flux(const Params& k, const VRec& L, const VRec& R, double unx, double uny) {
@@ -291,11 +274,11 @@ __device__ __forceinline__ Flx kepec_flux(const Params& k, const VRec& L, const 
 }
 
 __device__ __forceinline__ Flx kep_flux(const Params& k, const VRec& L, const VRec& R, double unx, double uny) {
-  // src/kep.cc:10-38 (pow(a, 2.0) is the square a*a; a^2 / (gamma - 1) as a^2 times 1/(gamma - 1))
-  double Hl = L.a * L.a * k.inv_gm1 + 0.5 * (L.u * L.u + L.v * L.v);
-  double Hr = R.a * R.a * k.inv_gm1 + 0.5 * (R.u * R.u + R.v * R.v);
+  // src/kep.cc:10-38; a^2/(gamma - 1) as gamma R T times 1/(gamma - 1)
+  const double Hl = k.gamma * k.R * L.x * k.inv_gm1 + 0.5 * (L.u * L.u + L.v * L.v);
+  const double Hr = k.gamma * k.R * R.x * k.inv_gm1 + 0.5 * (R.u * R.u + R.v * R.v);
   double p = 0.5 * (L.p + R.p);
-  double rho = 0.5 * (L.rho + R.rho);
+  double rho = 0.5 * (rec_rho(L) + rec_rho(R));
   double H = 0.5 * (Hl + Hr);
   double vx = L.u * 0.5 + R.u * 0.5, vy = L.v * 0.5 + R.v * 0.5;
   double vn = vx * unx + vy * uny;
@@ -313,7 +296,7 @@ __device__ __forceinline__ Flx roe_ec_flux(const Params& k, const VRec& L, const
   // the three divisions by z1b, the reciprocal of the z5 sum its ratio, and
   // (gamma + 1)/(gamma - 1) is a constant: two reciprocals and one division.
   double pl = L.p, pr = R.p;
-  double bl = L.b, br = R.b;
+  double bl = L.x, br = R.x;
   double z1b = 0.5 * (bl + br);
   double zx = L.u * (0.5 * bl) + R.u * (0.5 * br);
   double zy = L.v * (0.5 * bl) + R.v * (0.5 * br);
@@ -335,10 +318,11 @@ __device__ __forceinline__ Flx roe_ec_flux(const Params& k, const VRec& L, const
 
 __device__ __forceinline__ Flx avg_flux(const Params& k, const VRec& L, const VRec& R, double unx, double uny) {
   // src/simple_avg.cc:10-46
-  double El = 0.5 * L.rho * (L.u * L.u + L.v * L.v) + L.p / (k.gamma - 1);
-  double Er = 0.5 * R.rho * (R.u * R.u + R.v * R.v) + R.p / (k.gamma - 1);
+  const double rl = rec_rho(L), rr = rec_rho(R);
+  double El = 0.5 * rl * (L.u * L.u + L.v * L.v) + L.p / (k.gamma - 1);
+  double Er = 0.5 * rr * (R.u * R.u + R.v * R.v) + R.p / (k.gamma - 1);
   double vnl = L.u * unx + L.v * uny, vnr = R.u * unx + R.v * uny;
-  double ml = L.rho * vnl, mr = R.rho * vnr;
+  double ml = rl * vnl, mr = rr * vnr;
   Flx F;
   F.m = 0.0 + ml * 0.5;
   F.m += mr * 0.5;
@@ -400,16 +384,20 @@ __device__ __forceinline__ Flx tecno_flux(const Params& k, const VRec& L, const 
     if (ROE) {
       double vnl = L.u * unx + L.v * uny, vnr = Rp.u * unx + Rp.v * uny;
       double l2 = fabs(vn);
-      Lam[0] = (1 + k.ev_beta) * fabs(vn - a) + k.ev_alpha * fabs((vnl - L.a) - (vnr - Rp.a));
+      Lam[0] = (1 + k.ev_beta) * fabs(vn - a);
       Lam[1] = l2;
       Lam[2] = ssw > 0 ? dmax_(l2, a) : l2;
-      Lam[3] = (1 + k.ev_beta) * fabs(vn + a) + k.ev_alpha * fabs((vnl + L.a) - (vnr + Rp.a));
+      Lam[3] = (1 + k.ev_beta) * fabs(vn + a);
+      if (k.ev_alpha != 0.0) {
+        const double al = rec_sound(k, L), ar = rec_sound(k, Rp);
+        Lam[0] += k.ev_alpha * fabs((vnl - al) - (vnr - ar));
+        Lam[3] += k.ev_alpha * fabs((vnl + al) - (vnr + ar));
+      }
     } else {
       double lr = fabs(vn) + a;                  // a >= 0
       Lam[0] = Lam[1] = Lam[2] = Lam[3] = lr;
     }
-    double dV[4] = {Rp.V1 - L.V1, 2 * Rp.u * Rp.beta - 2 * L.u * L.beta, 2 * Rp.v * Rp.beta - 2 * L.v * L.beta,
-                    -2 * Rp.beta - -2 * L.beta};
+    double dV[4] = {Rp.V1 - L.V1, L.u * L.V5 - Rp.u * Rp.V5, L.v * L.V5 - Rp.v * Rp.V5, Rp.V5 - L.V5};
     double gl[4], gr[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -454,18 +442,22 @@ __device__ __forceinline__ Flx tecno_flux(const Params& k, const VRec& L, const 
   if (ROE) {
     double vnl = L.u * unx + L.v * uny, vnr = Rp.u * unx + Rp.v * uny;
     double l2 = fabs(vn);
-    Lam[0] = (1 + k.ev_beta) * fabs(vn - a) + k.ev_alpha * fabs((vnl - L.a) - (vnr - Rp.a));
+    Lam[0] = (1 + k.ev_beta) * fabs(vn - a);
     Lam[1] = l2;
     Lam[2] = ssw > 0 ? dmax_(l2, a) : l2;   // Liou's modification (src/kepes_tecno_roe.cc:85-87)
-    Lam[3] = (1 + k.ev_beta) * fabs(vn + a) + k.ev_alpha * fabs((vnl + L.a) - (vnr + Rp.a));
+    Lam[3] = (1 + k.ev_beta) * fabs(vn + a);
+    if (k.ev_alpha != 0.0) {
+      const double al = rec_sound(k, L), ar = rec_sound(k, Rp);
+      Lam[0] += k.ev_alpha * fabs((vnl - al) - (vnr - ar));
+      Lam[3] += k.ev_alpha * fabs((vnl + al) - (vnr + ar));
+    }
   } else {
     double lr = fabs(vn) + fabs(a);
     Lam[0] = Lam[1] = Lam[2] = Lam[3] = lr;
   }
   // Every reconstruction reads Z_l, Z_r only through Z_r - Z_l (src/reconstruct.cc:31-96),
   // so the jump is formed as R^T (V_r - V_l) with one product instead of two.
-  double dV[4] = {Rp.V1 - L.V1, 2 * Rp.u * Rp.beta - 2 * L.u * L.beta, 2 * Rp.v * Rp.beta - 2 * L.v * L.beta,
-                  -2 * Rp.beta - -2 * L.beta};
+  double dV[4] = {Rp.V1 - L.V1, L.u * L.V5 - Rp.u * Rp.V5, L.v * L.V5 - Rp.v * Rp.V5, Rp.V5 - L.V5};
   double h = (RECON == RECON_TVB_MINMOD) ? sqrt(dx * dx + dy * dy) : 0.0;
   double gl[4], gr[4];
 #pragma unroll

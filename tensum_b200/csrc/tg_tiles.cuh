@@ -1,26 +1,25 @@
 // tg_tiles.cuh -- tiled stage kernels of the FP64 single-solve path.
 //
 // A tile is a contiguous range of owned vertices (Hilbert order) plus every
-// vertex one edge away (periodic copies' neighbourhoods included).  One CTA
-// per tile stages everything the tile needs -- the gathered vertex data, the
-// tile's edge arrays and the owned vertices' gather lists -- into shared
-// memory with asynchronous copies issued all at once (cp.async), so a CTA has
-// its whole working set in flight before it waits.  Then:
-//   * each vertex's derived quantities (density, beta, entropy variables,
-//     sound speed, logs) are evaluated once per staged copy instead of once
-//     per incident edge,
-//   * each edge flux is computed once per tile and written over the edge's own
-//     (already consumed) geometry slots, and
-//   * every owned vertex sums its edge fluxes in a fixed order
-//     (deterministic; no flux buffer in HBM).
+// vertex one edge away (periodic copies' neighbourhoods included).  A CTA
+// gathers a tile's vertex records and gather lists into shared memory,
+// computes each edge flux of the tile once, and every owned vertex sums its
+// edge fluxes in a fixed order (deterministic; no flux buffer in HBM).
 //
-// k_tile_grad   compute_gradients (src/fv.cc:699-1059) for the owned vertices;
-//               at the first stage of a step it also evaluates the local time
-//               step (src/fv.cc:1499-1598) and U_old (src/fv.cc:1626-1630).
+// The gathers are a chain of dependent memory accesses (tile record -> vertex
+// indices -> records), and with one tile per CTA a warp spent 60 % of its life
+// waiting on them.  So a CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...
+// (the grid fills the chip once) and runs the chain of the next tile behind the
+// current one: its record and indices are read into registers during the edge
+// loop, its vertex records are copied while the owned vertices gather and
+// update.
+//
+// k_tile_grad   compute_gradients (src/fv.cc:699-1059) for the owned vertices.
 // k_tile_flux   compute_inviscid_residual + residual assembly
 //               (src/fv.cc:1066-1192, 1467-1494) and, in MODE_UPDATE, the
-//               SSP-RK3 update (src/fv.cc:1641-1652) with the residual norm
-//               partial sums; writes the new state into the next buffer.
+//               RK update (src/fv.cc:1641-1652); the last stage also forms the
+//               next step's local time step (src/fv.cc:1499-1598) and the
+//               residual norm; writes the new state into the next buffer.
 #pragma once
 
 #include "tg_kernels.cuh"
@@ -34,41 +33,61 @@
 #ifndef TG_TILE_ECAP
 #define TG_TILE_ECAP 512       // edges per tile
 #endif
-// resident flux CTAs per SM the register budget is sized for: TeCNO fluxes / central fluxes.
-// Measured at KH 1025^2: 7 central / gradient CTAs (72 / 70 registers, a 48-byte spill in
-// the update-mode central kernels) beat 6 (80 / 74 registers) by 5% a step, 8 (64
-// registers, 100+ bytes of spills) lose; 5 TeCNO CTAs spill and lose.
+// resident flux CTAs per SM the register budget is sized for: TeCNO fluxes / central fluxes,
+// and gradient CTAs.  With the next tile's loads behind the current one, fewer CTAs with
+// more registers win: KH 1025^2 steps of TeCNO-Rusanov / KEPEC / KEP in us with
+// (TeCNO, central, gradient) CTAs (4, 7, 7): 732 / 274 / 246, (4, 6, 5): 678 / 256 / 246,
+// (4, 5, 6): 724 / 271 / 264, (3, 5, 5): 706 / 271 / 266; gradient pass 78 / 68 / 60 / 59 us
+// with 7 (spills) / 3 / 5 / 4.
 #ifndef TG_FLUX_MINB
 #define TG_FLUX_MINB 4
 #endif
 #ifndef TG_FLUX_MINB_CENTRAL
-#define TG_FLUX_MINB_CENTRAL 7
+#define TG_FLUX_MINB_CENTRAL 6
 #endif
 #ifndef TG_GRAD_MINB
-#define TG_GRAD_MINB 7         // resident gradient / dt CTAs per SM the register budget is sized for
+#define TG_GRAD_MINB 5
 #endif
 
 namespace tg {
 
+// One tile: its ranges in the local vertex table (L vertices, nown of them owned, packed
+// L | nown << 16), the edge arrays, the owned vertices, the list offsets and the gather
+// lists (start a multiple of 8); bit 30 of nent: some owned vertex has boundary or viscous
+// entries.  A partition's records are in its tile order: frontier tiles first.
+struct alignas(32) TileRec {
+  int l0, sizes, e0, NE, vb, rel, cb, nent;
+  __host__ __device__ int L() const { return sizes & 0xffff; }
+  __host__ __device__ int nown() const { return sizes >> 16; }
+};
+constexpr int kTileBnd = 1 << 30;
+
 struct TileView {
-  const int *vbeg, *loff, *eoff, *lv;
-  const unsigned int* ab;
-  const double *nx, *ny, *g0x, *g0y, *g1x, *g1y;
-  const double *ux, *uy, *ar;   // unit normal and |n| per tile edge
+  const TileRec* rec;
+  const int* lv;                // local vertex table (owned vertices first)
+  const unsigned int* ab;       // local endpoints per tile edge
+  const double2* u;             // unit normal per tile edge
+  const double2* n;             // normal
+  const double* ar;             // |n|
   const double* r;              // radius per tile edge (axisymmetric runs)
-  const int* cv_off;            // per vertex (nv + 1); cv_ent has an even length
-  const unsigned short* cv_ent;
-  const double *x, *y;          // vertex coordinates (device order)
-  // ordered launches (ORD kernels: a partition's frontier or interior tiles): block b
-  // works on tile order[base + b], and total counts the tiles of every launch of the
-  // pass; the other kernels work on tile blockIdx.x over one launch of all tiles
-  const int* order;
-  int base, total;
+  const unsigned short* crel;   // per tile (owned + 1) offsets into its lists, at rel
+  const unsigned short* cent;   // (tile edge << 1) | side
+  const double2* gjg;           // the same entries in lane order for the gradients: weights,
+  const unsigned int* gji;      // and other | self << 16 (local vertices)
+  const double2* xy;            // vertex coordinates (device order)
+  // a launch works on tiles base .. base + count; total is the number of CTAs of every
+  // launch of the pass and pbase this launch's first one (norm partials)
+  int base, count, pbase, total;
 };
 
-template <bool ORD>
-__device__ __forceinline__ int tile_of_block(const TileView& t) {
-  return ORD ? t.order[t.base + blockIdx.x] : (int)blockIdx.x;
+__device__ __forceinline__ TileRec load_rec(const TileView& t, int i) {
+  const int4* p = reinterpret_cast<const int4*>(t.rec + t.base + i);
+  const int4 a = __ldg(p), b = __ldg(p + 1);
+  return TileRec{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+}
+// Global index of local vertex i of a tile (0 past its end): only the halo is tabled.
+__device__ __forceinline__ int local_vertex(const TileView& t, const TileRec& R, int i) {
+  return i < R.nown() ? R.vb + i : (i < R.L() ? t.lv[R.l0 + i] : 0);
 }
 
 #ifndef TG_TILE_THREADS
@@ -77,6 +96,10 @@ __device__ __forceinline__ int tile_of_block(const TileView& t) {
 constexpr int kTileThreads = TG_TILE_THREADS;
 
 // ---- asynchronous global -> shared copies (sm_80+ cp.async)
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
@@ -85,525 +108,477 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-__device__ __forceinline__ unsigned long long block_min_u64(unsigned long long bits) {
-  bits = warp_min_u64(bits);
-  __shared__ unsigned long long wmin[kTileThreads / 32];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) wmin[w] = bits;
-  __syncthreads();
-  if (w == 0) {
-    bits = lane < (int)(blockDim.x >> 5) ? wmin[lane] : 0x7ff0000000000000ull;
-    bits = warp_min_u64(bits);
-  }
-  return bits;
-}
-
-// Stage the owned vertices' gather lists: the entries, in whole 4-byte words
-// from the even entry at or below the tile's first one (returned as the base
-// the offsets are taken relative to), and the offsets.
-__device__ __forceinline__ int stage_lists(const TileView& t, int vb, int nown, unsigned int* sC, int* sO) {
-  const int base = t.cv_off[vb] & ~1;
-  const int nwords = (t.cv_off[vb + nown] - base + 1) >> 1;
-  const unsigned int* src = reinterpret_cast<const unsigned int*>(t.cv_ent + base);
-  for (int i = threadIdx.x; i < nwords; i += blockDim.x) cp_async4(sC + i, src + i);
-  for (int i = threadIdx.x; i <= nown; i += blockDim.x) cp_async4(sO + i, t.cv_off + vb + i);
-  return base;
-}
-
-__device__ __forceinline__ int list_entry(const unsigned int* sC, int j) {
-  return (int)((sC[j >> 1] >> ((j & 1) * 16)) & 0xffffu);
-}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // ---------------------------------------------------------------- gradients
-// Shared memory: W (4 per local vertex) [+ T, u, v at FIRST];
-// per edge: gradient weights (4) [+ normal (2) at FIRST] + endpoints (4 bytes);
-// gather lists.
-__host__ __device__ constexpr int grad_vertex_doubles(bool first) { return first ? 7 : 4; }
-__host__ __device__ constexpr int grad_edge_doubles(bool first) { return first ? 6 : 4; }
+// Entropy-variable gradients of the owned vertices.  The next tile's S and V1 are read
+// into registers and its gather entries (weights and local indices in lane order, so
+// copies and reads are consecutive words) into the other half of a double buffer while
+// this tile is summed; the records go to shared memory as the pairs (V2, V3), (V1, V5).
+__host__ __device__ inline size_t tile_grad_smem(int lmax, int cmax) {
+  return (size_t)lmax * 2 * sizeof(double2) + 2 * (size_t)cmax * (sizeof(double2) + sizeof(unsigned int));
+}
 
-// warm_only (gradient kernels at a step's first stage): runs only when the
-// previous step's last stage has already formed dt and U_old for this state,
-// the first-stage kernel (FIRST) only when it has not.
-template <bool FIRST, bool GRAD, bool ORD = false>
-__global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB) k_tile_grad(Params k, MeshView m, TileView t, StateView s,
-                                                            Scalars* sc, int lmax, int emax,
-                                                            const int* __restrict__ done, int warm_only) {
-  if (*done) return;
-  const bool warm = k.fuse_dt && sc->dt_next;
-  if ((FIRST && warm) || (warm_only && !warm)) return;
-  const bool dt_here = FIRST;
-  extern __shared__ double sm[];
-  const int tile = tile_of_block<ORD>(t);
-  const int l0 = t.loff[tile], L = t.loff[tile + 1] - l0;
-  const int e0 = t.eoff[tile], NE = t.eoff[tile + 1] - e0;
-  const int vb = t.vbeg[tile], nown = t.vbeg[tile + 1] - vb;
-  const int nv = m.nv;
-  double* sW = sm;                                   // 4 * L
-  double* sU = sm + 4 * lmax;                        // FIRST: T, u, v -> c, u, v (3 * L)
-  double* sE = sm + grad_vertex_doubles(FIRST) * lmax;   // g0x g0y g1x g1y [nx ny]
-  unsigned int* sAB = reinterpret_cast<unsigned int*>(sE + grad_edge_doubles(FIRST) * emax);
-  int* sO = reinterpret_cast<int*>(sAB + emax);      // nown + 1
-  unsigned int* sC = reinterpret_cast<unsigned int*>(sO + kTileThreads + 2);
+struct GradVertex {
+  D4 q;
+  double V1;
+  double2 w;     // V2, V3 (strong conditions)
+};
+__device__ __forceinline__ GradVertex load_grad_vertex(const Params& k, const StateView& s, int g) {
+  GradVertex x;
+  x.q = ld4(s.S + g);
+  x.V1 = s.V1[g];
+  x.w = k.strong ? s.W23[g] : make_double2(0.0, 0.0);
+  return x;
+}
 
-  for (int i = threadIdx.x; i < L; i += blockDim.x) {
-    int g = t.lv[l0 + i];
-    if (GRAD)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) cp_async8(sW + c * L + i, s.W + (size_t)c * nv + g);
-    if (dt_here) {
-      cp_async8(sU + i, s.P + g);                              // T
-      cp_async8(sU + L + i, s.P + (size_t)nv + g);             // u
-      cp_async8(sU + 2 * L + i, s.P + (size_t)2 * nv + g);     // v
-    }
-  }
-  for (int le = threadIdx.x; le < NE; le += blockDim.x) {
-    if (GRAD) {
-      cp_async8(sE + le, t.g0x + e0 + le);
-      cp_async8(sE + NE + le, t.g0y + e0 + le);
-      cp_async8(sE + 2 * NE + le, t.g1x + e0 + le);
-      cp_async8(sE + 3 * NE + le, t.g1y + e0 + le);
-    }
-    if (dt_here) {
-      cp_async8(sE + 4 * NE + le, t.nx + e0 + le);
-      cp_async8(sE + 5 * NE + le, t.ny + e0 + le);
-    }
-    cp_async4(sAB + le, t.ab + e0 + le);
-  }
-  const int cbase = stage_lists(t, vb, nown, sC, sO);
-  cp_async_wait_all();
-  __syncthreads();
-  if (dt_here) {
-    for (int i = threadIdx.x; i < L; i += blockDim.x) {
-      Prim q;
-      q.T = sU[i];
-      sU[i] = sound_speed(k, q);
-    }
-    __syncthreads();
-  }
+__global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
+    k_tile_grad(Params k, MeshView m, TileView t, StateView s, int lmax, int cmax, const int* __restrict__ done) {
+  const int stop = *done;
+  extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
-  const int v = vb + tid;
-  unsigned long long bits = 0x7ff0000000000000ull;
-  if (tid < nown) {
+  double2* sA = reinterpret_cast<double2*>(smem);             // (V2, V3)
+  double2* sB = sA + lmax;                                    // (V1, V5)
+  double2* sE0 = sB + lmax;                                   // weights per entry, two buffers
+  unsigned int* sI0 = reinterpret_cast<unsigned int*>(sE0 + 2 * (size_t)cmax);   // local indices per entry
+  int at = blockIdx.x;
+  TileRec R = load_rec(t, at);
+  if (stop) return;
+  auto entries = [&](const TileRec& r, int buf) {
+    const int n = r.nent & ~kTileBnd;
+    double2* e = sE0 + (size_t)buf * cmax;
+    unsigned int* i4 = sI0 + (size_t)buf * cmax;
+    for (int i = tid; i < n; i += kTileThreads) cp_async16(e + i, t.gjg + r.cb + i);
+    for (int i = tid; 4 * i < n; i += kTileThreads) cp_async16(i4 + 4 * i, t.gji + r.cb + 4 * i);
+    cp_async_commit();
+  };
+  entries(R, 0);
+  GradVertex x0 = load_grad_vertex(k, s, local_vertex(t, R, tid));
+  GradVertex x1 = load_grad_vertex(k, s, local_vertex(t, R, tid + kTileThreads));
+  for (int buf = 0;; buf ^= 1) {
+    const unsigned short* rel = t.crel + R.rel;
+    const int j0 = tid < R.nown() ? rel[tid] : 0, deg = tid < R.nown() ? rel[tid + 1] - j0 : 0;
+    const double f = tid < R.nown() ? m.inv6mc[R.vb + tid] : 0.0;
+    at += gridDim.x;
+    const bool more = at < t.count;
+    const TileRec N = more ? load_rec(t, at) : R;
+    auto put = [&](int i, const GradVertex& x) {
+      if (i >= R.L()) return;
+      sA[i] = k.strong ? x.w : make_double2(-x.q.w * x.q.x, -x.q.w * x.q.y);
+      sB[i] = make_double2(x.V1, x.q.w);
+    };
+    put(tid, x0);
+    put(tid + kTileThreads, x1);
+    for (int i = tid + 2 * kTileThreads; i < R.L(); i += kTileThreads)
+      put(i, load_grad_vertex(k, s, local_vertex(t, R, i)));
+    const double2 *sE = sE0 + (size_t)buf * cmax;
+    const unsigned int* sI = sI0 + (size_t)buf * cmax;
+    cp_async_wait<0>();
+    __syncthreads();
+    if (more) {
+      entries(N, buf ^ 1);
+      x0 = load_grad_vertex(k, s, local_vertex(t, N, tid));
+      x1 = load_grad_vertex(k, s, local_vertex(t, N, tid + kTileThreads));
+    }
+    const double2 wa = sA[tid < R.nown() ? tid : 0], wb = sB[tid < R.nown() ? tid : 0];
     double acc[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[c] = 0.0;
-    double lam = 0.0;
-    const int j0 = sO[tid] - cbase, j1 = sO[tid + 1] - cbase;
-    for (int j = j0; j < j1; ++j) {
-      int ent = list_entry(sC, j);
-      int le = ent >> 1, side = ent & 1;
-      unsigned int ab = sAB[le];
-      int la = ab & 0xffff, lb = ab >> 16;
-      int self = side ? lb : la, other = side ? la : lb;
-      if (GRAD) {
-        double gx = sE[(side ? 2 : 0) * NE + le];
-        double gy = sE[(side ? 3 : 1) * NE + le];
+    int p = __shfl_sync(0xffffffffu, j0, 0);       // the warp's first entry
+    const unsigned below = (1u << (tid & 31)) - 1u;
+    for (int n = 0;; ++n) {
+      const unsigned have = __ballot_sync(0xffffffffu, n < deg);
+      if (!have) break;
+      if (n < deg) {
+        const int e = p + __popc(have & below);
+        const unsigned idx = sI[e];
+        const double2 g = sE[e];
+        const int o = idx & 0xffff, self = idx >> 16;
+        const double2 oa = sA[o], ob = sB[o];
+        double2 ca = wa, cb = wb;
+        if (self != tid) { ca = sA[self]; cb = sB[self]; }   // a periodic copy's entry
+        const double d1 = ob.x - cb.x, d2 = oa.x - ca.x, d3 = oa.y - ca.y, d5 = ob.y - cb.y;
+        acc[0] += g.x * d1; acc[1] += g.y * d1;
+        acc[2] += g.x * d2; acc[3] += g.y * d2;
+        acc[4] += g.x * d3; acc[5] += g.y * d3;
+        acc[6] += g.x * d5; acc[7] += g.y * d5;
+      }
+      p += __popc(have);
+    }
+    if (tid < R.nown()) {
+      const int v = R.vb + tid;
+      if (R.nent & kTileBnd)
+        for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
+          const int ent = m.cb_ent[j];
+          if ((ent & 3) != 1) continue;
+          const int idx = ent >> 2;
+          double dW[4];
+          bface_grad_corr(k, m, s, idx, dW);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          double dW = sW[c * L + other] - sW[c * L + self];
-          acc[2 * c] += gx * dW;
-          acc[2 * c + 1] += gy * dW;
+          for (int c = 0; c < 4; ++c) {
+            acc[2 * c] += m.b_nx[idx] * dW[c];
+            acc[2 * c + 1] += m.b_ny[idx] * dW[c];
+          }
         }
-      }
-      if (dt_here) {
-        double nx = sE[4 * NE + le], ny = sE[5 * NE + le];
-        double area = face_area(nx, ny);
-        lam += face_radius(sU[L + self], sU[2 * L + self], nx, ny, sU[self], area) * 1.0;
-      }
+      st4(s.G + 2 * (size_t)v, acc[0] * f, acc[1] * f, acc[2] * f, acc[3] * f);
+      st4(s.G + 2 * (size_t)v + 1, acc[4] * f, acc[5] * f, acc[6] * f, acc[7] * f);
     }
-    for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
-      int ent = m.cb_ent[j];
-      int type = ent & 3, idx = ent >> 2;
-      if (GRAD && type == 1) {
-        double dW[4];
-        bface_grad_corr(k, m, s, idx, dW);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          acc[2 * c] += m.b_nx[idx] * dW[c];
-          acc[2 * c + 1] += m.b_ny[idx] * dW[c];
-        }
-      } else if (dt_here && type == 0) {
-        int d = idx >> 1;
-        int selfg = (idx & 1) ? m.b_v1[d] : m.b_v0[d];
-        Prim q = load_prim(s.P, nv, selfg);
-        double nx = m.b_nx[d], ny = m.b_ny[d];
-        double area = face_area(nx, ny);
-        lam += 0.5 * face_radius(q.u, q.v, nx, ny, sound_speed(k, q), area);
-      }
-    }
-    if (GRAD) {
-      double f = m.inv6mc[v];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) s.G[(size_t)c * nv + v] = acc[c] * f;
-    }
-    if (dt_here) {
-      if (k.model == 1) {
-        for (int j = j0; j < j1; ++j) {
-          int ent = list_entry(sC, j);
-          int le = ent >> 1, side = ent & 1;
-          unsigned int ab = sAB[le];
-          int la = ab & 0xffff, lb = ab >> 16;
-          int selfg = t.lv[l0 + (side ? lb : la)];
-          int ga = t.lv[l0 + la], gb = t.lv[l0 + lb];
-          Prim q = load_prim(s.P, nv, selfg);
-          double nx = sE[4 * NE + le], ny = sE[5 * NE + le];
-          double area = face_area(nx, ny);
-          double dx = t.x[gb] - t.x[ga], dy = t.y[gb] - t.y[ga];
-          double dl = face_area(dx, dy);
-          lam += (viscosity(k, q.T) * area / dl / density(k, q)) * 1.0;
-        }
-      }
-      double dtv = k.cfl * m.dcarea[v] / lam;
-      s.dt[v] = dtv;
-      bits = (unsigned long long)__double_as_longlong(dtv);
-      if (!(dtv > 0.0)) bits = 0x7ff0000000000000ull;
-      Cons c = prim2con(k, load_prim(s.P, nv, v));
-      s.Uold[v] = c.r; s.Uold[nv + v] = c.mx; s.Uold[2 * nv + v] = c.my; s.Uold[3 * nv + v] = c.E;
-    }
-  }
-  if (dt_here) {
-    bits = block_min_u64(bits);
-    if (threadIdx.x == 0) atomicMin(&sc->dtmin_bits, bits);
+    if (!more) break;
+    R = N;
+    __syncthreads();      // the records are rewritten for the next tile
   }
 }
 
 // --------------------------------------------------------------------- fluxes
 enum : int { MODE_RESIDUAL = 0, MODE_UPDATE = 1 };
 
-// Shared-memory slots of the per-vertex record fields each flux reads (-1:
-// unused), and where the raw inputs are staged before the record is formed in
-// place: p, u, v from P, the entropy variables V1 (W0) and V5 = -2 beta (W3)
-// from W, and T where a sound speed is needed.
-template <int FLUX> struct VLayout;
-template <> struct VLayout<FLUX_TECNO_ROE> { enum { rho = 0, u = 1, v = 2, p = -1, beta = 3, V1 = 4, a = 5, b = -1, n = 6,
-                                                    Rp = 0, Ru = 1, Rv = 2, RW3 = 3, RW0 = 4, RT = 5 }; };
-template <> struct VLayout<FLUX_TECNO_RUSANOV> { enum { rho = 0, u = 1, v = 2, p = -1, beta = 3, V1 = 4, a = -1, b = -1, n = 5,
-                                                        Rp = 0, Ru = 1, Rv = 2, RW3 = 3, RW0 = 4, RT = -1 }; };
-template <> struct VLayout<FLUX_KEPEC> { enum { rho = 0, u = 1, v = 2, p = -1, beta = 3, V1 = -1, a = -1, b = -1, n = 4,
-                                                Rp = 0, Ru = 1, Rv = 2, RW3 = 3, RW0 = -1, RT = -1 }; };
-template <> struct VLayout<FLUX_KEP> { enum { rho = 0, u = 1, v = 2, p = 3, beta = -1, V1 = -1, a = 4, b = -1, n = 5,
-                                              Rp = 3, Ru = 1, Rv = 2, RW3 = 0, RW0 = -1, RT = 4 }; };
-template <> struct VLayout<FLUX_ROE_EC> { enum { rho = -1, u = 0, v = 1, p = 2, beta = -1, V1 = -1, a = -1, b = 3, n = 4,
-                                                 Rp = 2, Ru = 0, Rv = 1, RW3 = 3, RW0 = -1, RT = -1 }; };
-template <> struct VLayout<FLUX_AVG> { enum { rho = 0, u = 1, v = 2, p = 3, beta = -1, V1 = -1, a = -1, b = -1, n = 4,
-                                              Rp = 3, Ru = 1, Rv = 2, RW3 = 0, RW0 = -1, RT = -1 }; };
-
+template <int FLUX>
+__host__ __device__ constexpr bool is_tecno() {
+  return FLUX == FLUX_TECNO_ROE || FLUX == FLUX_TECNO_RUSANOV;
+}
 template <int FLUX, int RECON>
 __host__ __device__ constexpr bool flux_needs_grad() {
-  return (FLUX == FLUX_TECNO_ROE || FLUX == FLUX_TECNO_RUSANOV) && RECON != RECON_FIRST;
+  return is_tecno<FLUX>() && RECON != RECON_FIRST;
 }
-// doubles per staged vertex: record fields [+ gradient (8) + coordinates (2)]
+
+// Shared memory of a staged vertex: the pairs (u, v) and (p, V5), one single (V1 for the
+// TeCNO fluxes, T for KEP, sqrt(-V5) for Roe-EC), and for the gradient fluxes four pairs of
+// the gradient and the coordinates.
+template <int FLUX>
+__host__ __device__ constexpr int vertex_singles() {
+  return is_tecno<FLUX>() || FLUX == FLUX_KEP || FLUX == FLUX_ROE_EC ? 1 : 0;
+}
 template <int FLUX, int RECON>
-__host__ __device__ constexpr int flux_vertex_doubles() {
-  return VLayout<FLUX>::n + (flux_needs_grad<FLUX, RECON>() ? 10 : 0);
+__host__ __device__ constexpr int vertex_pairs() {
+  return 2 + (flux_needs_grad<FLUX, RECON>() ? 5 : 0);
 }
 
 template <int FLUX>
-__device__ __forceinline__ void store_vrec(double* sV, int L, int i, const VRec& q) {
-  typedef VLayout<FLUX> Y;
-  if (Y::rho >= 0) sV[Y::rho * L + i] = q.rho;
-  if (Y::u >= 0) sV[Y::u * L + i] = q.u;
-  if (Y::v >= 0) sV[Y::v * L + i] = q.v;
-  if (Y::p >= 0) sV[Y::p * L + i] = q.p;
-  if (Y::beta >= 0) sV[Y::beta * L + i] = q.beta;
-  if (Y::V1 >= 0) sV[Y::V1 * L + i] = q.V1;
-  if (Y::a >= 0) sV[Y::a * L + i] = q.a;
-  if (Y::b >= 0) sV[Y::b * L + i] = q.b;
-}
-
-template <int FLUX>
-__device__ __forceinline__ VRec load_vrec(const double* sV, int L, int i) {
-  typedef VLayout<FLUX> Y;
+__device__ __forceinline__ VRec load_vrec(const double2* sA, const double2* sB, const double* s1, int i) {
   VRec q;
-  q.rho = Y::rho >= 0 ? sV[(Y::rho >= 0 ? Y::rho : 0) * L + i] : 0.0;
-  q.u = Y::u >= 0 ? sV[(Y::u >= 0 ? Y::u : 0) * L + i] : 0.0;
-  q.v = Y::v >= 0 ? sV[(Y::v >= 0 ? Y::v : 0) * L + i] : 0.0;
-  q.p = Y::p >= 0 ? sV[(Y::p >= 0 ? Y::p : 0) * L + i] : 0.0;
-  q.beta = Y::beta >= 0 ? sV[(Y::beta >= 0 ? Y::beta : 0) * L + i] : 0.0;
-  q.V1 = Y::V1 >= 0 ? sV[(Y::V1 >= 0 ? Y::V1 : 0) * L + i] : 0.0;
-  q.a = Y::a >= 0 ? sV[(Y::a >= 0 ? Y::a : 0) * L + i] : 0.0;
-  q.b = Y::b >= 0 ? sV[(Y::b >= 0 ? Y::b : 0) * L + i] : 0.0;
+  const double2 a = sA[i], b = sB[i];
+  q.u = a.x; q.v = a.y; q.p = b.x; q.V5 = b.y;
+  q.V1 = is_tecno<FLUX>() ? s1[i] : 0.0;
+  q.x = (FLUX == FLUX_KEP || FLUX == FLUX_ROE_EC) ? s1[i] : 0.0;
   return q;
 }
 
-// Whether a stage update stores only V5 of the entropy variables: the central fluxes
+// Whether a stage update forms V5 alone of the entropy variables: the central fluxes
 // read no other, and an inviscid run forms no gradients inside its steps.  Strong
-// conditions keep all four: they reset P after the update and leave the entropy
-// variables of the reset vertices as the update formed them, as the reference does.
+// conditions keep all four: they reset the primitive state after the update and leave the
+// entropy variables of the reset vertices as the update formed them, as the reference does.
 template <int FLUX>
 __device__ __forceinline__ bool w3_only(const Params& k) {
-  return FLUX != FLUX_TECNO_ROE && FLUX != FLUX_TECNO_RUSANOV && k.model == 0 && !k.strong;
+  return !is_tecno<FLUX>() && k.model == 0 && !k.strong;
 }
 
-template <int FLUX, int RECON, int MODE, bool ORD = false>
-__global__ void __launch_bounds__(kTileThreads, (FLUX == FLUX_TECNO_ROE || FLUX == FLUX_TECNO_RUSANOV)
-                                                    ? TG_FLUX_MINB : TG_FLUX_MINB_CENTRAL)
+// Sums of four values and a minimum over the block's warps, valid in thread 0
+// (fixed order).
+__device__ __forceinline__ void block_sum4_min(double* x, unsigned long long& lo) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
+  lo = warp_min_u64(lo);
+  __shared__ double ws[kTileThreads / 32][4];
+  __shared__ unsigned long long wl[kTileThreads / 32];
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) ws[w][c] = x[c];
+    wl[w] = lo;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int i = 1; i < kTileThreads / 32; ++i) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) x[c] += ws[i][c];
+      lo = wl[i] < lo ? wl[i] : lo;
+    }
+}
+
+// Shared-memory layout of k_tile_flux, in bytes (host and device agree on it).
+template <int FLUX, int RECON>
+struct FluxSmem {
+  size_t xy, g, f, n, single, list, ssw, bytes;
+  __host__ __device__ FluxSmem(int lmax, int emax, int cmax, bool dt) {
+    size_t o = 2 * (size_t)lmax * sizeof(double2);            // (u, v), (p, V5)
+    g = o;
+    if (flux_needs_grad<FLUX, RECON>()) o += 4 * (size_t)lmax * sizeof(double2);
+    xy = o;
+    if (flux_needs_grad<FLUX, RECON>()) o += (size_t)lmax * sizeof(double2);
+    f = o;                                                    // (mass, x), (y, energy) per edge
+    o += 2 * (size_t)emax * sizeof(double2);
+    n = o;                                                    // normals (runs that fuse dt)
+    if (dt) o += (size_t)emax * sizeof(double2);
+    list = o;                                                 // gather lists, two buffers
+    o += 2 * (size_t)cmax * sizeof(unsigned short);
+    single = o;
+    o += (size_t)(vertex_singles<FLUX>() * lmax) * sizeof(double);
+    ssw = o;
+    if (FLUX == FLUX_TECNO_ROE) o += (size_t)lmax * sizeof(int);
+    const size_t red = 4 * kTileThreads * sizeof(double);     // norm_and_step_end's buffer
+    bytes = o > red ? o : red;
+  }
+};
+
+template <int FLUX, int RECON, int MODE>
+__global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB : TG_FLUX_MINB_CENTRAL)
     k_tile_flux(Params k, MeshView m, TileView t, StateView s, Control ctl, Scalars* sc, int r, int do_norm,
-                double* __restrict__ Pout, double* __restrict__ Wout, int lmax, int emax,
-                const int* __restrict__ done) {
-  if (*done) return;
-  extern __shared__ double sm[];
-  typedef VLayout<FLUX> Y;
-  const int tile = tile_of_block<ORD>(t);
-  const int l0 = t.loff[tile], L = t.loff[tile + 1] - l0;
-  const int e0 = t.eoff[tile], NE = t.eoff[tile + 1] - e0;
-  const int vb = t.vbeg[tile], nown = t.vbeg[tile + 1] - vb;
-  const int nv = m.nv;
+                StateView out, int lmax, int emax, int cmax, const int* __restrict__ done) {
+  const int stop = *done;
+  extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool kGrad = flux_needs_grad<FLUX, RECON>();
-  double* sV = sm;                                          // Y::n * L
-  double* sG = sm + Y::n * lmax;                            // 8 * L (gradient fluxes only)
-  double* sX = sG + 8 * lmax;                               // 2 * L
-  double* sE = sm + flux_vertex_doubles<FLUX, RECON>() * lmax;   // 4 * NE: ux uy ar ab -> fluxes
   constexpr bool kRoe = (FLUX == FLUX_TECNO_ROE);
-  int* sS = reinterpret_cast<int*>(sE + 4 * emax);                 // Liou switch of the local vertices (Roe)
-  int* sO = sS + (kRoe ? lmax : 0);
-  unsigned int* sC = reinterpret_cast<unsigned int*>(sO + kTileThreads + 2);
+  const int nv = m.nv, tid = threadIdx.x;
+  const FluxSmem<FLUX, RECON> lay(lmax, emax, cmax, k.fuse_dt);
+  double2* sA = reinterpret_cast<double2*>(smem);
+  double2* sB = sA + lmax;
+  double2* sG = reinterpret_cast<double2*>(smem + lay.g);              // 4 * lmax
+  double2* sX = reinterpret_cast<double2*>(smem + lay.xy);
+  double2* sF = reinterpret_cast<double2*>(smem + lay.f);
+  double2* sF2 = sF + emax;
+  double2* sN = reinterpret_cast<double2*>(smem + lay.n);
+  double* s1 = reinterpret_cast<double*>(smem + lay.single);
+  unsigned short* sC = reinterpret_cast<unsigned short*>(smem + lay.list);
+  int* sS = reinterpret_cast<int*>(smem + lay.ssw);                    // Liou switch of the local vertices
 
-  // ---- stage: vertex gathers, edge arrays, gather lists (all in flight at once)
-  for (int i = threadIdx.x; i < L; i += blockDim.x) {
-    int g = t.lv[l0 + i];
-    cp_async8(sV + Y::Ru * L + i, s.P + (size_t)nv + g);
-    cp_async8(sV + Y::Rv * L + i, s.P + (size_t)2 * nv + g);
-    cp_async8(sV + Y::Rp * L + i, s.P + (size_t)3 * nv + g);
-    cp_async8(sV + Y::RW3 * L + i, s.W + (size_t)3 * nv + g);
-    if (Y::RW0 >= 0) cp_async8(sV + (Y::RW0 >= 0 ? Y::RW0 : 0) * L + i, s.W + g);
-    if (Y::RT >= 0) cp_async8(sV + (Y::RT >= 0 ? Y::RT : 0) * L + i, s.P + g);
+  int at = blockIdx.x;
+  TileRec R = load_rec(t, at);
+  if (stop) return;
+  auto stage_vertex = [&](int i, int g) {
+    const double2* q = reinterpret_cast<const double2*>(s.S + g);
+    cp_async16(sA + i, q);
+    cp_async16(sB + i, q + 1);
+    if (is_tecno<FLUX>()) cp_async8(s1 + i, s.V1 + g);
+    if (FLUX == FLUX_KEP) cp_async8(s1 + i, s.T + g);
     if (kGrad) {
+      const double2* q = reinterpret_cast<const double2*>(s.G + 2 * (size_t)g);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) cp_async8(sG + c * L + i, s.G + (size_t)c * nv + g);
-      cp_async8(sX + i, t.x + g);
-      cp_async8(sX + L + i, t.y + g);
+      for (int c = 0; c < 4; ++c) cp_async16(sG + c * lmax + i, q + c);
+      cp_async16(sX + i, t.xy + g);
     }
-    if (kRoe) {
-      if (k.liou) cp_async4(sS + i, s.ssw + g);
-      else sS[i] = 0;
-    }
-  }
-  for (int le = threadIdx.x; le < NE; le += blockDim.x) {
-    cp_async8(sE + le, t.ux + e0 + le);
-    cp_async8(sE + NE + le, t.uy + e0 + le);
-    cp_async8(sE + 2 * NE + le, t.ar + e0 + le);
-    cp_async4(sE + 3 * NE + le, t.ab + e0 + le);
-  }
-  const int cbase = stage_lists(t, vb, nown, sC, sO);
-  cp_async_wait_all();
-  __syncthreads();
+    if (kRoe && k.liou) cp_async4(sS + i, s.ssw + g);
+  };
+  // copies a tile's vertex records (global ids of the thread's first two given) and lists
+  auto stage = [&](const TileRec& T, int g0, int g1, int buf) {
+    if (tid < T.L()) stage_vertex(tid, g0);
+    if (tid + kTileThreads < T.L()) stage_vertex(tid + kTileThreads, g1);
+    for (int i = tid + 2 * kTileThreads; i < T.L(); i += kTileThreads) stage_vertex(i, local_vertex(t, T, i));
+    unsigned short* c = sC + (size_t)buf * cmax;
+    for (int i = tid; 8 * i < (T.nent & ~kTileBnd); i += kTileThreads) cp_async16(c + 8 * i, t.cent + T.cb + 8 * i);
+    cp_async_commit();
+  };
+  stage(R, local_vertex(t, R, tid), local_vertex(t, R, tid + kTileThreads), 0);
 
-  // ---- per-vertex records, in place
-  for (int i = threadIdx.x; i < L; i += blockDim.x) {
-    double u = sV[Y::Ru * L + i], v = sV[Y::Rv * L + i], p = sV[Y::Rp * L + i], w3 = sV[Y::RW3 * L + i];
-    double w0 = Y::RW0 >= 0 ? sV[(Y::RW0 >= 0 ? Y::RW0 : 0) * L + i] : 0.0;
-    double T = Y::RT >= 0 ? sV[(Y::RT >= 0 ? Y::RT : 0) * L + i] : 0.0;
-    const int g = k.strong ? t.lv[l0 + i] : 0;
-    if (k.strong && (m.sflag[g] & 1)) {
-      // a strong condition reset this vertex's primitive state but not its entropy
-      // variables: the flux reads the primitive state, as the reference does
-      Prim q;
-      q.T = Y::RT >= 0 ? T : s.P[g]; q.u = u; q.v = v; q.p = p;
-      store_vrec<FLUX>(sV, L, i, make_vrec<FLUX>(k, q));
-    } else {
-      store_vrec<FLUX>(sV, L, i, make_vrec_w<FLUX>(k, u, v, p, T, w0, w3));
-    }
-  }
-  __syncthreads();
-
-  // ---- edge fluxes; each result overwrites its edge's geometry slots
-  for (int le = threadIdx.x; le < NE; le += blockDim.x) {
-    double unx = sE[le], uny = sE[NE + le], area = sE[2 * NE + le];
-    unsigned int ab = *reinterpret_cast<const unsigned int*>(sE + 3 * NE + le);
-    int la = ab & 0xffff, lb = ab >> 16;
-    VRec A = load_vrec<FLUX>(sV, L, la), B = load_vrec<FLUX>(sV, L, lb);
-    double gl[8], gr[8], dx = 0.0, dy = 0.0;
-    if (kGrad) {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) { gl[c] = sG[c * L + la]; gr[c] = sG[c * L + lb]; }
-      dx = sX[lb] - sX[la];
-      dy = sX[L + lb] - sX[L + la];
-    }
-    Flx F = num_flux_unit<FLUX, RECON>(k, A, B, unx, uny, area, dx, dy, gl, gr, kRoe ? sS[la] + sS[lb] : 0);
-    if (k.axi) {   // residual[cl] += flux * r_f, residual[cr] -= flux * r_f (src/fv.cc:1095-1096)
-      const double rf = t.r[e0 + le];
-      F.m *= rf; F.x *= rf; F.y *= rf; F.e *= rf;
-    }
-    sE[le] = F.m; sE[NE + le] = F.x; sE[2 * NE + le] = F.y; sE[3 * NE + le] = F.e;
-  }
-  __syncthreads();
-
-  // ---- owned vertices: fixed-order sum, then residual or RK update
-  const int tid = threadIdx.x;
-  const int v = vb + tid;
-  double nrm[4] = {0.0, 0.0, 0.0, 0.0};
-  // last stage with fuse_dt: the next step's local dt and U_old from the new state
+  // last stage with fuse_dt: the next step's local dt from the new state
   const bool next_dt = MODE == MODE_UPDATE && do_norm && k.fuse_dt;
+  double nrm[4] = {0.0, 0.0, 0.0, 0.0};
   unsigned long long dbits = 0x7ff0000000000000ull;
-  Prim qn;                                   // the owned vertex's new state (next_dt)
-  if (tid < nown) {
-    Prim q0;
-    double uo[4], area = 0.0, w = 0.0, dtl = 0.0;
-    if (MODE == MODE_UPDATE) {   // issue the update's loads before the gather
-      q0 = load_prim(s.P, nv, v);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) uo[c] = s.Uold[(size_t)c * nv + v];
-      area = m.dcarea[v];
-      w = m.pweight[v];
-      if (!(ctl.time_mode == 1 || ctl.time_step > 0.0)) dtl = s.dt[v];
-    }
-    double r0 = 0.0, r1 = 0.0, r2 = 0.0, r3 = 0.0;
-    const int j0 = sO[tid] - cbase, j1 = sO[tid + 1] - cbase;
-    for (int j = j0; j < j1; ++j) {
-      int ent = list_entry(sC, j);
-      int le = ent >> 1;
-      double sg = (ent & 1) ? -1.0 : 1.0;
-      r0 += sE[le] * sg; r1 += sE[NE + le] * sg; r2 += sE[2 * NE + le] * sg; r3 += sE[3 * NE + le] * sg;
-    }
-    const int n2 = 2 * m.nb, n3 = 3 * m.nvu;
-    for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
-      int ent = m.cb_ent[j];
-      int type = ent & 3, idx = ent >> 2;
-      // axisymmetric weights (src/fv.cc:1151, 1187, 1226-1228, 1280-1282, 1315-1316): half the
-      // radius of the boundary-face vertex, of the viscous unit's cell, of the vertex
-      if (type == 0) {
-        const double w = k.axi ? 0.5 * m.v_r[(idx & 1) ? m.b_v1[idx >> 1] : m.b_v0[idx >> 1]] : 0.5;
-        r0 += s.Fb[idx] * w; r1 += s.Fb[n2 + idx] * w; r2 += s.Fb[2 * n2 + idx] * w; r3 += s.Fb[3 * n2 + idx] * w;
-      } else if (type == 2 && k.model == 1) {
-        const double w = k.axi ? -(0.5 * m.u_r[idx / 3]) : -(0.5 * 1.0);
-        r1 += s.Fv[idx] * w; r2 += s.Fv[n3 + idx] * w; r3 += s.Fv[2 * n3 + idx] * w;
-      } else if (type == 3 && k.model == 1) {
-        const double w = k.axi ? 0.5 * m.v_r[v] : 0.5;
-        r1 += s.Fvb[idx] * w; r2 += s.Fvb[m.nb + idx] * w; r3 += s.Fvb[2 * m.nb + idx] * w;
-      }
-    }
-    // strong conditions: compute_residual_norm zeroes the no-slip momentum residual
-    // before the last stage's update (src/fv.cc:1805-1819)
-    if (MODE == MODE_UPDATE && do_norm && k.strong && (m.sflag[v] & 2)) { r1 = 0.0; r2 = 0.0; }
-    if (MODE == MODE_RESIDUAL) {
-      s.R[v] = r0; s.R[nv + v] = r1; s.R[2 * nv + v] = r2; s.R[3 * nv + v] = r3;
-    } else {
-      if (do_norm) {
-        double a0 = r0 / area, a1 = r1 / area, a2 = r2 / area, a3 = r3 / area;
-        nrm[0] = a0 * a0 * w; nrm[1] = a1 * a1 * w; nrm[2] = a2 * a2 * w; nrm[3] = a3 * a3 * w;
-      }
-      double dtv = (ctl.time_mode == 1 || ctl.time_step > 0.0) ? sc->dt_global : dtl;
-      double factor = dtv / (vertex_radius(k, m, v) * area);
-      Cons c = rk_stage(k, ctl, s, nv, v, r, q0, uo, factor, r0, r1, r2, r3);
-      Prim q = con2prim(k, c);
-      Pout[v] = q.T; Pout[nv + v] = q.u; Pout[2 * nv + v] = q.v; Pout[3 * nv + v] = q.p;
-      if (w3_only<FLUX>(k)) {
-        // inviscid central fluxes read only V5 = -2 beta: the other entropy variables
-        // (two logarithms) are formed from P by whatever later needs them (refresh_w)
-        Wout[3 * nv + v] = prim2ent_v5(k, q);
-      } else {
-        Ent e = prim2ent(k, q);
-        Wout[v] = e.f; Wout[nv + v] = e.vx; Wout[2 * nv + v] = e.vy; Wout[3 * nv + v] = e.l;
-      }
-      bool ok = isfinite(q.T) && isfinite(q.u) && isfinite(q.v) && isfinite(q.p) && q.p > 0.0 && c.r > 0.0;
-      if (!ok) atomicOr(&sc->bad, 1);
-      if (next_dt) qn = q;
-    }
-  }
-  if (next_dt) {
-    // compute_dt (src/fv.cc:1499-1598) and store_conserved_old (src/fv.cc:1626-1630) of
-    // the coming step, with the operands and order of k_tile_grad<true, *>: the tile's
-    // dual normals are staged over the consumed fluxes in one wave of copies
+  const double dtg = MODE == MODE_UPDATE && (ctl.time_mode == 1 || ctl.time_step > 0.0) ? sc->dt_global : 0.0;
+
+  for (int buf = 0;; buf ^= 1) {
+    at += gridDim.x;
+    const bool more = at < t.count;
+    const TileRec N = more ? load_rec(t, at) : R;
+    const int e0 = R.e0, NE = R.NE;
+    // the thread's first edge and its list's range, read while the copies are in flight
+    double2 un = make_double2(0.0, 0.0);
+    double ar = 0.0;
+    unsigned ab = 0;
+    if (tid < NE) { un = t.u[e0 + tid]; ar = t.ar[e0 + tid]; ab = t.ab[e0 + tid]; }
+    const bool own = tid < R.nown();
+    const int v = R.vb + (own ? tid : 0);
+    const unsigned short* rel = t.crel + R.rel;
+    const int j0 = own ? rel[tid] : 0, j1 = own ? rel[tid + 1] : 0;
+    cp_async_wait<0>();
     __syncthreads();
-    for (int le = threadIdx.x; le < NE; le += blockDim.x) {
-      cp_async8(sE + le, t.nx + e0 + le);
-      cp_async8(sE + NE + le, t.ny + e0 + le);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    if (tid < nown) {
-      const double cs = sound_speed(k, qn);
-      const int j0 = sO[tid] - cbase, j1 = sO[tid + 1] - cbase;
-      double lam = 0.0;
-      for (int j = j0; j < j1; ++j) {
-        const int le = list_entry(sC, j) >> 1;
-        const double nx = sE[le], ny = sE[NE + le];
-        const double ar = face_area(nx, ny);
-        lam += face_radius(qn.u, qn.v, nx, ny, cs, ar) * 1.0;
-      }
-      for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
-        const int ent = m.cb_ent[j];
-        if ((ent & 3) != 0) continue;
-        const int d = ent >> 3;
-        const double nx = m.b_nx[d], ny = m.b_ny[d];
-        const double ar = face_area(nx, ny);
-        lam += 0.5 * face_radius(qn.u, qn.v, nx, ny, cs, ar);
-      }
-      if (k.model == 1) {
-        for (int j = j0; j < j1; ++j) {
-          const int le = list_entry(sC, j) >> 1;
-          const unsigned int ab = t.ab[e0 + le];
-          const int ga = t.lv[l0 + (int)(ab & 0xffff)], gb = t.lv[l0 + (int)(ab >> 16)];
-          const double nx = sE[le], ny = sE[NE + le];
-          const double ar = face_area(nx, ny);
-          const double dx = t.x[gb] - t.x[ga], dy = t.y[gb] - t.y[ga];
-          const double dl = face_area(dx, dy);
-          lam += (viscosity(k, qn.T) * ar / dl / density(k, qn)) * 1.0;
+    if (FLUX == FLUX_ROE_EC || k.strong) {
+      for (int i = tid; i < R.L(); i += kTileThreads) {
+        if (FLUX == FLUX_ROE_EC) s1[i] = sqrt(-sB[i].y);
+        const int g = k.strong ? local_vertex(t, R, i) : 0;
+        if (k.strong && (m.sflag[g] & 1)) {
+          // a strong condition reset this vertex's primitive state but not its entropy
+          // variables: the flux reads the primitive state, as the reference does
+          Prim q;
+          q.T = s.T[g]; q.u = sA[i].x; q.v = sA[i].y; q.p = sB[i].x;
+          const VRec x = make_vrec<FLUX>(k, q);
+          sB[i] = make_double2(x.p, x.V5);
+          if (is_tecno<FLUX>()) s1[i] = x.V1;
+          if (FLUX == FLUX_ROE_EC) s1[i] = x.x;
         }
       }
-      const double dtn = k.cfl * m.dcarea[v] / lam;
-      s.dt[v] = dtn;
-      dbits = (unsigned long long)__double_as_longlong(dtn);
-      if (!(dtn > 0.0)) dbits = 0x7ff0000000000000ull;
-      const Cons un = prim2con(k, qn);
-      s.Uold[v] = un.r; s.Uold[nv + v] = un.mx; s.Uold[2 * nv + v] = un.my; s.Uold[3 * nv + v] = un.E;
-    }
-    dbits = block_min_u64(dbits);
-    if (threadIdx.x == 0) {
-      atomicMin(&sc->dtmin_next, dbits);
-      if (blockIdx.x == 0) sc->dt_next = 1;
-    }
-  }
-  if (MODE == MODE_UPDATE && do_norm) {
-    // the tile buffers are no longer needed: reuse them for the block reduction
-    __syncthreads();
-    double* red = sm;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) red[c * kTileThreads + threadIdx.x] = nrm[c];
-    __syncthreads();
-    for (int o = kTileThreads / 2; o > 0; o >>= 1) {
-      if ((int)threadIdx.x < o)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) red[c * kTileThreads + threadIdx.x] += red[c * kTileThreads + threadIdx.x + o];
       __syncthreads();
     }
-    if (threadIdx.x == 0)
+    const int g0 = more ? local_vertex(t, N, tid) : 0, g1 = more ? local_vertex(t, N, tid + kTileThreads) : 0;
+
+    // ---- edge fluxes
+    for (int le = tid; le < NE; le += kTileThreads) {
+      const int la = ab & 0xffff, lb = ab >> 16;
+      const double2 u = un;
+      const double area = ar;
+      const int nx = le + kTileThreads;
+      if (nx < NE) { un = t.u[e0 + nx]; ar = t.ar[e0 + nx]; ab = t.ab[e0 + nx]; }
+      const VRec A = load_vrec<FLUX>(sA, sB, s1, la), B = load_vrec<FLUX>(sA, sB, s1, lb);
+      double gl[8], gr[8], dx = 0.0, dy = 0.0;
+      if (kGrad) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) s.part[(size_t)((ORD ? t.base : 0) + blockIdx.x) * 4 + c] = red[c * kTileThreads];
-    // the last block to finish forms the norms and ends the step
+        for (int c = 0; c < 4; ++c) {
+          const double2 x = sG[c * lmax + la], y = sG[c * lmax + lb];
+          gl[2 * c] = x.x; gl[2 * c + 1] = x.y;
+          gr[2 * c] = y.x; gr[2 * c + 1] = y.y;
+        }
+        const double2 xa = sX[la], xb = sX[lb];
+        dx = xb.x - xa.x;
+        dy = xb.y - xa.y;
+      }
+      Flx F = num_flux_unit<FLUX, RECON>(k, A, B, u.x, u.y, area, dx, dy, gl, gr,
+                                         kRoe && k.liou ? sS[la] + sS[lb] : 0);
+      if (k.axi) {   // residual[cl] += flux * r_f, residual[cr] -= flux * r_f (src/fv.cc:1095-1096)
+        const double rf = t.r[e0 + le];
+        F.m *= rf; F.x *= rf; F.y *= rf; F.e *= rf;
+      }
+      sF[le] = make_double2(F.m, F.x);
+      sF2[le] = make_double2(F.y, F.e);
+    }
+    // what the update reads, in flight across the barrier; the vertex's own record is staged
+    D4 q0{0.0, 0.0, 0.0, 0.0}, qo = q0;
+    double ia = 0.0, w = 0.0, dtl = dtg;
+    const bool old = MODE == MODE_UPDATE && (ctl.scheme == 1 || r > 0);   // the stage adds U_old
+    if (MODE == MODE_UPDATE && own) {
+      const double2 a = sA[tid], b = sB[tid];
+      q0 = D4{a.x, a.y, b.x, b.y};
+      if (old) qo = ld4(s.S0 + v);
+      ia = m.inv_area[v];
+      if (do_norm) w = m.pweight[v];
+      if (!(ctl.time_mode == 1 || ctl.time_step > 0.0)) dtl = s.dt[v];
+    }
+    __syncthreads();
+    if (next_dt) {
+      for (int le = tid; le < NE; le += kTileThreads) cp_async16(sN + le, t.n + e0 + le);
+      cp_async_commit();
+    }
+    if (more) stage(N, g0, g1, buf ^ 1);
+
+    // ---- owned vertices: fixed-order sum, then residual or RK update
+    const unsigned short* list = sC + (size_t)buf * cmax;
+    Prim qn{0.0, 0.0, 0.0, 0.0};               // the owned vertex's new state
+    if (own) {
+      double r0 = 0.0, r1 = 0.0, r2 = 0.0, r3 = 0.0;
+      for (int j = j0; j < j1; ++j) {
+        const int ent = list[j], le = ent >> 1;
+        const double sg = (ent & 1) ? -1.0 : 1.0;
+        const double2 f = sF[le], f2 = sF2[le];
+        r0 += f.x * sg; r1 += f.y * sg; r2 += f2.x * sg; r3 += f2.y * sg;
+      }
+      if (R.nent & kTileBnd) {
+        const int n2 = 2 * m.nb, n3 = 3 * m.nvu;
+        for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
+          int ent = m.cb_ent[j];
+          int type = ent & 3, idx = ent >> 2;
+          // axisymmetric weights (src/fv.cc:1151, 1187, 1226-1228, 1280-1282, 1315-1316): half the
+          // radius of the boundary-face vertex, of the viscous unit's cell, of the vertex
+          if (type == 0) {
+            const double w = k.axi ? 0.5 * m.v_r[(idx & 1) ? m.b_v1[idx >> 1] : m.b_v0[idx >> 1]] : 0.5;
+            r0 += s.Fb[idx] * w; r1 += s.Fb[n2 + idx] * w; r2 += s.Fb[2 * n2 + idx] * w; r3 += s.Fb[3 * n2 + idx] * w;
+          } else if (type == 2 && k.model == 1) {
+            const double w = k.axi ? -(0.5 * m.u_r[idx / 3]) : -(0.5 * 1.0);
+            r1 += s.Fv[idx] * w; r2 += s.Fv[n3 + idx] * w; r3 += s.Fv[2 * n3 + idx] * w;
+          } else if (type == 3 && k.model == 1) {
+            const double w = k.axi ? 0.5 * m.v_r[v] : 0.5;
+            r1 += s.Fvb[idx] * w; r2 += s.Fvb[m.nb + idx] * w; r3 += s.Fvb[2 * m.nb + idx] * w;
+          }
+        }
+      }
+      // strong conditions: compute_residual_norm zeroes the no-slip momentum residual
+      // before the last stage's update (src/fv.cc:1805-1819)
+      if (MODE == MODE_UPDATE && do_norm && k.strong && (m.sflag[v] & 2)) { r1 = 0.0; r2 = 0.0; }
+      if (MODE == MODE_RESIDUAL) {
+        s.R[v] = r0; s.R[nv + v] = r1; s.R[2 * nv + v] = r2; s.R[3 * nv + v] = r3;
+      } else {
+        if (do_norm) {
+          const double a0 = r0 * ia, a1 = r1 * ia, a2 = r2 * ia, a3 = r3 * ia;
+          nrm[0] += a0 * a0 * w; nrm[1] += a1 * a1 * w; nrm[2] += a2 * a2 * w; nrm[3] += a3 * a3 * w;
+        }
+        double factor = dtl * ia;
+        if (k.axi) factor /= m.v_r[v];
+        // conserved records from the stored ones: rho = -V5 p, no division; strong runs read
+        // T, since V5 lags a reset state
+        auto conserved = [&](const D4& q, const double* T) {
+          const double rho = k.strong ? density(k, Prim{T[v], q.x, q.y, q.z}) : -q.w * q.z;
+          return Cons{rho, q.x * rho, q.y * rho, fma(0.5 * fma(q.x, q.x, q.y * q.y), rho, q.z * k.inv_gm1)};
+        };
+        double uo[4] = {0.0, 0.0, 0.0, 0.0};
+        if (old) {
+          const Cons c = conserved(qo, s.T0);
+          uo[0] = c.r; uo[1] = c.mx; uo[2] = c.my; uo[3] = c.E;
+        }
+        const Cons c = rk_stage(ctl, s, nv, v, r, conserved(q0, s.T), uo, factor, r0, r1, r2, r3);
+        qn = con2prim(k, c);
+        if (w3_only<FLUX>(k)) {
+          // inviscid central fluxes read only V5 = -2 beta: V1 (two logarithms) is formed
+          // from the state by whatever later needs it (refresh_w)
+          st4(out.S + v, qn.u, qn.v, qn.p, prim2ent_v5(k, qn));
+          out.T[v] = qn.T;
+        } else {
+          store_state(k, out, v, qn, prim2ent(k, qn));
+        }
+        bool ok = isfinite(qn.T) && isfinite(qn.u) && isfinite(qn.v) && isfinite(qn.p) && qn.p > 0.0 && c.r > 0.0;
+        if (!ok) atomicOr(&sc->bad, 1);
+      }
+    }
+    if (next_dt) {
+      // compute_dt (src/fv.cc:1499-1598) of the coming step, as k_dt forms it
+      if (more) cp_async_wait<1>();
+      else cp_async_wait<0>();
+      __syncthreads();
+      if (own) {
+        double lam = 0.0;
+        for (int j = j0; j < j1; ++j) {
+          const double2 n = sN[list[j] >> 1];
+          lam += fabs(fma(qn.u, n.x, qn.v * n.y));
+        }
+        if (R.nent & kTileBnd)
+          for (int j = m.cb_off[v]; j < m.cb_off[v + 1]; ++j) {
+            const int ent = m.cb_ent[j];
+            if ((ent & 3) != 0) continue;
+            const int d = ent >> 3;
+            lam += 0.5 * fabs(fma(qn.u, m.b_nx[d], qn.v * m.b_ny[d]));
+          }
+        lam = spectral_sum(k, m, v, qn, lam);
+        const double dtn = k.cfl * m.dcarea[v] / lam;
+        if (ctl.time_mode == 0) s.dt[v] = dtn;     // unsteady runs read the minimum only
+        unsigned long long bits = (unsigned long long)__double_as_longlong(dtn);
+        if (!(dtn > 0.0)) bits = 0x7ff0000000000000ull;
+        dbits = bits < dbits ? bits : dbits;
+      }
+    }
+    if (!more) break;
+    R = N;
+  }
+  if (MODE == MODE_UPDATE && do_norm) {
+    block_sum4_min(nrm, dbits);
     __shared__ int last;
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
+      if (next_dt) {
+        atomicMin(&sc->dtmin_next, dbits);
+        if (blockIdx.x == 0) sc->dt_next = 1;
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s.part[(size_t)(t.pbase + blockIdx.x) * 4 + c] = nrm[c];
+      // the last block to finish forms the norms and ends the step
       __threadfence();
-      last = atomicAdd(&sc->blocks_done, 1u) == (ORD ? (unsigned)t.total : gridDim.x) - 1;
+      last = atomicAdd(&sc->blocks_done, 1u) == (unsigned)t.total - 1;
     }
     __syncthreads();
     if (last) {
       __threadfence();
-      norm_and_step_end(s, ORD ? t.total : (int)gridDim.x, nv, sc, ctl, red, kTileThreads);
-      if (threadIdx.x == 0) sc->blocks_done = 0;
+      norm_and_step_end(s, t.total, nv, sc, ctl, reinterpret_cast<double*>(smem), kTileThreads);
+      if (tid == 0) sc->blocks_done = 0;
     }
   }
-}
-
-// gather-list words (cmax entries, two per word) + offsets
-inline size_t tile_list_bytes(int cmax) {
-  return (kTileThreads + 2) * sizeof(int) + (size_t)((cmax + 2) / 2 + 1) * sizeof(unsigned int);
-}
-
-inline size_t tile_grad_smem(int lmax, int emax, int cmax, bool first) {
-  return ((size_t)lmax * grad_vertex_doubles(first) + (size_t)emax * grad_edge_doubles(first)) * sizeof(double) +
-         (size_t)emax * sizeof(unsigned int) + tile_list_bytes(cmax);
-}
-
-template <int FLUX, int RECON>
-size_t tile_flux_smem_t(int lmax, int emax, int cmax) {
-  size_t a = ((size_t)lmax * flux_vertex_doubles<FLUX, RECON>() + 4 * (size_t)emax) * sizeof(double) +
-             (FLUX == FLUX_TECNO_ROE ? (size_t)lmax * sizeof(int) : 0) + tile_list_bytes(cmax);
-  size_t b = 4 * kTileThreads * sizeof(double);
-  return a > b ? a : b;
 }
 
 }  // namespace tg
