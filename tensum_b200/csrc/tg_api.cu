@@ -60,20 +60,22 @@ struct tg_handle {
   double* V1b[3] = {nullptr, nullptr, nullptr};
   double2* W23b[3] = {nullptr, nullptr, nullptr};
   size_t smem_grad = 0, smem_flux = 0;
+  bool pdl = false;            // a step's kernels are dependent launches (pdl_wait)
   int grid_grad = 1, grid_flux = 1, grid_res = 1;   // CTAs that fill the chip once (the kernels walk tiles)
   Scalars* sc = nullptr;       // device
   int* done = nullptr;         // device flag written by k_step_begin
   int* never = nullptr;        // device zero, used by single-phase calls
-  double* tinst = nullptr;
+  std::vector<double> tinst_host;              // output times
   std::vector<void*> allocs;
   std::string err;
   int nblocks_v = 0;
   bool viscous = false;
   bool grads_needed = false;
-  cudaGraph_t graph = nullptr;                 // a step that forms its own dt (any state)
-  cudaGraphExec_t graph_exec = nullptr;
-  cudaGraph_t wgraph = nullptr;                // a step whose dt the previous step formed
-  cudaGraphExec_t wgraph_exec = nullptr;
+  // captured steps, each made at its first use: one that forms its own dt (any state), one
+  // whose dt the previous step formed, and kManySteps of the latter in a row
+  enum { kCold = 0, kWarm = 1, kMany = 2, kGraphs = 3 };
+  cudaGraph_t graph[kGraphs] = {};
+  cudaGraphExec_t graph_exec[kGraphs] = {};
   bool cold = true;                            // the next step may not find dt_next set
   bool w_partial[3] = {false, false, false};   // a step left this buffer's V1 unformed (refresh_w)
   bool uold_stale = false;                     // steps ran since Uold was stored (they form U_old themselves)
@@ -164,8 +166,24 @@ tg_status dev_alloc(tg_handle* h, size_t n, T** out) {
 
 inline int nblk(int n) { return (n + kBlock - 1) / kBlock; }
 
+// A launch on `st`, dependent on the stream's previous kernel by pdl_wait when pdl is set.
+template <class... P, class... A>
+void launch(bool pdl, void (*f)(P...), int grid, int block, size_t smem, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&c, f, P(a)...);
+}
+
 // ---- kernel dispatch over (flux, reconstruction)
-typedef void (*BfluxKernel)(Params, MeshView, StateView, const int*);
+typedef void (*BfluxKernel)(Params, MeshView, StateView, const int*, int);
 // Entry points that step or read the whole mesh: a partition handle steps through tg_part_*.
 #define TG_WHOLE_MESH(h) \
   if ((h) && (h)->part.n_parts > 0) return fail((h), TG_NOT_SUPPORTED, "a partition handle steps through tg_part_*");
@@ -280,30 +298,30 @@ int tiles(const tg_handle* h, int base, int count, int grid, TileView* v) {
   return std::min(count, grid);
 }
 
-void enqueue_gradient(tg_handle* h, int b, const int* done, int base = 0, int count = -1) {
+void enqueue_gradient(tg_handle* h, int b, const int* done, int base = 0, int count = -1, bool pdl = false) {
   TileView v;
   const int grid = tiles(h, base, count, h->grid_grad, &v);
   if (grid == 0) return;
-  k_tile_grad<<<grid, kTileThreads, h->smem_grad, h->stream>>>(
-      h->prm, h->mv, v, view(h, b), h->L.lmax, h->L.cmax, done);
+  launch(pdl, k_tile_grad, grid, kTileThreads, h->smem_grad, h->stream, h->prm, h->mv, v, view(h, b), h->L.lmax,
+         h->L.cmax, done);
 }
 
-// boundary-face and viscous contributions, gathered by the tiled flux kernel
-void enqueue_boundary(tg_handle* h, int b, const int* done) {
+// boundary-face and viscous contributions, gathered by the tiled flux kernel; with pdl, behind
+// the gradient pass of the same state where the run forms gradients
+void enqueue_boundary(tg_handle* h, int b, const int* done, bool pdl = false) {
   if (h->mv.nb > 0)
-    bflux_kernel(h->prm.flux, h->prm.recon)<<<nblk(2 * h->mv.nb), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, b),
-                                                                                            done);
-  if (h->viscous) k_viscous<<<nblk(h->mv.nvu), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, b), done);
+    launch(pdl, bflux_kernel(h->prm.flux, h->prm.recon), nblk(2 * h->mv.nb), kBlock, 0, h->stream, h->prm, h->mv,
+           view(h, b), done, pdl && h->grads_needed ? 1 : 0);
+  if (h->viscous) launch(pdl, k_viscous, nblk(h->mv.nvu), kBlock, 0, h->stream, h->prm, h->mv, view(h, b), done);
 }
 
 void enqueue_tile_flux(tg_handle* h, int b, int mode, int r, bool norm, int bout, const int* done, int base = 0,
-                       int count = -1) {
+                       int count = -1, bool pdl = false) {
   TileView v;
   const int grid = tiles(h, base, count, mode == MODE_UPDATE ? h->grid_flux : h->grid_res, &v);
   if (grid == 0) return;
-  tile_kernel(h->prm.flux, h->prm.recon, mode)<<<grid, kTileThreads, h->smem_flux, h->stream>>>(
-      h->prm, h->mv, v, view(h, b), h->ctl, h->sc, r, norm ? 1 : 0, view(h, bout), h->L.lmax, h->L.emax,
-      h->L.cmax, done);
+  launch(pdl, tile_kernel(h->prm.flux, h->prm.recon, mode), grid, kTileThreads, h->smem_flux, h->stream, h->prm, h->mv,
+         v, view(h, b), h->ctl, h->sc, r, norm ? 1 : 0, view(h, bout), h->L.lmax, h->L.emax, h->L.cmax, done);
 }
 
 // Inviscid central-flux steps without strong conditions leave V1 unformed (w3_only in
@@ -361,7 +379,7 @@ void enqueue_norm_final(tg_handle* h, int nblocks, bool use_sc_iter, long long i
 // (its last block).  warm: the previous step's last update formed this step's dt
 // (dt_next set), so the dt pass and k_dt_final are left out.
 void enqueue_step(tg_handle* h, bool warm) {
-  k_step_begin<<<1, 1, 0, h->stream>>>(h->ctl, h->sc, h->done, warm ? 1 : 0);
+  launch(h->pdl, k_step_begin, 1, 1, 0, h->stream, h->ctl, h->sc, h->done, warm ? 1 : 0);
   // stage r reads buffer bin and writes bout: ssprk3 0->1->2->0, rk4 0->1->2->1->0,
   // so a step always ends in buffer 0 and no stage writes the buffer it reads
   const int rk4_in[4] = {0, 1, 2, 1}, rk4_out[4] = {1, 2, 1, 0};
@@ -370,42 +388,56 @@ void enqueue_step(tg_handle* h, bool warm) {
     const int bin = h->ctl.scheme == 1 ? rk4_in[r] : r, bout = h->ctl.scheme == 1 ? rk4_out[r] : (r + 1) % 3;
     if (first && !warm) {
       if (h->ctl.time_step <= 0.0)
-        k_dt<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), h->sc, h->done, 1);
-      k_dt_final<<<1, 1, 0, h->stream>>>(h->ctl, h->sc, h->done);
+        launch(h->pdl, k_dt, nblk(h->mv.nv), kBlock, 0, h->stream, h->prm, h->mv, view(h, 0), h->sc, h->done, 1);
+      launch(h->pdl, k_dt_final, 1, 1, 0, h->stream, h->ctl, h->sc, h->done);
     }
-    if (h->grads_needed) enqueue_gradient(h, bin, h->done);
     if (first) enqueue_ssw(h, h->done);
-    enqueue_boundary(h, bin, h->done);
-    enqueue_tile_flux(h, bin, MODE_UPDATE, r, last, bout, h->done);
+    if (h->grads_needed) enqueue_gradient(h, bin, h->done, 0, -1, h->pdl);
+    enqueue_boundary(h, bin, h->done, h->pdl);
+    enqueue_tile_flux(h, bin, MODE_UPDATE, r, last, bout, h->done, 0, -1, h->pdl);
     if (h->prm.strong && h->mv.nsb > 0)
-      k_strong_bc<<<nblk(h->mv.nsb), kBlock, 0, h->stream>>>(h->mv, view(h, bout), h->done);
+      launch(h->pdl, k_strong_bc, nblk(h->mv.nsb), kBlock, 0, h->stream, h->mv, view(h, bout), h->done);
   }
 }
 
-// The captured step to replay: the warm one once the previous step has formed dt for the
-// current state (cold is cleared only then).
-cudaGraphExec_t step_graph(const tg_handle* h) {
-  return (h->prm.fuse_dt && !h->cold && h->wgraph_exec) ? h->wgraph_exec : h->graph_exec;
+// Warm steps in the longest captured run: a replay's own launch latency, and the full
+// dependency between two replays, fall on one step in so many.
+constexpr int kManySteps = 8;
+
+tg_status capture(tg_handle* h, int which) {
+  if (h->graph_exec[which]) return TG_OK;
+  TG_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  for (int i = 0; i < (which == tg_handle::kMany ? kManySteps : 1); ++i) enqueue_step(h, which != tg_handle::kCold);
+  cudaError_t e = cudaStreamEndCapture(h->stream, &h->graph[which]);
+  if (e != cudaSuccess) return fail(h, TG_CUDA_ERROR, std::string("graph capture: ") + cudaGetErrorString(e));
+  TG_CUDA(h, cudaGraphInstantiate(&h->graph_exec[which], h->graph[which], 0));
+  return TG_OK;
 }
 
-// n replays of the captured step.  A cold step leaves dt_next set (or its loop test ended
-// the run, and the later steps' tests do too), so only the first of them forms its own dt.
+// n steps by replays: warm ones once the previous step has formed dt for the current state.
+// A cold step leaves dt_next set (or its loop test ended the run, and the later steps' tests
+// do too), so only the first of them forms its own dt.
 tg_status launch_steps(tg_handle* h, long n) {
-  for (long i = 0; i < n; ++i) {
-    TG_CUDA(h, cudaGraphLaunch(step_graph(h), h->stream));
+  for (long i = 0; i < n;) {
+    const bool warm = h->prm.fuse_dt && !h->cold, many = warm && n - i >= kManySteps;
+    const int which = many ? tg_handle::kMany : warm ? tg_handle::kWarm : tg_handle::kCold;
+    const tg_status st = capture(h, which);
+    if (st != TG_OK) return st;
+    TG_CUDA(h, cudaGraphLaunch(h->graph_exec[which], h->stream));
     h->cold = false;
+    i += many ? kManySteps : 1;
   }
   if (n > 0) mark_steps(h);
   return TG_OK;
 }
 
 void drop_graphs(tg_handle* h) {
-  if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
-  if (h->graph) cudaGraphDestroy(h->graph);
-  if (h->wgraph_exec) cudaGraphExecDestroy(h->wgraph_exec);
-  if (h->wgraph) cudaGraphDestroy(h->wgraph);
-  h->graph_exec = h->wgraph_exec = nullptr;
-  h->graph = h->wgraph = nullptr;
+  for (int i = 0; i < tg_handle::kGraphs; ++i) {
+    if (h->graph_exec[i]) cudaGraphExecDestroy(h->graph_exec[i]);
+    if (h->graph[i]) cudaGraphDestroy(h->graph[i]);
+    h->graph_exec[i] = nullptr;
+    h->graph[i] = nullptr;
+  }
 }
 
 // The state changed outside a captured step: the next step forms dt itself.
@@ -579,19 +611,6 @@ tg_status check_bad(tg_handle* h) {
 
 }  // namespace
 
-tg_status capture_step_graph(tg_handle* h) {
-  if (h->graph_exec) return TG_OK;
-  for (int w = 0; w < (h->prm.fuse_dt ? 2 : 1); ++w) {
-    cudaGraph_t* g = w ? &h->wgraph : &h->graph;
-    TG_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    enqueue_step(h, w == 1);
-    cudaError_t e = cudaStreamEndCapture(h->stream, g);
-    if (e != cudaSuccess) return fail(h, TG_CUDA_ERROR, std::string("graph capture: ") + cudaGetErrorString(e));
-    TG_CUDA(h, cudaGraphInstantiate(w ? &h->wgraph_exec : &h->graph_exec, *g, 0));
-  }
-  return TG_OK;
-}
-
 void enqueue_phase(tg_handle* h, int phase) {
   switch (phase) {
     case TG_PHASE_GRADIENT: enqueue_gradient(h, 0, h->never); break;
@@ -601,10 +620,7 @@ void enqueue_phase(tg_handle* h, int phase) {
       break;
     case TG_PHASE_UPDATE: enqueue_update(h, 1, false, h->never); break;
     case TG_PHASE_DT: enqueue_dt(h, h->never); break;
-    default:
-      cudaGraphLaunch(step_graph(h), h->stream);
-      mark_steps(h);
-      break;
+    default: launch_steps(h, 1); break;
   }
 }
 
@@ -701,7 +717,12 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
       return fail(nullptr, TG_INVALID_ARG, msg);
     }
   }
-  msg = build_tiles(h->L, TG_TILE_OWNED, TG_TILE_LCAP, TG_TILE_ECAP);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  const bool tecno = mat->flux_scheme == FLUX_TECNO_ROE || mat->flux_scheme == FLUX_TECNO_RUSANOV;
+  const int n_own = h->L.n_owned >= 0 ? h->L.n_owned : h->L.nv;
+  msg = build_tiles(h->L, tile_owned(n_own, sms * (tecno ? TG_FLUX_MINB : TG_FLUX_MINB_CENTRAL)), TG_TILE_LCAP,
+                    TG_TILE_ECAP);
   if (!msg.empty()) {
     delete h;
     return fail(nullptr, TG_INVALID_ARG, msg);
@@ -859,8 +880,6 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
       tg_destroy(h);
       return fail(nullptr, TG_CUDA_ERROR, "tile kernels need more shared memory than the device allows");
     }
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     auto fill = [&](const void* f, size_t smem) {
       int per = 1;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kTileThreads, smem) != cudaSuccess || per < 1) per = 1;
@@ -868,6 +887,12 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
     };
     h->grid_grad = fill((const void*)k_tile_grad, h->smem_grad);
     h->grid_flux = fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_UPDATE), h->smem_flux);
+    // Dependent launches where the passes of a step fill the chip at most once, or where no
+    // gradient pass alternates with the flux pass.  Past that the early CTAs of one pass
+    // between the last ones of the other leave register holes too small for its fourth
+    // CTA per SM, and a round more (TeCNO-Rusanov on 1025^2 671 -> 1027 us, 513^2 209 -> 241;
+    // one round: 65^2 46 -> 40, the 128 x 256 cylinder 131 -> 116; KEPEC 387^2 55 -> 51).
+    h->pdl = L.ntiles <= h->grid_flux || !h->grads_needed;
     h->grid_res = fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_RESIDUAL), h->smem_flux);
   }
   if ((st = dev_alloc(h, 1, &h->sc)) != TG_OK) { tg_destroy(h); return st; }
@@ -884,6 +909,7 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   }
   const double* tip = nullptr;
   if ((st = dev_upload(h, ti, &tip)) != TG_OK) { tg_destroy(h); return st; }
+  h->tinst_host = ti;
   Control& c = h->ctl;
   c.time_mode = opt->time_mode; c.n_rks = opt->time_scheme == TG_TIME_RK4 ? 4 : 3;
   c.scheme = opt->time_scheme == TG_TIME_RK4 ? 1 : 0;
@@ -1183,9 +1209,8 @@ tg_status tg_step(tg_handle* h, int n_steps, double* info4) {
   TG_WHOLE_MESH(h)
   if (!h) return fail(h, TG_INVALID_ARG, "NULL handle");
   if (n_steps < 0) return fail(h, TG_INVALID_ARG, "n_steps < 0");
-  tg_status st = capture_step_graph(h);
+  tg_status st = take_queued_input(h);
   if (st != TG_OK) return st;
-  if ((st = take_queued_input(h)) != TG_OK) return st;
   if ((st = launch_steps(h, n_steps)) != TG_OK) return st;
   Scalars s;
   st = read_scalars(h, &s);
@@ -1229,9 +1254,8 @@ tg_status tg_advance(tg_handle* h, int instance, long max_steps, double* info5) 
   TG_WHOLE_MESH(h)
   if (!h) return fail(h, TG_INVALID_ARG, "NULL handle");
   if (max_steps < 0) return fail(h, TG_INVALID_ARG, "max_steps < 0");
-  tg_status st = capture_step_graph(h);
+  tg_status st = take_queued_input(h);
   if (st != TG_OK) return st;
-  if ((st = take_queued_input(h)) != TG_OK) return st;
   int stop = instance;
   TG_CUDA(h, cudaMemcpyAsync(&h->sc->stop_counter, &stop, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   Scalars s;
@@ -1239,7 +1263,15 @@ tg_status tg_advance(tg_handle* h, int instance, long max_steps, double* info5) 
   if ((st = queued_input_refused(h)) != TG_OK) return st;
   long launched = 0;
   while (launched < max_steps && !s.bad && s.counter <= instance && !run_over(h, s)) {
-    const long chunk = std::min<long>(16, max_steps - launched);
+    // about as many steps as the output time is away at the coming step's dt, then the rest
+    // one by one: a replay past it does nothing but costs its launches
+    double dt = 0.0;
+    if (h->ctl.time_step > 0.0) dt = h->ctl.time_step;
+    else if (s.dt_next) std::memcpy(&dt, &s.dtmin_next, sizeof(dt));
+    const double away = h->ctl.time_mode == 1 && dt > 0.0 && s.counter < h->ctl.ntinst
+                            ? (h->tinst_host[s.counter] - s.elapsed) / dt : 16.0;
+    const long want = away < 1.0 ? 1 : away < 256.0 ? (long)std::ceil(away) : 256;
+    const long chunk = std::min<long>(want, max_steps - launched);
     if ((st = launch_steps(h, chunk)) != TG_OK) return st;
     launched += chunk;
     if ((st = read_scalars(h, &s)) != TG_OK) return st;
@@ -1509,16 +1541,14 @@ tg_status tg_stream(tg_handle* h, void** out) {
 tg_status tg_time_phase(tg_handle* h, int phase, int reps, double* ms) {
   TG_WHOLE_MESH(h)
   if (!h || !ms || reps <= 0 || phase < 0 || phase > 4) return fail(h, TG_INVALID_ARG, "bad argument");
-  if (phase == TG_PHASE_STEP) {
-    tg_status st = capture_step_graph(h);
-    if (st != TG_OK) return st;
-  }
   cudaEvent_t a, b;
   TG_CUDA(h, cudaEventCreate(&a));
   TG_CUDA(h, cudaEventCreate(&b));
   enqueue_phase(h, phase);
   TG_CUDA(h, cudaEventRecord(a, h->stream));
-  for (int i = 0; i < reps; ++i) enqueue_phase(h, phase);
+  if (phase == TG_PHASE_STEP) launch_steps(h, reps);
+  else
+    for (int i = 0; i < reps; ++i) enqueue_phase(h, phase);
   TG_CUDA(h, cudaEventRecord(b, h->stream));
   tg_status st = sync(h);
   float t = 0.0f;

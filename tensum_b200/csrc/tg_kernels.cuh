@@ -48,6 +48,18 @@ __device__ __forceinline__ double vertex_radius(const Params& k, const MeshView&
   return k.axi ? m.v_r[v] : 1.0;
 }
 
+// Dependent launches.  The kernels of a step are launched with programmatic stream
+// serialization: a kernel's CTAs may start once every CTA of its predecessor has called
+// pdl_trigger (or ended) and an SM has room, and pdl_wait returns when the predecessor has
+// completed and its writes are visible.  Every such kernel waits before it reads or writes
+// anything a step changes -- so its own completion implies that of all kernels before it --
+// and reads mesh data only ahead of that, behind the predecessor's tail.  The kernels of a
+// stage that do not depend on each other (gradients, boundary faces, viscous units) trigger
+// after their wait and let the next of them run at once: pdl_wait at its end keeps the
+// completion chain.  Launched without the attribute both calls do nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // A 32-byte record: one sector, moved by one 256-bit access per thread.
 struct alignas(32) D4 {
   double x, y, z, w;
@@ -263,11 +275,9 @@ __global__ void k_store_old(Params k, MeshView m, StateView s, const int* __rest
 }
 
 // Boundary-face inviscid fluxes (src/fv.cc:1100-1188): one thread per (face, vertex).
+// with_grad: launched right behind the gradient pass and independent of it (pdl_wait).
 template <int FLUX, int RECON>
-__global__ void k_bflux(Params k, MeshView m, StateView s, const int* __restrict__ done) {
-  if (*done) return;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2 * m.nb) return;
+__device__ __forceinline__ void bflux_one(const Params& k, const MeshView& m, const StateView& s, int t) {
   int d = t >> 1, q = t & 1;
   int c = q ? m.b_v1[d] : m.b_v0[d];
   Prim s0 = load_prim(s, c), s1 = s0;
@@ -284,12 +294,17 @@ __global__ void k_bflux(Params k, MeshView m, StateView s, const int* __restrict
   const int n2 = 2 * m.nb;
   s.Fb[t] = F.m; s.Fb[n2 + t] = F.x; s.Fb[2 * n2 + t] = F.y; s.Fb[3 * n2 + t] = F.e;
 }
+template <int FLUX, int RECON>
+__global__ void k_bflux(Params k, MeshView m, StateView s, const int* __restrict__ done, int with_grad) {
+  pdl_trigger();
+  if (!with_grad) pdl_wait();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < 2 * m.nb && !*done) bflux_one<FLUX, RECON>(k, m, s, t);
+  pdl_wait();
+}
 
 // Viscous residual units (src/fv.cc:1197-1320): interior cells and boundary faces.
-__global__ void k_viscous(Params k, MeshView m, StateView s, const int* __restrict__ done) {
-  if (*done) return;
-  int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= m.nvu) return;
+__device__ __forceinline__ void viscous_one(const Params& k, const MeshView& m, const StateView& s, int u) {
   int c = m.u_cell[u];
   int v[3] = {m.c_v[3 * c], m.c_v[3 * c + 1], m.c_v[3 * c + 2]};
   const double* n = m.c_n + 6 * (size_t)c;
@@ -355,6 +370,13 @@ __global__ void k_viscous(Params k, MeshView m, StateView s, const int* __restri
     s.Fvb[d] = F.x; s.Fvb[m.nb + d] = F.y; s.Fvb[2 * m.nb + d] = F.e - Cor;
   }
 }
+// Launched behind the gradient pass (viscous runs always form gradients), independent of it.
+__global__ void k_viscous(Params k, MeshView m, StateView s, const int* __restrict__ done) {
+  pdl_trigger();
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u < m.nvu && !*done) viscous_one(k, m, s, u);
+  pdl_wait();
+}
 
 // |n| and the face spectral radius |u.n| + c |n| of the local time step
 // (src/fv.cc:1512-1580), with their multiply-adds written out so that every
@@ -386,6 +408,8 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x)
 // Local time step (src/fv.cc:1499-1598): spectral-radius gather, dt = cfl A / sum,
 // block minimum by warp shuffles, then one atomicMin on the (positive) bit pattern.
 __global__ void k_dt(Params k, MeshView m, StateView s, Scalars* sc, const int* __restrict__ done, int in_step) {
+  pdl_trigger();
+  pdl_wait();
   if (*done) return;
   if (in_step && k.fuse_dt && sc->dt_next) return;   // the previous step's last update formed it
   int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -457,6 +481,8 @@ __global__ void k_dt(Params k, MeshView m, StateView s, Scalars* sc, const int* 
 // (all faces, boundary ones included) across which u.n - a|n| or u.n + a|n|
 // changes sign from positive to negative.  Writers only ever store 1.
 __global__ void k_ssw(Params k, MeshView m, StateView s, const int* __restrict__ done) {
+  pdl_trigger();
+  pdl_wait();
   if (*done) return;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.ne) return;
@@ -479,6 +505,8 @@ __global__ void k_ssw(Params k, MeshView m, StateView s, const int* __restrict__
 // order; the entropy variables keep their values (the reference does not
 // recompute them), so gradients see the pre-condition state.
 __global__ void k_strong_bc(MeshView m, StateView s, const int* __restrict__ done) {
+  pdl_trigger();
+  pdl_wait();
   if (*done) return;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= m.nsb) return;
@@ -522,6 +550,8 @@ __device__ __forceinline__ void dt_final(const Control& ctl, Scalars* sc) {
 }
 
 __global__ void k_dt_final(Control ctl, Scalars* sc, const int* __restrict__ done) {
+  pdl_trigger();
+  pdl_wait();
   if (*done) return;
   dt_final(ctl, sc);
 }
@@ -531,6 +561,8 @@ __global__ void k_dt_final(Control ctl, Scalars* sc, const int* __restrict__ don
 // when dt_next is set.  warm (a step captured without the first-stage dt pass,
 // launched only when dt_next is set): the dt clamp happens here too.
 __global__ void k_step_begin(Control ctl, Scalars* sc, int* done, int warm) {
+  pdl_trigger();
+  pdl_wait();
   // unsteady runs never advance the iteration bound (term_iter stays 0, src/fv.cc:2266-2268)
   bool go = sc->rtotal > ctl.min_residue && (ctl.time_mode == 1 || sc->iter < ctl.max_iter) &&
             sc->elapsed < ctl.final_time && sc->counter <= sc->stop_counter;

@@ -25,7 +25,7 @@
 #include "tg_kernels.cuh"
 
 #ifndef TG_TILE_OWNED
-#define TG_TILE_OWNED 128      // owned vertices per tile (<= kTileThreads)
+#define TG_TILE_OWNED 128      // most owned vertices per tile (<= kTileThreads)
 #endif
 #ifndef TG_TILE_LCAP
 #define TG_TILE_LCAP 256       // local (owned + halo) vertices per tile
@@ -95,6 +95,22 @@ __device__ __forceinline__ int local_vertex(const TileView& t, const TileRec& R,
 #endif
 constexpr int kTileThreads = TG_TILE_THREADS;
 
+// Owned vertices per tile of a mesh of nv vertices on a chip that holds `ctas` flux CTAs at
+// once.  A large mesh takes full tiles (the smallest halo).  Where full tiles would fill
+// the chip less than twice, they are made smaller so that its one or two rounds are full:
+// a CTA's time is a chain of latencies and grows with its edges per thread, so a chip half
+// filled with full tiles, or a nearly empty second round, costs as much as a full one.
+// Below 32 the halo outweighs the edges.  TeCNO-Roe step in us on n^2 vertices with 32 / 64 /
+// 96 / 128 owned: 65^2 33.4 / 32.7 / 36.5 / 40.3, 129^2 40.0 / 43.4 / 54.6 / 48.0, 193^2 62.7 /
+// 48.5 / 56.9 / 60.0, 225^2 81.8 / 68.8 / 57.4 / 65.4, 257^2 96.9 / 75.8 / 85.4 / 68.0,
+// 321^2 139 / 104 / 95.6 / 100; the 128 x 256 cylinder 129 / 91 / 103 / 116.
+inline int tile_owned(long nv, int ctas) {
+  const long full = (long)ctas * TG_TILE_OWNED, rounds = (nv + full - 1) / full;
+  if (rounds > 2) return TG_TILE_OWNED;
+  const long want = (nv + ctas * rounds - 1) / (ctas * rounds);
+  return (int)(want <= 32 ? 32 : want >= TG_TILE_OWNED ? TG_TILE_OWNED : (want + 15) / 16 * 16);
+}
+
 // ---- asynchronous global -> shared copies (sm_80+ cp.async)
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -136,7 +152,6 @@ __device__ __forceinline__ GradVertex load_grad_vertex(const Params& k, const St
 
 __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
     k_tile_grad(Params k, MeshView m, TileView t, StateView s, int lmax, int cmax, const int* __restrict__ done) {
-  const int stop = *done;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
   double2* sA = reinterpret_cast<double2*>(smem);             // (V2, V3)
@@ -145,7 +160,6 @@ __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
   unsigned int* sI0 = reinterpret_cast<unsigned int*>(sE0 + 2 * (size_t)cmax);   // local indices per entry
   int at = blockIdx.x;
   TileRec R = load_rec(t, at);
-  if (stop) return;
   auto entries = [&](const TileRec& r, int buf) {
     const int n = r.nent & ~kTileBnd;
     double2* e = sE0 + (size_t)buf * cmax;
@@ -155,8 +169,18 @@ __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
     cp_async_commit();
   };
   entries(R, 0);
-  GradVertex x0 = load_grad_vertex(k, s, local_vertex(t, R, tid));
-  GradVertex x1 = load_grad_vertex(k, s, local_vertex(t, R, tid + kTileThreads));
+  const int v0 = local_vertex(t, R, tid), v1 = local_vertex(t, R, tid + kTileThreads);
+  pdl_wait();
+  // after the wait: the boundary and viscous passes may run alongside; without them the
+  // flux pass follows, and its CTAs had better not take this pass's place (below)
+  if (m.nb > 0) pdl_trigger();
+  const int stop = *done;
+  GradVertex x0 = load_grad_vertex(k, s, v0);
+  GradVertex x1 = load_grad_vertex(k, s, v1);
+  if (stop) {
+    cp_async_wait<0>();
+    return;
+  }
   for (int buf = 0;; buf ^= 1) {
     const unsigned short* rel = t.crel + R.rel;
     const int j0 = tid < R.nown() ? rel[tid] : 0, deg = tid < R.nown() ? rel[tid + 1] - j0 : 0;
@@ -182,6 +206,7 @@ __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
       x0 = load_grad_vertex(k, s, local_vertex(t, N, tid));
       x1 = load_grad_vertex(k, s, local_vertex(t, N, tid + kTileThreads));
     }
+    else pdl_trigger();
     const double2 wa = sA[tid < R.nown() ? tid : 0], wb = sB[tid < R.nown() ? tid : 0];
     double acc[8];
 #pragma unroll
@@ -328,7 +353,6 @@ template <int FLUX, int RECON, int MODE>
 __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB : TG_FLUX_MINB_CENTRAL)
     k_tile_flux(Params k, MeshView m, TileView t, StateView s, Control ctl, Scalars* sc, int r, int do_norm,
                 StateView out, int lmax, int emax, int cmax, const int* __restrict__ done) {
-  const int stop = *done;
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool kGrad = flux_needs_grad<FLUX, RECON>();
   constexpr bool kRoe = (FLUX == FLUX_TECNO_ROE);
@@ -347,7 +371,6 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
 
   int at = blockIdx.x;
   TileRec R = load_rec(t, at);
-  if (stop) return;
   auto stage_vertex = [&](int i, int g) {
     const double2* q = reinterpret_cast<const double2*>(s.S + g);
     cp_async16(sA + i, q);
@@ -371,7 +394,16 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
     for (int i = tid; 8 * i < (T.nent & ~kTileBnd); i += kTileThreads) cp_async16(c + 8 * i, t.cent + T.cb + 8 * i);
     cp_async_commit();
   };
-  stage(R, local_vertex(t, R, tid), local_vertex(t, R, tid + kTileThreads), 0);
+  {
+    const int g0 = local_vertex(t, R, tid), g1 = local_vertex(t, R, tid + kTileThreads);
+    pdl_wait();
+    const int stop = *done;
+    stage(R, g0, g1, 0);
+    if (stop) {
+      cp_async_wait<0>();
+      return;
+    }
+  }
 
   // last stage with fuse_dt: the next step's local dt from the new state
   const bool next_dt = MODE == MODE_UPDATE && do_norm && k.fuse_dt;
@@ -461,6 +493,7 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
       cp_async_commit();
     }
     if (more) stage(N, g0, g1, buf ^ 1);
+    else pdl_trigger();   // this late, the next pass starts behind the last update only
 
     // ---- owned vertices: fixed-order sum, then residual or RK update
     const unsigned short* list = sC + (size_t)buf * cmax;
