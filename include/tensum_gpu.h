@@ -540,6 +540,10 @@ tg_status tg_mlp_train(tg_mlp* m, const float* X, const float* T, int n, int epo
                        float* losses);
 /* precision 0: FP32, 1: BF16 tensor cores; on_device: X and Y are device pointers. */
 tg_status tg_mlp_predict(tg_mlp* m, const float* X, int n, float* Y, int precision, int on_device);
+/* From and to physical units, host arrays in FP64: Y = ym + ys net((X - xm) / xs), xm and xs of
+ * length din, ym and ys of length dout; every operation rounded as written. */
+tg_status tg_mlp_predict_scaled(tg_mlp* m, const double* X, int n, const double* xm, const double* xs,
+                                const double* ym, const double* ys, double* Y, int precision);
 
 /* ---- allocation-free residual norm ------------------------------------ */
 

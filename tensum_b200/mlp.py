@@ -27,8 +27,9 @@ def _lib():
         L.tg_mlp_loss_grad.argtypes = [vp, fp, fp, i, fp, fp]
         L.tg_mlp_train.argtypes = [vp, fp, fp, i, i, i, C.c_float, fp]
         L.tg_mlp_predict.argtypes = [vp, vp, i, vp, i, i]
+        L.tg_mlp_predict_scaled.argtypes = [vp, vp, i, vp, vp, vp, vp, vp, i]
         for n in ("tg_mlp_create", "tg_mlp_destroy", "tg_mlp_get_params", "tg_mlp_set_params", "tg_mlp_loss_grad",
-                  "tg_mlp_train", "tg_mlp_predict"):
+                  "tg_mlp_train", "tg_mlp_predict", "tg_mlp_predict_scaled"):
             getattr(L, n).restype = i
         _bound = True
     return L
@@ -111,5 +112,13 @@ class MLP:
 
     def predict(self, X, precision: int = 1) -> np.ndarray:
         """Surrogate QoIs for inputs X (physical units); precision 1 = BF16 tensor cores."""
-        Xn = (np.asarray(X, np.float64) - self.xm) / self.xs
-        return self.raw_predict(Xn, precision).astype(np.float64) * self.ys + self.ym
+        X = np.ascontiguousarray(X, np.float64)
+        if X.ndim != 2 or X.shape[1] != self.din:      # whatever broadcasts against the input scaling
+            Xn = (X - self.xm) / self.xs
+            return self.raw_predict(Xn, precision).astype(np.float64) * self.ys + self.ym
+        sc = [np.ascontiguousarray(np.broadcast_to(np.asarray(a, np.float64), (k,)))
+              for a, k in ((self.xm, self.din), (self.xs, self.din), (self.ym, self.dout), (self.ys, self.dout))]
+        Y = np.empty((X.shape[0], self.dout))
+        self._chk(self.L.tg_mlp_predict_scaled(self.h, X.ctypes.data, X.shape[0], *[a.ctypes.data for a in sc],
+                                               Y.ctypes.data, precision))
+        return Y
