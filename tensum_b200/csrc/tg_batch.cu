@@ -48,7 +48,7 @@ struct tg_batch {
   BParams prm{};
   int* stop = nullptr;           // device stop counter (read by kb_step_begin)
   double* tinst = nullptr;
-  int shape = 0;                 // index into kShapes
+  int shape = 1;                 // index into kShapes (the usual winner of tg_batch_tune)
   bool bnd = false;              // walls / far field or Navier-Stokes: the boundary and viscous passes run
   int dt_chunks = 1;
   cudaGraphExec_t graph_exec = nullptr;
@@ -124,8 +124,11 @@ template <int ST, int H>
 long long layout_warps_pair(Batch& B, int kind) {
   long long w = 0;
   for (int l = 0; l < B.nlev; ++l) {
+    const int n = item_count(B.lev[l].m, kind);
     B.lev[l].w_begin = w;
-    w += level_warps_pair<ST, H>(item_count(B.lev[l].m, kind), B.lev[l].S);
+    B.lev[l].w_items = (unsigned)std::max<long long>(1, level_warps_pair<ST, H>(n, ST));
+    B.lev[l].w_magic = (unsigned)(((1ull << 32) + B.lev[l].w_items - 1) / B.lev[l].w_items);
+    w += level_warps_pair<ST, H>(n, B.lev[l].S);
   }
   B.work = w;
   return w;
@@ -219,6 +222,20 @@ int max_samples(const tg_batch* b) {
   return m;
 }
 
+// The edge pass's shared memory (its limit raised at capture) and its grid: blocks that fill
+// the chip once.
+size_t edge_smem_of(const tg_batch* b, int bs) {
+  return needs_grad(b) ? edge_smem<FLUX_TECNO_ROE, RECON_TVD_MINMOD>(bs) : edge_smem<FLUX_KEPEC, RECON_FIRST>(bs);
+}
+unsigned edge_grid(const tg_batch* b, FluxK f, int bs) {
+  const size_t smem = edge_smem_of(b, bs);
+  cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per = 1, sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)f, bs, smem) != cudaSuccess || per < 1) per = 1;
+  return (unsigned)(per * sms);
+}
+
 unsigned blocks_of(const Batch& B, int bs) { return (unsigned)((B.work * 32 + bs - 1) / bs); }
 
 // One full step of every level on b->stream.
@@ -238,13 +255,14 @@ void enqueue_step(tg_batch* b) {
   else kb_dt<8, false><<<(unsigned)dt_blocks, 256, 0, b->stream>>>(B, b->prm, b->dt_chunks);
   kb_dt_final<<<gs, 256, 0, b->stream>>>(B, b->prm);
   FluxK fk = flux_kernel(b->prm.flux, b->prm.recon, b->shape);
+  const unsigned fill = edge_grid(b, fk, sh.bs);
   FluxK gk = gather_kernel(b->shape, b->bnd);
   GradK rk = grad_kernel(sh.st, b->bnd);
   for (int r = 0; r < 3; ++r) {
     if (needs_grad(b)) rk<<<blocks_of(BG, sh.bs), sh.bs, 0, b->stream>>>(BG, b->prm, r, 0);
     if (b->bnd && BB.work > 0) bflux_kernel(b->prm.flux, b->shape)<<<blocks_of(BB, sh.bs), sh.bs, 0, b->stream>>>(BB, b->prm, r);
     if (b->prm.model == 1) viscous_kernel(b->shape)<<<blocks_of(BU, sh.bs), sh.bs, 0, b->stream>>>(BU, b->prm, r);
-    fk<<<blocks_of(BE, sh.bs), sh.bs, 0, b->stream>>>(BE, b->prm, r);
+    fk<<<std::min(blocks_of(BE, sh.bs), fill), sh.bs, edge_smem_of(b, sh.bs), b->stream>>>(BE, b->prm, r);
     gk<<<blocks_of(B, sh.bs), sh.bs, 0, b->stream>>>(B, b->prm, r);
   }
   kb_step_end<<<gs, 256, 0, b->stream>>>(B, b->prm);
@@ -370,7 +388,10 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
     LevelMesh& m = V.m;
     m.nv = L.nv; m.ne = L.ne;
     // geometry formed in FP64, stored in FP32
-    std::vector<double> ux(L.ne), uy(L.ne), ar(L.ne), aw(L.nv), visw(L.nv, 0.0);
+    std::vector<double> aw(L.nv), visw(L.nv, 0.0);
+    std::vector<EdgeRec> ed(L.ne);
+    std::vector<GradRec> ge(L.ce_ent.size() + 2, GradRec{0, 0.0f, 0.0f, 0.0f});
+    std::vector<DtRec> de(L.ce_ent.size());
     for (int v = 0; v < L.nv; ++v) aw[v] = L.dcarea[v] * L.pweight[v];
     for (int v = 0; v < L.nv; ++v)
       for (int j = L.ce_off[v]; j < L.ce_off[v + 1]; ++j) {
@@ -381,13 +402,19 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
     for (int e = 0; e < L.ne; ++e) {
       const double a = std::sqrt(L.e_nx[e] * L.e_nx[e] + L.e_ny[e] * L.e_ny[e]);
       const double ia = a > 0.0 ? 1.0 / a : 0.0;   // gradient-only edges carry no flux
-      ux[e] = L.e_nx[e] * ia; uy[e] = L.e_ny[e] * ia; ar[e] = a;
+      ed[e] = EdgeRec{L.e_a[e], L.e_b[e], (float)(L.e_nx[e] * ia), (float)(L.e_ny[e] * ia), (float)L.e_dx[e],
+                      (float)L.e_dy[e], (float)a, 0.0f};
+    }
+    for (size_t j = 0; j < L.ce_ent.size(); ++j) {
+      const int e = L.ce_ent[j] >> 1;
+      const bool side = L.ce_ent[j] & 1;
+      ge[j] = GradRec{side ? L.e_a[e] : L.e_b[e], (float)(side ? L.e_g1x[e] : L.e_g0x[e]),
+                      (float)(side ? L.e_g1y[e] : L.e_g0y[e]), 0.0f};
+      de[j] = DtRec{(float)L.e_nx[e], (float)L.e_ny[e], ed[e].ar, 0.0f};
     }
 #define BU(vec, field) \
     if ((st = bupload(b, vec, &m.field)) != TG_OK) { tg_batch_destroy(b); return st; }
-    BU(L.e_a, e_a) BU(L.e_b, e_b) BU(ux, ux) BU(uy, uy) BU(ar, ar) BU(L.e_nx, nx) BU(L.e_ny, ny)
-    BU(L.e_dx, dx) BU(L.e_dy, dy) BU(L.e_g0x, g0x) BU(L.e_g0y, g0y) BU(L.e_g1x, g1x) BU(L.e_g1y, g1y)
-    BU(L.ce_off, ce_off) BU(L.ce_ent, ce_ent) BU(L.dcarea, area) BU(L.inv6mc, inv6mc) BU(visw, visw) BU(L.x, x) BU(L.y, y) BU(aw, aw)
+    BU(ed, ed) BU(ge, ge) BU(de, de) BU(L.ce_off, ce_off) BU(L.ce_ent, ce_ent) BU(L.dcarea, area) BU(L.inv6mc, inv6mc) BU(visw, visw) BU(L.x, x) BU(L.y, y) BU(aw, aw)
     m.nb = L.nb; m.nvu = L.nvu; m.nic = L.n_int_cells;
     BU(L.b_v0, b_v0) BU(L.b_v1, b_v1) BU(L.b_kind, b_kind) BU(L.b_adiab, b_adiab) BU(L.b_nx, b_nx) BU(L.b_ny, b_ny)
     BU(L.cb_off, cb_off) BU(L.cb_ent, cb_ent)
@@ -398,7 +425,6 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
     const size_t vs = (size_t)L.nv * V.P;
     for (int r = 0; r < 3; ++r)
       if ((st = balloc(b, kQ * vs, &V.Q[r])) != TG_OK) { tg_batch_destroy(b); return st; }
-    if ((st = balloc(b, 4 * vs, &V.Uold)) != TG_OK) { tg_batch_destroy(b); return st; }
     if ((st = balloc(b, 4 * (size_t)L.ne * V.P, &V.F)) != TG_OK) { tg_batch_destroy(b); return st; }
     if ((mat->reconstruct_scheme != RECON_FIRST && mat->flux_scheme != FLUX_KEPEC) || L.nb > 0 || mat->model == 1) {
       if ((st = balloc(b, kG * vs, &V.G)) != TG_OK) { tg_batch_destroy(b); return st; }
@@ -449,7 +475,7 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
   if ((st = bupload(b, ti, &tip)) != TG_OK) { tg_batch_destroy(b); return st; }
   k.tinst = tip;
   k.ntinst = (int)ti.size();
-  if ((st = balloc(b, 1, &b->stop)) != TG_OK) { tg_batch_destroy(b); return st; }
+  if ((st = balloc(b, 1, &b->stop)) != TG_OK || (st = balloc(b, 1, &k.live)) != TG_OK) { tg_batch_destroy(b); return st; }
   k.stop_counter = INT_MAX;
   k.stop = b->stop;
   int inf = INT_MAX;

@@ -36,14 +36,29 @@ constexpr int kQ = 5;        // stored per vertex-sample: u, v, p, V1, V5
 constexpr int kG = 8;        // dV1/dx, dV1/dy, dV2/dx, dV2/dy, dV3/dx, dV3/dy, dV5/dx, dV5/dy
 
 // Mesh of one level (device order of the single-solve layout, tg_mesh.cc).
+// What a pass reads of an edge, or of an entry of a vertex's gather list, is one record
+// of 16-byte words, so that an item's index chain is one broadcast load per entry and the
+// entry after it can be on its way; arrays indexed through the edge cost two dependent
+// loads and an address each.  Geometry is formed in FP64.
+struct EdgeRec {
+  int a, b;                        // endpoints
+  float ux, uy;                    // unit dual normal
+  float dx, dy;                    // x_b - x_a
+  float ar, pad;                   // |n|
+};
+struct GradRec {
+  int other;                       // the entry's other endpoint
+  float gx, gy, pad;               // P1 gradient weights of this side
+};
+struct DtRec {
+  float nx, ny, ar, pad;           // dual normal and |n|
+};
 struct LevelMesh {
   int nv, ne;
-  const int *e_a, *e_b;            // edge endpoints
-  const float *ux, *uy, *ar;       // unit dual normal and |n| (formed in FP64)
-  const float *nx, *ny;            // dual normal (for the time step)
-  const float *dx, *dy;            // x_b - x_a
-  const float *g0x, *g0y, *g1x, *g1y;   // P1 gradient weights of the a / b side
+  const EdgeRec* ed;
   const int *ce_off, *ce_ent;      // per-vertex gather: (edge << 1) | side
+  const GradRec* ge;               // per entry
+  const DtRec* de;                 // per entry
   const float *area, *inv6mc;      // dual area, 1 / (6 median area)
   const float* visw;               // sum over the vertex's edges of |n| / |x_b - x_a| (viscous time step)
   const double* aw;                // dual area x periodic-copy weight (integrals)
@@ -79,8 +94,7 @@ struct Level {
   LevelClock c;
   int S;                           // samples (a multiple of 32)
   int P;                           // row pitch in floats: S plus a pad that breaks power-of-two strides
-  float* Q[3];                     // rotating states, nv x kQ x S
-  float* Uold;                     // nv x 4 x S
+  float* Q[3];                     // rotating states, nv x kQ x S (U_old is formed from Q[0])
   float* G;                        // nv x kG x S
   float* F;                        // ne x 4 x S: area-weighted edge fluxes of the current stage
   // boundaries / Navier-Stokes (null on periodic Euler levels)
@@ -90,6 +104,7 @@ struct Level {
   float* Fv;                       // nvu x 9 x S: viscous fluxes (x, y, energy) toward the cell's 3 vertices
   float* Fvb;                      // nb x 3 x S: viscous boundary fluxes
   long long w_begin;               // first warp of this level in a fused launch (set per launch shape)
+  unsigned w_items, w_magic;       // warps per sample tile and ceil(2^32 / w_items) mod 2^32 (set per launch shape)
 };
 
 struct Batch {
@@ -107,6 +122,7 @@ struct BParams {
   int ntinst;
   int stop_counter;                // unused on the device: the live value is *stop
   const int* stop;                 // samples hold once their output counter exceeds it
+  int* live;                       // nonzero while some sample of the batch advances in this step
   int flux, recon;
 };
 
@@ -442,15 +458,43 @@ __device__ __forceinline__ f2 rcp2(f2 a) { return make_float2(rcp_apx(a.x), rcp_
 __device__ __forceinline__ f2 sqrt2(f2 a) { return make_float2(sqrt_apx(a.x), sqrt_apx(a.y)); }
 __device__ __forceinline__ f2 ld2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
 __device__ __forceinline__ void st2(float* p, f2 v) { *reinterpret_cast<float2*>(p) = v; }
+// H neighbouring pairs by one load or store (H = 2: 16 bytes; sample indices are multiples
+// of 2 H and rows of 32 samples)
+template <int H>
+__device__ __forceinline__ void ldh(const float* p, f2* o) {
+  if (H == 2) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(p));
+    o[0] = make_float2(x.x, x.y);
+    o[H - 1] = make_float2(x.z, x.w);
+  } else {
+    o[0] = ld2(p);
+  }
+}
+template <int H>
+__device__ __forceinline__ void sth(float* p, const f2* v) {
+  if (H == 2) *reinterpret_cast<float4*>(p) = make_float4(v[0].x, v[0].y, v[H - 1].x, v[H - 1].y);
+  else st2(p, v[0]);
+}
 
-// F of the Ismail-Roe log mean of one component (src/material.h:24-42), the
-// near-equal series in FP64; 1 / (a + b) from the approximate FP32 reciprocal
-// refined by one Newton-Raphson step in FP64 (relative error about 2^-46).
-__device__ __forceinline__ float logF1(float a, float b) {
+// F of the Ismail-Roe log mean of one component (src/material.h:24-42) where a and b are
+// near (far is set where they are not and logF_far has the value): the series in FP64,
+// 1 / (a + b) from the approximate FP32 reciprocal refined by one Newton-Raphson step in
+// FP64 (relative error about 2^-46).
+__device__ __forceinline__ double logF_ratio(float a, float b) {
   const double da = a, db = b;
   const double d = db + da;                      // exact in FP64, as is db - da
-  const double y0 = (double)rcp_apx((float)d);
-  const double f = (db - da) * (y0 * ::fma(-d, y0, 2.0));
+  const double y0 = (double)rcp_apx(a + b);      // (float)d
+  return (db - da) * (y0 * ::fma(-d, y0, 2.0));
+}
+__device__ __forceinline__ float logF_near(float a, float b, bool& far) {
+  const double f = logF_ratio(a, b);
+  const double u = f * f;
+  far = far || !(u < 1.0e-2);
+  const double u2 = u * u;
+  return (float)::fma(u2 * u, 1.0 / 7.0, ::fma(u2, 1.0 / 5.0, ::fma(u, 1.0 / 3.0, 1.0)));
+}
+__device__ __forceinline__ float logF1(float a, float b) {
+  const double f = logF_ratio(a, b);
   const double u = f * f;
   if (u < 1.0e-2) {
     const double u2 = u * u;
@@ -459,10 +503,20 @@ __device__ __forceinline__ float logF1(float a, float b) {
   return logf(b / a) / (2.0f * (float)f);
 }
 
-// minmod (src/limiter.h:14-27) of one component
-__device__ __forceinline__ float minmod1(float a, float b) {
-  const float m = fminf(fabsf(a), fabsf(b));
-  return ((a > 0.0f && b > 0.0f) || (a < 0.0f && b < 0.0f)) ? copysignf(m, a) : 0.0f;
+// Z_ji - Z_ij = d - minmod(2 s_r - d, d) / 2 - minmod(2 s_l - d, d) / 2 (src/limiter.h:14-27,
+// src/reconstruct.cc:139-188).  minmod(-a, -b) = -minmod(a, b), so everything is formed with
+// d's sign taken out: the limiter is then a clamp to [0, |d|], two instructions instead of the
+// sign tests and selects, and each rounding is the mirror image of the unflipped one.
+__device__ __forceinline__ float xsign(float x, unsigned s) { return __uint_as_float(__float_as_uint(x) ^ s); }
+__device__ __forceinline__ f2 limited_jump(f2 d, f2 sl, f2 sr) {
+  const unsigned s0 = __float_as_uint(d.x) & 0x80000000u, s1 = __float_as_uint(d.y) & 0x80000000u;
+  const f2 D = make_float2(xsign(d.x, s0), xsign(d.y, s1)), nD = neg2(D);
+  const f2 xr = fma2(sp(2.0f), make_float2(xsign(sr.x, s0), xsign(sr.y, s1)), nD);
+  const f2 xl = fma2(sp(2.0f), make_float2(xsign(sl.x, s0), xsign(sl.y, s1)), nD);
+  const f2 mr = make_float2(fmaxf(0.0f, fminf(xr.x, D.x)), fmaxf(0.0f, fminf(xr.y, D.y)));
+  const f2 ml = make_float2(fmaxf(0.0f, fminf(xl.x, D.x)), fmaxf(0.0f, fminf(xl.y, D.y)));
+  const f2 q = fma2(sp(-0.5f), ml, fma2(sp(-0.5f), mr, D));
+  return make_float2(xsign(q.x, s0), xsign(q.y, s1));
 }
 
 struct PRec { f2 rho, u, v, p, beta, V1; };
@@ -482,8 +536,15 @@ __device__ __forceinline__ PRec prec(f2 u, f2 v, f2 p, f2 V1, f2 V5) {
 // KEPEC central flux (src/kepec.cc:10-38) on a unit normal, with its averages.
 __device__ __forceinline__ PFlx kepec2(const BParams& k, const PRec& L, const PRec& R, float unx, float uny, PAvg& A) {
   const f2 sr = add2(L.rho, R.rho), sb = add2(L.beta, R.beta);
-  const f2 Fr = make_float2(logF1(L.rho.x, R.rho.x), logF1(L.rho.y, R.rho.y));
-  const f2 Fb = make_float2(logF1(L.beta.x, R.beta.x), logF1(L.beta.y, R.beta.y));
+  // the four log means by their series; one branch for the edges where some pair is far
+  // apart, which forms all four again
+  bool far = false;
+  f2 Fr = make_float2(logF_near(L.rho.x, R.rho.x, far), logF_near(L.rho.y, R.rho.y, far));
+  f2 Fb = make_float2(logF_near(L.beta.x, R.beta.x, far), logF_near(L.beta.y, R.beta.y, far));
+  if (far) {
+    Fr = make_float2(logF1(L.rho.x, R.rho.x), logF1(L.rho.y, R.rho.y));
+    Fb = make_float2(logF1(L.beta.x, R.beta.x), logF1(L.beta.y, R.beta.y));
+  }
   const f2 hs = mul2(sp(0.5f), sr);
   const f2 isb = rcp2(sb);
   A.rho = mul2(hs, rcp2(Fr));          // (rho_l + rho_r) / 2 / F_rho
@@ -504,9 +565,11 @@ __device__ __forceinline__ PFlx kepec2(const BParams& k, const PRec& L, const PR
 
 // KEPES-TeCNO (src/kepes_tecno_roe.cc:11-173, src/kepes_tecno_rusanov.cc:11-164)
 // in the unscaled form of ftecno: S^2 (Lambda jump(R0^T V)), first order or minmod.
-template <int ROE, int RECON>
-__device__ __forceinline__ PFlx tecno2(const BParams& k, const PRec& L, const PRec& R, float unx, float uny, float dx,
-                                       float dy, const f2* gL, const f2* gR) {
+// grads(gl, gr) gives the entropy-variable gradients along the edge, V1, V2, V3, V5; it is
+// called once, after the central flux, so that they need not be held before.
+template <int ROE, int RECON, class Grads>
+__device__ __forceinline__ PFlx tecno2(const BParams& k, const PRec& L, const PRec& R, float unx, float uny,
+                                       Grads&& grads) {
   static_assert(RECON == RECON_FIRST || RECON == RECON_TVD_MINMOD, "ensembles run first order or minmod");
   PAvg A;
   PFlx F = kepec2(k, L, R, unx, uny, A);
@@ -547,21 +610,11 @@ __device__ __forceinline__ PFlx tecno2(const BParams& k, const PRec& L, const PR
   RT(dV, q);
   if (RECON != RECON_FIRST) {
     f2 gl[4], gr[4], sl[4], sr[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      gl[i] = fma2(gL[2 * i + 1], sp(dy), mul2(gL[2 * i], sp(dx)));
-      gr[i] = fma2(gR[2 * i + 1], sp(dy), mul2(gR[2 * i], sp(dx)));
-    }
+    grads(gl, gr);
     RT(gl, sl);
     RT(gr, sr);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {   // Z_ji - Z_ij = d - minmod(2 s_r - d, d) / 2 - minmod(2 s_l - d, d) / 2
-      const f2 d = q[i], nd = neg2(d);
-      const f2 xr = fma2(sp(2.0f), sr[i], nd), xl = fma2(sp(2.0f), sl[i], nd);
-      const f2 mr = make_float2(minmod1(xr.x, d.x), minmod1(xr.y, d.y));
-      const f2 ml = make_float2(minmod1(xl.x, d.x), minmod1(xl.y, d.y));
-      q[i] = fma2(sp(-0.5f), ml, fma2(sp(-0.5f), mr, d));
-    }
+    for (int i = 0; i < 4; ++i) q[i] = limited_jump(q[i], sl[i], sr[i]);
   }
   const f2 s01 = mul2(A.rho, sp(k.inv_gamma));
   const f2 hs01 = mul2(sp(0.5f), s01);
@@ -578,11 +631,11 @@ __device__ __forceinline__ PFlx tecno2(const BParams& k, const PRec& L, const PR
   return F;
 }
 
-template <int FLUX, int RECON>
-__device__ __forceinline__ PFlx pflux(const BParams& k, const PRec& L, const PRec& R, float unx, float uny, float dx,
-                                      float dy, const f2* gL, const f2* gR) {
-  if (FLUX == FLUX_TECNO_ROE) return tecno2<1, RECON>(k, L, R, unx, uny, dx, dy, gL, gR);
-  if (FLUX == FLUX_TECNO_RUSANOV) return tecno2<0, RECON>(k, L, R, unx, uny, dx, dy, gL, gR);
+template <int FLUX, int RECON, class Grads>
+__device__ __forceinline__ PFlx pflux(const BParams& k, const PRec& L, const PRec& R, float unx, float uny,
+                                      Grads&& grads) {
+  if (FLUX == FLUX_TECNO_ROE) return tecno2<1, RECON>(k, L, R, unx, uny, grads);
+  if (FLUX == FLUX_TECNO_RUSANOV) return tecno2<0, RECON>(k, L, R, unx, uny, grads);
   PAvg A;
   return kepec2(k, L, R, unx, uny, A);
 }
@@ -650,8 +703,9 @@ __device__ __forceinline__ Item item_of_pair(const Batch& B, unsigned w, int lan
     if (i < B.nlev && (long long)w >= B.lev[i].w_begin) l = i;
   const unsigned r = w - (unsigned)B.lev[l].w_begin;
   const unsigned n = (unsigned)item_count(B.lev[l].m, KIND);
-  const unsigned nvw = (n + IPW - 1) / IPW;
-  const unsigned tile = r / nvw;
+  const unsigned nvw = B.lev[l].w_items;
+  unsigned tile = nvw == 1 ? r : __umulhi(r, B.lev[l].w_magic);   // r / nvw, or one more
+  if (tile * nvw > r) --tile;
   it.l = l;
   it.s = (int)(tile * ST) + 2 * H * (int)(lane % LPI);
   it.v = (int)((r - tile * nvw) * IPW) + (int)(lane / LPI);
@@ -659,6 +713,27 @@ __device__ __forceinline__ Item item_of_pair(const Batch& B, unsigned w, int lan
   return it;
 }
 
+// Register budgets of the paired passes as resident threads per SM.  All wait on memory more
+// than on anything else, so more warps win until they spill.  Step in ms of 768 samples of
+// Kelvin-Helmholtz 257^2 / 128 of the 128 x 256 cylinder, 128-thread blocks: gather + update at
+// 512, 768, 1024 threads 13.2 / 2.05, 12.3 / 1.94, 12.1 / 1.94 (96 samples of 65^2 123, 121, 126
+// us); gradients of meshes with boundaries at 512, 768, 1024: 2.02, 1.93, 1.88; viscous units
+// at 512, 768: 2.17, 1.99.
+#ifndef TG_BATCH_GRAD_BLOCK
+#define TG_BATCH_GRAD_BLOCK 256      // largest block of the launch shapes
+#endif
+#ifndef TG_BATCH_GRAD_MINB
+#define TG_BATCH_GRAD_MINB 3
+#endif
+#ifndef TG_BATCH_GRAD_MINB_BND
+#define TG_BATCH_GRAD_MINB_BND 4
+#endif
+#ifndef TG_BATCH_GATHER_THREADS
+#define TG_BATCH_GATHER_THREADS 768
+#endif
+#ifndef TG_BATCH_VISC_THREADS
+#define TG_BATCH_VISC_THREADS 768
+#endif
 // Pairs per lane of the gradient and gather passes.
 #ifndef TG_BATCH_LANE_PAIRS
 #define TG_BATCH_LANE_PAIRS 2
@@ -679,10 +754,11 @@ __global__ void kb_step_begin(Batch B, BParams k) {
   const bool go = !L.c.bad[s] && L.c.elapsed[s] < k.final_time && L.c.counter[s] <= *k.stop;
   L.c.active[s] = go ? 1 : 0;
   L.c.dtmin_bits[s] = 0x7f800000u;
+  if (go) *k.live = 1;             // cleared by the previous step's end
 }
 
 // Local time step (src/fv.cc:1499-1580) of every vertex and the running
-// per-sample minimum; U_old (src/fv.cc:1626-1630).  Each lane keeps a pair of
+// per-sample minimum.  Each lane keeps a pair of
 // samples (a group of 64; the last group of a level whose sample count is an
 // odd multiple of 32 leaves its upper half-warp idle) and walks a strided set of
 // vertices, so one atomic per block and sample remains.  BND adds the
@@ -692,6 +768,7 @@ __host__ __device__ __forceinline__ int dt_groups(int S) { return (S + 63) / 64;
 
 template <int VT, bool BND>
 __global__ void __launch_bounds__(32 * VT) kb_dt(Batch B, BParams k, int chunks) {
+  if (!*k.live) return;
   const int lane = threadIdx.x & 31, vg = threadIdx.x >> 5;
   // blockIdx.x: (level, sample group, chunk)
   long long bid = blockIdx.x;
@@ -722,9 +799,9 @@ __global__ void __launch_bounds__(32 * VT) kb_dt(Batch B, BParams k, int chunks)
       const f2 c = make_float2(sqrtf(gp.x / rho.x), sqrtf(gp.y / rho.y));
       f2 lam = sp(0.0f);
       for (int j = L.m.ce_off[v]; j < L.m.ce_off[v + 1]; ++j) {
-        const int e = L.m.ce_ent[j] >> 1;
-        const f2 vn = fma2(w, sp(L.m.ny[e]), mul2(u, sp(L.m.nx[e])));
-        lam = add2(lam, fma2(c, sp(L.m.ar[e]), abs2(vn)));
+        const float4 n = __ldg(reinterpret_cast<const float4*>(L.m.de + j));   // nx, ny, |n|
+        const f2 vn = fma2(w, sp(n.y), mul2(u, sp(n.x)));
+        lam = add2(lam, fma2(c, sp(n.z), abs2(vn)));
       }
       if (BND) {
         for (int j = L.m.cb_off[v]; j < L.m.cb_off[v + 1]; ++j) {
@@ -743,12 +820,6 @@ __global__ void __launch_bounds__(32 * VT) kb_dt(Batch B, BParams k, int chunks)
       const f2 dtv = make_float2(ca / lam.x, ca / lam.y);
       m.x = fminf(m.x, dtv.x > 0.0f ? dtv.x : inf);
       m.y = fminf(m.y, dtv.y > 0.0f ? dtv.y : inf);
-      // U_old
-      float* uo = L.Uold + rows(v, 4, P) + s;
-      st2(uo, rho);
-      st2(uo + P, mul2(rho, u));
-      st2(uo + 2 * P, mul2(rho, w));
-      st2(uo + 3 * P, fma2(p, sp(k.inv_gm1), mul2(mul2(sp(0.5f), fma2(w, w, mul2(u, u))), rho)));
     }
   }
   __shared__ float2 red[VT][32];
@@ -787,7 +858,8 @@ __global__ void kb_dt_final(Batch B, BParams k) {
 // samples, held ones included (forces); otherwise a thread whose samples are
 // all held skips.
 template <int ST, bool BND, int H = BND ? 1 : kLanePairs>
-__global__ void kb_grad(Batch B, BParams k, int r, int every) {
+__global__ void __launch_bounds__(TG_BATCH_GRAD_BLOCK, BND ? TG_BATCH_GRAD_MINB_BND : TG_BATCH_GRAD_MINB) kb_grad(Batch B, BParams k, int r, int every) {
+  if (!every && !*k.live) return;
   const unsigned w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const Item it = item_of_pair<ST, IT_VERTEX, H>(B, w, threadIdx.x & 31);
   if (!it.ok) return;
@@ -804,28 +876,43 @@ __global__ void kb_grad(Batch B, BParams k, int r, int every) {
   }
   const int S = L.P;   // row pitch
   const float* Q = L.Q[r] + s;
-  auto W = [&](int x, f2 (*o)[4]) {   // V2 = 2 beta u = -V5 u
+  struct Raw { f2 u[H], v[H], V1[H], V5[H]; };
+  auto load = [&](int x, Raw& o) {
     const float* q = Q + rows(x, kQ, S);
+    ldh<H>(q, o.u); ldh<H>(q + S, o.v); ldh<H>(q + 3 * S, o.V1); ldh<H>(q + 4 * S, o.V5);
+  };
+  auto ent = [&](const Raw& x, f2 (*o)[4]) {   // V2 = 2 beta u = -V5 u
 #pragma unroll
     for (int h = 0; h < H; ++h) {
-      const f2 V5 = ld2(q + 4 * S + 2 * h), nV5 = neg2(V5);
-      o[h][0] = ld2(q + 3 * S + 2 * h); o[h][1] = mul2(nV5, ld2(q + 2 * h)); o[h][2] = mul2(nV5, ld2(q + S + 2 * h));
-      o[h][3] = V5;
+      const f2 nV5 = neg2(x.V5[h]);
+      o[h][0] = x.V1[h]; o[h][1] = mul2(nV5, x.u[h]); o[h][2] = mul2(nV5, x.v[h]); o[h][3] = x.V5[h];
     }
   };
+  auto W = [&](int x, f2 (*o)[4]) {
+    Raw q;
+    load(x, q);
+    ent(q, o);
+  };
+  // the coming neighbour's state is on its way while this one's is used, its entry one further
+  const int j0 = L.m.ce_off[v], j1 = L.m.ce_off[v + 1];
+  const int4* ge = reinterpret_cast<const int4*>(L.m.ge);
+  int4 e = __ldg(ge + j0), nx = __ldg(ge + j0 + 1);   // the arrays end with two spare entries
   f2 ws[H][4];
   W(v, ws);
+  Raw cur, nxt;
+  load(e.x, cur);
   f2 acc[H][kG];
 #pragma unroll
   for (int h = 0; h < H; ++h)
 #pragma unroll
     for (int c = 0; c < kG; ++c) acc[h][c] = sp(0.0f);
-  for (int j = L.m.ce_off[v]; j < L.m.ce_off[v + 1]; ++j) {
-    const int ent = L.m.ce_ent[j], e = ent >> 1, side = ent & 1;
-    const int o = side ? L.m.e_a[e] : L.m.e_b[e];
-    const f2 gx = sp(side ? L.m.g1x[e] : L.m.g0x[e]), gy = sp(side ? L.m.g1y[e] : L.m.g0y[e]);
+  for (int j = j0; j < j1; ++j) {
+    load(nx.x, nxt);
+    const f2 gx = sp(__int_as_float(e.y)), gy = sp(__int_as_float(e.z));
+    e = nx;
+    nx = __ldg(ge + min(j + 2, j1));
     f2 wo[H][4];
-    W(o, wo);
+    ent(cur, wo);
 #pragma unroll
     for (int h = 0; h < H; ++h)
 #pragma unroll
@@ -834,6 +921,7 @@ __global__ void kb_grad(Batch B, BParams k, int r, int every) {
         acc[h][2 * c] = fma2(gx, d, acc[h][2 * c]);
         acc[h][2 * c + 1] = fma2(gy, d, acc[h][2 * c + 1]);
       }
+    cur = nxt;
   }
   if (BND) {
     for (int j = L.m.cb_off[v]; j < L.m.cb_off[v + 1]; ++j) {
@@ -873,54 +961,146 @@ __global__ void kb_grad(Batch B, BParams k, int r, int every) {
   const f2 f = sp(L.m.inv6mc[v]);
   float* G = L.G + rows(v, kG, S) + s;
 #pragma unroll
-  for (int h = 0; h < H; ++h)
+  for (int c = 0; c < kG; ++c) {
+    f2 o[H];
 #pragma unroll
-    for (int c = 0; c < kG; ++c) st2(G + c * S + 2 * h, mul2(acc[h][c], f));
+    for (int h = 0; h < H; ++h) o[h] = mul2(acc[h][c], f);
+    sth<H>(G + c * S, o);
+  }
 }
 
 // Edge fluxes of one stage (src/fv.cc:1066-1192, src/material.cc:27-74): one
-// edge and a pair of samples per thread, the flux of the edge's own
-// orientation (a left, b right) times |n|, stored for the gather.  A pair
-// whose two samples are both held skips.
-// Resident threads per SM the edge pass is compiled for (0: the compiler's choice).
+// edge and a pair of samples per lane, the flux of the edge's own
+// orientation (a left, b right) times |n|, stored for the gather.  A warp
+// whose samples are all held skips.
+//
+// With one edge per thread the pass waited on its 26 rows of endpoint data half the
+// time (long scoreboard 6.5 of 12 warp cycles per issue at 24 warps).  So a warp walks edges, and the
+// coming edge's rows are copied to shared memory once the current one's have been
+// read: the state first, the gradients after the central flux, so that neither is held in
+// registers longer than it is used.  60 % of the issue slots are used at 17 warps (44 % before),
+// and the limits are the FP32 pipes and the fixed latencies: 0.79 -> 0.72 ms on 256 samples of
+// 257^2.
+// Resident threads per SM the edge pass is compiled for, with and without gradients.
 #ifndef TG_BATCH_EDGE_THREADS
-#define TG_BATCH_EDGE_THREADS 896
+#define TG_BATCH_EDGE_THREADS 640
 #endif
-#if TG_BATCH_EDGE_THREADS > 0
-#define TG_EDGE_BOUNDS(BS) __launch_bounds__(BS, TG_BATCH_EDGE_THREADS / (BS))
-#else
-#define TG_EDGE_BOUNDS(BS) __launch_bounds__(BS)
+#ifndef TG_BATCH_EDGE_THREADS_FIRST
+#define TG_BATCH_EDGE_THREADS_FIRST 896
 #endif
+// Rows a pair of edge endpoints brings: five state components, and the gradients where the
+// reconstruction reads them.
+template <int FLUX, int RECON>
+__host__ __device__ constexpr bool edge_grads() {
+  return RECON != RECON_FIRST && (FLUX == FLUX_TECNO_ROE || FLUX == FLUX_TECNO_RUSANOV);
+}
+template <int FLUX, int RECON>
+__host__ __device__ constexpr int edge_rows() {
+  return kQ + (edge_grads<FLUX, RECON>() ? kG : 0);
+}
+// Shared memory of a block: per warp the row segments of its 64 / ST edges.
+template <int FLUX, int RECON>
+__host__ __device__ constexpr size_t edge_smem(int bs) {
+  return (size_t)(bs / 32) * 64 * 2 * edge_rows<FLUX, RECON>() * sizeof(float);
+}
+
 template <int FLUX, int RECON, int ST, int BS>
-__global__ void TG_EDGE_BOUNDS(BS) kb_edge_flux(Batch B, BParams k, int r) {
-  const unsigned w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const Item it = item_of_pair<ST, IT_EDGE>(B, w, threadIdx.x & 31);
-  if (!it.ok) return;
-  const Level& L = B.lev[it.l];
-  const int e = it.v, s = it.s;
-  const int2 act = *reinterpret_cast<const int2*>(L.c.active + s);
-  if (!act.x && !act.y) return;
-  constexpr bool kGr = (RECON != RECON_FIRST) && (FLUX == FLUX_TECNO_ROE || FLUX == FLUX_TECNO_RUSANOV);
-  const int S = L.P;   // row pitch
-  const int ia = L.m.e_a[e], ib = L.m.e_b[e];
-  const float* qa = L.Q[r] + rows(ia, kQ, S) + s;
-  const float* qb = L.Q[r] + rows(ib, kQ, S) + s;
-  const PRec A = prec(ld2(qa), ld2(qa + S), ld2(qa + 2 * S), ld2(qa + 3 * S), ld2(qa + 4 * S));
-  const PRec Bv = prec(ld2(qb), ld2(qb + S), ld2(qb + 2 * S), ld2(qb + 3 * S), ld2(qb + 4 * S));
-  f2 ga[kG], gb[kG];
-  if (kGr) {
-    const float* Ga = L.G + rows(ia, kG, S) + s;
-    const float* Gb = L.G + rows(ib, kG, S) + s;
+__global__ void __launch_bounds__(BS, (edge_grads<FLUX, RECON>() ? TG_BATCH_EDGE_THREADS : TG_BATCH_EDGE_THREADS_FIRST) / BS)
+    kb_edge_flux(Batch B, BParams k, int r) {
+  constexpr int NR = edge_rows<FLUX, RECON>(), LPI = ST / 2, CPR = ST / 4;   // rows, lanes per edge, 16-byte words per row
+  constexpr bool kGr = edge_grads<FLUX, RECON>();
+  extern __shared__ __align__(16) float sm[];
+  const int lane = threadIdx.x & 31;
+  const unsigned stride = gridDim.x * (BS / 32);
+  unsigned w = blockIdx.x * (BS / 32) + (threadIdx.x >> 5);
+  float* buf = sm + (size_t)(threadIdx.x >> 5) * 64 * 2 * NR + (lane / LPI) * 2 * NR * ST;   // the lane's edge
+  const int live = *k.live;
+  // the coming edge: its item, record and row segments, in the order a's state components
+  // 0 .. 3 and gradients, b's, and component 4 of both
+  auto record = [&](const Item& it, int4& e0, float4& e1) {
+    if (!it.ok) return;
+    const EdgeRec* e = B.lev[it.l].m.ed + it.v;
+    e0 = __ldg(reinterpret_cast<const int4*>(e));
+    e1 = __ldg(reinterpret_cast<const float4*>(e) + 1);
+  };
+  auto copy = [&](const Item& it, const int4& e0) {
+    if (!it.ok) return;
+    const Level& L = B.lev[it.l];
+    const int S = L.P, s0 = it.s - 2 * (lane % LPI) + 4 * (lane % CPR);
+    const int sub = (lane % LPI) / CPR;       // which of the two rows a copy takes
+    unsigned d = (unsigned)__cvta_generic_to_shared(buf + sub * ST + 4 * (lane % CPR));
+    auto put = [&](const float* p, int n) {   // rows p, p + S, ... as n pairs
 #pragma unroll
-    for (int c = 0; c < kG; ++c) { ga[c] = ld2(Ga + c * S); gb[c] = ld2(Gb + c * S); }
-  } else {
-#pragma unroll
-    for (int c = 0; c < kG; ++c) ga[c] = gb[c] = sp(0.0f);
+      for (int i = 0; i < n; ++i, p += 2 * S, d += 2 * ST * 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(p) : "memory");
+    };
+    const float* qa = L.Q[r] + rows(e0.x, kQ, S) + s0;
+    const float* qb = L.Q[r] + rows(e0.y, kQ, S) + s0;
+    put(qa + sub * S, 2);
+    if (kGr) put(L.G + rows(e0.x, kG, S) + s0 + sub * S, 4);
+    put(qb + sub * S, 2);
+    if (kGr) put(L.G + rows(e0.y, kG, S) + s0 + sub * S, 4);
+    put((sub ? qb : qa) + 4 * S, 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (!live || (long long)w >= B.work) return;
+  Item it = item_of_pair<ST, IT_EDGE>(B, w, lane);
+  int4 e0 = make_int4(0, 0, 0, 0);
+  float4 e1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  record(it, e0, e1);
+  copy(it, e0);
+  Item nx{0, 0, 0, false};
+  int4 n0 = e0;
+  float4 n1 = e1;
+  bool more = stride < (unsigned long long)B.work - w;
+  if (more) {
+    nx = item_of_pair<ST, IT_EDGE>(B, w + stride, lane);
+    record(nx, n0, n1);
   }
-  const PFlx F = pflux<FLUX, RECON>(k, A, Bv, L.m.ux[e], L.m.uy[e], L.m.dx[e], L.m.dy[e], ga, gb);
-  const f2 ar = sp(L.m.ar[e]);
-  float* Fo = L.F + rows(e, 4, S) + s;
-  st2(Fo, mul2(F.m, ar)); st2(Fo + S, mul2(F.x, ar)); st2(Fo + 2 * S, mul2(F.y, ar)); st2(Fo + 3 * S, mul2(F.e, ar));
+  for (;;) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    auto x = [&](int c) { return *reinterpret_cast<const float2*>(buf + c * ST + 2 * (lane % LPI)); };
+    auto next = [&]() {        // the buffer has been read: the coming edge's rows
+      __syncwarp();
+      if (more) copy(nx, n0);
+    };
+    int2 act = make_int2(0, 0);
+    if (it.ok) act = *reinterpret_cast<const int2*>(B.lev[it.l].c.active + it.s);
+    const bool on = act.x || act.y;
+    if (__any_sync(0xffffffffu, on)) {
+      const PRec A = prec(x(0), x(1), x(2), x(3), x(2 * NR - 2));
+      const PRec Bv = prec(x(NR - 1), x(NR), x(NR + 1), x(NR + 2), x(2 * NR - 1));
+      if (!kGr) next();
+      const PFlx F = pflux<FLUX, RECON>(k, A, Bv, __int_as_float(e0.z), __int_as_float(e0.w), [&](f2* gl, f2* gr) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          gl[i] = fma2(x(4 + 2 * i + 1), sp(e1.y), mul2(x(4 + 2 * i), sp(e1.x)));
+          gr[i] = fma2(x(NR + 3 + 2 * i + 1), sp(e1.y), mul2(x(NR + 3 + 2 * i), sp(e1.x)));
+        }
+        next();
+      });
+      if (on) {
+        const Level& L = B.lev[it.l];
+        const int S = L.P;
+        const f2 ar = sp(e1.z);
+        float* Fo = L.F + rows(it.v, 4, S) + it.s;
+        st2(Fo, mul2(F.m, ar)); st2(Fo + S, mul2(F.x, ar)); st2(Fo + 2 * S, mul2(F.y, ar)); st2(Fo + 3 * S, mul2(F.e, ar));
+      }
+    } else {
+      next();
+    }
+    if (!more) break;
+    w += stride;
+    it = nx;
+    e0 = n0;
+    e1 = n1;
+    more = stride < (unsigned long long)B.work - w;
+    if (more) {
+      nx = item_of_pair<ST, IT_EDGE>(B, w + stride, lane);
+      record(nx, n0, n1);
+    }
+  }
 }
 
 // Boundary-face fluxes (src/fv.cc:1100-1188): one (face vertex, sample) per
@@ -928,6 +1108,7 @@ __global__ void TG_EDGE_BOUNDS(BS) kb_edge_flux(Batch B, BParams k, int r) {
 // order (the reference passes zero gradients); otherwise inviscid_bflux.
 template <int FLUX, int ST, int BS>
 __global__ void __launch_bounds__(BS) kb_bflux(Batch B, BParams k, int r) {
+  if (!*k.live) return;
   const unsigned w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const Item it = item_of<ST, IT_BSLOT>(B, w, threadIdx.x & 31);
   if (!it.ok) return;
@@ -1013,7 +1194,8 @@ __device__ __forceinline__ void pviscous_apply(const PViscK& K, float nx, float 
 }
 
 template <int ST, int BS>
-__global__ void __launch_bounds__(BS) kb_viscous(Batch B, BParams k, int r) {
+__global__ void __launch_bounds__(BS, TG_BATCH_VISC_THREADS / BS) kb_viscous(Batch B, BParams k, int r) {
+  if (!*k.live) return;
   const unsigned w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const Item it = item_of_pair<ST, IT_UNIT>(B, w, threadIdx.x & 31);
   if (!it.ok) return;
@@ -1122,16 +1304,17 @@ __global__ void __launch_bounds__(BS) kb_viscous(Batch B, BParams k, int r) {
 // pairs of samples per thread.  Held or finished samples copy their state
 // through.
 template <int ST, int BS, bool BND, int H = kLanePairs>
-__global__ void __launch_bounds__(BS) kb_gather_update(Batch B, BParams k, int r) {
+__global__ void __launch_bounds__(BS, TG_BATCH_GATHER_THREADS / BS) kb_gather_update(Batch B, BParams k, int r) {
+  if (!*k.live) return;            // nothing advances: Q[0] stays the state
   const unsigned w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const Item it = item_of_pair<ST, IT_VERTEX, H>(B, w, threadIdx.x & 31);
   if (!it.ok) return;
   const Level& L = B.lev[it.l];
   const int v = it.v, s = it.s;
   const int S = L.P;   // row pitch
-  const size_t ov = rows(v, kQ, S) + s;
-  const float* Q = L.Q[r] + ov;
-  float* Qn = L.Q[(r + 1) % 3] + ov;
+  const size_t ov_ = rows(v, kQ, S) + s;
+  const float* Q = L.Q[r] + ov_;
+  float* Qn = L.Q[(r + 1) % 3] + ov_;
   int2 act[H];
   bool any = false;
 #pragma unroll
@@ -1141,9 +1324,11 @@ __global__ void __launch_bounds__(BS) kb_gather_update(Batch B, BParams k, int r
   }
   if (!any) {
 #pragma unroll
-    for (int h = 0; h < H; ++h)
-#pragma unroll
-      for (int c = 0; c < kQ; ++c) st2(Qn + c * S + 2 * h, ld2(Q + c * S + 2 * h));
+    for (int c = 0; c < kQ; ++c) {
+      f2 x[H];
+      ldh<H>(Q + c * S, x);
+      sth<H>(Qn + c * S, x);
+    }
     return;
   }
   f2 r0[H], r1[H], r2[H], r3[H];
@@ -1155,10 +1340,12 @@ __global__ void __launch_bounds__(BS) kb_gather_update(Batch B, BParams k, int r
     const int ent = L.m.ce_ent[j];
     const float* Fe = L.F + rows(ent >> 1, 4, S) + s;
     const f2 sg = sp((ent & 1) ? -1.0f : 1.0f);
+    f2 f0[H], f1[H], f2_[H], f3[H];
+    ldh<H>(Fe, f0); ldh<H>(Fe + S, f1); ldh<H>(Fe + 2 * S, f2_); ldh<H>(Fe + 3 * S, f3);
 #pragma unroll
     for (int h = 0; h < H; ++h) {
-      r0[h] = fma2(ld2(Fe + 2 * h), sg, r0[h]); r1[h] = fma2(ld2(Fe + S + 2 * h), sg, r1[h]);
-      r2[h] = fma2(ld2(Fe + 2 * S + 2 * h), sg, r2[h]); r3[h] = fma2(ld2(Fe + 3 * S + 2 * h), sg, r3[h]);
+      r0[h] = fma2(f0[h], sg, r0[h]); r1[h] = fma2(f1[h], sg, r1[h]);
+      r2[h] = fma2(f2_[h], sg, r2[h]); r3[h] = fma2(f3[h], sg, r3[h]);
     }
   }
   if (BND) {   // boundary and viscous contributions in list order (src/fv.cc:1100-1188, 1197-1320)
@@ -1188,18 +1375,29 @@ __global__ void __launch_bounds__(BS) kb_gather_update(Batch B, BParams k, int r
   const f2 a_rk = sp(r == 0 ? 0.0f : (r == 1 ? 0.75f : 1.0f / 3.0f));
   const f2 b_rk = sp(r == 0 ? 1.0f : (r == 1 ? 0.25f : 2.0f / 3.0f));
   const float area = L.m.area[v];
-  const float* Uo = L.Uold + rows(v, 4, S) + s;
+  f2 qu[H], qv[H], qp[H], qw[H], ou[H], ov[H], op[H], ow[H], res[kQ][H];
+  ldh<H>(Q, qu); ldh<H>(Q + S, qv); ldh<H>(Q + 2 * S, qp); ldh<H>(Q + 4 * S, qw);
+  if (r > 0) {   // U_old from the state the step started from; stage 0 does not use it
+    const float* O = L.Q[0] + ov_;
+    ldh<H>(O, ou); ldh<H>(O + S, ov); ldh<H>(O + 2 * S, op); ldh<H>(O + 4 * S, ow);
+  }
+  auto conserved = [&](f2 u, f2 v, f2 p, f2 V5, f2* c) {
+    c[0] = mul2(neg2(V5), p);
+    c[1] = mul2(c[0], u);
+    c[2] = mul2(c[0], v);
+    c[3] = fma2(p, sp(k.inv_gm1), mul2(mul2(sp(0.5f), fma2(v, v, mul2(u, u))), c[0]));
+  };
 #pragma unroll
   for (int h = 0; h < H; ++h) {
     const int o = 2 * h;
-    const f2 u0 = ld2(Q + o), v0 = ld2(Q + S + o), p0 = ld2(Q + 2 * S + o), V50 = ld2(Q + 4 * S + o);
-    const f2 rho0 = mul2(neg2(V50), p0);
+    f2 c0[4], uo[4] = {sp(0.0f), sp(0.0f), sp(0.0f), sp(0.0f)};
+    conserved(qu[h], qv[h], qp[h], qw[h], c0);
+    if (r > 0) conserved(ou[h], ov[h], op[h], ow[h], uo);
     const f2 c2 = mul2(make_float2((float)L.c.dt[s + o] / area, (float)L.c.dt[s + o + 1] / area), neg2(b_rk));
-    const f2 cr = fma2(r0[h], c2, fma2(ld2(Uo + o), a_rk, mul2(rho0, b_rk)));
-    const f2 cx = fma2(r1[h], c2, fma2(ld2(Uo + S + o), a_rk, mul2(mul2(rho0, u0), b_rk)));
-    const f2 cy = fma2(r2[h], c2, fma2(ld2(Uo + 2 * S + o), a_rk, mul2(mul2(rho0, v0), b_rk)));
-    const f2 E0 = fma2(p0, sp(k.inv_gm1), mul2(mul2(sp(0.5f), fma2(v0, v0, mul2(u0, u0))), rho0));
-    const f2 cE = fma2(r3[h], c2, fma2(ld2(Uo + 3 * S + o), a_rk, mul2(E0, b_rk)));
+    const f2 cr = fma2(r0[h], c2, fma2(uo[0], a_rk, mul2(c0[0], b_rk)));
+    const f2 cx = fma2(r1[h], c2, fma2(uo[1], a_rk, mul2(c0[1], b_rk)));
+    const f2 cy = fma2(r2[h], c2, fma2(uo[2], a_rk, mul2(c0[2], b_rk)));
+    const f2 cE = fma2(r3[h], c2, fma2(uo[3], a_rk, mul2(c0[3], b_rk)));
     const f2 ir = make_float2(1.0f / cr.x, 1.0f / cr.y);
     const f2 u = mul2(cx, ir), vv = mul2(cy, ir);
     const f2 p = mul2(sp(k.gamma - 1.0f), fma2(sp(-0.5f), fma2(cy, vv, mul2(cx, u)), cE));
@@ -1217,12 +1415,14 @@ __global__ void __launch_bounds__(BS) kb_gather_update(Batch B, BParams k, int r
       }
     }
 #pragma unroll
-    for (int c = 0; c < kQ; ++c) st2(Qn + c * S + o, out[c]);
+    for (int c = 0; c < kQ; ++c) res[c][h] = out[c];
     if (act[h].x && (!(p.x > 0.0f) || !(cr.x > 0.0f) || !isfinite(u.x) || !isfinite(vv.x) || !isfinite(p.x)))
       L.c.bad[s + o] = 1;
     if (act[h].y && (!(p.y > 0.0f) || !(cr.y > 0.0f) || !isfinite(u.y) || !isfinite(vv.y) || !isfinite(p.y)))
       L.c.bad[s + o + 1] = 1;
   }
+#pragma unroll
+  for (int c = 0; c < kQ; ++c) sth<H>(Qn + c * S, res[c]);
 }
 
 // Per-sample step end (src/fv.cc:2307-2336).
@@ -1231,6 +1431,7 @@ __global__ void kb_step_end(Batch B, BParams k) {
   if (l >= B.nlev) return;
   const Level& L = B.lev[l];
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s == 0 && l == 0) *k.live = 0;
   if (s >= L.S || !L.c.active[s]) return;
   L.c.elapsed[s] += L.c.dt[s];
   if (L.c.reached[s]) {
