@@ -22,26 +22,13 @@
 #include "tg_expr.cuh"
 #include "tg_tiles.cuh"
 #include "tg_mesh.h"
+#include "tg_stage.h"
 
 using namespace tg;
 
 namespace {
 
 thread_local std::string g_last_error;
-
-// Pinned staging for state transfers from and to pageable caller buffers: up to
-// kMaxLanes host threads, each with its own stream and two kSlot slots, so the
-// host memcpy into one slot overlaps the DMA of the other.  Pinned caller
-// buffers bypass it (one cudaMemcpyAsync on the handle's stream).
-struct Stager {
-  static constexpr int kMaxLanes = 8;
-  static constexpr size_t kSlot = size_t(2) << 20;
-  int lanes = 0;
-  char* slots = nullptr;   // pinned, lanes * 2 * kSlot bytes
-  cudaStream_t st[kMaxLanes] = {};
-  cudaEvent_t ev[kMaxLanes][2] = {};
-  char* slot(int lane, int k) const { return slots + (2 * (size_t)lane + k) * kSlot; }
-};
 
 }  // namespace
 
@@ -85,6 +72,8 @@ struct tg_handle {
   int* bad = nullptr;                 // device flag of k_state_check
   cudaEvent_t raw_ready = nullptr;
   Stager stage;
+  void* work = nullptr;               // see reserve()
+  size_t work_bytes = 0;
   // output snapshots (tg_output_begin / tg_output_wait)
   double* snap = nullptr;             // 5 * nv: PrimVar records in the caller's order
   double* snap_grad = nullptr;        // 15 * nv: dE records in the caller's order
@@ -165,6 +154,18 @@ tg_status dev_alloc(tg_handle* h, size_t n, T** out) {
 }
 
 inline int nblk(int n) { return (n + kBlock - 1) / kBlock; }
+
+// The handle's workspace of small uploads and results, grown on demand: work that used it is
+// complete whenever a call that reserves it returns.
+cudaError_t reserve(tg_handle* h, size_t bytes) {
+  if (bytes <= h->work_bytes) return cudaSuccess;
+  cudaFree(h->work);
+  h->work = nullptr;
+  h->work_bytes = 0;
+  const cudaError_t e = cudaMalloc(&h->work, bytes);
+  if (e == cudaSuccess) h->work_bytes = bytes;
+  return e;
+}
 
 // A launch on `st`, dependent on the stream's previous kernel by pdl_wait when pdl is set.
 template <class... P, class... A>
@@ -452,73 +453,6 @@ tg_status sync(tg_handle* h) {
   return TG_OK;
 }
 
-bool host_pinned(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeHost;
-}
-
-// One lane of a staged host->device copy of len bytes.
-cudaError_t lane_h2d(const tg_handle* h, int lane, char* dst, const char* src, size_t len) {
-  const Stager& S = h->stage;
-  cudaError_t e = cudaSetDevice(h->device);
-  for (size_t off = 0, k = 0; e == cudaSuccess && off < len; off += Stager::kSlot, ++k) {
-    const int s = (int)(k & 1);
-    const size_t n = std::min(Stager::kSlot, len - off);
-    if (k >= 2 && (e = cudaEventSynchronize(S.ev[lane][s])) != cudaSuccess) break;
-    std::memcpy(S.slot(lane, s), src + off, n);
-    if ((e = cudaMemcpyAsync(dst + off, S.slot(lane, s), n, cudaMemcpyHostToDevice, S.st[lane])) != cudaSuccess) break;
-    e = cudaEventRecord(S.ev[lane][s], S.st[lane]);
-  }
-  cudaError_t e2 = cudaStreamSynchronize(S.st[lane]);
-  return e != cudaSuccess ? e : e2;
-}
-
-// One lane of a staged device->host copy; the lane's stream first waits for `ready`.
-cudaError_t lane_d2h(const tg_handle* h, int lane, char* dst, const char* src, size_t len, cudaEvent_t ready) {
-  const Stager& S = h->stage;
-  cudaError_t e = cudaSetDevice(h->device);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(S.st[lane], ready, 0);
-  const size_t nk = (len + Stager::kSlot - 1) / Stager::kSlot;
-  auto issue = [&](size_t k) {
-    const int s = (int)(k & 1);
-    const size_t n = std::min(Stager::kSlot, len - k * Stager::kSlot);
-    cudaError_t ei = cudaMemcpyAsync(S.slot(lane, s), src + k * Stager::kSlot, n, cudaMemcpyDeviceToHost, S.st[lane]);
-    return ei != cudaSuccess ? ei : cudaEventRecord(S.ev[lane][s], S.st[lane]);
-  };
-  for (size_t k = 0; e == cudaSuccess && k < std::min<size_t>(2, nk); ++k) e = issue(k);
-  for (size_t k = 0; e == cudaSuccess && k < nk; ++k) {
-    const int s = (int)(k & 1);
-    if ((e = cudaEventSynchronize(S.ev[lane][s])) != cudaSuccess) break;
-    std::memcpy(dst + k * Stager::kSlot, S.slot(lane, s), std::min(Stager::kSlot, len - k * Stager::kSlot));
-    if (k + 2 < nk) e = issue(k + 2);
-  }
-  cudaError_t e2 = cudaStreamSynchronize(S.st[lane]);
-  return e != cudaSuccess ? e : e2;
-}
-
-// Splits a staged copy over the lanes (lane 0 on the calling thread).
-template <class Lane>
-cudaError_t run_lanes(const tg_handle* h, size_t bytes, Lane lane) {
-  const int n = (int)std::max<size_t>(1, std::min<size_t>(h->stage.lanes, bytes / (2 * Stager::kSlot)));
-  const size_t per = ((bytes + n - 1) / n + 255) & ~size_t(255);
-  std::vector<cudaError_t> errs(n, cudaSuccess);
-  std::vector<std::thread> th;
-  for (int t = 1; t < n; ++t) {
-    const size_t off = t * per;
-    if (off >= bytes) break;
-    th.emplace_back([&, t, off] { errs[t] = lane(t, off, std::min(per, bytes - off)); });
-  }
-  errs[0] = lane(0, 0, std::min(per, bytes));
-  for (auto& x : th) x.join();
-  for (cudaError_t e : errs)
-    if (e != cudaSuccess) return e;
-  return cudaSuccess;
-}
-
 // Caller buffer -> h->raw, ordered before the next work on h->stream.
 tg_status state_h2d(tg_handle* h, const double* prim, size_t bytes) {
   if (host_pinned(prim)) {
@@ -526,25 +460,19 @@ tg_status state_h2d(tg_handle* h, const double* prim, size_t bytes) {
     return TG_OK;
   }
   TG_CUDA(h, cudaStreamSynchronize(h->stream));   // h->raw may still be read by an earlier transfer
-  const char* src = (const char*)prim;
-  char* dst = (char*)h->raw;
-  TG_CUDA(h, run_lanes(h, bytes, [&](int t, size_t off, size_t len) { return lane_h2d(h, t, dst + off, src + off, len); }));
+  TG_CUDA(h, h->stage.in(h->raw, prim, bytes));
   return TG_OK;
 }
 
-// h->raw -> caller buffer, after the work enqueued so far on h->stream; returns when the data is in `prim`.
-tg_status state_d2h(tg_handle* h, double* prim, size_t bytes) {
-  if (host_pinned(prim)) {
-    TG_CUDA(h, cudaMemcpyAsync(prim, h->raw, bytes, cudaMemcpyDeviceToHost, h->stream));
+// Device -> caller buffer, after the work enqueued so far on h->stream; returns when the data is there.
+tg_status dev_out(tg_handle* h, void* dst, const void* src, size_t bytes) {
+  if (host_pinned(dst)) {
+    TG_CUDA(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
     TG_CUDA(h, cudaStreamSynchronize(h->stream));
     return TG_OK;
   }
   TG_CUDA(h, cudaEventRecord(h->raw_ready, h->stream));
-  const char* src = (const char*)h->raw;
-  char* dst = (char*)prim;
-  TG_CUDA(h, run_lanes(h, bytes, [&](int t, size_t off, size_t len) {
-    return lane_d2h(h, t, dst + off, src + off, len, h->raw_ready);
-  }));
+  TG_CUDA(h, h->stage.out(dst, src, bytes, h->raw_ready));
   return TG_OK;
 }
 
@@ -930,14 +858,7 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   if ((st = dev_alloc(h, 1, &h->bad)) != TG_OK) { tg_destroy(h); return st; }
   if ((st = dev_upload(h, L.old_of_new, &h->old_of_new)) != TG_OK) { tg_destroy(h); return st; }
   {
-    Stager& S = h->stage;
-    const size_t bytes = 5 * (size_t)h->n_caller * sizeof(double);
-    S.lanes = (int)std::max<size_t>(1, std::min<size_t>(Stager::kMaxLanes, bytes / (2 * Stager::kSlot)));
-    cudaError_t ep = cudaMallocHost((void**)&S.slots, 2 * (size_t)S.lanes * Stager::kSlot);
-    for (int t = 0; t < S.lanes && ep == cudaSuccess; ++t) {
-      ep = cudaStreamCreateWithFlags(&S.st[t], cudaStreamNonBlocking);
-      for (int k = 0; k < 2 && ep == cudaSuccess; ++k) ep = cudaEventCreateWithFlags(&S.ev[t][k], cudaEventDisableTiming);
-    }
+    cudaError_t ep = h->stage.init(h->device, 5 * (size_t)h->n_caller * sizeof(double));
     if (ep == cudaSuccess) ep = cudaEventCreateWithFlags(&h->raw_ready, cudaEventDisableTiming);
     if (ep != cudaSuccess) { tg_destroy(h); return fail(nullptr, TG_CUDA_ERROR, cudaGetErrorString(ep)); }
   }
@@ -971,13 +892,8 @@ tg_status tg_destroy(tg_handle* h) {
   for (void* p : h->allocs) cudaFree(p);
   if (h->mom) cudaFree(h->mom);
   if (h->mom_in) cudaFree(h->mom_in);
-  for (int t = 0; t < Stager::kMaxLanes; ++t) {
-    if (h->stage.st[t]) cudaStreamSynchronize(h->stage.st[t]);
-    for (int k = 0; k < 2; ++k)
-      if (h->stage.ev[t][k]) cudaEventDestroy(h->stage.ev[t][k]);
-    if (h->stage.st[t]) cudaStreamDestroy(h->stage.st[t]);
-  }
-  if (h->stage.slots) cudaFreeHost(h->stage.slots);
+  cudaFree(h->work);
+  h->stage.release();
   if (h->raw_ready) cudaEventDestroy(h->raw_ready);
   if (h->out_stream) cudaStreamSynchronize(h->out_stream);
   if (h->in_stream) cudaStreamSynchronize(h->in_stream);
@@ -1015,18 +931,19 @@ tg_status tg_set_state_expr(tg_handle* h, const tg_expr* const* fields, const do
   std::vector<int> code, off;
   std::vector<double> k;
   expr::pack5(fields, nullptr, code, off, k);
-  int *dcode = nullptr, *doff = nullptr, *derr = nullptr;
-  double *dk = nullptr, *drnd = nullptr;
-  cudaError_t e = cudaMalloc((void**)&dcode, code.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&doff, off.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&dk, std::max<size_t>(1, k.size()) * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&drnd, std::max(1, n_rnd) * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&derr, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dcode, code.data(), code.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(doff, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess && !k.empty()) e = cudaMemcpyAsync(dk, k.data(), k.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess && n_rnd > 0) e = cudaMemcpyAsync(drnd, rnd, n_rnd * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(derr, 0, sizeof(int), h->stream);
+  // one upload into the handle's workspace: constants, random numbers, programs, offsets, and
+  // the error word (zero)
+  const size_t nd = k.size() + n_rnd, ni = code.size() + off.size() + 1;
+  std::vector<double> pack(nd + (ni + 1) / 2, 0.0);
+  if (!k.empty()) std::memcpy(pack.data(), k.data(), k.size() * sizeof(double));
+  if (n_rnd > 0) std::memcpy(pack.data() + k.size(), rnd, n_rnd * sizeof(double));
+  int* pi = reinterpret_cast<int*>(pack.data() + nd);
+  std::memcpy(pi, code.data(), code.size() * sizeof(int));
+  std::memcpy(pi + code.size(), off.data(), off.size() * sizeof(int));
+  cudaError_t e = reserve(h, pack.size() * sizeof(double));
+  double *dk = (double*)h->work, *drnd = dk + k.size();
+  int *dcode = (int*)(dk + nd), *doff = dcode + code.size(), *derr = doff + off.size();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h->work, pack.data(), pack.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
   int err = 0;
   if (e == cudaSuccess) {
     const int nv = h->L.nv;
@@ -1035,7 +952,6 @@ tg_status tg_set_state_expr(tg_handle* h, const tg_expr* const* fields, const do
     e = cudaMemcpyAsync(&err, derr, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   }
-  cudaFree(dcode); cudaFree(doff); cudaFree(dk); cudaFree(drnd); cudaFree(derr);
   if (e != cudaSuccess) return fail(h, TG_CUDA_ERROR, cudaGetErrorString(e));
   if (err) return fail(h, TG_INVALID_ARG, "pert: unknown type or random-number index out of range");
   return take_raw_state(h, t0);
@@ -1084,7 +1000,7 @@ tg_status tg_get_state(tg_handle* h, double* prim, int n_vertex) {
   const int nv = h->L.nv;
   k_state_out<<<nblk(nv), kBlock, 0, h->stream>>>(nv, view(h, 0), h->old_of_new, h->raw);
   TG_CUDA(h, cudaGetLastError());
-  return state_d2h(h, prim, 5 * (size_t)nv * sizeof(double));
+  return dev_out(h, prim, h->raw, 5 * (size_t)nv * sizeof(double));
 }
 
 tg_status tg_store_conserved_old(tg_handle* h) {
@@ -1377,27 +1293,21 @@ tg_status tg_forces(tg_handle* h, int n_forces, const int* n_tags, const int* ta
   std::vector<int> rec4, off;
   const std::string msg = force_faces(h->L, n_forces, n_tags, tags, rec4, off);
   if (!msg.empty()) return fail(h, TG_INVALID_ARG, msg);
-  std::vector<int4> rec(rec4.size() / 4);
-  for (size_t i = 0; i < rec.size(); ++i) rec[i] = make_int4(rec4[4 * i], rec4[4 * i + 1], rec4[4 * i + 2], rec4[4 * i + 3]);
-  tg_status st;
-  const int4* drec = nullptr;
-  const int* doff = nullptr;
-  double* dout = nullptr;
-  int4* r = nullptr;
-  int* o = nullptr;
-  TG_CUDA(h, cudaMalloc((void**)&r, rec.size() * sizeof(int4)));
-  TG_CUDA(h, cudaMalloc((void**)&o, off.size() * sizeof(int)));
-  TG_CUDA(h, cudaMalloc((void**)&dout, 4 * (size_t)n_forces * sizeof(double)));
-  drec = r; doff = o;
-  TG_CUDA(h, cudaMemcpyAsync(r, rec.data(), rec.size() * sizeof(int4), cudaMemcpyHostToDevice, h->stream));
-  TG_CUDA(h, cudaMemcpyAsync(o, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  // the handle's workspace: face records, offsets (padded), results
+  const size_t n_in = rec4.size() + off.size();
+  rec4.insert(rec4.end(), off.begin(), off.end());
+  const size_t out_at = (n_in * sizeof(int) + 15) / 16 * 16;
+  TG_CUDA(h, reserve(h, out_at + 4 * (size_t)n_forces * sizeof(double)));
+  const int4* drec = (const int4*)h->work;
+  const int* doff = (const int*)h->work + (n_in - off.size());
+  double* dout = (double*)((char*)h->work + out_at);
+  TG_CUDA(h, cudaMemcpyAsync(h->work, rec4.data(), n_in * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   // Navier-Stokes forces recompute the gradients of the current state (src/force.cc:123)
   if (h->prm.model == 1) enqueue_gradient(h, 0, h->never);
   k_forces<<<n_forces, kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, 0), drec, doff, dout);
   std::vector<double> hout(4 * (size_t)n_forces);
   cudaError_t e = cudaMemcpyAsync(hout.data(), dout, hout.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-  st = sync(h);
-  cudaFree(r); cudaFree(o); cudaFree(dout);
+  const tg_status st = sync(h);
   if (e != cudaSuccess) return fail(h, TG_CUDA_ERROR, cudaGetErrorString(e));
   if (st != TG_OK) return st;
   std::memcpy(out, hout.data(), hout.size() * sizeof(double));
@@ -1446,21 +1356,15 @@ tg_status tg_moments_increment(tg_handle* h, int instance, long k) {
 tg_status tg_moments_get(tg_handle* h, int instance, double* fm, double* sm, double* m2) {
   tg_status st = mom_check(h, instance);
   if (st != TG_OK) return st;
-  const size_t nv = h->L.nv, nvar = h->mom_nvar;
-  std::vector<double> buf(3 * nvar * nv);
-  TG_CUDA(h, cudaMemcpyAsync(buf.data(), mom_array(h, instance, 0), buf.size() * sizeof(double),
-                             cudaMemcpyDeviceToHost, h->stream));
-  if ((st = sync(h)) != TG_OK) return st;
+  const size_t n = (size_t)h->mom_nvar * h->L.nv;
+  if (!h->mom_in) TG_CUDA(h, cudaMalloc((void**)&h->mom_in, 3 * n * sizeof(double)));
+  k_moments_out<<<dim3(nblk(h->L.nv), 3), kBlock, 0, h->stream>>>(h->L.nv, h->mom_nvar, mom_array(h, instance, 0),
+                                                                    h->old_of_new, h->mom_in);
+  TG_CUDA(h, cudaGetLastError());
   double* out[3] = {fm, sm, m2};
-  for (int w = 0; w < 3; ++w) {
-    if (!out[w]) continue;
-    const double* src = buf.data() + (size_t)w * nvar * nv;
-    for (size_t i = 0; i < nv; ++i) {
-      double* d = out[w] + nvar * (size_t)h->L.old_of_new[i];
-      for (size_t c = 0; c < nvar; ++c) d[c] = src[c * nv + i];
-    }
-  }
-  return TG_OK;
+  for (int w = 0; w < 3; ++w)
+    if (out[w] && (st = dev_out(h, out[w], h->mom_in + w * n, n * sizeof(double))) != TG_OK) return st;
+  return sync(h);
 }
 
 tg_status tg_moments_export(tg_handle* h, int instance, void* dev_dst) {

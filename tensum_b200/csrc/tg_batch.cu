@@ -13,11 +13,13 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/tensum_gpu.h"
 #include "tg_batch.cuh"
 #include "tg_mesh.h"
+#include "tg_stage.h"
 
 using namespace tg;
 using namespace tg::batch;
@@ -29,7 +31,7 @@ thread_local std::string g_batch_error;
 struct LevelHost {
   HostLayout L;
   int S = 0;
-  std::vector<void*> allocs;
+  const int* old_of_new = nullptr;   // device copy
 };
 
 struct Shape {
@@ -56,6 +58,13 @@ struct tg_batch {
   std::vector<void*> allocs;
   std::string err;
   size_t device_bytes = 0;
+  std::vector<double> tinst_host;
+  // workspace of uploads and results, grown on demand (every call that uses it ends
+  // synchronised), and the staging of large results to pageable memory
+  void* work = nullptr;
+  size_t work_bytes = 0;
+  Stager stage;
+  cudaEvent_t ready = nullptr;
 };
 
 namespace {
@@ -92,8 +101,12 @@ tg_status bupload(tg_batch* b, const std::vector<U>& v, const T** out) {
   T* p = nullptr;
   tg_status st = balloc(b, v.size(), &p);
   if (st != TG_OK) return st;
-  std::vector<T> tmp(v.begin(), v.end());
-  if (!tmp.empty()) TB_CUDA(b, cudaMemcpy(p, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if constexpr (std::is_same<T, U>::value) {
+    if (!v.empty()) TB_CUDA(b, cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+  } else {
+    std::vector<T> tmp(v.begin(), v.end());
+    if (!tmp.empty()) TB_CUDA(b, cudaMemcpy(p, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice));
+  }
   *out = p;
   return TG_OK;
 }
@@ -101,6 +114,31 @@ tg_status bupload(tg_batch* b, const std::vector<U>& v, const T** out) {
 tg_status bsync(tg_batch* b) {
   TB_CUDA(b, cudaGetLastError());
   TB_CUDA(b, cudaStreamSynchronize(b->stream));
+  return TG_OK;
+}
+
+tg_status work_reserve(tg_batch* b, size_t bytes) {
+  if (bytes <= b->work_bytes) return TG_OK;
+  cudaFree(b->work);
+  b->work = nullptr;
+  b->work_bytes = 0;
+  TB_CUDA(b, cudaMalloc(&b->work, bytes));
+  b->work_bytes = bytes;
+  return TG_OK;
+}
+
+// Device -> caller memory after the work on b->stream so far; large pageable targets through
+// the staging threads.
+tg_status copy_out(tg_batch* b, void* dst, const void* src, size_t bytes) {
+  if (bytes < 2 * Stager::kPerLane || host_pinned(dst)) {
+    TB_CUDA(b, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, b->stream));
+    return bsync(b);
+  }
+  TB_CUDA(b, cudaGetLastError());
+  if (!b->ready) TB_CUDA(b, cudaEventCreateWithFlags(&b->ready, cudaEventDisableTiming));
+  TB_CUDA(b, b->stage.init(b->device, bytes));
+  TB_CUDA(b, cudaEventRecord(b->ready, b->stream));
+  TB_CUDA(b, b->stage.out(dst, src, bytes, b->ready));
   return TG_OK;
 }
 
@@ -299,28 +337,37 @@ tg_status capture(tg_batch* b) {
 struct ClockHost {
   std::vector<double> elapsed;
   std::vector<int> counter, bad;
+  std::vector<float> dt;     // the last step's time step before the clamp to an output time
 };
 
 tg_status read_clock(tg_batch* b, int l, ClockHost& c) {
   const int S = b->B.lev[l].S;
-  c.elapsed.resize(S); c.counter.resize(S); c.bad.resize(S);
+  c.elapsed.resize(S); c.counter.resize(S); c.bad.resize(S); c.dt.resize(S);
+  TB_CUDA(b, cudaMemcpyAsync(c.dt.data(), b->B.lev[l].c.dtmin_bits, S * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
   TB_CUDA(b, cudaMemcpyAsync(c.elapsed.data(), b->B.lev[l].c.elapsed, S * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   TB_CUDA(b, cudaMemcpyAsync(c.counter.data(), b->B.lev[l].c.counter, S * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
   TB_CUDA(b, cudaMemcpyAsync(c.bad.data(), b->B.lev[l].c.bad, S * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
   return bsync(b);
 }
 
-// Every sample of every level is past output `instance`, finished, or bad.
-tg_status all_reached(tg_batch* b, int instance, bool* yes, int* nbad) {
+// Every sample of every level is past output `instance`, finished, or bad; else about how
+// many steps the slowest one needs (8 where no step has been taken yet).
+tg_status all_reached(tg_batch* b, int instance, bool* yes, int* nbad, double* steps) {
   *yes = true;
   *nbad = 0;
+  *steps = 1.0;
+  const double target = instance < (int)b->tinst_host.size() && instance >= 0
+                            ? std::min(b->tinst_host[instance], b->prm.final_time) : b->prm.final_time;
   for (int l = 0; l < b->nlev; ++l) {
     ClockHost c;
     tg_status st = read_clock(b, l, c);
     if (st != TG_OK) return st;
     for (int s = 0; s < b->B.lev[l].S; ++s) {
       if (c.bad[s]) { ++*nbad; continue; }
-      if (c.counter[s] <= instance && c.elapsed[s] < b->prm.final_time) *yes = false;
+      if (c.counter[s] > instance || !(c.elapsed[s] < b->prm.final_time)) continue;
+      *yes = false;
+      const double dt = c.dt[s];
+      *steps = std::max(*steps, dt > 0.0 && std::isfinite(dt) ? (target - c.elapsed[s]) / dt : 8.0);
     }
   }
   return TG_OK;
@@ -422,6 +469,7 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
     BU(L.c_nbr_off, c_nbr_off) BU(L.c_nbr, c_nbr) BU(L.bf_face_nx, bf_nx) BU(L.bf_face_ny, bf_ny)
     BU(L.bf_face_v0, bf_v0) BU(L.bf_face_v1, bf_v1)
 #undef BU
+    if ((st = bupload(b, L.old_of_new, &H.old_of_new)) != TG_OK) { tg_batch_destroy(b); return st; }
     const size_t vs = (size_t)L.nv * V.P;
     for (int r = 0; r < 3; ++r)
       if ((st = balloc(b, kQ * vs, &V.Q[r])) != TG_OK) { tg_batch_destroy(b); return st; }
@@ -475,6 +523,7 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
   if ((st = bupload(b, ti, &tip)) != TG_OK) { tg_batch_destroy(b); return st; }
   k.tinst = tip;
   k.ntinst = (int)ti.size();
+  b->tinst_host = ti;
   if ((st = balloc(b, 1, &b->stop)) != TG_OK || (st = balloc(b, 1, &k.live)) != TG_OK) { tg_batch_destroy(b); return st; }
   k.stop_counter = INT_MAX;
   k.stop = b->stop;
@@ -512,6 +561,9 @@ tg_status tg_batch_destroy(tg_batch* b) {
   drop_graph(b);
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (void* p : b->allocs) cudaFree(p);
+  cudaFree(b->work);
+  b->stage.release();
+  if (b->ready) cudaEventDestroy(b->ready);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return TG_OK;
@@ -550,19 +602,11 @@ tg_status tg_batch_get_state(tg_batch* b, int level, int sample, double* prim_ao
   const Level& V = b->B.lev[level];
   const HostLayout& L = b->lh[level].L;
   if (sample < 0 || sample >= V.S || n_vertex != L.nv) return bfail(b, TG_INVALID_ARG, "bad sample or vertex count");
-  std::vector<float> q((size_t)kQ * L.nv);
-  TB_CUDA(b, cudaMemcpy2DAsync(q.data(), sizeof(float), V.Q[0] + sample, V.P * sizeof(float), sizeof(float),
-                               (size_t)kQ * L.nv, cudaMemcpyDeviceToHost, b->stream));
-  tg_status st = bsync(b);
+  const size_t bytes = 5 * (size_t)L.nv * sizeof(double);
+  const tg_status st = work_reserve(b, bytes);
   if (st != TG_OK) return st;
-  for (int i = 0; i < L.nv; ++i) {
-    double* p = prim_aos + 5 * (size_t)L.old_of_new[i];
-    const float* r = q.data() + (size_t)kQ * i;
-    const double u = r[0], v = r[1], pr = r[2], V5 = r[4];
-    const double rho = -V5 * pr;
-    p[0] = pr / (b->prm.R * rho); p[1] = pr; p[2] = u; p[3] = v; p[4] = 0.0;
-  }
-  return TG_OK;
+  kb_state_out<<<(L.nv + 255) / 256, 256, 0, b->stream>>>(V, b->prm, sample, b->lh[level].old_of_new, (double*)b->work);
+  return copy_out(b, prim_aos, b->work, bytes);
 }
 
 tg_status tg_batch_set_parameters(tg_batch* b, int level, const double* mu_ref, const double* bface_values) {
@@ -615,16 +659,12 @@ tg_status tg_batch_set_uniform(tg_batch* b, int level, const double* prim) {
     rec[3 * (size_t)S + s] = (float)((g - ent) / (g - 1.0) - (u * u + v * v) * beta);
     rec[4 * (size_t)S + s] = (float)(-2.0 * beta);
   }
-  float* d = nullptr;
-  TB_CUDA(b, cudaMalloc((void**)&d, rec.size() * sizeof(float)));
-  cudaError_t e = cudaMemcpyAsync(d, rec.data(), rec.size() * sizeof(float), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) {
-    const long long t = (long long)V.m.nv * S;
-    kb_ic_uniform<<<(unsigned)((t + 255) / 256), 256, 0, b->stream>>>(V, d);
-    e = cudaStreamSynchronize(b->stream);
-  }
-  cudaFree(d);
-  if (e != cudaSuccess) return bfail(b, TG_CUDA_ERROR, cudaGetErrorString(e));
+  tg_status st = work_reserve(b, rec.size() * sizeof(float));
+  if (st != TG_OK) return st;
+  TB_CUDA(b, cudaMemcpyAsync(b->work, rec.data(), rec.size() * sizeof(float), cudaMemcpyHostToDevice, b->stream));
+  const long long t = (long long)V.m.nv * S;
+  kb_ic_uniform<<<(unsigned)((t + 255) / 256), 256, 0, b->stream>>>(V, (const float*)b->work);
+  if ((st = bsync(b)) != TG_OK) return st;
   return reset_clock(b, level, 0, S);
 }
 
@@ -641,26 +681,18 @@ tg_status tg_batch_forces(tg_batch* b, int level, int n_forces, const int* n_tag
   Batch B = b->B;
   layout_pair(B, sh.st, IT_VERTEX, 1);   // kb_grad<*, true> takes one pair per lane
   if (b->prm.model == 1) grad_kernel(sh.st, true)<<<blocks_of(B, sh.bs), sh.bs, 0, b->stream>>>(B, b->prm, 0, 1);
-  int* drec = nullptr;
-  int* doff = nullptr;
-  double* dout = nullptr;
-  const size_t nout = (size_t)V.S * n_forces * 4;
-  TB_CUDA(b, cudaMalloc((void**)&drec, rec4.size() * sizeof(int)));
-  cudaError_t e = cudaMalloc((void**)&doff, off.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&dout, nout * sizeof(double));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(drec, rec4.data(), rec4.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(doff, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) {
-    kb_forces<8><<<(unsigned)(n_forces * (V.S >> 5)), 256, 0, b->stream>>>(V, b->prm, (const int4*)drec, doff, n_forces, dout);
-    e = cudaMemcpyAsync(out, dout, nout * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  if (e == cudaSuccess) e = cudaGetLastError();
-  cudaFree(drec);
-  cudaFree(doff);
-  cudaFree(dout);
-  if (e != cudaSuccess) return bfail(b, TG_CUDA_ERROR, cudaGetErrorString(e));
-  return TG_OK;
+  // workspace: face records, offsets (padded), results
+  const size_t nout = (size_t)V.S * n_forces * 4, n_in = rec4.size() + off.size();
+  const int* doff = nullptr;
+  rec4.insert(rec4.end(), off.begin(), off.end());
+  const size_t out_at = (n_in * sizeof(int) + 15) / 16 * 16;
+  const tg_status st = work_reserve(b, out_at + nout * sizeof(double));
+  if (st != TG_OK) return st;
+  doff = (const int*)b->work + (n_in - off.size());
+  double* dout = (double*)((char*)b->work + out_at);
+  TB_CUDA(b, cudaMemcpyAsync(b->work, rec4.data(), n_in * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+  kb_forces<8><<<(unsigned)(n_forces * (V.S >> 5)), 256, 0, b->stream>>>(V, b->prm, (const int4*)b->work, doff, n_forces, dout);
+  return copy_out(b, out, dout, nout * sizeof(double));
 }
 
 namespace {
@@ -750,17 +782,13 @@ tg_status tg_batch_set_kh(tg_batch* b, int level, const double* rows, int n_rnd)
   if (!b || !rows || level < 0 || level >= b->nlev || n_rnd < 2 || n_rnd % 2)
     return bfail(b, TG_INVALID_ARG, "bad level, NULL rows or odd row length");
   const Level& V = b->B.lev[level];
-  double* d = nullptr;
   const size_t n = (size_t)V.S * n_rnd;
-  TB_CUDA(b, cudaMalloc((void**)&d, n * sizeof(double)));
-  cudaError_t e = cudaMemcpyAsync(d, rows, n * sizeof(double), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess) {
-    const long long t = (long long)V.m.nv * V.S;
-    kb_ic_kh<<<(unsigned)((t + 255) / 256), 256, 0, b->stream>>>(V, b->prm, d, n_rnd);
-    e = cudaStreamSynchronize(b->stream);
-  }
-  cudaFree(d);
-  if (e != cudaSuccess) return bfail(b, TG_CUDA_ERROR, cudaGetErrorString(e));
+  tg_status st = work_reserve(b, n * sizeof(double));
+  if (st != TG_OK) return st;
+  TB_CUDA(b, cudaMemcpyAsync(b->work, rows, n * sizeof(double), cudaMemcpyHostToDevice, b->stream));
+  const long long t = (long long)V.m.nv * V.S;
+  kb_ic_kh<<<(unsigned)((t + 255) / 256), 256, 0, b->stream>>>(V, b->prm, (const double*)b->work, n_rnd);
+  if ((st = bsync(b)) != TG_OK) return st;
   return reset_clock(b, level, 0, V.S);
 }
 
@@ -773,12 +801,13 @@ tg_status tg_batch_advance(tg_batch* b, int instance, long max_steps, double* in
   bool done = false;
   int nbad = 0;
   long launched = 0;
-  if ((st = all_reached(b, instance, &done, &nbad)) != TG_OK) return st;
+  double steps = 1.0;
+  if ((st = all_reached(b, instance, &done, &nbad, &steps)) != TG_OK) return st;
   while (!done && launched < max_steps) {
-    const long chunk = std::min<long>(8, max_steps - launched);
+    const long chunk = std::min<long>(steps < 64.0 ? (long)std::ceil(steps) : 64, max_steps - launched);
     for (long i = 0; i < chunk; ++i) TB_CUDA(b, cudaGraphLaunch(b->graph_exec, b->stream));
     launched += chunk;
-    if ((st = all_reached(b, instance, &done, &nbad)) != TG_OK) return st;
+    if ((st = all_reached(b, instance, &done, &nbad, &steps)) != TG_OK) return st;
   }
   int inf = INT_MAX;
   TB_CUDA(b, cudaMemcpyAsync(b->stop, &inf, sizeof(int), cudaMemcpyHostToDevice, b->stream));
@@ -815,45 +844,33 @@ tg_status tg_batch_moments(tg_batch* b, int level, int extras, double* fm, doubl
   const HostLayout& L = b->lh[level].L;
   const int nvar = 5 + (extras & 1) + ((extras >> 1) & 1) + ((extras >> 2) & 1);
   const size_t n = (size_t)nvar * L.nv;
-  double* d = nullptr;
-  TB_CUDA(b, cudaMalloc((void**)&d, 3 * n * sizeof(double)));
-  kb_moments<<<(unsigned)((n + 127) / 128), 128, 0, b->stream>>>(V, b->prm, extras, nvar, d, d + n, d + 2 * n);
-  std::vector<double> h(3 * n);
-  cudaError_t e = cudaMemcpyAsync(h.data(), d, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  cudaFree(d);
-  if (e != cudaSuccess) return bfail(b, TG_CUDA_ERROR, cudaGetErrorString(e));
+  tg_status st = work_reserve(b, 3 * n * sizeof(double));
+  if (st != TG_OK) return st;
+  typedef void (*MomentsK)(Level, BParams, const int*, double*, double*, double*);
+  static const MomentsK kernels[8] = {kb_moments<0>, kb_moments<1>, kb_moments<2>, kb_moments<3>,
+                                      kb_moments<4>, kb_moments<5>, kb_moments<6>, kb_moments<7>};
+  double* d = (double*)b->work;
+  kernels[extras]<<<(L.nv + 7) / 8, 256, 0, b->stream>>>(V, b->prm, b->lh[level].old_of_new, d, d + n, d + 2 * n);
   double* out[3] = {fm, sm, m2};
-  for (int w = 0; w < 3; ++w) {
-    if (!out[w]) continue;
-    for (int i = 0; i < L.nv; ++i) {
-      double* dst = out[w] + (size_t)nvar * L.old_of_new[i];
-      for (int c = 0; c < nvar; ++c) dst[c] = h[(size_t)w * n + (size_t)c * L.nv + i];
-    }
-  }
-  return TG_OK;
+  for (int w = 0; w < 3; ++w)
+    if (out[w] && (st = copy_out(b, out[w], d + w * n, n * sizeof(double))) != TG_OK) return st;
+  return bsync(b);
 }
 
 tg_status tg_batch_integrals(tg_batch* b, int level, double* out) {
   if (!b || !out || level < 0 || level >= b->nlev) return bfail(b, TG_INVALID_ARG, "bad level or NULL output");
   const Level& V = b->B.lev[level];
-  const int chunks = 16;
-  double* d = nullptr;
-  const size_t n = (size_t)chunks * V.S * 3;
-  TB_CUDA(b, cudaMalloc((void**)&d, n * sizeof(double)));
-  kb_integrals<8><<<(V.S >> 5) * chunks, 256, 0, b->stream>>>(V, b->prm, chunks, d);
-  std::vector<double> h(n);
-  cudaError_t e = cudaMemcpyAsync(h.data(), d, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-  cudaFree(d);
-  if (e != cudaSuccess) return bfail(b, TG_CUDA_ERROR, cudaGetErrorString(e));
-  for (int s = 0; s < V.S; ++s)
-    for (int c = 0; c < 3; ++c) {
-      double acc = 0.0;
-      for (int ch = 0; ch < chunks; ++ch) acc += h[((size_t)ch * V.S + s) * 3 + c];
-      out[(size_t)s * 3 + c] = acc;
-    }
-  return TG_OK;
+  // enough blocks for the chip whatever the number of sample groups
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+  const int groups = V.S >> 5, chunks = std::min(std::max(16, (8 * sms + groups - 1) / groups), std::max(16, V.m.nv / 64));
+  const size_t n = 3 * (size_t)V.S;
+  const tg_status st = work_reserve(b, (size_t)(chunks + 1) * n * sizeof(double));
+  if (st != TG_OK) return st;
+  double* d = (double*)b->work;
+  kb_integrals<8><<<groups * chunks, 256, 0, b->stream>>>(V, b->prm, chunks, d);
+  kb_integrals_sum<<<(unsigned)((n + 255) / 256), 256, 0, b->stream>>>((int)n, chunks, d, d + chunks * n);
+  return copy_out(b, out, d + chunks * n, n * sizeof(double));
 }
 
 tg_status tg_batch_set_shape(tg_batch* b, int shape) {

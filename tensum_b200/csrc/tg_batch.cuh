@@ -1598,61 +1598,94 @@ __global__ void kb_bc_expr(Level L, expr::Field5 f, int mask, const int* __restr
   if (e) atomicOr(err, e);
 }
 
+// One sample's state as PrimVar records (T, p, u, v, w) in the caller's vertex order.
+__global__ void kb_state_out(Level L, BParams k, int sample, const int* __restrict__ old_of_new, double* __restrict__ out) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= L.m.nv) return;
+  const float* q = L.Q[0] + rows(v, kQ, L.P) + sample;
+  const double u = q[0], w = q[L.P], p = q[2 * L.P], V5 = q[4 * L.P];
+  const double rho = -V5 * p;
+  double* o = out + 5 * (size_t)old_of_new[v];
+  o[0] = p / ((double)k.R * rho); o[1] = p; o[2] = u; o[3] = w; o[4] = 0.0;
+}
+
 // Ensemble moments of one level at its current state, FP64: Welford mean and
-// sum of squared deviations in sample order (the per-group recurrence of
-// increment_moments, src/fv.cc:595-694) and a Kahan-compensated sum of
-// squares.  One thread per (component, vertex); record layout as
-// tg_moments_*: PrimVar (T, p, u, v, w), then density, mach, entropy.
-__global__ void kb_moments(Level L, BParams k, int extras, int nvar, double* __restrict__ fm, double* __restrict__ sm,
-                           double* __restrict__ m2) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)nvar * L.m.nv) return;
-  const int c = (int)(t / L.m.nv), v = (int)(t % L.m.nv);
-  // which derived quantity component c is
-  int kind = c;   // 0 T, 1 p, 2 u, 3 v, 4 w, 5+ extras in bit order
-  if (c >= 5) {
-    int want = c - 5, b = 0;
-    for (; b < 4; ++b)
-      if ((extras >> b) & 1) { if (want == 0) break; --want; }
-    kind = 5 + b;
-  }
-  double mean = 0.0, ssd = 0.0, sq = 0.0, comp = 0.0;
-  for (int s = 0; s < L.S; ++s) {
-    const float* q = L.Q[0] + rows(v, kQ, L.P) + s;
-    const double u = q[0], w = q[L.P], p = q[2 * L.P];
-    const double V5 = q[4 * L.P];
+// sum of squared deviations (the per-group recurrence of increment_moments,
+// src/fv.cc:595-694) and a Kahan-compensated sum of squares.  A warp per vertex, its lanes
+// over the samples, so that a row is read once, coalesced, for every component; the lanes'
+// equal groups are merged pairwise by reduce_moments' rule (src/reduce_moments.cc:36-113).
+// One thread per component and vertex read a sector per sample, twice the divisions and
+// every row once per component: 5.62 -> 1.09 ms on 768 samples of 257^2 with every extra.
+// Bound by FP64 arithmetic (two logarithms, two roots and four divisions a sample); the rows
+// alone would take 0.12 ms.  Record layout as
+// tg_moments_*: PrimVar (T, p, u, v, w), then density, mach, entropy by EX's bits, in the
+// caller's vertex order.
+template <int EX>
+__global__ void __launch_bounds__(256) kb_moments(Level L, BParams k, const int* __restrict__ old_of_new,
+                                                  double* __restrict__ fm, double* __restrict__ sm,
+                                                  double* __restrict__ m2) {
+  constexpr int NX = 4 + (EX & 1) + ((EX >> 1) & 1) + ((EX >> 2) & 1);    // without w
+  const int v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (v >= L.m.nv) return;
+  const int P = L.P;
+  double mean[NX], ssd[NX], sq[NX], comp[NX];
+#pragma unroll
+  for (int c = 0; c < NX; ++c) mean[c] = ssd[c] = sq[c] = comp[c] = 0.0;
+  const float* row = L.Q[0] + rows(v, kQ, P) + lane;
+  const int n = L.S >> 5;
+  for (int i = 0; i < n; ++i, row += 32) {
+    const double u = row[0], w = row[P], p = row[2 * P], V5 = row[4 * P];
     const double rho = -V5 * p;
-    double x;
-    switch (kind) {
-      case 0: x = p / ((double)k.R * rho); break;
-      case 1: x = p; break;
-      case 2: x = u; break;
-      case 3: x = w; break;
-      case 4: x = 0.0; break;
-      case 5: x = rho; break;
-      case 6: x = sqrt(u * u + w * w) / sqrt((double)k.gamma * p / rho); break;
-      default: x = log(p) - (double)k.gamma * log(rho); break;
+    double x[NX];
+    x[0] = p / ((double)k.R * rho);
+    x[1] = p; x[2] = u; x[3] = w;
+    int j = 4;
+    if (EX & 1) x[j++] = rho;
+    if (EX & 2) x[j++] = sqrt(u * u + w * w) / sqrt((double)k.gamma * p / rho);
+    if (EX & 4) x[j++] = log(p) - (double)k.gamma * log(rho);
+    const double r = 1.0 / (double)(i + 1);
+#pragma unroll
+    for (int c = 0; c < NX; ++c) {
+      const double d = x[c] - mean[c];
+      mean[c] = i == 0 ? x[c] : mean[c] + d * r;
+      if (i > 0) ssd[c] += d * (x[c] - mean[c]);
+      const double y = x[c] * x[c] - comp[c];       // Kahan
+      const double t = sq[c] + y;
+      comp[c] = (t - sq[c]) - y;
+      sq[c] = t;
     }
-    const double kk = (double)(s + 1);
-    const double prev = mean;
-    mean = s == 0 ? x : (c < 5 ? x * (1.0 / kk) + prev * ((kk - 1.0) / kk) : prev + (x - prev) / kk);
-    if (s > 0) ssd += (x - prev) * (x - mean);
-    const double y = x * x - comp;       // Kahan
-    const double tsum = sq + y;
-    comp = (tsum - sq) - y;
-    sq = tsum;
   }
-  const size_t o = (size_t)c * L.m.nv + v;
-  fm[o] = mean;
-  sm[o] = sq;
-  m2[o] = ssd;
+  double cnt = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1, cnt *= 2.0)
+#pragma unroll
+    for (int c = 0; c < NX; ++c) {
+      const double mo = __shfl_xor_sync(0xffffffffu, mean[c], o), so = __shfl_xor_sync(0xffffffffu, ssd[c], o);
+      const double qo = __shfl_xor_sync(0xffffffffu, sq[c], o), co = __shfl_xor_sync(0xffffffffu, comp[c], o);
+      const double d = mo - mean[c];
+      mean[c] += 0.5 * d;
+      ssd[c] += so + d * d * (0.5 * cnt);
+      const double y = qo - (comp[c] + co), t = sq[c] + y;
+      comp[c] = (t - sq[c]) - y;
+      sq[c] = t;
+    }
+  if (lane == 0) {      // lane 0's merge order is fixed
+    const size_t o = (size_t)(NX + 1) * old_of_new[v];
+#pragma unroll
+    for (int c = 0; c <= NX; ++c) {
+      const int q = c < 4 ? c : c - 1;
+      fm[o + c] = c == 4 ? 0.0 : mean[q];
+      sm[o + c] = c == 4 ? 0.0 : sq[q];
+      m2[o + c] = c == 4 ? 0.0 : ssd[q];
+    }
+  }
 }
 
 // Per-sample integrals (FP64) of one level's current states, the
 // compute_global quantities (src/fv.cc:2186-2203) plus the vertical kinetic
 // energy: q0 = sum 0.5 rho v^2 A w, q1 = sum 0.5 rho u^2 A w,
 // q2 = sum -rho s / (gamma - 1) A w.  Block (sample group, vertex chunk);
-// partial[chunk][sample][3], summed over chunks in order by the host.
+// partial[chunk][sample][3], summed over chunks in order by kb_integrals_sum.
 template <int VT>
 __global__ void __launch_bounds__(32 * VT) kb_integrals(Level L, BParams k, int chunks, double* __restrict__ partial) {
   const int lane = threadIdx.x & 31, vg = threadIdx.x >> 5;
@@ -1681,6 +1714,15 @@ __global__ void __launch_bounds__(32 * VT) kb_integrals(Level L, BParams k, int 
 #pragma unroll
     for (int c = 0; c < 3; ++c) partial[((size_t)ch * L.S + s) * 3 + c] = q[c];
   }
+}
+
+__global__ void kb_integrals_sum(int n, int chunks, const double* __restrict__ partial, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double acc = 0.0;
+#pragma unroll 8
+  for (int ch = 0; ch < chunks; ++ch) acc += partial[(size_t)ch * n + i];
+  out[i] = acc;
 }
 
 }  // namespace batch

@@ -904,6 +904,16 @@ __global__ void k_moments_increment(Params k, int nv, StateView s, int extras, i
   }
 }
 
+// The three moment arrays [nvar][nv] of an instance -> [vertex][nvar] in the caller's order.
+__global__ void k_moments_out(int nv, int nvar, const double* __restrict__ mom, const int* __restrict__ old_of_new,
+                              double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nv) return;
+  const size_t n = (size_t)nvar * nv * blockIdx.y;
+  double* o = out + n + (size_t)nvar * old_of_new[i];
+  for (int c = 0; c < nvar; ++c) o[c] = mom[n + (size_t)c * nv + i];
+}
+
 // One received group of reduce_moments (src/reduce_moments.cc:36-113).
 __global__ void k_moments_merge(size_t n, double fact1, double fact2, double* __restrict__ fm,
                                 double* __restrict__ sm, double* __restrict__ m2, const double* __restrict__ fo,

@@ -151,34 +151,51 @@ std::string build_layout(const tg_mesh& m, const tg_bc_table* bc, bool need_visc
   std::vector<double> fnrm(m.face_normal, m.face_normal + 2 * (size_t)nf);
   std::vector<int> flc(m.face_lcell, m.face_lcell + nf), frc(m.face_rcell, m.face_rcell + nf);
   {
-    auto pkey = [](int a, int b) { return ((uint64_t)(uint32_t)std::min(a, b) << 32) | (uint32_t)std::max(a, b); };
-    std::unordered_map<uint64_t, int> seen;
-    seen.reserve(2 * (size_t)nf);
-    for (int f = 0; f < nf; ++f) seen.emplace(pkey(m.face_vertex[2 * f], m.face_vertex[2 * f + 1]), -1);
+    // faces by their lower vertex; an edge that is none of them is found by a cell
+    std::vector<int> off(nv + 1, 0), other(nf);
+    for (int f = 0; f < nf; ++f) ++off[std::min(m.face_vertex[2 * f], m.face_vertex[2 * f + 1]) + 1];
+    for (int i = 0; i < nv; ++i) off[i + 1] += off[i];
+    {
+      std::vector<int> at(off.begin(), off.end() - 1);
+      for (int f = 0; f < nf; ++f) {
+        const int a = m.face_vertex[2 * f], b = m.face_vertex[2 * f + 1];
+        other[at[std::min(a, b)]++] = std::max(a, b);
+      }
+    }
+    std::unordered_map<uint64_t, int> extra;
     for (int c = 0; c < nc; ++c)
       for (int k = 0; k < 3; ++k) {
         const int a = m.cell_vertex[3 * c + k], b = m.cell_vertex[3 * c + (k + 1) % 3];
-        auto it = seen.find(pkey(a, b));
-        if (it == seen.end()) {
-          seen.emplace(pkey(a, b), (int)flc.size());
+        const int lo = std::min(a, b), hi = std::max(a, b);
+        bool face = false;
+        if (lo >= 0 && lo < nv)
+          for (int j = off[lo]; j < off[lo + 1] && !face; ++j) face = other[j] == hi;
+        if (face) continue;
+        auto [it, fresh] = extra.emplace(((uint64_t)(uint32_t)lo << 32) | (uint32_t)hi, (int)flc.size());
+        if (fresh) {
           fvx.push_back(a); fvx.push_back(b);
           fnrm.push_back(0.0); fnrm.push_back(0.0);
           flc.push_back(c); frc.push_back(-1);
-        } else if (it->second >= 0) {
+        } else {
           frc[it->second] = c;
         }
       }
   }
   const int nfa = (int)flc.size();
+  // edges by their lower, then their higher vertex in device order, ties in face order: buckets
+  // of the lower vertex
   std::vector<int> eorder(nfa);
-  std::iota(eorder.begin(), eorder.end(), 0);
-  auto lo = [&](int f) { return std::min(N[fvx[2 * f]], N[fvx[2 * f + 1]]); };
-  auto hi = [&](int f) { return std::max(N[fvx[2 * f]], N[fvx[2 * f + 1]]); };
-  std::stable_sort(eorder.begin(), eorder.end(), [&](int a, int b) {
-    int la = lo(a), lb = lo(b);
-    if (la != lb) return la < lb;
-    return hi(a) < hi(b);
-  });
+  {
+    std::vector<int> off(nv + 1, 0);
+    auto lo = [&](int f) { return std::min(N[fvx[2 * f]], N[fvx[2 * f + 1]]); };
+    auto hi = [&](int f) { return std::max(N[fvx[2 * f]], N[fvx[2 * f + 1]]); };
+    for (int f = 0; f < nfa; ++f) ++off[lo(f) + 1];
+    for (int i = 0; i < nv; ++i) off[i + 1] += off[i];
+    std::vector<int> at(off.begin(), off.end() - 1);
+    for (int f = 0; f < nfa; ++f) eorder[at[lo(f)]++] = f;
+    for (int i = 0; i < nv; ++i)
+      std::stable_sort(eorder.begin() + off[i], eorder.begin() + off[i + 1], [&](int a, int b) { return hi(a) < hi(b); });
+  }
   L.ne = nfa;
   L.e_a.resize(nfa); L.e_b.resize(nfa); L.e_face.resize(nfa);
   L.e_nx.resize(nfa); L.e_ny.resize(nfa); L.e_dx.resize(nfa); L.e_dy.resize(nfa);
@@ -221,25 +238,33 @@ std::string build_layout(const tg_mesh& m, const tg_bc_table* bc, bool need_visc
   };
 
   // per reference vertex incident edges (in edge order)
-  std::vector<std::vector<int>> inc(nv);
+  std::vector<int> inc_off(nv + 1, 0), inc(2 * (size_t)nfa);
   for (int e = 0; e < nfa; ++e) {
-    inc[fvx[2 * L.e_face[e]]].push_back(e << 1);
-    inc[fvx[2 * L.e_face[e] + 1]].push_back((e << 1) | 1);
+    ++inc_off[fvx[2 * L.e_face[e]] + 1];
+    ++inc_off[fvx[2 * L.e_face[e] + 1] + 1];
+  }
+  for (int i = 0; i < nv; ++i) inc_off[i + 1] += inc_off[i];
+  {
+    std::vector<int> at(inc_off.begin(), inc_off.end() - 1);
+    for (int e = 0; e < nfa; ++e) {
+      inc[at[fvx[2 * L.e_face[e]]]++] = e << 1;
+      inc[at[fvx[2 * L.e_face[e] + 1]]++] = (e << 1) | 1;
+    }
   }
   L.ce_off.assign(nv + 1, 0);
   std::vector<int> g;
   for (int i = 0; i < nv; ++i) {
     group(L.old_of_new[i], g);
-    size_t cnt = 0;
-    for (int o : g) cnt += inc[o].size();
-    L.ce_off[i + 1] = L.ce_off[i] + (int)cnt;
+    int cnt = 0;
+    for (int o : g) cnt += inc_off[o + 1] - inc_off[o];
+    L.ce_off[i + 1] = L.ce_off[i] + cnt;
   }
   L.ce_ent.resize(L.ce_off[nv]);
   for (int i = 0; i < nv; ++i) {
     group(L.old_of_new[i], g);
     int p = L.ce_off[i];
     for (int o : g)
-      for (int x : inc[o]) L.ce_ent[p++] = x;
+      for (int j = inc_off[o]; j < inc_off[o + 1]; ++j) L.ce_ent[p++] = inc[j];
   }
 
   // ---- non-periodic boundary faces

@@ -1,0 +1,142 @@
+// tg_stage.h -- copies between pageable caller buffers and the device.
+//
+// Up to kMaxLanes host threads, each with its own stream and two pinned kSlot slots, so that
+// the host memcpy of one slot (and the page faults of a buffer that is touched for the first
+// time) overlaps the DMA of the other and the other lanes'.  Pinned caller buffers need none
+// of it: one cudaMemcpyAsync.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+#include <system_error>
+#include <thread>
+#include <vector>
+
+namespace tg {
+
+inline bool host_pinned(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+struct Stager {
+  static constexpr int kMaxLanes = 8;
+  static constexpr size_t kSlot = size_t(512) << 10, kPerLane = 2 * kSlot;
+  int device = 0, lanes = 0;
+  char* slots = nullptr;   // pinned, lanes * 2 * kSlot bytes
+  cudaStream_t st[kMaxLanes] = {};
+  cudaEvent_t ev[kMaxLanes][2] = {};
+
+  static int lanes_for(size_t bytes) {
+    return (int)std::max<size_t>(1, std::min<size_t>(kMaxLanes, bytes / kPerLane));
+  }
+  // lanes for transfers of up to `bytes`; a later call may ask for more
+  cudaError_t init(int dev, size_t bytes) {
+    device = dev;
+    const int want = lanes_for(bytes);
+    if (want <= lanes) return cudaSuccess;
+    release();
+    cudaError_t e = cudaMallocHost((void**)&slots, (size_t)want * kPerLane);
+    for (int t = 0; t < want && e == cudaSuccess; ++t) {
+      e = cudaStreamCreateWithFlags(&st[t], cudaStreamNonBlocking);
+      for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ev[t][k], cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) lanes = want;
+    else release();
+    return e;
+  }
+  void release() {
+    for (int t = 0; t < kMaxLanes; ++t) {
+      if (st[t]) cudaStreamSynchronize(st[t]);
+      for (int k = 0; k < 2; ++k) {
+        if (ev[t][k]) cudaEventDestroy(ev[t][k]);
+        ev[t][k] = nullptr;
+      }
+      if (st[t]) cudaStreamDestroy(st[t]);
+      st[t] = nullptr;
+    }
+    if (slots) cudaFreeHost(slots);
+    slots = nullptr;
+    lanes = 0;
+  }
+  char* slot(int lane, int k) const { return slots + (2 * (size_t)lane + k) * kSlot; }
+
+  // One lane of a host -> device copy of len bytes.
+  cudaError_t lane_in(int lane, char* dst, const char* src, size_t len) const {
+    cudaError_t e = cudaSetDevice(device);
+    for (size_t off = 0, k = 0; e == cudaSuccess && off < len; off += kSlot, ++k) {
+      const int s = (int)(k & 1);
+      const size_t n = std::min(kSlot, len - off);
+      if (k >= 2 && (e = cudaEventSynchronize(ev[lane][s])) != cudaSuccess) break;
+      std::memcpy(slot(lane, s), src + off, n);
+      if ((e = cudaMemcpyAsync(dst + off, slot(lane, s), n, cudaMemcpyHostToDevice, st[lane])) != cudaSuccess) break;
+      e = cudaEventRecord(ev[lane][s], st[lane]);
+    }
+    cudaError_t e2 = cudaStreamSynchronize(st[lane]);
+    return e != cudaSuccess ? e : e2;
+  }
+
+  // One lane of a device -> host copy; the lane's stream first waits for `ready`.
+  cudaError_t lane_out(int lane, char* dst, const char* src, size_t len, cudaEvent_t ready) const {
+    cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st[lane], ready, 0);
+    const size_t nk = (len + kSlot - 1) / kSlot;
+    auto issue = [&](size_t k) {
+      const int s = (int)(k & 1);
+      const size_t n = std::min(kSlot, len - k * kSlot);
+      cudaError_t ei = cudaMemcpyAsync(slot(lane, s), src + k * kSlot, n, cudaMemcpyDeviceToHost, st[lane]);
+      return ei != cudaSuccess ? ei : cudaEventRecord(ev[lane][s], st[lane]);
+    };
+    for (size_t k = 0; e == cudaSuccess && k < std::min<size_t>(2, nk); ++k) e = issue(k);
+    for (size_t k = 0; e == cudaSuccess && k < nk; ++k) {
+      const int s = (int)(k & 1);
+      if ((e = cudaEventSynchronize(ev[lane][s])) != cudaSuccess) break;
+      std::memcpy(dst + k * kSlot, slot(lane, s), std::min(kSlot, len - k * kSlot));
+      if (k + 2 < nk) e = issue(k + 2);
+    }
+    cudaError_t e2 = cudaStreamSynchronize(st[lane]);
+    return e != cudaSuccess ? e : e2;
+  }
+
+  // Splits a copy over the lanes (lane 0 on the calling thread; where no thread is to be had,
+  // the calling one does the rest).
+  template <class Lane>
+  cudaError_t run(size_t bytes, Lane lane) const {
+    const int n = std::min(lanes, lanes_for(bytes));
+    const size_t per = ((bytes + n - 1) / n + 255) & ~size_t(255);
+    cudaError_t errs[kMaxLanes] = {};
+    std::thread th[kMaxLanes];
+    auto work = [&](int t) {
+      const size_t off = t * per;
+      if (off < bytes) errs[t] = lane(t, off, std::min(per, bytes - off));
+    };
+    int started = 1;
+    try {
+      for (; started < n; ++started) th[started] = std::thread(work, started);
+    } catch (const std::system_error&) {
+    }
+    work(0);
+    for (int t = started; t < n; ++t) work(t);
+    for (int t = 1; t < started; ++t) th[t].join();
+    for (cudaError_t e : errs)
+      if (e != cudaSuccess) return e;
+    return cudaSuccess;
+  }
+
+  cudaError_t in(void* dst, const void* src, size_t bytes) const {
+    return run(bytes, [&](int t, size_t off, size_t len) { return lane_in(t, (char*)dst + off, (const char*)src + off, len); });
+  }
+  cudaError_t out(void* dst, const void* src, size_t bytes, cudaEvent_t ready) const {
+    return run(bytes, [&](int t, size_t off, size_t len) {
+      return lane_out(t, (char*)dst + off, (const char*)src + off, len, ready);
+    });
+  }
+};
+
+}  // namespace tg
