@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
     __syncthreads();
     if (FLUX == FLUX_ROE_EC || k.strong) {
       for (int i = tid; i < R.L(); i += kTileThreads) {
-        if (FLUX == FLUX_ROE_EC) s1[i] = sqrt(-sB[i].y);
+        if (FLUX == FLUX_ROE_EC) s1[i] = sqrt_nr(-sB[i].y);
         const int g = k.strong ? local_vertex(t, R, i) : 0;
         if (k.strong && (m.sflag[g] & 1)) {
           // a strong condition reset this vertex's primitive state but not its entropy
