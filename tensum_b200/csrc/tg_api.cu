@@ -46,9 +46,9 @@ struct tg_handle {
   double* Tb[3] = {nullptr, nullptr, nullptr};
   double* V1b[3] = {nullptr, nullptr, nullptr};
   double2* W23b[3] = {nullptr, nullptr, nullptr};
-  size_t smem_grad = 0, smem_flux = 0;
+  size_t smem_grad = 0, smem_flux[3] = {0, 0, 0};   // flux: by mode
   bool pdl = false;            // a step's kernels are dependent launches (pdl_wait)
-  int grid_grad = 1, grid_flux = 1, grid_res = 1;   // CTAs that fill the chip once (the kernels walk tiles)
+  int grid_grad = 1, grid_flux[3] = {1, 1, 1};   // CTAs that fill the chip once (the kernels walk tiles)
   Scalars* sc = nullptr;       // device
   int* done = nullptr;         // device flag written by k_step_begin
   int* never = nullptr;        // device zero, used by single-phase calls
@@ -266,7 +266,9 @@ cudaError_t raise_smem(const void* f, size_t bytes) {
 }
 
 TileFluxKernel tile_kernel(int flux, int recon, int mode) {
-  return mode == MODE_UPDATE ? tile_kernel_m<MODE_UPDATE>(flux, recon) : tile_kernel_m<MODE_RESIDUAL>(flux, recon);
+  return mode == MODE_RESIDUAL ? tile_kernel_m<MODE_RESIDUAL>(flux, recon)
+         : mode == MODE_UPDATE ? tile_kernel_m<MODE_UPDATE>(flux, recon)
+                               : tile_kernel_m<MODE_LAST>(flux, recon);
 }
 
 // state view of buffer b (the three buffers rotate through the stages)
@@ -316,13 +318,15 @@ void enqueue_boundary(tg_handle* h, int b, const int* done, bool pdl = false) {
   if (h->viscous) launch(pdl, k_viscous, nblk(h->mv.nvu), kBlock, 0, h->stream, h->prm, h->mv, view(h, b), done);
 }
 
-void enqueue_tile_flux(tg_handle* h, int b, int mode, int r, bool norm, int bout, const int* done, int base = 0,
+void enqueue_tile_flux(tg_handle* h, int b, int mode, int r, int bout, const int* done, int base = 0,
                        int count = -1, bool pdl = false) {
+  const int norm = mode == MODE_LAST;
+  if (mode == MODE_UPDATE && h->prm.flux == FLUX_TECNO_ROE) mode = MODE_LAST;
   TileView v;
-  const int grid = tiles(h, base, count, mode == MODE_UPDATE ? h->grid_flux : h->grid_res, &v);
+  const int grid = tiles(h, base, count, h->grid_flux[mode], &v);
   if (grid == 0) return;
-  launch(pdl, tile_kernel(h->prm.flux, h->prm.recon, mode), grid, kTileThreads, h->smem_flux, h->stream, h->prm, h->mv,
-         v, view(h, b), h->ctl, h->sc, r, norm ? 1 : 0, view(h, bout), h->L.lmax, h->L.emax, h->L.cmax, done);
+  launch(pdl, tile_kernel(h->prm.flux, h->prm.recon, mode), grid, kTileThreads, h->smem_flux[mode], h->stream, h->prm,
+         h->mv, v, view(h, b), h->ctl, h->sc, r, norm, view(h, bout), h->L.lmax, h->L.emax, h->L.cmax, done);
 }
 
 // Inviscid central-flux steps without strong conditions leave V1 unformed (w3_only in
@@ -349,7 +353,7 @@ int residual_kernels(const tg_handle* h) {
 void enqueue_residual(tg_handle* h, const int* done) {
   enqueue_gradient(h, 0, done);
   enqueue_boundary(h, 0, done);
-  enqueue_tile_flux(h, 0, MODE_RESIDUAL, 0, false, 0, done);
+  enqueue_tile_flux(h, 0, MODE_RESIDUAL, 0, 0, done);
 }
 
 // compute_ssw follows compute_dt in FiniteVolume::solve (src/fv.cc:2282-2285)
@@ -395,7 +399,7 @@ void enqueue_step(tg_handle* h, bool warm) {
     if (first) enqueue_ssw(h, h->done);
     if (h->grads_needed) enqueue_gradient(h, bin, h->done, 0, -1, h->pdl);
     enqueue_boundary(h, bin, h->done, h->pdl);
-    enqueue_tile_flux(h, bin, MODE_UPDATE, r, last, bout, h->done, 0, -1, h->pdl);
+    enqueue_tile_flux(h, bin, last ? MODE_LAST : MODE_UPDATE, r, bout, h->done, 0, -1, h->pdl);
     if (h->prm.strong && h->mv.nsb > 0)
       launch(h->pdl, k_strong_bc, nblk(h->mv.nsb), kBlock, 0, h->stream, h->mv, view(h, bout), h->done);
   }
@@ -544,7 +548,7 @@ void enqueue_phase(tg_handle* h, int phase) {
     case TG_PHASE_GRADIENT: enqueue_gradient(h, 0, h->never); break;
     case TG_PHASE_FLUX:
       enqueue_boundary(h, 0, h->never);
-      enqueue_tile_flux(h, 0, MODE_RESIDUAL, 0, false, 0, h->never);
+      enqueue_tile_flux(h, 0, MODE_RESIDUAL, 0, 0, h->never);
       break;
     case TG_PHASE_UPDATE: enqueue_update(h, 1, false, h->never); break;
     case TG_PHASE_DT: enqueue_dt(h, h->never); break;
@@ -797,14 +801,16 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   h->sv.S0 = h->Sb[0];
   h->sv.T0 = h->Tb[0];
   h->smem_grad = tile_grad_smem(L.lmax, L.cmax);
-  h->smem_flux = flux_smem(mat->flux_scheme, mat->reconstruct_scheme, L.lmax, L.emax, L.cmax, k.fuse_dt);
   {
+    const int modes[3] = {MODE_RESIDUAL, MODE_UPDATE, MODE_LAST};
     cudaError_t ea = raise_smem((const void*)k_tile_grad, h->smem_grad);
-    cudaError_t ec = raise_smem((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_UPDATE),
-                                h->smem_flux);
-    cudaError_t ed = raise_smem((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_RESIDUAL),
-                                h->smem_flux);
-    if (ea != cudaSuccess || ec != cudaSuccess || ed != cudaSuccess) {
+    for (int mode : modes) {
+      h->smem_flux[mode] = flux_smem(mat->flux_scheme, mat->reconstruct_scheme, L.lmax, L.emax, L.cmax,
+                                     mode == MODE_LAST && k.fuse_dt);
+      if (ea == cudaSuccess)
+        ea = raise_smem((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, mode), h->smem_flux[mode]);
+    }
+    if (ea != cudaSuccess) {
       tg_destroy(h);
       return fail(nullptr, TG_CUDA_ERROR, "tile kernels need more shared memory than the device allows");
     }
@@ -814,14 +820,15 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
       return per * sms;
     };
     h->grid_grad = fill((const void*)k_tile_grad, h->smem_grad);
-    h->grid_flux = fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_UPDATE), h->smem_flux);
+    for (int mode : modes)
+      h->grid_flux[mode] =
+          fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, mode), h->smem_flux[mode]);
     // Dependent launches where the passes of a step fill the chip at most once, or where no
     // gradient pass alternates with the flux pass.  Past that the early CTAs of one pass
     // between the last ones of the other leave register holes too small for its fourth
     // CTA per SM, and a round more (TeCNO-Rusanov on 1025^2 671 -> 1027 us, 513^2 209 -> 241;
     // one round: 65^2 46 -> 40, the 128 x 256 cylinder 131 -> 116; KEPEC 387^2 55 -> 51).
-    h->pdl = L.ntiles <= h->grid_flux || !h->grads_needed;
-    h->grid_res = fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, MODE_RESIDUAL), h->smem_flux);
+    h->pdl = L.ntiles <= h->grid_flux[MODE_LAST] || !h->grads_needed;
   }
   if ((st = dev_alloc(h, 1, &h->sc)) != TG_OK) { tg_destroy(h); return st; }
   if ((st = dev_alloc(h, 1, &h->done)) != TG_OK) { tg_destroy(h); return st; }
@@ -1619,7 +1626,7 @@ tg_status tg_part_flux(tg_handle* h, int r, int which) {
   // boundary-face sides depend only on their own vertex's state: the faces are formed with
   // the interior (or all) tiles, and the frontier tiles, launched after, gather them too
   if (which != TG_TILES_FRONTIER) enqueue_boundary(h, bin, h->done);
-  enqueue_tile_flux(h, bin, MODE_UPDATE, r, last, bout, h->done, base, count);
+  enqueue_tile_flux(h, bin, last ? MODE_LAST : MODE_UPDATE, r, bout, h->done, base, count);
   if (which != TG_TILES_INTERIOR) {
     h->part.cur = bout;
     if (last) h->part.norms_pending = true;

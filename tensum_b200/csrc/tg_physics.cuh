@@ -526,6 +526,15 @@ __device__ __forceinline__ Flx num_flux_unit(const Params& k, const VRec& L, con
   return F;
 }
 
+// The central fluxes are linear in the normal, so n itself serves: no |n|, no unit normal.
+template <int FLUX>
+__device__ __forceinline__ Flx central_flux(const Params& k, const VRec& L, const VRec& R, double nx, double ny) {
+  if (FLUX == FLUX_KEPEC) return kepec_flux(k, L, R, nx, ny);
+  if (FLUX == FLUX_KEP) return kep_flux(k, L, R, nx, ny);
+  if (FLUX == FLUX_ROE_EC) return roe_ec_flux(k, L, R, nx, ny);
+  return avg_flux(k, L, R, nx, ny);
+}
+
 template <int FLUX, int RECON>
 __device__ __forceinline__ Flx num_flux(const Params& k, const VRec& L, const VRec& R, double nx, double ny, double dx,
                                         double dy, const double* dEl, const double* dEr) {

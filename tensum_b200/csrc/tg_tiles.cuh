@@ -38,12 +38,17 @@
 // more registers win: KH 1025^2 steps of TeCNO-Rusanov / KEPEC / KEP in us with
 // (TeCNO, central, gradient) CTAs (4, 7, 7): 732 / 274 / 246, (4, 6, 5): 678 / 256 / 246,
 // (4, 5, 6): 724 / 271 / 264, (3, 5, 5): 706 / 271 / 266; gradient pass 78 / 68 / 60 / 59 us
-// with 7 (spills) / 3 / 5 / 4.
+// with 7 (spills) / 3 / 5 / 4.  Since then, the central fluxes' normals staged, CTAs of a
+// step's earlier / last updates 6 / 6, 6 / 5, 5 / 5: KEPEC 240 / 227 / 243, KEP 236 / 234 / 236,
+// Roe-EC 259 / 248 / 251.
 #ifndef TG_FLUX_MINB
 #define TG_FLUX_MINB 4
 #endif
 #ifndef TG_FLUX_MINB_CENTRAL
 #define TG_FLUX_MINB_CENTRAL 6
+#endif
+#ifndef TG_FLUX_MINB_CENTRAL_LAST
+#define TG_FLUX_MINB_CENTRAL_LAST 5
 #endif
 #ifndef TG_GRAD_MINB
 #define TG_GRAD_MINB 5
@@ -257,7 +262,17 @@ __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
 }
 
 // --------------------------------------------------------------------- fluxes
-enum : int { MODE_RESIDUAL = 0, MODE_UPDATE = 1 };
+// MODE_LAST is a step's last update: it also forms the residual norm and the next local time
+// step.  It is a kernel of its own, except for TeCNO-Roe, whose every update runs it (norm
+// tells the last one): without that code the others spill less, but Roe's earlier stages
+// come out slower.  Steps on 1025^2 in us, one kernel / two: TeCNO-Rusanov 651 / 638, KEPEC
+// 246 / 227, Roe-EC 261 / 248 (both with the staged normals), TeCNO-Roe 657 / 677.
+enum : int { MODE_RESIDUAL = 0, MODE_UPDATE = 1, MODE_LAST = 2 };
+template <int FLUX>
+__host__ __device__ constexpr bool own_last() {
+  return FLUX != FLUX_TECNO_ROE;
+}
+
 
 template <int FLUX>
 __host__ __device__ constexpr bool is_tecno() {
@@ -327,7 +342,8 @@ __device__ __forceinline__ void block_sum4_min(double* x, unsigned long long& lo
 // Shared-memory layout of k_tile_flux, in bytes (host and device agree on it).
 template <int FLUX, int RECON>
 struct FluxSmem {
-  size_t xy, g, f, n, single, list, ssw, bytes;
+  size_t xy, g, f, n, ab, single, list, ssw, bytes;
+  static constexpr bool kStage = !is_tecno<FLUX>();
   __host__ __device__ FluxSmem(int lmax, int emax, int cmax, bool dt) {
     size_t o = 2 * (size_t)lmax * sizeof(double2);            // (u, v), (p, V5)
     g = o;
@@ -336,8 +352,10 @@ struct FluxSmem {
     if (flux_needs_grad<FLUX, RECON>()) o += (size_t)lmax * sizeof(double2);
     f = o;                                                    // (mass, x), (y, energy) per edge
     o += 2 * (size_t)emax * sizeof(double2);
-    n = o;                                                    // normals (runs that fuse dt)
-    if (dt) o += (size_t)emax * sizeof(double2);
+    n = o;                                                    // normals (TeCNO: where dt is fused)
+    if (dt || kStage) o += (size_t)emax * sizeof(double2);
+    ab = o;                                                   // central fluxes: endpoints
+    if (kStage) o += (((size_t)emax + 3) & ~(size_t)3) * sizeof(unsigned int);
     list = o;                                                 // gather lists, two buffers
     o += 2 * (size_t)cmax * sizeof(unsigned short);
     single = o;
@@ -350,14 +368,23 @@ struct FluxSmem {
 };
 
 template <int FLUX, int RECON, int MODE>
-__global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB : TG_FLUX_MINB_CENTRAL)
-    k_tile_flux(Params k, MeshView m, TileView t, StateView s, Control ctl, Scalars* sc, int r, int do_norm,
+__global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>()    ? TG_FLUX_MINB
+                                                : MODE == MODE_LAST ? TG_FLUX_MINB_CENTRAL_LAST
+                                                                    : TG_FLUX_MINB_CENTRAL)
+    k_tile_flux(Params k, MeshView m, TileView t, StateView s, Control ctl, Scalars* sc, int r, int norm,
                 StateView out, int lmax, int emax, int cmax, const int* __restrict__ done) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool kGrad = flux_needs_grad<FLUX, RECON>();
+  // The central fluxes are short and linear in the normal: a tile's normals (no |n|) and
+  // endpoints are copied with its records, 20 bytes an edge instead of 28, and the next dt
+  // finds them there.  The TeCNO fluxes leave no shared memory for that and read an edge
+  // ahead into registers.
+  constexpr bool kStage = !is_tecno<FLUX>();
   constexpr bool kRoe = (FLUX == FLUX_TECNO_ROE);
+  constexpr bool kUpdate = MODE != MODE_RESIDUAL;
+  const bool do_norm = MODE == MODE_LAST && (own_last<FLUX>() || norm);
   const int nv = m.nv, tid = threadIdx.x;
-  const FluxSmem<FLUX, RECON> lay(lmax, emax, cmax, k.fuse_dt);
+  const FluxSmem<FLUX, RECON> lay(lmax, emax, cmax, MODE == MODE_LAST && k.fuse_dt);
   double2* sA = reinterpret_cast<double2*>(smem);
   double2* sB = sA + lmax;
   double2* sG = reinterpret_cast<double2*>(smem + lay.g);              // 4 * lmax
@@ -365,6 +392,7 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
   double2* sF = reinterpret_cast<double2*>(smem + lay.f);
   double2* sF2 = sF + emax;
   double2* sN = reinterpret_cast<double2*>(smem + lay.n);
+  unsigned int* sAB = reinterpret_cast<unsigned int*>(smem + lay.ab);
   double* s1 = reinterpret_cast<double*>(smem + lay.single);
   unsigned short* sC = reinterpret_cast<unsigned short*>(smem + lay.list);
   int* sS = reinterpret_cast<int*>(smem + lay.ssw);                    // Liou switch of the local vertices
@@ -385,20 +413,28 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
     }
     if (kRoe && k.liou) cp_async4(sS + i, s.ssw + g);
   };
-  // copies a tile's vertex records (global ids of the thread's first two given) and lists
+  auto stage_normals = [&](const TileRec& T) {
+    for (int le = tid; le < T.NE; le += kTileThreads) cp_async16(sN + le, t.n + T.e0 + le);
+  };
+  // copies a tile's vertex records (global ids of the thread's first two given), endpoints
+  // and lists
   auto stage = [&](const TileRec& T, int g0, int g1, int buf) {
+    if (kStage)
+      for (int le = tid; le < T.NE; le += kTileThreads) cp_async4(sAB + le, t.ab + T.e0 + le);
     if (tid < T.L()) stage_vertex(tid, g0);
     if (tid + kTileThreads < T.L()) stage_vertex(tid + kTileThreads, g1);
     for (int i = tid + 2 * kTileThreads; i < T.L(); i += kTileThreads) stage_vertex(i, local_vertex(t, T, i));
     unsigned short* c = sC + (size_t)buf * cmax;
     for (int i = tid; 8 * i < (T.nent & ~kTileBnd); i += kTileThreads) cp_async16(c + 8 * i, t.cent + T.cb + 8 * i);
-    cp_async_commit();
+    if (!kStage) cp_async_commit();
   };
   {
     const int g0 = local_vertex(t, R, tid), g1 = local_vertex(t, R, tid + kTileThreads);
+    if (kStage) stage_normals(R);
     pdl_wait();
     const int stop = *done;
     stage(R, g0, g1, 0);
+    if (kStage) cp_async_commit();
     if (stop) {
       cp_async_wait<0>();
       return;
@@ -406,21 +442,21 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
   }
 
   // last stage with fuse_dt: the next step's local dt from the new state
-  const bool next_dt = MODE == MODE_UPDATE && do_norm && k.fuse_dt;
+  const bool next_dt = do_norm && k.fuse_dt;
   double nrm[4] = {0.0, 0.0, 0.0, 0.0};
   unsigned long long dbits = 0x7ff0000000000000ull;
-  const double dtg = MODE == MODE_UPDATE && (ctl.time_mode == 1 || ctl.time_step > 0.0) ? sc->dt_global : 0.0;
+  const double dtg = kUpdate && (ctl.time_mode == 1 || ctl.time_step > 0.0) ? sc->dt_global : 0.0;
 
   for (int buf = 0;; buf ^= 1) {
     at += gridDim.x;
     const bool more = at < t.count;
     const TileRec N = more ? load_rec(t, at) : R;
     const int e0 = R.e0, NE = R.NE;
-    // the thread's first edge and its list's range, read while the copies are in flight
+    // the thread's first edge (TeCNO) and its list's range, read while the copies are in flight
     double2 un = make_double2(0.0, 0.0);
     double ar = 0.0;
     unsigned ab = 0;
-    if (tid < NE) { un = t.u[e0 + tid]; ar = t.ar[e0 + tid]; ab = t.ab[e0 + tid]; }
+    if (!kStage && tid < NE) { un = t.u[e0 + tid]; ar = t.ar[e0 + tid]; ab = t.ab[e0 + tid]; }
     const bool own = tid < R.nown();
     const int v = R.vb + (own ? tid : 0);
     const unsigned short* rel = t.crel + R.rel;
@@ -448,11 +484,12 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
 
     // ---- edge fluxes
     for (int le = tid; le < NE; le += kTileThreads) {
+      if (kStage) ab = sAB[le];
       const int la = ab & 0xffff, lb = ab >> 16;
-      const double2 u = un;
+      const double2 u = kStage ? sN[le] : un;
       const double area = ar;
       const int nx = le + kTileThreads;
-      if (nx < NE) { un = t.u[e0 + nx]; ar = t.ar[e0 + nx]; ab = t.ab[e0 + nx]; }
+      if (!kStage && nx < NE) { un = t.u[e0 + nx]; ar = t.ar[e0 + nx]; ab = t.ab[e0 + nx]; }
       const VRec A = load_vrec<FLUX>(sA, sB, s1, la), B = load_vrec<FLUX>(sA, sB, s1, lb);
       double gl[8], gr[8], dx = 0.0, dy = 0.0;
       if (kGrad) {
@@ -466,8 +503,9 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
         dx = xb.x - xa.x;
         dy = xb.y - xa.y;
       }
-      Flx F = num_flux_unit<FLUX, RECON>(k, A, B, u.x, u.y, area, dx, dy, gl, gr,
-                                         kRoe && k.liou ? sS[la] + sS[lb] : 0);
+      Flx F = kStage ? central_flux<FLUX>(k, A, B, u.x, u.y)
+                     : num_flux_unit<FLUX, RECON>(k, A, B, u.x, u.y, area, dx, dy, gl, gr,
+                                                  kRoe && k.liou ? sS[la] + sS[lb] : 0);
       if (k.axi) {   // residual[cl] += flux * r_f, residual[cr] -= flux * r_f (src/fv.cc:1095-1096)
         const double rf = t.r[e0 + le];
         F.m *= rf; F.x *= rf; F.y *= rf; F.e *= rf;
@@ -478,8 +516,8 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
     // what the update reads, in flight across the barrier; the vertex's own record is staged
     D4 q0{0.0, 0.0, 0.0, 0.0}, qo = q0;
     double ia = 0.0, w = 0.0, dtl = dtg;
-    const bool old = MODE == MODE_UPDATE && (ctl.scheme == 1 || r > 0);   // the stage adds U_old
-    if (MODE == MODE_UPDATE && own) {
+    const bool old = kUpdate && (ctl.scheme == 1 || r > 0);   // the stage adds U_old
+    if (kUpdate && own) {
       const double2 a = sA[tid], b = sB[tid];
       q0 = D4{a.x, a.y, b.x, b.y};
       if (old) qo = ld4(s.S0 + v);
@@ -488,11 +526,14 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
       if (!(ctl.time_mode == 1 || ctl.time_step > 0.0)) dtl = s.dt[v];
     }
     __syncthreads();
-    if (next_dt) {
+    if (!kStage && next_dt) {
       for (int le = tid; le < NE; le += kTileThreads) cp_async16(sN + le, t.n + e0 + le);
       cp_async_commit();
     }
-    if (more) stage(N, g0, g1, buf ^ 1);
+    if (more) {
+      stage(N, g0, g1, buf ^ 1);
+      if (kStage && !next_dt) stage_normals(N);
+    }
     else pdl_trigger();   // this late, the next pass starts behind the last update only
 
     // ---- owned vertices: fixed-order sum, then residual or RK update
@@ -527,7 +568,7 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
       }
       // strong conditions: compute_residual_norm zeroes the no-slip momentum residual
       // before the last stage's update (src/fv.cc:1805-1819)
-      if (MODE == MODE_UPDATE && do_norm && k.strong && (m.sflag[v] & 2)) { r1 = 0.0; r2 = 0.0; }
+      if (do_norm && k.strong && (m.sflag[v] & 2)) { r1 = 0.0; r2 = 0.0; }
       if (MODE == MODE_RESIDUAL) {
         s.R[v] = r0; s.R[nv + v] = r1; s.R[2 * nv + v] = r2; s.R[3 * nv + v] = r3;
       } else {
@@ -564,9 +605,11 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
     }
     if (next_dt) {
       // compute_dt (src/fv.cc:1499-1598) of the coming step, as k_dt forms it
-      if (more) cp_async_wait<1>();
-      else cp_async_wait<0>();
-      __syncthreads();
+      if (!kStage) {
+        if (more) cp_async_wait<1>();
+        else cp_async_wait<0>();
+        __syncthreads();
+      }
       if (own) {
         double lam = 0.0;
         for (int j = j0; j < j1; ++j) {
@@ -587,11 +630,16 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>() ? TG_FLUX_MINB 
         if (!(dtn > 0.0)) bits = 0x7ff0000000000000ull;
         dbits = bits < dbits ? bits : dbits;
       }
+      if (kStage && more) {
+        __syncthreads();      // the normals are read until here
+        stage_normals(N);
+      }
     }
     if (!more) break;
+    if (kStage) cp_async_commit();
     R = N;
   }
-  if (MODE == MODE_UPDATE && do_norm) {
+  if (do_norm) {
     block_sum4_min(nrm, dbits);
     __shared__ int last;
     if (tid == 0) {
