@@ -52,7 +52,7 @@ struct tg_batch {
   double* tinst = nullptr;
   int shape = 1;                 // index into kShapes (the usual winner of tg_batch_tune)
   bool bnd = false;              // walls / far field or Navier-Stokes: the boundary and viscous passes run
-  int dt_chunks = 1;
+  int dt_per = 1;                // vertices per block of the time step's pass: four blocks per SM
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraph_t graph = nullptr;
   std::vector<void*> allocs;
@@ -288,9 +288,9 @@ void enqueue_step(tg_batch* b) {
   const dim3 gs((max_samples(b) + 255) / 256, b->nlev);
   kb_step_begin<<<gs, 256, 0, b->stream>>>(B, b->prm);
   long long dt_blocks = 0;
-  for (int l = 0; l < b->nlev; ++l) dt_blocks += (long long)dt_groups(B.lev[l].S) * b->dt_chunks;
-  if (b->bnd) kb_dt<8, true><<<(unsigned)dt_blocks, 256, 0, b->stream>>>(B, b->prm, b->dt_chunks);
-  else kb_dt<8, false><<<(unsigned)dt_blocks, 256, 0, b->stream>>>(B, b->prm, b->dt_chunks);
+  for (int l = 0; l < b->nlev; ++l) dt_blocks += (long long)dt_groups(B.lev[l].S) * dt_chunks(B.lev[l].m.nv, b->dt_per);
+  if (b->bnd) kb_dt<8, true><<<(unsigned)dt_blocks, 256, 0, b->stream>>>(B, b->prm, b->dt_per);
+  else kb_dt<8, false><<<(unsigned)dt_blocks, 256, 0, b->stream>>>(B, b->prm, b->dt_per);
   kb_dt_final<<<gs, 256, 0, b->stream>>>(B, b->prm);
   FluxK fk = flux_kernel(b->prm.flux, b->prm.recon, b->shape);
   const unsigned fill = edge_grid(b, fk, sh.bs);
@@ -530,11 +530,11 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
   int inf = INT_MAX;
   cudaMemcpy(b->stop, &inf, sizeof(int), cudaMemcpyHostToDevice);
   // dt kernel: about four blocks per SM over all sample groups
-  long long groups = 0;
-  for (int l = 0; l < n_levels; ++l) groups += dt_groups(b->B.lev[l].S);
+  long long work = 0;
+  for (int l = 0; l < n_levels; ++l) work += dt_groups(b->B.lev[l].S) * (long long)b->B.lev[l].m.nv;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-  b->dt_chunks = (int)std::max<long long>(1, (4LL * sms + groups - 1) / groups);
+  b->dt_per = (int)std::max<long long>(1, (work + 4LL * sms - 1) / (4LL * sms));
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { tg_batch_destroy(b); return bfail(nullptr, TG_CUDA_ERROR, cudaGetErrorString(e)); }
   for (int l = 0; l < n_levels; ++l)
