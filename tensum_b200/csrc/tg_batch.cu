@@ -459,13 +459,23 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
                       (float)(side ? L.e_g1y[e] : L.e_g0y[e]), 0.0f};
       de[j] = DtRec{(float)L.e_nx[e], (float)L.e_ny[e], ed[e].ar, 0.0f};
     }
+    std::vector<UnitRec> un(L.nvu);
+    for (int u = 0; u < L.nvu; ++u) {
+      const int c = L.u_cell[u];
+      UnitRec& x = un[u];
+      for (int i = 0; i < 3; ++i) x.v[i] = L.c_v[3 * c + i];
+      x.cell = c | (L.c_bf_off[c + 1] > L.c_bf_off[c] ? kUnitBf : 0);
+      for (int i = 0; i < 6; ++i) x.n[i] = (float)L.c_n[6 * (size_t)c + i];
+      x.inv2a = (float)L.c_inv2a[c];
+      x.pad = 0.0f;
+    }
 #define BU(vec, field) \
     if ((st = bupload(b, vec, &m.field)) != TG_OK) { tg_batch_destroy(b); return st; }
     BU(ed, ed) BU(ge, ge) BU(de, de) BU(L.ce_off, ce_off) BU(L.ce_ent, ce_ent) BU(L.dcarea, area) BU(L.inv6mc, inv6mc) BU(visw, visw) BU(L.x, x) BU(L.y, y) BU(aw, aw)
     m.nb = L.nb; m.nvu = L.nvu; m.nic = L.n_int_cells;
     BU(L.b_v0, b_v0) BU(L.b_v1, b_v1) BU(L.b_kind, b_kind) BU(L.b_adiab, b_adiab) BU(L.b_nx, b_nx) BU(L.b_ny, b_ny)
     BU(L.cb_off, cb_off) BU(L.cb_ent, cb_ent)
-    BU(L.u_cell, u_cell) BU(L.c_v, c_v) BU(L.c_n, c_n) BU(L.c_inv2a, c_inv2a) BU(L.c_bf_off, c_bf_off) BU(L.c_bf, c_bf)
+    BU(un, un) BU(L.c_bf_off, c_bf_off) BU(L.c_bf, c_bf)
     BU(L.c_nbr_off, c_nbr_off) BU(L.c_nbr, c_nbr) BU(L.bf_face_nx, bf_nx) BU(L.bf_face_ny, bf_ny)
     BU(L.bf_face_v0, bf_v0) BU(L.bf_face_v1, bf_v1)
 #undef BU

@@ -46,6 +46,15 @@ struct EdgeRec {
   float dx, dy;                    // x_b - x_a
   float ar, pad;                   // |n|
 };
+// A viscous unit; its cell's vertices, normals and area were three dependent arrays (the
+// 128 x 256 cylinder, 128 samples: the pass 150 -> 131 us).
+struct UnitRec {
+  int v[3];                        // the cell's vertices
+  int cell;                        // the cell, kUnitBf set where it has boundary faces
+  float n[6];                      // its P1 normals
+  float inv2a, pad;                // 1 / (2 cell area)
+};
+constexpr int kUnitBf = 1 << 30;
 struct GradRec {
   int other;                       // the entry's other endpoint
   float gx, gy, pad;               // P1 gradient weights of this side
@@ -70,8 +79,7 @@ struct LevelMesh {
   const float *b_nx, *b_ny;
   const int *cb_off, *cb_ent;
   // viscous units: interior cells, then one boundary cell per boundary face
-  const int *u_cell, *c_v;         // cell of a unit; 3 vertices per cell
-  const float *c_n, *c_inv2a;      // 6 P1 normals per cell; 1 / (2 cell area)
+  const UnitRec* un;               // viscous units
   const int *c_bf_off, *c_bf;      // boundary faces with the cell on their left (gradient corrections)
   const int *c_nbr_off, *c_nbr;    // the cell's boundary faces in cell.face slot order
   const float *bf_nx, *bf_ny;      // face-list normal of a boundary face
@@ -718,7 +726,10 @@ __device__ __forceinline__ Item item_of_pair(const Batch& B, unsigned w, int lan
 // Kelvin-Helmholtz 257^2 / 128 of the 128 x 256 cylinder, 128-thread blocks: gather + update at
 // 512, 768, 1024 threads 13.2 / 2.05, 12.3 / 1.94, 12.1 / 1.94 (96 samples of 65^2 123, 121, 126
 // us); gradients of meshes with boundaries at 512, 768, 1024: 2.02, 1.93, 1.88; viscous units
-// at 512, 768: 2.17, 1.99.
+// at 512, 768: 2.17, 1.99.  Since then, a unit's mesh data one record and the next boundary or
+// viscous entry's rows on their way: gather + update of meshes with boundaries at 768, 896,
+// 1024: 1.81, 1.77, 1.78 (without boundaries 96 samples of 65^2 124, 127, 128 us), viscous
+// units at 512, 640, 768, 896, 1024: 1.92, 1.87, 1.83, 1.78, 1.77.
 #ifndef TG_BATCH_GRAD_BLOCK
 #define TG_BATCH_GRAD_BLOCK 256      // largest block of the launch shapes
 #endif
@@ -731,8 +742,11 @@ __device__ __forceinline__ Item item_of_pair(const Batch& B, unsigned w, int lan
 #ifndef TG_BATCH_GATHER_THREADS
 #define TG_BATCH_GATHER_THREADS 768
 #endif
+#ifndef TG_BATCH_GATHER_THREADS_BND
+#define TG_BATCH_GATHER_THREADS_BND 896
+#endif
 #ifndef TG_BATCH_VISC_THREADS
-#define TG_BATCH_VISC_THREADS 768
+#define TG_BATCH_VISC_THREADS 1024
 #endif
 // Pairs per lane of the gradient and gather passes.
 #ifndef TG_BATCH_LANE_PAIRS
@@ -794,14 +808,25 @@ __global__ void __launch_bounds__(32 * VT) kb_dt(Batch B, BParams k, int per) {
     const int P = L.P;
     const int v0 = ch * per, v1 = min(L.m.nv, v0 + per);
     const f2 mu = BND && k.model == 1 ? make_float2(L.mu[s], L.mu[s + 1]) : sp(0.0f);
-    for (int v = v0 + vg; v < v1; v += VT) {
+    // the coming vertex's rows and entry range are on their way while this one's are used
+    f2 nu = sp(0.0f), nw = nu, np = nu, n5 = nu;
+    int nj0 = 0, nj1 = 0;
+    auto load = [&](int v) {
       const float* q = L.Q[0] + rows(v, kQ, P) + s;
-      const f2 u = ld2(q), w = ld2(q + P), p = ld2(q + 2 * P), V5 = ld2(q + 4 * P);
+      nu = ld2(q); nw = ld2(q + P); np = ld2(q + 2 * P); n5 = ld2(q + 4 * P);
+      nj0 = L.m.ce_off[v]; nj1 = L.m.ce_off[v + 1];
+    };
+    if (v0 + vg < v1) load(v0 + vg);
+    for (int v = v0 + vg; v < v1; v += VT) {
+      const f2 u = nu, w = nw, p = np, V5 = n5;
+      const int j0 = nj0, j1 = nj1;
+      if (v + VT < v1) load(v + VT);
       const f2 rho = mul2(neg2(V5), p);
       const f2 gp = mul2(sp(k.gamma), p);
       const f2 c = make_float2(sqrtf(gp.x / rho.x), sqrtf(gp.y / rho.y));
       f2 lam = sp(0.0f);
-      for (int j = L.m.ce_off[v]; j < L.m.ce_off[v + 1]; ++j) {
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) {
         const float4 n = __ldg(reinterpret_cast<const float4*>(L.m.de + j));   // nx, ny, |n|
         const f2 vn = fma2(w, sp(n.y), mul2(u, sp(n.x)));
         lam = add2(lam, fma2(c, sp(n.z), abs2(vn)));
@@ -1213,18 +1238,22 @@ __global__ void __launch_bounds__(BS, TG_BATCH_VISC_THREADS / BS) kb_viscous(Bat
     const f2 V5 = ld2(q + 4 * S), nV5 = neg2(V5);
     o[0] = ld2(q + 3 * S); o[1] = mul2(nV5, ld2(q)); o[2] = mul2(nV5, ld2(q + S)); o[3] = V5;
   };
-  const int c = L.m.u_cell[u];
-  const float* n = L.m.c_n + 6 * (size_t)c;
+  const int4 ra = __ldg(reinterpret_cast<const int4*>(L.m.un + u));
+  const float4 rb = __ldg(reinterpret_cast<const float4*>(L.m.un + u) + 1), rc = __ldg(reinterpret_cast<const float4*>(L.m.un + u) + 2);
+  const int c = ra.w & ~kUnitBf;
+  const float n[6] = {rb.x, rb.y, rb.z, rb.w, rc.x, rc.y};
   f2 wv[3][4];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) W(L.m.c_v[3 * c + i], wv[i]);
+  W(ra.x, wv[0]);
+  W(ra.y, wv[1]);
+  W(ra.z, wv[2]);
   f2 dE[kG];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     dE[2 * i] = fma2(sp(n[4]), wv[2][i], fma2(sp(n[2]), wv[1][i], mul2(sp(n[0]), wv[0][i])));
     dE[2 * i + 1] = fma2(sp(n[5]), wv[2][i], fma2(sp(n[3]), wv[1][i], mul2(sp(n[1]), wv[0][i])));
   }
-  for (int j = L.m.c_bf_off[c]; j < L.m.c_bf_off[c + 1]; ++j) {
+  const bool bf = (ra.w & kUnitBf) != 0;
+  for (int j = bf ? L.m.c_bf_off[c] : 0, end = bf ? L.m.c_bf_off[c + 1] : 0; j < end; ++j) {
     const int d = L.m.c_bf[j];
     const int kind = L.m.b_kind[d], ad = L.m.b_adiab[d];
     const float nx = L.m.b_nx[d], ny = L.m.b_ny[d];
@@ -1251,7 +1280,7 @@ __global__ void __launch_bounds__(BS, TG_BATCH_VISC_THREADS / BS) kb_viscous(Bat
       dE[2 * i + 1] = fma2(sp(ny), dW, dE[2 * i + 1]);
     }
   }
-  const f2 f = sp(L.m.c_inv2a[c]);
+  const f2 f = sp(rc.z);
 #pragma unroll
   for (int i = 0; i < kG; ++i) dE[i] = mul2(dE[i], f);
   f2 avg[4];
@@ -1307,7 +1336,7 @@ __global__ void __launch_bounds__(BS, TG_BATCH_VISC_THREADS / BS) kb_viscous(Bat
 // pairs of samples per thread.  Held or finished samples copy their state
 // through.
 template <int ST, int BS, bool BND, int H = kLanePairs>
-__global__ void __launch_bounds__(BS, TG_BATCH_GATHER_THREADS / BS) kb_gather_update(Batch B, BParams k, int r) {
+__global__ void __launch_bounds__(BS, (BND ? TG_BATCH_GATHER_THREADS_BND : TG_BATCH_GATHER_THREADS) / BS) kb_gather_update(Batch B, BParams k, int r) {
   if (!*k.live) return;            // nothing advances: Q[0] stays the state
   const unsigned w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const Item it = item_of_pair<ST, IT_VERTEX, H>(B, w, threadIdx.x & 31);
@@ -1352,25 +1381,40 @@ __global__ void __launch_bounds__(BS, TG_BATCH_GATHER_THREADS / BS) kb_gather_up
     }
   }
   if (BND) {   // boundary and viscous contributions in list order (src/fv.cc:1100-1188, 1197-1320)
-    for (int j = L.m.cb_off[v]; j < L.m.cb_off[v + 1]; ++j) {
-      const int ent = L.m.cb_ent[j];
+    // the coming entry's rows are on their way while this one's are used, its index one further
+    const int b0 = L.m.cb_off[v], b1 = L.m.cb_off[v + 1];
+    f2 x[3][H];
+    auto load = [&](int ent) {
+      const int type = ent & 3;
+      if (type == 1 || (type != 0 && k.model != 1)) return;
+      const float* p = type == 0 ? L.Fb + rows(ent >> 2, 4, S) + S : (type == 2 ? L.Fv : L.Fvb) + rows(ent >> 2, 3, S);
+      p += s;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ldh<H>(p + c * S, x[c]);
+    };
+    int ent = b0 < b1 ? L.m.cb_ent[b0] : 1, nx = b0 + 1 < b1 ? L.m.cb_ent[b0 + 1] : 1;   // 1: gradients only
+    load(ent);
+    for (int j = b0; j < b1; ++j) {
       const int type = ent & 3, idx = ent >> 2;
+      f2 y[3][H];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int h = 0; h < H; ++h) y[c][h] = x[c][h];
+      ent = nx;
+      nx = j + 2 < b1 ? L.m.cb_ent[j + 2] : 1;
+      load(ent);
+      if (type == 1 || (type != 0 && k.model != 1)) continue;
+      const f2 hf = sp(type == 2 ? -0.5f : 0.5f);
       if (type == 0) {
-        const float* Fe = L.Fb + rows(idx, 4, S) + s;
-        const f2 hf = sp(0.5f);
+        f2 x0[H];
+        ldh<H>(L.Fb + rows(idx, 4, S) + s, x0);
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
-          r0[h] = fma2(ld2(Fe + 2 * h), hf, r0[h]); r1[h] = fma2(ld2(Fe + S + 2 * h), hf, r1[h]);
-          r2[h] = fma2(ld2(Fe + 2 * S + 2 * h), hf, r2[h]); r3[h] = fma2(ld2(Fe + 3 * S + 2 * h), hf, r3[h]);
-        }
-      } else if ((type == 2 || type == 3) && k.model == 1) {
-        const float* Fe = (type == 2 ? L.Fv : L.Fvb) + rows(idx, 3, S) + s;
-        const f2 hf = sp(type == 2 ? -0.5f : 0.5f);
+        for (int h = 0; h < H; ++h) r0[h] = fma2(x0[h], hf, r0[h]);
+      }
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
-          r1[h] = fma2(ld2(Fe + 2 * h), hf, r1[h]); r2[h] = fma2(ld2(Fe + S + 2 * h), hf, r2[h]);
-          r3[h] = fma2(ld2(Fe + 2 * S + 2 * h), hf, r3[h]);
-        }
+      for (int h = 0; h < H; ++h) {
+        r1[h] = fma2(y[0][h], hf, r1[h]); r2[h] = fma2(y[1][h], hf, r2[h]); r3[h] = fma2(y[2][h], hf, r3[h]);
       }
     }
   }
