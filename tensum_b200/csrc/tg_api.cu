@@ -63,6 +63,7 @@ struct tg_handle {
   enum { kCold = 0, kWarm = 1, kMany = 2, kGraphs = 3 };
   cudaGraph_t graph[kGraphs] = {};
   cudaGraphExec_t graph_exec[kGraphs] = {};
+  long steps_run = 0;                          // steps launched on this handle
   bool cold = true;                            // the next step may not find dt_next set
   bool w_partial[3] = {false, false, false};   // a step left this buffer's V1 unformed (refresh_w)
   bool uold_stale = false;                     // steps ran since Uold was stored (they form U_old themselves)
@@ -408,6 +409,9 @@ void enqueue_step(tg_handle* h, bool warm) {
 // Warm steps in the longest captured run: a replay's own launch latency, and the full
 // dependency between two replays, fall on one step in so many.
 constexpr int kManySteps = 8;
+// Capturing that run costs as much as it saves in some tens of steps (0.4 ms, 4 ms the first
+// time in a process), so a handle that steps a few times only does without it.
+constexpr long kManyAfter = 32;
 
 tg_status capture(tg_handle* h, int which) {
   if (h->graph_exec[which]) return TG_OK;
@@ -424,13 +428,15 @@ tg_status capture(tg_handle* h, int which) {
 // do too), so only the first of them forms its own dt.
 tg_status launch_steps(tg_handle* h, long n) {
   for (long i = 0; i < n;) {
-    const bool warm = h->prm.fuse_dt && !h->cold, many = warm && n - i >= kManySteps;
+    const bool warm = h->prm.fuse_dt && !h->cold;
+    const bool many = warm && n - i >= kManySteps && h->steps_run >= kManyAfter;
     const int which = many ? tg_handle::kMany : warm ? tg_handle::kWarm : tg_handle::kCold;
     const tg_status st = capture(h, which);
     if (st != TG_OK) return st;
     TG_CUDA(h, cudaGraphLaunch(h->graph_exec[which], h->stream));
     h->cold = false;
     i += many ? kManySteps : 1;
+    h->steps_run += many ? kManySteps : 1;
   }
   if (n > 0) mark_steps(h);
   return TG_OK;
