@@ -110,14 +110,19 @@ class MLP:
         self._chk(self.L.tg_mlp_predict(self.h, X.ctypes.data, X.shape[0], Y.ctypes.data, precision, 0))
         return Y
 
+    @staticmethod
+    def _vec(a, k):
+        a = np.asarray(a, np.float64)
+        return a if a.shape == (k,) and a.flags.c_contiguous else np.ascontiguousarray(np.broadcast_to(a, (k,)))
+
     def predict(self, X, precision: int = 1) -> np.ndarray:
         """Surrogate QoIs for inputs X (physical units); precision 1 = BF16 tensor cores."""
         X = np.ascontiguousarray(X, np.float64)
         if X.ndim != 2 or X.shape[1] != self.din:      # whatever broadcasts against the input scaling
             Xn = (X - self.xm) / self.xs
             return self.raw_predict(Xn, precision).astype(np.float64) * self.ys + self.ym
-        sc = [np.ascontiguousarray(np.broadcast_to(np.asarray(a, np.float64), (k,)))
-              for a, k in ((self.xm, self.din), (self.xs, self.din), (self.ym, self.dout), (self.ys, self.dout))]
+        sc = [self._vec(a, k) for a, k in ((self.xm, self.din), (self.xs, self.din), (self.ym, self.dout),
+                                           (self.ys, self.dout))]
         Y = np.empty((X.shape[0], self.dout))
         self._chk(self.L.tg_mlp_predict_scaled(self.h, X.ctypes.data, X.shape[0], *[a.ctypes.data for a in sc],
                                                Y.ctypes.data, precision))

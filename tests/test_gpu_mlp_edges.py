@@ -45,3 +45,15 @@ def test_scaled_prediction_is_the_scaled_call(din, dout, n, precision):
     X = rng.normal(size=(n, din))
     want = net.raw_predict((X - net.xm) / net.xs, precision).astype(np.float64) * net.ys + net.ym
     assert np.array_equal(net.predict(X, precision), want)
+
+
+def test_scaled_predictions_of_growing_and_shrinking_calls():
+    """One net's calls share a workspace that grows; up to 2048 doubles the scaling and the
+    rows travel in one copy (678 rows of three inputs and outputs)."""
+    net, _, rng = _net(3, 3, 7)
+    X = rng.normal(size=(33000, 3))
+    net.ym, net.ys = rng.normal(size=3), rng.uniform(0.5, 2.0, 3)
+    for n in (1, 256, 257, 678, 679, 5000, 2, 33000, 300):
+        net.xm, net.xs = rng.normal(size=3), rng.uniform(0.5, 2.0, 3)
+        want = net.raw_predict((X[:n] - net.xm) / net.xs, 1).astype(np.float64) * net.ys + net.ym
+        assert np.array_equal(net.predict(X[:n], 1), want), n
