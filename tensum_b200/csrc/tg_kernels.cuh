@@ -112,9 +112,9 @@ struct Scalars {
   int bad;
   unsigned long long dtmin_bits;
   int stop_counter;    // steps stop once counter exceeds it (output-time stepping)
-  // Set by a last-stage update that also formed dt, U_old and their minimum
+  // Set by a last-stage update that also formed dt and its minimum
   // (dtmin_next) for the state it wrote; cleared whenever the state changes by
-  // any other route, so the next step's first stage then forms them itself.
+  // any other route, so the next step then forms them itself.
   int dt_next;
   unsigned long long dtmin_next;
   unsigned int blocks_done;   // blocks of the last stage's launch that have written their norm partials

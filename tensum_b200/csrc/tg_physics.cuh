@@ -39,7 +39,7 @@ struct Params {
   int nd, visc, heat;
   int liou;       // Liou's carbuncle switch active (liou_fix with kepes_tecno_roe)
   int strong;     // bc_scheme strong
-  int fuse_dt;    // the last stage's update also forms the next step's local dt and U_old
+  int fuse_dt;    // the last stage's update also forms the next step's local dt
   int axi;        // axisymmetric: residual contributions and the update weighted by radii
 };
 
