@@ -48,7 +48,7 @@ struct tg_handle {
   double2* W23b[3] = {nullptr, nullptr, nullptr};
   size_t smem_grad = 0, smem_flux[3] = {0, 0, 0};   // flux: by mode
   bool pdl = false;            // a step's kernels are dependent launches (pdl_wait)
-  int grid_grad = 1, grid_flux[3] = {1, 1, 1};   // CTAs that fill the chip once (the kernels walk tiles)
+  int grid_grad = 1, grid_head = 1, grid_flux[3] = {1, 1, 1};   // CTAs that fill the chip once (the kernels walk tiles)
   Scalars* sc = nullptr;       // device
   int* done = nullptr;         // device flag written by k_step_begin
   int* never = nullptr;        // device zero, used by single-phase calls
@@ -185,7 +185,8 @@ void launch(bool pdl, void (*f)(P...), int grid, int block, size_t smem, cudaStr
 }
 
 // ---- kernel dispatch over (flux, reconstruction)
-typedef void (*BfluxKernel)(Params, MeshView, StateView, const int*, int);
+typedef void (*BfluxKernel)(Params, MeshView, StateView, const int*);
+typedef void (*HeadKernel)(Params, MeshView, TileView, StateView, int, int, const int*, int, int);
 // Entry points that step or read the whole mesh: a partition handle steps through tg_part_*.
 #define TG_WHOLE_MESH(h) \
   if ((h) && (h)->part.n_parts > 0) return fail((h), TG_NOT_SUPPORTED, "a partition handle steps through tg_part_*");
@@ -193,26 +194,35 @@ typedef void (*BfluxKernel)(Params, MeshView, StateView, const int*, int);
 typedef void (*TileFluxKernel)(Params, MeshView, TileView, StateView, Control, Scalars*, int, int, StateView, int, int,
                                int, const int*);
 
+// The boundary faces' kernel and the gradient pass that does them too (k_stage_head).
+struct BndKernels {
+  BfluxKernel bflux;
+  HeadKernel head;
+};
+template <int F, int R>
+BndKernels bnd_pair() {
+  return {k_bflux<F, R>, k_stage_head<F, R>};
+}
 template <int F>
-BfluxKernel pick_bflux(int recon) {
+BndKernels pick_bnd(int recon) {
   switch (recon) {
-    case RECON_FIRST: return k_bflux<F, RECON_FIRST>;
-    case RECON_SECOND: return k_bflux<F, RECON_SECOND>;
-    case RECON_SECOND_MUSCL: return k_bflux<F, RECON_SECOND_MUSCL>;
-    case RECON_VAN_ALBADA: return k_bflux<F, RECON_VAN_ALBADA>;
-    case RECON_TVD_MINMOD: return k_bflux<F, RECON_TVD_MINMOD>;
-    case RECON_TVB_MINMOD: return k_bflux<F, RECON_TVB_MINMOD>;
-    default: return k_bflux<F, RECON_ENO2>;
+    case RECON_FIRST: return bnd_pair<F, RECON_FIRST>();
+    case RECON_SECOND: return bnd_pair<F, RECON_SECOND>();
+    case RECON_SECOND_MUSCL: return bnd_pair<F, RECON_SECOND_MUSCL>();
+    case RECON_VAN_ALBADA: return bnd_pair<F, RECON_VAN_ALBADA>();
+    case RECON_TVD_MINMOD: return bnd_pair<F, RECON_TVD_MINMOD>();
+    case RECON_TVB_MINMOD: return bnd_pair<F, RECON_TVB_MINMOD>();
+    default: return bnd_pair<F, RECON_ENO2>();
   }
 }
-BfluxKernel bflux_kernel(int flux, int recon) {
-  switch (flux) {
-    case FLUX_TECNO_ROE: return pick_bflux<FLUX_TECNO_ROE>(recon);
-    case FLUX_TECNO_RUSANOV: return pick_bflux<FLUX_TECNO_RUSANOV>(recon);
-    case FLUX_KEPEC: return k_bflux<FLUX_KEPEC, RECON_FIRST>;
-    case FLUX_KEP: return k_bflux<FLUX_KEP, RECON_FIRST>;
-    case FLUX_ROE_EC: return k_bflux<FLUX_ROE_EC, RECON_FIRST>;
-    default: return k_bflux<FLUX_AVG, RECON_FIRST>;
+BndKernels bnd_kernels(const Params& k) {
+  switch (k.flux) {
+    case FLUX_TECNO_ROE: return pick_bnd<FLUX_TECNO_ROE>(k.recon);
+    case FLUX_TECNO_RUSANOV: return pick_bnd<FLUX_TECNO_RUSANOV>(k.recon);
+    case FLUX_KEPEC: return bnd_pair<FLUX_KEPEC, RECON_FIRST>();
+    case FLUX_KEP: return bnd_pair<FLUX_KEP, RECON_FIRST>();
+    case FLUX_ROE_EC: return bnd_pair<FLUX_ROE_EC, RECON_FIRST>();
+    default: return bnd_pair<FLUX_AVG, RECON_FIRST>();
   }
 }
 
@@ -310,13 +320,28 @@ void enqueue_gradient(tg_handle* h, int b, const int* done, int base = 0, int co
          h->L.cmax, done);
 }
 
-// boundary-face and viscous contributions, gathered by the tiled flux kernel; with pdl, behind
-// the gradient pass of the same state where the run forms gradients
+// boundary-face and viscous contributions, gathered by the tiled flux kernel
 void enqueue_boundary(tg_handle* h, int b, const int* done, bool pdl = false) {
   if (h->mv.nb > 0)
-    launch(pdl, bflux_kernel(h->prm.flux, h->prm.recon), nblk(2 * h->mv.nb), kBlock, 0, h->stream, h->prm, h->mv,
-           view(h, b), done, pdl && h->grads_needed ? 1 : 0);
-  if (h->viscous) launch(pdl, k_viscous, nblk(h->mv.nvu), kBlock, 0, h->stream, h->prm, h->mv, view(h, b), done);
+    launch(pdl, bnd_kernels(h->prm).bflux, nblk(2 * h->mv.nb), kBlock, 0, h->stream, h->prm, h->mv, view(h, b), done);
+  if (h->viscous) k_viscous<<<nblk(h->mv.nvu), kBlock, 0, h->stream>>>(h->prm, h->mv, view(h, b), done);
+}
+
+// Whether the stages of a step form gradients, boundary faces and viscous units in one launch.
+bool stage_head(const tg_handle* h) { return h->pdl && h->grads_needed && (h->mv.nb > 0 || h->viscous); }
+
+// Everything a stage forms ahead of its flux pass.
+void enqueue_stage_head(tg_handle* h, int b, const int* done) {
+  if (!stage_head(h)) {
+    if (h->grads_needed) enqueue_gradient(h, b, done, 0, -1, h->pdl);
+    enqueue_boundary(h, b, done, h->pdl);
+    return;
+  }
+  TileView v;
+  const int ctas = tiles(h, 0, -1, h->grid_head, &v), nvu = h->viscous ? h->mv.nvu : 0;
+  const int units = (2 * h->mv.nb + nvu + kTileThreads - 1) / kTileThreads;
+  launch(true, bnd_kernels(h->prm).head, ctas + units, kTileThreads, h->smem_grad, h->stream, h->prm, h->mv, v,
+         view(h, b), h->L.lmax, h->L.cmax, done, ctas, nvu);
 }
 
 void enqueue_tile_flux(tg_handle* h, int b, int mode, int r, int bout, const int* done, int base = 0,
@@ -398,8 +423,7 @@ void enqueue_step(tg_handle* h, bool warm) {
       launch(h->pdl, k_dt_final, 1, 1, 0, h->stream, h->ctl, h->sc, h->done);
     }
     if (first) enqueue_ssw(h, h->done);
-    if (h->grads_needed) enqueue_gradient(h, bin, h->done, 0, -1, h->pdl);
-    enqueue_boundary(h, bin, h->done, h->pdl);
+    enqueue_stage_head(h, bin, h->done);
     enqueue_tile_flux(h, bin, last ? MODE_LAST : MODE_UPDATE, r, bout, h->done, 0, -1, h->pdl);
     if (h->prm.strong && h->mv.nsb > 0)
       launch(h->pdl, k_strong_bc, nblk(h->mv.nsb), kBlock, 0, h->stream, h->mv, view(h, bout), h->done);
@@ -810,6 +834,8 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   {
     const int modes[3] = {MODE_RESIDUAL, MODE_UPDATE, MODE_LAST};
     cudaError_t ea = raise_smem((const void*)k_tile_grad, h->smem_grad);
+    const void* head = (const void*)bnd_kernels(k).head;
+    if (ea == cudaSuccess) ea = raise_smem(head, h->smem_grad);
     for (int mode : modes) {
       h->smem_flux[mode] = flux_smem(mat->flux_scheme, mat->reconstruct_scheme, L.lmax, L.emax, L.cmax,
                                      mode == MODE_LAST && k.fuse_dt);
@@ -826,6 +852,7 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
       return per * sms;
     };
     h->grid_grad = fill((const void*)k_tile_grad, h->smem_grad);
+    h->grid_head = fill(head, h->smem_grad);
     for (int mode : modes)
       h->grid_flux[mode] =
           fill((const void*)tile_kernel(mat->flux_scheme, mat->reconstruct_scheme, mode), h->smem_flux[mode]);
@@ -858,12 +885,13 @@ static tg_status create_handle(const tg_mesh* mesh, const tg_material* mat, cons
   c.min_residue = opt->min_residue; c.max_iter = opt->max_iter; c.final_time = opt->final_time; c.tinst = tip;
 
   h->kernels_per_flux = residual_kernels(h);
-  // launches of a replayed step: step_begin + gradient passes + per stage (boundary,
-  // viscous, tiled flux; the last also forms the norms and ends the step) + Liou /
-  // strong-condition kernels; a step that forms its own dt adds the dt pass and dt_final,
-  // a fixed time step dt_final alone.
+  // launches of a replayed step: step_begin + gradient passes + per stage (boundary and
+  // viscous units unless the gradient pass does them, tiled flux; the last also forms the norms
+  // and ends the step) + Liou / strong-condition kernels; a step that forms its own dt adds the
+  // dt pass and dt_final, a fixed time step dt_final alone.
   // The count is that of the steady state: warm steps when the next dt is fused.
-  const int tail = (k.liou ? 1 : 0) + (k.strong && h->mv.nsb > 0 ? c.n_rks : 0) + c.n_rks * residual_kernels(h);
+  const int tail = (k.liou ? 1 : 0) + (k.strong && h->mv.nsb > 0 ? c.n_rks : 0) +
+                   c.n_rks * (stage_head(h) ? 1 : residual_kernels(h));
   const int grads = h->grads_needed ? c.n_rks : 0;
   if (k.fuse_dt) h->kernels_per_step = 1 + grads + tail;
   else h->kernels_per_step = 1 + (c.time_step > 0.0 ? 0 : 1) + grads + 1 + tail;

@@ -51,12 +51,11 @@ __device__ __forceinline__ double vertex_radius(const Params& k, const MeshView&
 // Dependent launches.  The kernels of a step are launched with programmatic stream
 // serialization: a kernel's CTAs may start once every CTA of its predecessor has called
 // pdl_trigger (or ended) and an SM has room, and pdl_wait returns when the predecessor has
-// completed and its writes are visible.  Every such kernel waits before it reads or writes
-// anything a step changes -- so its own completion implies that of all kernels before it --
-// and reads mesh data only ahead of that, behind the predecessor's tail.  The kernels of a
-// stage that do not depend on each other (gradients, boundary faces, viscous units) trigger
-// after their wait and let the next of them run at once: pdl_wait at its end keeps the
-// completion chain.  Launched without the attribute both calls do nothing.
+// completed and its writes are visible.  Nothing else makes them visible: a trigger orders
+// the launch in time and no memory.  So every such kernel waits before it reads or writes
+// anything a step changes -- its own completion then implies that of all kernels before it --
+// and reads mesh data only ahead of that, behind the predecessor's tail.  Launched without
+// the attribute both calls do nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -275,7 +274,6 @@ __global__ void k_store_old(Params k, MeshView m, StateView s, const int* __rest
 }
 
 // Boundary-face inviscid fluxes (src/fv.cc:1100-1188): one thread per (face, vertex).
-// with_grad: launched right behind the gradient pass and independent of it (pdl_wait).
 template <int FLUX, int RECON>
 __device__ __forceinline__ void bflux_one(const Params& k, const MeshView& m, const StateView& s, int t) {
   int d = t >> 1, q = t & 1;
@@ -295,12 +293,11 @@ __device__ __forceinline__ void bflux_one(const Params& k, const MeshView& m, co
   s.Fb[t] = F.m; s.Fb[n2 + t] = F.x; s.Fb[2 * n2 + t] = F.y; s.Fb[3 * n2 + t] = F.e;
 }
 template <int FLUX, int RECON>
-__global__ void k_bflux(Params k, MeshView m, StateView s, const int* __restrict__ done, int with_grad) {
+__global__ void k_bflux(Params k, MeshView m, StateView s, const int* __restrict__ done) {
   pdl_trigger();
-  if (!with_grad) pdl_wait();
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < 2 * m.nb && !*done) bflux_one<FLUX, RECON>(k, m, s, t);
-  pdl_wait();
 }
 
 // Viscous residual units (src/fv.cc:1197-1320): interior cells and boundary faces.
@@ -370,12 +367,9 @@ __device__ __forceinline__ void viscous_one(const Params& k, const MeshView& m, 
     s.Fvb[d] = F.x; s.Fvb[m.nb + d] = F.y; s.Fvb[2 * m.nb + d] = F.e - Cor;
   }
 }
-// Launched behind the gradient pass (viscous runs always form gradients), independent of it.
 __global__ void k_viscous(Params k, MeshView m, StateView s, const int* __restrict__ done) {
-  pdl_trigger();
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u < m.nvu && !*done) viscous_one(k, m, s, u);
-  pdl_wait();
 }
 
 // |n| and the face spectral radius |u.n| + c |n| of the local time step
