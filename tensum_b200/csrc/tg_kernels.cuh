@@ -54,8 +54,10 @@ __device__ __forceinline__ double vertex_radius(const Params& k, const MeshView&
 // completed and its writes are visible.  Nothing else makes them visible: a trigger orders
 // the launch in time and no memory.  So every such kernel waits before it reads or writes
 // anything a step changes -- its own completion then implies that of all kernels before it --
-// and reads mesh data only ahead of that, behind the predecessor's tail.  Launched without
-// the attribute both calls do nothing.
+// and reads mesh data only ahead of that, behind the predecessor's tail.  A kernel may be
+// resident while its predecessor writes what it will read, so none of its parameters is
+// declared __restrict__ (read-only data the compiler may fetch at any time).  Launched
+// without the attribute both calls do nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -293,7 +295,7 @@ __device__ __forceinline__ void bflux_one(const Params& k, const MeshView& m, co
   s.Fb[t] = F.m; s.Fb[n2 + t] = F.x; s.Fb[2 * n2 + t] = F.y; s.Fb[3 * n2 + t] = F.e;
 }
 template <int FLUX, int RECON>
-__global__ void k_bflux(Params k, MeshView m, StateView s, const int* __restrict__ done) {
+__global__ void k_bflux(Params k, MeshView m, StateView s, const int* done) {
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -401,7 +403,7 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x)
 
 // Local time step (src/fv.cc:1499-1598): spectral-radius gather, dt = cfl A / sum,
 // block minimum by warp shuffles, then one atomicMin on the (positive) bit pattern.
-__global__ void k_dt(Params k, MeshView m, StateView s, Scalars* sc, const int* __restrict__ done, int in_step) {
+__global__ void k_dt(Params k, MeshView m, StateView s, Scalars* sc, const int* done, int in_step) {
   pdl_trigger();
   pdl_wait();
   if (*done) return;
@@ -474,7 +476,7 @@ __global__ void k_dt(Params k, MeshView m, StateView s, Scalars* sc, const int* 
 // compute_ssw (src/compute_ssw.cc:7-38): flags both endpoints of every edge
 // (all faces, boundary ones included) across which u.n - a|n| or u.n + a|n|
 // changes sign from positive to negative.  Writers only ever store 1.
-__global__ void k_ssw(Params k, MeshView m, StateView s, const int* __restrict__ done) {
+__global__ void k_ssw(Params k, MeshView m, StateView s, const int* done) {
   pdl_trigger();
   pdl_wait();
   if (*done) return;
@@ -498,7 +500,7 @@ __global__ void k_ssw(Params k, MeshView m, StateView s, const int* __restrict__
 // boundary face's condition applied to its vertices' primitive state in face
 // order; the entropy variables keep their values (the reference does not
 // recompute them), so gradients see the pre-condition state.
-__global__ void k_strong_bc(MeshView m, StateView s, const int* __restrict__ done) {
+__global__ void k_strong_bc(MeshView m, StateView s, const int* done) {
   pdl_trigger();
   pdl_wait();
   if (*done) return;
@@ -543,7 +545,7 @@ __device__ __forceinline__ void dt_final(const Control& ctl, Scalars* sc) {
   sc->dt_global = dtg;
 }
 
-__global__ void k_dt_final(Control ctl, Scalars* sc, const int* __restrict__ done) {
+__global__ void k_dt_final(Control ctl, Scalars* sc, const int* done) {
   pdl_trigger();
   pdl_wait();
   if (*done) return;

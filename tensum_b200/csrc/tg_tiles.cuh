@@ -260,7 +260,7 @@ __device__ __forceinline__ void tile_grad(const Params& k, const MeshView& m, co
 }
 
 __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
-    k_tile_grad(Params k, MeshView m, TileView t, StateView s, int lmax, int cmax, const int* __restrict__ done) {
+    k_tile_grad(Params k, MeshView m, TileView t, StateView s, int lmax, int cmax, const int* done) {
   tile_grad(k, m, t, s, lmax, cmax, done, gridDim.x);
 }
 
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
 // cylinder 7.00 (own launches, no wait) -> 6.38 ms.
 template <int FLUX, int RECON>
 __global__ void __launch_bounds__(kTileThreads, TG_GRAD_MINB)
-    k_stage_head(Params k, MeshView m, TileView t, StateView s, int lmax, int cmax, const int* __restrict__ done,
+    k_stage_head(Params k, MeshView m, TileView t, StateView s, int lmax, int cmax, const int* done,
                  int ctas, int nvu) {
   if (blockIdx.x < ctas) {
     tile_grad(k, m, t, s, lmax, cmax, done, ctas);
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kTileThreads, is_tecno<FLUX>()    ? TG_FLUX_MI
                                                 : MODE == MODE_LAST ? TG_FLUX_MINB_CENTRAL_LAST
                                                                     : TG_FLUX_MINB_CENTRAL)
     k_tile_flux(Params k, MeshView m, TileView t, StateView s, Control ctl, Scalars* sc, int r, int norm,
-                StateView out, int lmax, int emax, int cmax, const int* __restrict__ done) {
+                StateView out, int lmax, int emax, int cmax, const int* done) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool kGrad = flux_needs_grad<FLUX, RECON>();
   // The central fluxes are short and linear in the normal: a tile's normals (no |n|) and

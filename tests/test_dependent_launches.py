@@ -64,3 +64,11 @@ def test_waits_before_it_reads_the_state(name, args, body):
     assert m, f"{name} has no unconditional pdl_wait()"
     early = STATE.search(body[:m.end()])
     assert not early, f"{name} reads {early.group(0)!r} before pdl_wait()"
+
+
+@pytest.mark.parametrize("name,args,body", DEPENDENT, ids=[n for n, _, _ in DEPENDENT])
+def test_promises_no_read_only_memory(name, args, body):
+    """It may be resident while its predecessor writes: __restrict__ and __ldg let a load move
+    ahead of the wait (the tile records, which no kernel writes, are read by load_rec)."""
+    assert "__restrict__" not in args
+    assert "__ldg" not in body
