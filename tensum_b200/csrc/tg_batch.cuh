@@ -467,7 +467,18 @@ __device__ __forceinline__ f2 sqrt2(f2 a) { return make_float2(sqrt_apx(a.x), sq
 __device__ __forceinline__ f2 ld2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
 __device__ __forceinline__ void st2(float* p, f2 v) { *reinterpret_cast<float2*>(p) = v; }
 // H neighbouring pairs by one load or store (H = 2: 16 bytes; sample indices are multiples
-// of 2 H and rows of 32 samples)
+// of 2 H and rows of 32 samples).  ldh, like ld2, is for memory that its kernel does not
+// write (__ldg: such a load may move past any store); ldh_rw is for memory that it does.
+template <int H>
+__device__ __forceinline__ void ldh_rw(const float* p, f2* o) {
+  if (H == 2) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    o[0] = make_float2(x.x, x.y);
+    o[H - 1] = make_float2(x.z, x.w);
+  } else {
+    o[0] = *reinterpret_cast<const float2*>(p);
+  }
+}
 template <int H>
 __device__ __forceinline__ void ldh(const float* p, f2* o) {
   if (H == 2) {
@@ -1424,9 +1435,9 @@ __global__ void __launch_bounds__(BS, (BND ? TG_BATCH_GATHER_THREADS_BND : TG_BA
   const float area = L.m.area[v];
   f2 qu[H], qv[H], qp[H], qw[H], ou[H], ov[H], op[H], ow[H], res[kQ][H];
   ldh<H>(Q, qu); ldh<H>(Q + S, qv); ldh<H>(Q + 2 * S, qp); ldh<H>(Q + 4 * S, qw);
-  if (r > 0) {   // U_old from the state the step started from; stage 0 does not use it
+  if (r > 0) {   // U_old from the state the step started from (the last stage overwrites it); stage 0 does not use it
     const float* O = L.Q[0] + ov_;
-    ldh<H>(O, ou); ldh<H>(O + S, ov); ldh<H>(O + 2 * S, op); ldh<H>(O + 4 * S, ow);
+    ldh_rw<H>(O, ou); ldh_rw<H>(O + S, ov); ldh_rw<H>(O + 2 * S, op); ldh_rw<H>(O + 4 * S, ow);
   }
   auto conserved = [&](f2 u, f2 v, f2 p, f2 V5, f2* c) {
     c[0] = mul2(neg2(V5), p);
