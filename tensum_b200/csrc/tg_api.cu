@@ -447,20 +447,38 @@ tg_status capture(tg_handle* h, int which) {
   return TG_OK;
 }
 
-// n steps by replays: warm ones once the previous step has formed dt for the current state.
-// A cold step leaves dt_next set (or its loop test ended the run, and the later steps' tests
-// do too), so only the first of them forms its own dt.
+// The graph the next of `left` steps replays, `run` steps after the handle's first, and the
+// steps it takes: a warm one once the previous step has formed dt for the current state.
+int next_graph(const tg_handle* h, bool cold, long run, long left) {
+  if (!h->prm.fuse_dt || cold) return tg_handle::kCold;
+  return left >= kManySteps && run >= kManyAfter ? tg_handle::kMany : tg_handle::kWarm;
+}
+constexpr long steps_of(int graph) { return graph == tg_handle::kMany ? kManySteps : 1; }
+
+// Captures every graph that n more steps replay.
+tg_status capture_ahead(tg_handle* h, long n) {
+  bool cold = h->cold;
+  for (long i = 0; i < n;) {
+    const int which = next_graph(h, cold, h->steps_run + i, n - i);
+    const tg_status st = capture(h, which);
+    if (st != TG_OK) return st;
+    cold = false;
+    i += steps_of(which);
+  }
+  return TG_OK;
+}
+
+// n steps by replays.  A cold step leaves dt_next set (or its loop test ended the run, and
+// the later steps' tests do too), so only the first of them forms its own dt.
 tg_status launch_steps(tg_handle* h, long n) {
   for (long i = 0; i < n;) {
-    const bool warm = h->prm.fuse_dt && !h->cold;
-    const bool many = warm && n - i >= kManySteps && h->steps_run >= kManyAfter;
-    const int which = many ? tg_handle::kMany : warm ? tg_handle::kWarm : tg_handle::kCold;
+    const int which = next_graph(h, h->cold, h->steps_run, n - i);
     const tg_status st = capture(h, which);
     if (st != TG_OK) return st;
     TG_CUDA(h, cudaGraphLaunch(h->graph_exec[which], h->stream));
     h->cold = false;
-    i += many ? kManySteps : 1;
-    h->steps_run += many ? kManySteps : 1;
+    i += steps_of(which);
+    h->steps_run += steps_of(which);
   }
   if (n > 0) mark_steps(h);
   return TG_OK;
@@ -573,7 +591,7 @@ tg_status check_bad(tg_handle* h) {
 
 }  // namespace
 
-void enqueue_phase(tg_handle* h, int phase) {
+tg_status enqueue_phase(tg_handle* h, int phase) {
   switch (phase) {
     case TG_PHASE_GRADIENT: enqueue_gradient(h, 0, h->never); break;
     case TG_PHASE_FLUX:
@@ -582,8 +600,9 @@ void enqueue_phase(tg_handle* h, int phase) {
       break;
     case TG_PHASE_UPDATE: enqueue_update(h, 1, false, h->never); break;
     case TG_PHASE_DT: enqueue_dt(h, h->never); break;
-    default: launch_steps(h, 1); break;
+    default: return launch_steps(h, 1);
   }
+  return TG_OK;
 }
 
 // InitialCondition::value (src/ic.h:79-104) at every vertex, on the device, written
@@ -1489,13 +1508,17 @@ tg_status tg_time_phase(tg_handle* h, int phase, int reps, double* ms) {
   cudaEvent_t a, b;
   TG_CUDA(h, cudaEventCreate(&a));
   TG_CUDA(h, cudaEventCreate(&b));
-  enqueue_phase(h, phase);
-  TG_CUDA(h, cudaEventRecord(a, h->stream));
-  if (phase == TG_PHASE_STEP) launch_steps(h, reps);
-  else
-    for (int i = 0; i < reps; ++i) enqueue_phase(h, phase);
-  TG_CUDA(h, cudaEventRecord(b, h->stream));
-  tg_status st = sync(h);
+  tg_status st = enqueue_phase(h, phase);
+  if (st == TG_OK && phase == TG_PHASE_STEP) st = capture_ahead(h, reps);   // outside the timed region
+  cudaEventRecord(a, h->stream);
+  if (phase == TG_PHASE_STEP) {
+    if (st == TG_OK) st = launch_steps(h, reps);
+  } else {
+    for (int i = 0; i < reps && st == TG_OK; ++i) st = enqueue_phase(h, phase);
+  }
+  cudaEventRecord(b, h->stream);
+  const tg_status ended = sync(h);
+  if (st == TG_OK) st = ended;
   float t = 0.0f;
   if (st == TG_OK) {
     cudaError_t e = cudaEventElapsedTime(&t, a, b);
