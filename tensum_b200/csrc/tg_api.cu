@@ -63,7 +63,8 @@ struct tg_handle {
   enum { kCold = 0, kWarm = 1, kMany = 2, kGraphs = 3 };
   cudaGraph_t graph[kGraphs] = {};
   cudaGraphExec_t graph_exec[kGraphs] = {};
-  long steps_run = 0;                          // steps launched on this handle
+  long steps_run = 0;                          // steps launched since the graphs were last dropped
+  long steps_before = 0;                       // and between that and the time before
   bool cold = true;                            // the next step may not find dt_next set
   bool w_partial[3] = {false, false, false};   // a step left this buffer's V1 unformed (refresh_w)
   bool uold_stale = false;                     // steps ran since Uold was stored (they form U_old themselves)
@@ -433,8 +434,11 @@ void enqueue_step(tg_handle* h, bool warm) {
 // Warm steps in the longest captured run: a replay's own launch latency, and the full
 // dependency between two replays, fall on one step in so many.
 constexpr int kManySteps = 8;
-// Capturing that run costs as much as it saves in some tens of steps (0.4 ms, 4 ms the first
-// time in a process), so a handle that steps a few times only does without it.
+// Capturing that run costs as much as it saves in some tens of steps (0.15 ms on a cylinder of
+// 24 x 48 against 6 us a step; 4 ms the first time in a process), so it is made where at least
+// so many steps run on the same graphs: counting those still to run in the call, or as many as
+// the handle's last parameters had.  New ones (tg_update_parameters) drop the graphs, and
+// samples of a few steps do without it.
 constexpr long kManyAfter = 32;
 
 tg_status capture(tg_handle* h, int which) {
@@ -447,11 +451,11 @@ tg_status capture(tg_handle* h, int which) {
   return TG_OK;
 }
 
-// The graph the next of `left` steps replays, `run` steps after the handle's first, and the
-// steps it takes: a warm one once the previous step has formed dt for the current state.
+// The graph that the next of `left` steps replays, `run` steps after the graphs were last
+// dropped: a warm one once the previous step has formed dt for the current state.
 int next_graph(const tg_handle* h, bool cold, long run, long left) {
   if (!h->prm.fuse_dt || cold) return tg_handle::kCold;
-  return left >= kManySteps && run >= kManyAfter ? tg_handle::kMany : tg_handle::kWarm;
+  return left >= kManySteps && std::max(run + left, h->steps_before) >= kManyAfter ? tg_handle::kMany : tg_handle::kWarm;
 }
 constexpr long steps_of(int graph) { return graph == tg_handle::kMany ? kManySteps : 1; }
 
@@ -491,6 +495,8 @@ void drop_graphs(tg_handle* h) {
     h->graph_exec[i] = nullptr;
     h->graph[i] = nullptr;
   }
+  if (h->steps_run > 0) h->steps_before = h->steps_run;
+  h->steps_run = 0;
 }
 
 // The state changed outside a captured step: the next step forms dt itself.

@@ -4,7 +4,14 @@ tg_time_phase reports the time of the steps alone, whatever graphs it has to mak
 Capturing eight steps costs about as much as 16 steps of the 33 x 33 mesh take (0.4 ms), so
 a capture inside the timed region shows as a first result of about twice the second; the
 bound lies between the two.  The least of several fresh handles stands for all.
+
+tg_update_parameters drops the graphs.  A sample of nine steps must then cost one step more
+than a sample of eight (twice that is the bound) and not the capture of an eight-step run,
+which takes as long as several steps.  And whichever graphs a run takes, its steps are the
+same bit for bit, new parameters included.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -31,3 +38,51 @@ def test_a_timed_phase_holds_no_capture(before, reps):
         first = s.time_phase("step", reps)
         ratio.append(first / s.time_phase("step", reps))
     assert min(ratio) < 1.4, ratio
+
+
+def _cylinder(angle):
+    m = cases.cylinder_mesh(24, 48, 3)
+    return abi.Problem(preproc.preprocess(m), cases.cylinder_config(0.2, 100.0, angle, 1e9, 1)), cases.cylinder_ic(m.coords, 0.2, 1.0)
+
+
+def test_short_samples_make_no_long_graphs():
+    (P, prim), (Q, _) = _cylinder(0.5), _cylinder(1.0)
+    s = gpu.Solver(P)
+    s.set_state(prim)
+    s.step(64)
+
+    def sample(n):
+        t = []
+        for k in range(20):
+            a = time.perf_counter()
+            s.update_parameters(P if k % 2 else Q)
+            s.step(n)
+            t.append(time.perf_counter() - a)
+        return np.median(t[2:])
+
+    step = 1e-3 * s.time_phase("step", 4)
+    eight, nine = sample(8), sample(9)
+    assert nine - eight < 2.0 * step, (eight, nine, step)
+
+
+@pytest.mark.parametrize("case", ["kepec", "tecno", "cylinder"])
+def test_long_graphs_are_the_same_steps(case):
+    """50 steps in one call (one cold, six runs of eight, one warm) against 50 calls; then both
+    again with other parameters."""
+    if case == "cylinder":
+        (P, prim), (Q, _) = _cylinder(0.5), _cylinder(1.0)
+    else:
+        P, prim = _kh(65, *(("kepec", "first") if case == "kepec" else ("kepes_tecno_roe", "minmod")))
+        Q = P                                       # nothing to change: the graphs are dropped
+    a, b = gpu.Solver(P), gpu.Solver(P)
+    for s in (a, b):
+        s.set_state(prim)
+    for other in (False, True):
+        if other:
+            a.update_parameters(Q)
+            b.update_parameters(Q)
+        ia = a.step(50)
+        for _ in range(50):
+            ib = b.step(1)
+        assert np.array_equal(a.get_state(), b.get_state())
+        assert np.array_equal(ia, ib)
