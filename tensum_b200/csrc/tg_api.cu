@@ -1278,6 +1278,7 @@ tg_status tg_update_parameters(tg_handle* h, const tg_material* mat, const tg_bc
       mat->mu_model != k.mu_model)
     return fail(h, TG_NOT_SUPPORTED, "model, flux, reconstruction and viscosity law are fixed at tg_create");
   if (!(mat->gamma > 1.0) || !(mat->gas_const > 0.0)) return fail(h, TG_INVALID_ARG, "gamma must be > 1, gas_const > 0");
+  const bool gas = k.gamma != mat->gamma || k.R != mat->gas_const;
   k.gamma = mat->gamma; k.R = mat->gas_const; k.Cp = mat->gamma * mat->gas_const / (mat->gamma - 1.0);
   k.sqrt_gm1 = std::sqrt(mat->gamma - 1.0);
   k.inv_gamma = 1.0 / mat->gamma;
@@ -1298,6 +1299,12 @@ tg_status tg_update_parameters(tg_handle* h, const tg_material* mat, const tg_bc
     if (!L.b_val.empty())
       TG_CUDA(h, cudaMemcpyAsync(const_cast<double*>(h->mv.b_val), L.b_val.data(), L.b_val.size() * sizeof(double),
                                  cudaMemcpyHostToDevice, h->stream));
+  }
+  if (gas) {
+    // the state is (T, p, u, v); its entropy variables, from which the kernels take the density
+    // (rho = -V5 p), depend on the gas
+    k_prim2ent<<<nblk(h->mv.nv), kBlock, 0, h->stream>>>(k, h->mv.nv, view(h, 0), nullptr);
+    h->w_partial[0] = false;
   }
   // dt depends on the material; the captured step holds the parameters by value
   clear_dt_next(h);
