@@ -595,17 +595,19 @@ struct tg_mlp {
   float *X = nullptr, *T = nullptr, *A = nullptr, *Y = nullptr, *D = nullptr, *D4 = nullptr, *losses = nullptr;
   int cap_losses = 0;
   float2* corr = nullptr;           // kMaxBatches bias corrections
-  // tg_mlp_predict_scaled: scaling vectors followed by the rows of a call of one chunk (at most
-  // kRows), and, from its first larger call on, per-lane streams with pinned and device
-  // buffers of kRows rows
+  // tg_mlp_predict_scaled: scaling vectors followed by the rows of a call without staging, and
+  // the staging lanes: a stream each and equal parts of one pinned and one device block
   double* scale = nullptr;
-  int scale_rows = 0;
+  size_t scale_rows = 0;
   static constexpr int kLanes = 4, kRows = 32768, kFirstRows = 256;
   cudaStream_t lane[kLanes] = {};
-  double *pin[kLanes] = {}, *dev[kLanes] = {};
+  char *pin = nullptr, *dev = nullptr;
+  size_t lane_bytes = 0;
+  size_t plain_bytes = 0;           // moved without staging by calls of more than kRows rows
   std::string err;
 };
-constexpr int kMaxBatches = 4096;   // minibatches of one training launch (64 samples each: about 15 ms)
+constexpr int kMaxBatches = 4096;   // minibatches of one training launch (64 samples each: about 40 ms)
+constexpr size_t kPlainBytes = size_t(16) << 20;   // see tg_mlp_predict_scaled
 
 namespace {
 
@@ -730,11 +732,10 @@ tg_status tg_mlp_destroy(tg_mlp* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   cudaFree(h->theta); cudaFree(h->m); cudaFree(h->v); cudaFree(h->g); cudaFree(h->losses); cudaFree(h->corr);
   cudaFree(h->X); cudaFree(h->T); cudaFree(h->A); cudaFree(h->Y); cudaFree(h->D); cudaFree(h->D4); cudaFree(h->scale);
-  for (int i = 0; i < tg_mlp::kLanes; ++i) {
-    if (h->lane[i]) cudaStreamDestroy(h->lane[i]);
-    cudaFreeHost(h->pin[i]);
-    cudaFree(h->dev[i]);
-  }
+  for (cudaStream_t s : h->lane)
+    if (s) cudaStreamDestroy(s);
+  cudaFreeHost(h->pin);
+  cudaFree(h->dev);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return TG_OK;
@@ -845,23 +846,58 @@ tg_status tg_mlp_predict(tg_mlp* h, const float* X, int n, float* Y, int precisi
   return TG_OK;
 }
 
+// The staging lanes of a call that moves `bytes`: kLanes parts that take it in 32 chunks, 1 MiB
+// at least, a power of two.  False: no pinned memory to be had.
+static bool stage_lanes(tg_mlp* h, size_t bytes) {
+  const size_t most = (size_t)tg_mlp::kRows * (h->din + h->dout) * sizeof(double);
+  size_t want = size_t(1) << 20;
+  while (want < most && want < bytes / 32) want *= 2;
+  if (want <= h->lane_bytes) return true;
+  cudaFreeHost(h->pin);
+  cudaFree(h->dev);
+  h->pin = h->dev = nullptr;
+  h->lane_bytes = 0;
+  cudaError_t e = cudaMallocHost((void**)&h->pin, tg_mlp::kLanes * want);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&h->dev, tg_mlp::kLanes * want);
+  for (cudaStream_t& s : h->lane)
+    if (e == cudaSuccess && !s) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  h->lane_bytes = want;
+  return true;
+}
+
 // The same from and to physical units, host arrays in FP64: Y = ym + ys net((X - xm) / xs).
-// A large set goes in chunks through a few host threads, each copying its chunks into a pinned
-// buffer, so that copies both ways and the network overlap (2^20 inputs of 3: 35 ms with the
-// scaling in numpy and pageable copies, now 2.2).
+// A large set goes in chunks through a few host threads, each copying its chunks into pinned
+// memory, so that copies both ways and the network overlap.  Page-locking takes 1 to 4 ms and
+// more with its size, about what 16 MB lose by pageable copies, so a network gets that memory
+// once its large calls have moved so much: a study often makes one call.  ms of a new network's
+// first call / of later ones in FP32, with the scaling in numpy and pageable copies: 2^20 inputs
+// of 3 43 / 43, 100 000 of 20 9.4 / 8.7, 100 000 of 3 4.2 / 4.2; with four pinned buffers of
+// 32768 rows at the first large call 13 / 2.2, 20 / 1.1, 12.7 / 0.6; now 11 / 2.2, 6.3 / 0.9,
+// 1.3 / 0.4.
 tg_status tg_mlp_predict_scaled(tg_mlp* h, const double* X, int n, const double* xm, const double* xs, const double* ym,
                                 const double* ys, double* Y, int precision) {
   if (!h || !X || !Y || !xm || !xs || !ym || !ys || n < 1) return mfail(h, TG_INVALID_ARG, "bad prediction set");
   const int din = h->din, dout = h->dout;
-  const int chunks = (n + tg_mlp::kRows - 1) / tg_mlp::kRows, lanes = std::min<int>(tg_mlp::kLanes, chunks);
-  const int ns = 2 * (din + dout), want = chunks == 1 ? n : 0;
+  const size_t row = (din + dout) * sizeof(double), bytes = n * row;
+  bool plain = n <= tg_mlp::kRows;
+  if (!plain && !h->pin && h->plain_bytes + bytes < kPlainBytes) {
+    h->plain_bytes += bytes;
+    plain = true;
+  }
+  if (!plain) plain = !stage_lanes(h, bytes);
+  const int ns = 2 * (din + dout);
+  const size_t want = plain ? n : 0;
   if (!h->scale || want > h->scale_rows) {
     TM_CUDA(h, cudaStreamSynchronize(h->stream));
     cudaFree(h->scale);
     h->scale = nullptr;
     h->scale_rows = 0;
-    const int rows = std::max<int>(tg_mlp::kFirstRows, want);
-    TM_CUDA(h, cudaMalloc((void**)&h->scale, (ns + (size_t)rows * (din + dout)) * sizeof(double)));
+    const size_t rows = std::max<size_t>(tg_mlp::kFirstRows, want);
+    TM_CUDA(h, cudaMalloc((void**)&h->scale, ns * sizeof(double) + rows * row));
     h->scale_rows = rows;
   }
   const Scaling S{h->scale, h->scale + din, h->scale + 2 * din, h->scale + 2 * din + dout};
@@ -874,10 +910,10 @@ tg_status tg_mlp_predict_scaled(tg_mlp* h, const double* X, int n, const double*
   std::memcpy(in + 2 * din, ym, dout * sizeof(double));
   std::memcpy(in + 2 * din + dout, ys, dout * sizeof(double));
   const size_t nx = (size_t)n * din;
-  const bool one = chunks == 1 && ns + nx <= kOne;
+  const bool one = plain && ns + nx <= kOne;
   if (one) std::memcpy(in + ns, X, nx * sizeof(double));
   TM_CUDA(h, cudaMemcpyAsync(h->scale, in, (one ? ns + nx : ns) * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  if (chunks == 1) {
+  if (plain) {
     double *dx = h->scale + ns, *dy = dx + nx;
     cudaError_t e = one ? cudaSuccess : cudaMemcpyAsync(dx, X, nx * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
@@ -890,24 +926,19 @@ tg_status tg_mlp_predict_scaled(tg_mlp* h, const double* X, int n, const double*
     if (e != cudaSuccess || e2 != cudaSuccess) return mfail(h, TG_CUDA_ERROR, cudaGetErrorString(e != cudaSuccess ? e : e2));
     return TG_OK;
   }
-  const size_t bytes = (size_t)tg_mlp::kRows * (din + dout) * sizeof(double);
-  for (int i = 0; i < lanes; ++i) {
-    if (h->dev[i]) continue;
-    TM_CUDA(h, cudaStreamCreateWithFlags(&h->lane[i], cudaStreamNonBlocking));
-    TM_CUDA(h, cudaMallocHost((void**)&h->pin[i], bytes));
-    TM_CUDA(h, cudaMalloc((void**)&h->dev[i], bytes));
-  }
+  const int per = (int)(h->lane_bytes / row);       // rows of a lane's chunk
+  const int chunks = (int)((n + (long long)per - 1) / per), lanes = std::min<int>(tg_mlp::kLanes, chunks);
   TM_CUDA(h, cudaStreamSynchronize(h->stream));      // weights and scaling are in place
   int device = 0;
   TM_CUDA(h, cudaGetDevice(&device));
   std::vector<cudaError_t> errs(lanes, cudaSuccess);
   auto work = [&](int l) {
     cudaError_t e = cudaSetDevice(device);
-    double *pin = h->pin[l], *dev = h->dev[l];
-    double *pout = pin + (size_t)tg_mlp::kRows * din, *dout_ = dev + (size_t)tg_mlp::kRows * din;
+    double *pin = (double*)(h->pin + l * h->lane_bytes), *dev = (double*)(h->dev + l * h->lane_bytes);
+    double *pout = pin + (size_t)per * din, *dout_ = dev + (size_t)per * din;
     for (int c = l; c < chunks && e == cudaSuccess; c += lanes) {
-      const size_t r0 = (size_t)c * tg_mlp::kRows;
-      const int rows = (int)std::min<size_t>(tg_mlp::kRows, n - r0);
+      const size_t r0 = (size_t)c * per;
+      const int rows = (int)std::min<size_t>(per, n - r0);
       std::memcpy(pin, X + r0 * din, (size_t)rows * din * sizeof(double));
       e = cudaMemcpyAsync(dev, pin, (size_t)rows * din * sizeof(double), cudaMemcpyHostToDevice, h->lane[l]);
       if (e != cudaSuccess) break;
