@@ -112,17 +112,20 @@ class MLP:
 
     @staticmethod
     def _vec(a, k):
+        """a as k contiguous doubles; None where it broadcasts otherwise than one value per column."""
         a = np.asarray(a, np.float64)
+        if a.shape not in ((), (1,), (k,)):
+            return None
         return a if a.shape == (k,) and a.flags.c_contiguous else np.ascontiguousarray(np.broadcast_to(a, (k,)))
 
     def predict(self, X, precision: int = 1) -> np.ndarray:
         """Surrogate QoIs for inputs X (physical units); precision 1 = BF16 tensor cores."""
         X = np.ascontiguousarray(X, np.float64)
-        if X.ndim != 2 or X.shape[1] != self.din:      # whatever broadcasts against the input scaling
-            Xn = (X - self.xm) / self.xs
-            return self.raw_predict(Xn, precision).astype(np.float64) * self.ys + self.ym
         sc = [self._vec(a, k) for a, k in ((self.xm, self.din), (self.xs, self.din), (self.ym, self.dout),
                                            (self.ys, self.dout))]
+        if X.ndim != 2 or X.shape[1] != self.din or any(a is None for a in sc):   # whatever else broadcasts
+            Xn = (X - self.xm) / self.xs
+            return self.raw_predict(Xn, precision).astype(np.float64) * self.ys + self.ym
         Y = np.empty((X.shape[0], self.dout))
         self._chk(self.L.tg_mlp_predict_scaled(self.h, X.ctypes.data, X.shape[0], *[a.ctypes.data for a in sc],
                                                Y.ctypes.data, precision))
