@@ -57,8 +57,9 @@ __device__ __forceinline__ double dmax_(double a, double b) { return (a < b) ? b
 // one is a single fused rounding, so the result is the correctly rounded one up to rare
 // neighbours: over 8e8 arguments from 2^-900 to 2^900 both gave 1/x's and sqrt's bits every
 // time (the approximations are within 2^-19.9 there).  Unlike / and sqrt they do not branch
-// for zeros, infinities and subnormals: those give NaN, and a state that holds them is
-// flagged as bad either way.
+// for zeros, infinities and subnormals: those give NaN.  Callers pass temperatures, densities,
+// pressures and means of them, positive in a state that was accepted (T > 0 and p > 0) or left
+// by an update that was not flagged (isfinite, p > 0 and rho > 0); a flagged state has no value.
 // A third of the flux passes' instructions were integer and control work, much of it those
 // branches: steps on 1025^2 in us, / and sqrt / these: TeCNO-Rusanov 678 / 651, TeCNO-Roe
 // 711 / 657, KEPEC 249 / 246, Roe-EC 264 / 261; TeCNO-Roe on 65^2 33.4 / 32.1.
@@ -77,26 +78,6 @@ __device__ __forceinline__ double sqrt_nr(double a) {
   h = fma(h, r, h);
   return fma(fma(-g, g, a), h, g);
 }
-
-// Ismail-Roe logarithmic mean (a - b)/ln(a/b), src/material.h:24-42: returns
-// F with logmean = 0.5 (a + b) / F.  The reference forms f = (xi - 1)/(xi + 1)
-// from xi = b/a; f = (b - a)/(b + a) is the same quantity with one division
-// instead of two (and no cancellation in xi - 1), and the series divides by
-// 3, 5, 7 where multiplying by the reciprocals differs by at most an ulp.
-__device__ __forceinline__ double logavg_F(double a, double b) {
-  double f = (b - a) / (b + a);
-  double u = f * f;
-  if (u < 1.0e-2) {
-    double u2 = u * u;
-    double u3 = u2 * u;
-    return 1.0 + u * (1.0 / 3.0) + u2 * (1.0 / 5.0) + u3 * (1.0 / 7.0);
-  }
-  return log(b / a) / 2.0 / f;
-}
-
-__device__ __forceinline__ double logavg(double a, double b) { return 0.5 * (a + b) / logavg_F(a, b); }
-// 1 / logavg(a, b), for the callers that only ever divide by the log mean
-__device__ __forceinline__ double inv_logavg(double a, double b) { return logavg_F(a, b) / (0.5 * (a + b)); }
 
 // 1/(R T) = 2 beta: the one division density, beta and the conserved state share.
 __device__ __forceinline__ double inv_RT(const Params& k, const Prim& q) { return rcp_nr(k.R * q.T); }
@@ -263,10 +244,11 @@ __device__ __forceinline__ VRec make_vrec(const Params& k, const Prim& q) {
   return r;
 }
 
-// The averages the KEPEC and TeCNO fluxes share: the density log mean, the
-// inverse of the beta log mean and p = (rho_l + rho_r) / (2 (beta_l + beta_r)),
-// from two reciprocals and one division instead of five divisions: the reciprocal
-// of the V5 sum (-2 times beta's) serves beta's log-mean ratio f, 1/beta_ln and p.
+// Ismail-Roe logarithmic mean (a - b)/ln(a/b), src/material.h:24-42: returns F with
+// logmean = 0.5 (a + b) / F, given f = (b - a)/(b + a).  The reference forms f as
+// (xi - 1)/(xi + 1) from xi = b/a; this has one division instead of two (and no
+// cancellation in xi - 1), and the series divides by 3, 5, 7 where multiplying by the
+// reciprocals differs by at most an ulp.
 __device__ __forceinline__ double logavg_F_of(double f, double a, double b) {
   double u = f * f;
   if (u < 1.0e-2) {
@@ -276,6 +258,11 @@ __device__ __forceinline__ double logavg_F_of(double f, double a, double b) {
   }
   return log(b / a) / 2.0 / f;
 }
+
+// The averages the KEPEC and TeCNO fluxes share: the density log mean, the
+// inverse of the beta log mean and p = (rho_l + rho_r) / (2 (beta_l + beta_r)),
+// from two reciprocals and one division instead of five divisions: the reciprocal
+// of the V5 sum (-2 times beta's) serves beta's log-mean ratio f, 1/beta_ln and p.
 __device__ __forceinline__ void shared_means(const VRec& L, const VRec& R, double& rho, double& ibeta, double& p) {
   const double rl = rec_rho(L), rr = rec_rho(R);
   const double sr = rl + rr, sv = L.V5 + R.V5;
