@@ -29,24 +29,30 @@ struct Stager {
   static constexpr int kMaxLanes = 8;
   static constexpr size_t kPerLane = size_t(1) << 20;   // the least worth a lane
   int device = 0, lanes = 0;
-  // 512 KiB (page-locking memory is most of a small handle's creation), 1 MiB where every lane
-  // fills it several times: set_state + step + get_state of 1025^2 from pageable buffers with
-  // 512 KiB / 1 / 2 MiB 0.65 / 0.80 / 0.76e9 vertex-stage updates/s
   size_t slot_bytes = 0;
   char* slots = nullptr;   // pinned, lanes * 2 * slot_bytes
   cudaStream_t st[kMaxLanes] = {};
   cudaEvent_t ev[kMaxLanes][2] = {};
 
+  // A lane per MiB, but never two: one helper thread alone often wakes late, and its lane takes
+  // as long as the whole copy.  Medians in us of set_state / get_state from pageable buffers
+  // with one lane and two: 229^2 224 / 175 and 320 / 265, 257^2 258 / 210 and 370 / 310; of
+  // 300^2 with two and three 400 / 320 and 290 / 215.
   static int lanes_for(size_t bytes) {
-    return (int)std::max<size_t>(1, std::min<size_t>(kMaxLanes, bytes / kPerLane));
+    const size_t n = bytes / kPerLane;
+    return n < 3 ? 1 : (int)std::min<size_t>(kMaxLanes, n);
   }
+  // 512 KiB (page-locking memory is most of a small handle's creation), 1 MiB where every lane
+  // fills that twice: 513^2 590 / 435 us either way, 700^2 with 512 KiB / 1 MiB 945 / 780 and
+  // 805 / 725, 900^2 1480 / 1310 and 1150 / 1080.
+  static size_t slot_for(size_t bytes) { return bytes >= 2 * kMaxLanes * kPerLane ? kPerLane : kPerLane / 2; }
   // lanes for transfers of up to `bytes`; a later call may ask for more
   cudaError_t init(int dev, size_t bytes) {
     device = dev;
     const int want = lanes_for(bytes);
     if (want <= lanes) return cudaSuccess;
     release();
-    slot_bytes = bytes >= 4 * kMaxLanes * kPerLane ? kPerLane : kPerLane / 2;
+    slot_bytes = slot_for(bytes);
     cudaError_t e = cudaMallocHost((void**)&slots, 2 * (size_t)want * slot_bytes);
     for (int t = 0; t < want && e == cudaSuccess; ++t) {
       e = cudaStreamCreateWithFlags(&st[t], cudaStreamNonBlocking);
