@@ -440,6 +440,9 @@ constexpr int kManySteps = 8;
 // the handle's last parameters had.  New ones (tg_update_parameters) drop the graphs, and
 // samples of a few steps do without it.
 constexpr long kManyAfter = 32;
+// and behind so many single steps, whose time on the device hides the capture (the first 32 / 200
+// steps of a new handle of 65^2 1.42 / 6.67 ms with it ahead of them, 1.26 / 6.60 behind)
+constexpr long kManyFrom = 16;
 
 tg_status capture(tg_handle* h, int which) {
   if (h->graph_exec[which]) return TG_OK;
@@ -455,7 +458,8 @@ tg_status capture(tg_handle* h, int which) {
 // dropped: a warm one once the previous step has formed dt for the current state.
 int next_graph(const tg_handle* h, bool cold, long run, long left) {
   if (!h->prm.fuse_dt || cold) return tg_handle::kCold;
-  return left >= kManySteps && std::max(run + left, h->steps_before) >= kManyAfter ? tg_handle::kMany : tg_handle::kWarm;
+  const bool many = left >= kManySteps && run >= kManyFrom && std::max(run + left, h->steps_before) >= kManyAfter;
+  return many ? tg_handle::kMany : tg_handle::kWarm;
 }
 constexpr long steps_of(int graph) { return graph == tg_handle::kMany ? kManySteps : 1; }
 

@@ -27,7 +27,7 @@ def test_first_and_later_copies():
                                                 boundary={t: ("periodic", {}) for t in (1, 2, 3, 4)}))
     rows = np.stack([cases.kh_rnd_row(s) for s in range(32)])
     first, later = [], []
-    for _ in range(6):
+    for _ in range(12):
         b = batch.Batch([(P, 32)])
         b.set_kh(0, rows)
         b.advance(1, 1)
