@@ -132,7 +132,8 @@ tg_status work_reserve(tg_batch* b, size_t bytes) {
 // through the staging threads, once the batch has copied kPlainBytes to such targets directly:
 // page-locking the slots takes 1 to 4 ms and more, about what that much loses.  First and later
 // copies of one member's state in ms, slots made at the first one / now: 257^2 2.9 / 0.2 and
-// 0.8 / 0.2, 513^2 11 / 0.5 and 1.6 / 0.5.
+// 0.8 / 0.2, 513^2 11 / 0.5 and 1.6 / 0.5.  Slots of 512 KiB: 1 MiB ones gain a batch nothing
+// later, and a first call on levels of 129^2, 257^2 and 513^2 takes 47 ms with them, 40 without.
 constexpr size_t kPlainBytes = size_t(16) << 20;
 tg_status copy_out(tg_batch* b, void* dst, const void* src, size_t bytes) {
   bool plain = bytes < 2 * Stager::kPerLane || host_pinned(dst);
@@ -140,7 +141,7 @@ tg_status copy_out(tg_batch* b, void* dst, const void* src, size_t bytes) {
     b->plain_bytes += bytes;
     plain = true;
   }
-  if (!plain && b->stage.init(b->device, bytes) != cudaSuccess) {   // no pinned memory to be had
+  if (!plain && b->stage.init(b->device, bytes, Stager::kPerLane / 2) != cudaSuccess) {   // no pinned memory to be had
     cudaGetLastError();
     plain = true;
   }

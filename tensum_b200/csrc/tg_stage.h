@@ -46,13 +46,13 @@ struct Stager {
   // fills that twice: 513^2 590 / 435 us either way, 700^2 with 512 KiB / 1 MiB 945 / 780 and
   // 805 / 725, 900^2 1480 / 1310 and 1150 / 1080.
   static size_t slot_for(size_t bytes) { return bytes >= 2 * kMaxLanes * kPerLane ? kPerLane : kPerLane / 2; }
-  // lanes for transfers of up to `bytes`; a later call may ask for more
-  cudaError_t init(int dev, size_t bytes) {
+  // lanes for transfers of up to `bytes`, with slots of `most` at most; a later call may ask for more
+  cudaError_t init(int dev, size_t bytes, size_t most = kPerLane) {
     device = dev;
     const int want = lanes_for(bytes);
     if (want <= lanes) return cudaSuccess;
     release();
-    slot_bytes = slot_for(bytes);
+    slot_bytes = std::min(most, slot_for(bytes));
     cudaError_t e = cudaMallocHost((void**)&slots, 2 * (size_t)want * slot_bytes);
     for (int t = 0; t < want && e == cudaSuccess; ++t) {
       e = cudaStreamCreateWithFlags(&st[t], cudaStreamNonBlocking);
