@@ -30,6 +30,9 @@ def cuda_device_present() -> bool:
 
 
 def pytest_collection_modifyitems(config, items):
+    # the drop-in's tests need the reference's program, which is built where its sources are: last,
+    # so that a run that stops at the first failure has been through all others
+    items.sort(key=lambda it: it.path.name == "test_gpu_dropin.py")
     if cuda_device_present():
         return
     skip = pytest.mark.skip(reason="no CUDA device in this container")
