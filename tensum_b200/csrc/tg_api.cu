@@ -443,6 +443,13 @@ constexpr long kManyAfter = 32;
 // and behind so many single steps, whose time on the device hides the capture (the first 32 / 200
 // steps of a new handle of 65^2 1.42 / 6.67 ms with it ahead of them, 1.26 / 6.60 behind)
 constexpr long kManyFrom = 16;
+// It is also made behind so many steps of the same call, whose first steps have nothing on the
+// device ahead of them.  3 samples of a new handle, the second one making it at its second step /
+// at its ninth: KEPEC on 100^2, 16 steps each, 2.30 / 2.10 ms; TeCNO-Rusanov on 257^2, 24 steps
+// each, 7.25 / 7.07.
+constexpr long kManyBehind = 8;
+// Where calls are too short for that, the handle has it made after so many steps.
+constexpr long kManyAnyway = 64;
 
 tg_status capture(tg_handle* h, int which) {
   if (h->graph_exec[which]) return TG_OK;
@@ -454,12 +461,15 @@ tg_status capture(tg_handle* h, int which) {
   return TG_OK;
 }
 
-// The graph that the next of `left` steps replays, `run` steps after the graphs were last
-// dropped: a warm one once the previous step has formed dt for the current state.
-int next_graph(const tg_handle* h, bool cold, long run, long left) {
+// The graph that the next of `left` steps replays, `here` steps into a call and `run` steps after
+// the graphs were last dropped: a warm one once the previous step has formed dt for the
+// current state.
+int next_graph(const tg_handle* h, bool cold, long here, long run, long left) {
   if (!h->prm.fuse_dt || cold) return tg_handle::kCold;
-  const bool many = left >= kManySteps && run >= kManyFrom && std::max(run + left, h->steps_before) >= kManyAfter;
-  return many ? tg_handle::kMany : tg_handle::kWarm;
+  const bool made = h->graph_exec[tg_handle::kMany] != nullptr;
+  const bool pays = run >= kManyFrom && std::max(run + left, h->steps_before) >= kManyAfter &&
+                    (here >= kManyBehind || run >= kManyAnyway);
+  return left >= kManySteps && (made || pays) ? tg_handle::kMany : tg_handle::kWarm;
 }
 constexpr long steps_of(int graph) { return graph == tg_handle::kMany ? kManySteps : 1; }
 
@@ -467,7 +477,7 @@ constexpr long steps_of(int graph) { return graph == tg_handle::kMany ? kManySte
 tg_status capture_ahead(tg_handle* h, long n) {
   bool cold = h->cold;
   for (long i = 0; i < n;) {
-    const int which = next_graph(h, cold, h->steps_run + i, n - i);
+    const int which = next_graph(h, cold, i, h->steps_run + i, n - i);
     const tg_status st = capture(h, which);
     if (st != TG_OK) return st;
     cold = false;
@@ -480,7 +490,7 @@ tg_status capture_ahead(tg_handle* h, long n) {
 // the later steps' tests do too), so only the first of them forms its own dt.
 tg_status launch_steps(tg_handle* h, long n) {
   for (long i = 0; i < n;) {
-    const int which = next_graph(h, h->cold, h->steps_run, n - i);
+    const int which = next_graph(h, h->cold, i, h->steps_run, n - i);
     const tg_status st = capture(h, which);
     if (st != TG_OK) return st;
     TG_CUDA(h, cudaGraphLaunch(h->graph_exec[which], h->stream));
