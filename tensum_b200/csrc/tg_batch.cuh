@@ -735,12 +735,10 @@ __device__ __forceinline__ Item item_of_pair(const Batch& B, unsigned w, int lan
 // Register budgets of the paired passes as resident threads per SM.  All wait on memory more
 // than on anything else, so more warps win until they spill.  Step in ms of 768 samples of
 // Kelvin-Helmholtz 257^2 / 128 of the 128 x 256 cylinder, 128-thread blocks: gather + update at
-// 512, 768, 1024 threads 13.2 / 2.05, 12.3 / 1.94, 12.1 / 1.94 (96 samples of 65^2 123, 121, 126
-// us); gradients of meshes with boundaries at 512, 768, 1024: 2.02, 1.93, 1.88; viscous units
-// at 512, 768: 2.17, 1.99.  Since then, a unit's mesh data one record and the next boundary or
-// viscous entry's rows on their way: gather + update of meshes with boundaries at 768, 896,
-// 1024: 1.81, 1.77, 1.78 (without boundaries 96 samples of 65^2 124, 127, 128 us), viscous
-// units at 512, 640, 768, 896, 1024: 1.92, 1.87, 1.83, 1.78, 1.77.
+// 512, 768, 1024 threads 13.2 / 2.05, 12.3 / 1.94, 12.1 / 1.94; 96 samples of 65^2 at 768, 896,
+// 1024 124, 127, 128 us.  Cylinder alone: gradients at 512, 768, 1024: 2.02, 1.93, 1.88; gather
+// + update at 768, 896, 1024, its next entry's rows on their way: 1.81, 1.77, 1.78; viscous units,
+// mesh data in one record, at 512, 640, 768, 896, 1024: 1.92, 1.87, 1.83, 1.78, 1.77.
 #ifndef TG_BATCH_GRAD_BLOCK
 #define TG_BATCH_GRAD_BLOCK 256      // largest block of the launch shapes
 #endif

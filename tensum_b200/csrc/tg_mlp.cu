@@ -74,6 +74,10 @@ __device__ __forceinline__ void adam(float gp, float& th, float& m, float& v, fl
 // cluster: 256 samples, batch 64, 800 minibatches in 282 ms before and 7.9 ms now,
 // the same weights bit for bit.  What is left of a minibatch's 9.8 us is latency: L2 round
 // trips of weights, activations and deltas, the barriers, and chains of 64 multiply-adds.
+// Large batches stay on the 8 SMs too: thread-per-sample kernels over the whole chip were slower
+// at every size.  One loss and gradient of n samples in us, those / the cluster: 3 inputs and 3
+// outputs, n = 64, 1000, 4096, 65536: 377 / 56, 795 / 165, 1595 / 515, 21898 / 6889; 32 and 8:
+// 405 / 69, 845 / 263, 1626 / 855, 23781 / 13093.
 constexpr int kCl = 8, kTrainThreads = 256, kTile = 64;
 constexpr int kSmall = (8 * kMaxIn + 24 + 9 * kMaxOut + 2 * H - 1) / (2 * H);   // small gradients per thread
 // Weight rows padded so that lanes over rows read 16-byte words, and lanes over columns

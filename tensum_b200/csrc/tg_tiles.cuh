@@ -38,9 +38,9 @@
 // more registers win: KH 1025^2 steps of TeCNO-Rusanov / KEPEC / KEP in us with
 // (TeCNO, central, gradient) CTAs (4, 7, 7): 732 / 274 / 246, (4, 6, 5): 678 / 256 / 246,
 // (4, 5, 6): 724 / 271 / 264, (3, 5, 5): 706 / 271 / 266; gradient pass 78 / 68 / 60 / 59 us
-// with 7 (spills) / 3 / 5 / 4.  Since then, the central fluxes' normals staged, CTAs of a
-// step's earlier / last updates 6 / 6, 6 / 5, 5 / 5: KEPEC 240 / 227 / 243, KEP 236 / 234 / 236,
-// Roe-EC 259 / 248 / 251.
+// with 7 (spills) / 3 / 5 / 4.  With the central fluxes' normals staged too,
+// CTAs of a step's earlier / last updates 6 / 6, 6 / 5, 5 / 5: KEPEC 240 / 227 / 243, KEP 236 /
+// 234 / 236, Roe-EC 259 / 248 / 251.
 #ifndef TG_FLUX_MINB
 #define TG_FLUX_MINB 4
 #endif
@@ -105,10 +105,17 @@ constexpr int kTileThreads = TG_TILE_THREADS;
 // the chip less than twice, they are made smaller so that its one or two rounds are full:
 // a CTA's time is a chain of latencies and grows with its edges per thread, so a chip half
 // filled with full tiles, or a nearly empty second round, costs as much as a full one.
-// Below 32 the halo outweighs the edges.  TeCNO-Roe step in us on n^2 vertices with 32 / 64 /
-// 96 / 128 owned: 65^2 33.4 / 32.7 / 36.5 / 40.3, 129^2 40.0 / 43.4 / 54.6 / 48.0, 193^2 62.7 /
-// 48.5 / 56.9 / 60.0, 225^2 81.8 / 68.8 / 57.4 / 65.4, 257^2 96.9 / 75.8 / 85.4 / 68.0,
-// 321^2 139 / 104 / 95.6 / 100; the 128 x 256 cylinder 129 / 91 / 103 / 116.
+// Below 32 the halo outweighs the edges.  Steps in us on n^2 vertices with 32 / 64 / 96 / 112 / 128
+// owned, the rule's choice last.  TeCNO-Roe: 65^2 31.8 / 31.5 / 33.8 / 37.0 / 37.3, 32; 129^2 37.6 /
+// 41.4 / 51.5 / 43.8 / 43.6, 32; 193^2 62.1 / 46.4 / 53.3 / 55.9 / 54.5, 64; 225^2 81.5 / 70.1 / 54.0 /
+// 58.2 / 60.6, 96; 257^2 92.9 / 74.4 / 70.4 / 66.0 / 63.6, 112; 300^2 109 / 88.8 / 83.4 / 88.5 / 82.8,
+// 80 (86.5); 321^2 129 / 100 / 92.5 / 91.4 / 94.5, 96; 387^2 173 / 132 / 122 / 118 / 109, 128.
+// Where it is not the best, the chip is filled but the halo larger.  The central fluxes are sized
+// for their earlier updates (6 CTAs per SM); the last one runs 5, so its last round can be nearly
+// empty (257^2, 387^2).  KEPEC: 65^2 19.2 / 18.8 / 19.7 / 21.1 / 20.8, 32; 300^2 47.7 / 37.8 / 37.1 /
+// 35.8 / 33.3, 112; 387^2 66.9 / 50.4 / 47.0 / 46.4 / 46.6, 96; 450^2 85.3 / 63.3 / 57.3 / 55.6 / 55.2,
+// 128.  Roe-EC: 257^2 24.8 / 21.9 / 20.2 / 20.9 / 21.0, 80 (21.4); 387^2 68.8 / 52.2 / 48.4 / 47.9 /
+// 48.2, 96; 450^2 87.6 / 65.0 / 59.1 / 57.9 / 60.6, 128.
 inline int tile_owned(long nv, int ctas) {
   const long full = (long)ctas * TG_TILE_OWNED, rounds = (nv + full - 1) / full;
   if (rounds > 2) return TG_TILE_OWNED;
